@@ -441,10 +441,10 @@ cgs_status cgs_batch_create(const cgs_pair *pairs, int32_t n, const cgs_batch_pl
     if (gn > 0) {
         const size_t budget = 227 * 1024;
         const size_t fixed = span_kernel_smem(gplan.G, gplan.NW, gplan.TH, gplan.TX, gtiles, 0);
-        gcap = fixed + (size_t)kMinSpanCap * 32 > budget ? 0 : (int)((budget - fixed) / 32);
+        gcap = fixed + (size_t)kMinSpanCap * 16 * kWinStages > budget ? 0 : (int)((budget - fixed) / (16 * kWinStages));
         gcap = std::max(gcap, kMinSpanCap + gplan.TH * 32 * gplan.TX / 4);
         const size_t gsm = span_kernel_smem(gplan.G, gplan.NW, gplan.TH, gplan.TX, gtiles, gcap);
-        if (fixed + (size_t)kMinSpanCap * 32 > budget || gsm > budget) {
+        if (fixed + (size_t)kMinSpanCap * 16 * kWinStages > budget || gsm > budget) {
             for (int32_t i = 0; i < n; i++) pend[i].route = pend[i].route == 1 ? 0 : pend[i].route;
             gn = 0;  // cannot happen for the sizes span_plan admits; the pairs go to the persistent kernel
         }

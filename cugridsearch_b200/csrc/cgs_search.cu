@@ -714,8 +714,8 @@ bool span_plan(const cgs_image &mov, const cgs_image &fix, const cgs_options &o,
     sp->tiles_y = (fix.height + sp->TH - 1) / sp->TH;
     const int tiles = sp->tiles_x * sp->tiles_y;
     const size_t budget = 227 * 1024, fixed = span_kernel_smem(sp->G, sp->NW, sp->TH, sp->TX, tiles, 0);
-    if (fixed + (size_t)kMinSpanCap * 32 > budget) return false;
-    sp->cap = (int)((budget - fixed) / 32);
+    if (fixed + (size_t)kMinSpanCap * 16 * kWinStages > budget) return false;
+    sp->cap = (int)((budget - fixed) / (16 * kWinStages));
     // CGS_SPAN_CAP (quads) lowers the stage size, e.g. to exercise the global-memory path
     sp->cap = std::max(kMinSpanCap, std::min(sp->cap, env_int("CGS_SPAN_CAP", sp->cap)));
     sp->cap = std::max(sp->cap, kMinSpanCap + sp->TH * 32 * sp->TX / 4);  // room for the fixed rows

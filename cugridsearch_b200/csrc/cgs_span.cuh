@@ -24,10 +24,16 @@
 // every 32-column block of a tile the CTA's grid points map the block into a small region of
 // the moving image (the union of the block's quadrilateral images, points of one task being
 // neighbours in the locality order); the regions of a tile's blocks are copied from the staged
-// tap quads into one stage of a two-stage mbarrier pipeline by bulk copies, one per region row
-// (the next tile's copies overlap the current tile's sweep), and the sweep reads its 16-byte
-// quads from there.  A block whose region does not fit the stage reads global memory instead
-// (same values).  Blocks rather than whole tiles bound the regions of rotated maps.
+// tap quads into the window stage by bulk copies, one per region row, and the sweep reads its
+// 16-byte quads from there.  A block whose region does not fit the stage reads global memory
+// instead (same values).  Blocks rather than whole tiles bound the regions of rotated maps.
+//
+// One stage, filled by every warp.  The stage takes all the shared memory that is left (about
+// 12 K quads), which holds the eight windows of a 256 x 16 tile at +-20 degrees (8-11 K quads);
+// two stages of half the size sent a third of the blocks to global memory.  The next tile's
+// copies start at the barrier that ends a tile and run during the next band's span pass; a tile's
+// wait is then 0.5-2 K cycles of about 65 K.  Measured on the 256 x 256, 6^8 search: two stages
+// filled by one warp 133.3 ms, one stage filled by one warp 128.6 ms, by all warps 116.1 ms.
 //
 // Sweep.  Lane l takes the tile's columns x0 + l + 32 k; each warp evaluates its G grid points
 // at every pixel, two points per packed FP32x2 instruction.  Blocks inside every point's inner
@@ -50,7 +56,6 @@
 
 namespace cgs {
 
-constexpr int kWinStages = 2;
 // Moving images with (W + 8) H >= 2^22 are outside the span path: the quad index x + pitch y
 // (pitch at most W + 7) is formed exactly in FP32 below that.
 constexpr int64_t kSpanMaxQuads = (int64_t)1 << 22;
@@ -78,7 +83,7 @@ struct PairRow {
 // with row pitch `pitch` quads, `off` quads into the stage's window area; h == 0: no point
 // samples the block on the fast path; w < 0: the window does not fit the stage and the sweep
 // reads global memory.  For the sweep: rel = 16 (off - x0 - pitch y0 - kMagicBits) (mod 2^32),
-// so that quad (ix, iy) lies at stage window + rel + 16 bits(fy pitch + tx); pitchf = pitch.
+// so that quad (ix, iy) lies at stage window + rel + 16 bits(tx - nfy pitch); pitchf = -pitch.
 struct BlockWin {
     int16_t x0, y0, w, h;
     int32_t pitch, off;
@@ -198,42 +203,48 @@ __device__ __forceinline__ void block_extent(const SpanSlot &k, float x0, float 
     one(x1, y1);
 }
 
-// Issue (warp 0) the copies of tile t into stage `st`, completing on that stage's barrier: the
-// tile's rows of the staged fixed image (TH x TW floats at the stage's start; columns past the
-// image's right edge are not copied) and the windows of its blocks (quads, after the fixed tile).
+// Thread 0: announce the bytes of tile t's copies on stage `st`'s barrier (its one arrival).  It
+// comes before the CTA barrier after which every warp issues its part (issue_window).
 template <int TX>
+__device__ __forceinline__ void expect_window(const SearchParams &p, const SpanSmem &ss, int t, int st) {
+    constexpr int TW = 32 * TX;
+    const int x0 = (t % p.tiles_x) * TW, y0 = (t / p.tiles_x) * p.tile_h;
+    const BlockWin *bw = ss.wins + t * TX;
+    uint32_t bytes = (uint32_t)min(p.tile_h, p.fix.h - y0) * (uint32_t)((min(TW, p.fix.w - x0) * 4 + 15) & ~15);
+#pragma unroll
+    for (int c = 0; c < TX; c++)
+        if (bw[c].h > 0 && bw[c].w > 0) bytes += (uint32_t)bw[c].w * (uint32_t)bw[c].h * 16u;
+    mbar_arrive_expect_tx(&ss.bars[st], bytes);
+}
+
+// Issue (every warp its part) the copies of tile t into stage `st`, completing on that stage's
+// barrier: the tile's rows of the staged fixed image (TH x TW floats at the stage's start; columns
+// past the image's right edge are not copied) and the windows of its blocks (quads, after the
+// fixed tile).  A tile has about 220 row copies and a warp issues one in about 60 cycles, so one
+// warp would hold the others back for 14 K cycles per tile; shared by the CTA's warps it is 1 K.
+template <int NW, int TX>
 __device__ __forceinline__ void issue_window(const SearchParams &p, const SpanSmem &ss, int t, int st) {
     constexpr int TW = 32 * TX;
-    const int lane = threadIdx.x & 31;
+    constexpr int WB = NW / TX;  // warps per block window
+    static_assert(NW % TX == 0, "whole warps per block window");
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int TH = p.tile_h;
     const int x0 = (t % p.tiles_x) * TW, y0 = (t / p.tiles_x) * TH;
-    const int rows = min(TH, p.fix.h - y0);
-    const uint32_t row_bytes = (uint32_t)((min(TW, p.fix.w - x0) * 4 + 15) & ~15);  // within the row pitch
-    const BlockWin *bw = ss.wins + t * TX;
     uint64_t *bar = &ss.bars[st];
-    if (lane == 0) {
-        uint32_t bytes = (uint32_t)rows * row_bytes;
-#pragma unroll
-        for (int c = 0; c < TX; c++)
-            if (bw[c].h > 0 && bw[c].w > 0) bytes += (uint32_t)bw[c].w * (uint32_t)bw[c].h * 16u;
-        fence_proxy_async_smem();  // the stage's previous reads before the async refill
-        mbar_arrive_expect_tx(bar, bytes);
+    fence_proxy_async_smem();  // the stage's previous reads before the async refill
+    if (lane == 31) {
+        const int rows = min(TH, p.fix.h - y0);
+        const uint32_t row_bytes = (uint32_t)((min(TW, p.fix.w - x0) * 4 + 15) & ~15);  // within the row pitch
+        float *fdst = reinterpret_cast<float *>(ss.win + (size_t)st * ss.cap);
+        for (int j = warp; j < rows; j += NW)
+            bulk_g2s(fdst + j * TW, p.fix.data + (int64_t)(y0 + j) * p.fix.pitch + x0, row_bytes, bar);
     }
-    __syncwarp();
-    fence_proxy_async_smem();
-    float *fdst = reinterpret_cast<float *>(ss.win + (size_t)st * ss.cap);
-    for (int j = lane; j < rows; j += 32)
-        bulk_g2s(fdst + j * TW, p.fix.data + (int64_t)(y0 + j) * p.fix.pitch + x0, row_bytes, bar);
-    float4 *wdst = ss.win + (size_t)st * ss.cap + TH * TW / 4;
-#pragma unroll
-    for (int c = 0; c < TX; c++) {
-        const BlockWin b = bw[c];
-        if (b.h > 0 && b.w > 0) {
-            const float4 *src = p.mov_quad + (int64_t)b.y0 * p.quad_pitch + b.x0;
-            for (int j = lane; j < b.h; j += 32)
-                bulk_g2s(wdst + b.off + (size_t)j * b.pitch, src + (int64_t)j * p.quad_pitch, (uint32_t)b.w * 16u,
-                         bar);
-        }
+    const BlockWin b = ss.wins[t * TX + warp / WB];
+    if (b.h > 0 && b.w > 0) {
+        float4 *wdst = ss.win + (size_t)st * ss.cap + TH * TW / 4 + b.off;
+        const float4 *src = p.mov_quad + (int64_t)b.y0 * p.quad_pitch + b.x0;
+        for (int j = lane * WB + warp % WB; j < b.h; j += 32 * WB)
+            bulk_g2s(wdst + (size_t)j * b.pitch, src + (int64_t)j * p.quad_pitch, (uint32_t)b.w * 16u, bar);
     }
 }
 
@@ -355,7 +366,7 @@ __device__ __forceinline__ bool run_span_task(const SearchParams &p, uint32_t ta
                                 bw.off = used;
                                 bw.rel = 16u * ((uint32_t)used - (uint32_t)cx0 - (uint32_t)pitch * (uint32_t)cy0 -
                                                 (uint32_t)kMagicBits);
-                                bw.pitchf = (float)pitch;
+                                bw.pitchf = -(float)pitch;
                                 used += pitch * h;
                             } else {
                                 bw.w = -1;
@@ -368,9 +379,11 @@ __device__ __forceinline__ bool run_span_task(const SearchParams &p, uint32_t ta
         }
     }
     __syncthreads();
-    if (warp == 0) {
-        for (int t = 0; t < kWinStages && t < ntiles; t++) issue_window<TX>(p, ss, t, (int)((wit + t) % kWinStages));
-    }
+    if (threadIdx.x == 0)
+        for (int t = 0; t < kWinStages && t < ntiles; t++) expect_window<TX>(p, ss, t, (int)((wit + t) % kWinStages));
+    __syncthreads();
+    for (int t = 0; t < kWinStages && t < ntiles; t++)
+        issue_window<NW, TX>(p, ss, t, (int)((wit + t) % kWinStages));
 
     // ---- sweep
     float2 part[GP][3];  // {sum m', sum m'^2, sum f'm'} of each pair of points
@@ -380,12 +393,11 @@ __device__ __forceinline__ bool run_span_task(const SearchParams &p, uint32_t ta
         for (int j = 0; j < 3; j++) part[h][j] = make_float2(0.0f, 0.0f);
     InnerSpan *my_spans = ss.spans + warp * G * TH;
     RowRun *my_runs = ss.runs + warp * TH;
-    const float2 magic2 = make_float2(kMagic, kMagic), nmagic2 = make_float2(-kMagic, -kMagic);
-    const float2 minus1 = make_float2(-1.0f, -1.0f);
-    // quad index from floor bits: bits(ty + pitch fy) - kMagicBits = ix + pitch iy (exact below
-    // 2^22); global quad (ix, iy) at mqbase + 16 bits
+    const float2 magic2 = make_float2(kMagic, kMagic), minus1 = make_float2(-1.0f, -1.0f);
+    // quad index from floor bits: bits(tx - pitch nfy) - kMagicBits = ix + pitch iy (exact below
+    // 2^22; nfy = -floor y); global quad (ix, iy) at mqbase + 16 bits
     const uint64_t mqbase = reinterpret_cast<uint64_t>(p.mov_quad) - 16ull * (uint64_t)(uint32_t)kMagicBits;
-    const float2 qpitch2 = make_float2((float)p.quad_pitch, (float)p.quad_pitch);
+    const float2 qpitch2 = make_float2(-(float)p.quad_pitch, -(float)p.quad_pitch);
 
     for (int t = 0; t < ntiles; t++, wit++) {
         const int tx = t % tiles_x, ty = t / tiles_x;
@@ -542,17 +554,18 @@ __device__ __forceinline__ bool run_span_task(const SearchParams &p, uint32_t ta
                 const float2 xf2 = make_float2(xf, xf);
 #pragma unroll
                 for (int h = 0; h < GP; h++) {
-                    // both points of the pair in each FP32x2 operation: map, floor (round-down add
-                    // of 1.5 * 2^23 leaves floor(m) in the mantissa), fraction, quad index
+                    // both points of the pair in each FP32x2 operation: map, floor (the product X / w
+                    // added to 1.5 * 2^23 with one rounding down leaves floor(X / w) in the mantissa),
+                    // its negative, fraction (X / w - floor, one rounding), quad index; the product is
+                    // never rounded by itself, which saves two operations of twelve
                     const float2 w = __ffma2_rn(A2[h], xf2, byw[h]);
                     const float2 X = __ffma2_rn(C12[h], xf2, byx[h]);
                     const float2 Y = __ffma2_rn(D12[h], xf2, byy[h]);
                     const float2 rw = make_float2(rcp_approx(w.x), rcp_approx(w.y));
-                    const float2 mx = __fmul2_rn(X, rw), my = __fmul2_rn(Y, rw);
-                    const float2 tx2 = __fadd2_rd(mx, magic2), ty2 = __fadd2_rd(my, magic2);
-                    const float2 fx2 = __fadd2_rn(tx2, nmagic2), fy2 = __fadd2_rn(ty2, nmagic2);
-                    const float2 ax2 = __ffma2_rn(fx2, minus1, mx), ay2 = __ffma2_rn(fy2, minus1, my);
-                    const float2 qi = __ffma2_rn(fy2, pitch2, tx2);
+                    const float2 tx2 = __ffma2_rd(X, rw, magic2), ty2 = __ffma2_rd(Y, rw, magic2);
+                    const float2 nfx2 = __ffma2_rn(tx2, minus1, magic2), nfy2 = __ffma2_rn(ty2, minus1, magic2);
+                    const float2 ax2 = __ffma2_rn(X, rw, nfx2), ay2 = __ffma2_rn(Y, rw, nfy2);
+                    const float2 qi = __ffma2_rn(nfy2, pitch2, tx2);
                     bool in0 = true, in1 = true;
                     if constexpr (EDGE) {
                         const InnerSpan a = isp[2 * h], b = isp[2 * h + 1];
@@ -676,18 +689,20 @@ __device__ __forceinline__ bool run_span_task(const SearchParams &p, uint32_t ta
                     part[h][j] = make_float2(0.0f, 0.0f);
                 }
         }
+        const bool more = t + kWinStages < ntiles;
+        if (threadIdx.x == 0 && more) expect_window<TX>(p, ss, t + kWinStages, st);
         __syncthreads();  // every warp is done with this stage
         if (*ss.abort_flag) {
             // a wait gave up: let this stage's copies and the next stage's (already issued) land,
             // within the same bound, before the CTA stops
             if (threadIdx.x == 0) {
                 mbar_wait_bounded(&ss.bars[st], (wit / kWinStages) & 1u, kWaitLimitNs);
-                if (t + 1 < ntiles)
+                if (kWinStages > 1 && t + 1 < ntiles)
                     mbar_wait_bounded(&ss.bars[(wit + 1) % kWinStages], ((wit + 1) / kWinStages) & 1u, kWaitLimitNs);
             }
             return false;
         }
-        if (warp == 0 && t + kWinStages < ntiles) issue_window<TX>(p, ss, t + kWinStages, st);
+        if (more) issue_window<NW, TX>(p, ss, t + kWinStages, st);
     }
 
     // ---- per grid point: finalise, dump, argmin key (as the pixel-loop kernel)
