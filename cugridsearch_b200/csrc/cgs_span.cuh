@@ -160,29 +160,57 @@ __device__ __forceinline__ SpanSmem carve_span(unsigned char *smem, int TH, int 
     return s;
 }
 
-// Row span of one point: the integer x in [0, fw) satisfying the four half-plane conditions
-// m < X/w < W - m, m < Y/w < H - m (margins mx, my; negative margins widen), w of sign s.
-__device__ __forceinline__ void row_span(const SpanSlot &k, float yf, float s, int fw, float mw, float mh, float mx,
-                                         float my, int &xa, int &len) {
+// Spans of one row of one point: the inner span [xa, xa + len) and the outer span [pa, pa + plen),
+// which holds it.
+struct RowSpans {
+    int xa, len, pa, plen;
+};
+
+// The spans of row y (see the head of this file).  Each edge of the moving image gives a condition
+// s f(x) > 0 with f(x) = a x + b linear and s the sign of w; x = q solves f = 0.  f is the distance
+// to the edge in pixels times w, so with h = 1.5 g max|w| / |a| (max over the row) every x beyond
+// q + h lies at least 1.5 guard bands inside that edge and every x beyond q - h at least as far
+// outside it: one reciprocal gives both spans.  An edge that the row follows (a changes f by less
+// than a thousandth of the margin over the whole row) is decided by b alone.  Branch-free: the
+// reciprocals of the four edges overlap (IEEE divisions, one per edge and span, took 40 % of the
+// span pass).
+__device__ __forceinline__ RowSpans row_spans(const SpanSlot &k, float yf, int fw, float mw, float mh) {
     const float bw = fmaf(k.B, yf, k.PQ), bX = fmaf(k.C2, yf, k.RS), bY = fmaf(k.D2, yf, k.TU);
-    float lo = -1.0f, hi = (float)fw;  // open interval of admissible x, clamped to the row
-    bool none = false;
-    auto cons = [&](float a, float b) {  // s (a x + b) > 0
+    const float fwf = (float)fw, we = fmaf(k.A, fwf - 1.0f, bw);
+    const float s = bw > 0.0f ? 1.0f : -1.0f;  // the guard holds: w keeps its sign over the image
+    const float wmax = fmaxf(fabsf(bw), fabsf(we));
+    float ilo = -1.0f, ihi = fwf, olo = -1.0f, ohi = fwf;  // open intervals, clamped to the row
+    bool inone = false, onone = false;
+    auto edge = [&](float a, float b, float m) {  // m: the margin times max|w|
         a *= s;
         b *= s;
-        if (a > 0.0f) lo = fmaxf(lo, -b / a);
-        else if (a < 0.0f) hi = fminf(hi, -b / a);
-        else if (!(b > 0.0f)) none = true;
+        const bool flat = fabsf(a) * fwf < 1e-3f * m;
+        const float r = rcp_approx(a);
+        const float q0 = -b * r;
+        const float q = fmaf(fmaf(-q0, a, -b), r, q0), h = m * fabsf(r);
+        const bool up = !flat && a > 0.0f, down = !flat && a < 0.0f;
+        ilo = up ? fmaxf(ilo, q + h) : ilo;
+        olo = up ? fmaxf(olo, q - h) : olo;
+        ihi = down ? fminf(ihi, q - h) : ihi;
+        ohi = down ? fminf(ohi, q + h) : ohi;
+        inone = inone || (flat && !(b > 1.01f * m));
+        onone = onone || (flat && !(b > -1.01f * m));
     };
-    cons(fmaf(-mx, k.A, k.C1), fmaf(-mx, bw, bX));                    // X - m w > 0
-    cons(fmaf(mw - mx, k.A, -k.C1), fmaf(mw - mx, bw, -bX));          // (W - m) w - X > 0
-    cons(fmaf(-my, k.A, k.D1), fmaf(-my, bw, bY));                    // Y - m w > 0
-    cons(fmaf(mh - my, k.A, -k.D1), fmaf(mh - my, bw, -bY));          // (H - m) w - Y > 0
-    lo = fmaxf(lo, -1.0f);
-    hi = fminf(hi, (float)fw);
-    const int a0 = max(0, (int)floorf(lo) + 1), b0 = min(fw - 1, (int)ceilf(hi) - 1);
-    xa = a0;
-    len = (none || b0 < a0) ? 0 : b0 - a0 + 1;
+    const float gx = 1.5f * k.gx * wmax, gy = 1.5f * k.gy * wmax;
+    edge(k.C1, bX, gx);                                    // X > 0
+    edge(fmaf(mw, k.A, -k.C1), fmaf(mw, bw, -bX), gx);     // W w - X > 0
+    edge(k.D1, bY, gy);                                    // Y > 0
+    edge(fmaf(mh, k.A, -k.D1), fmaf(mh, bw, -bY), gy);     // H w - Y > 0
+    ilo = fmaxf(ilo, -1.0f);
+    olo = fmaxf(olo, -1.0f);
+    const int a0 = max(0, (int)floorf(fminf(ilo, fwf)) + 1), b0 = min(fw - 1, (int)ceilf(fmaxf(ihi, -1.0f)) - 1);
+    const int a1 = max(0, (int)floorf(fminf(olo, fwf)) + 1), b1 = min(fw - 1, (int)ceilf(fmaxf(ohi, -1.0f)) - 1);
+    RowSpans r;
+    r.xa = a0;
+    r.len = (inone || b0 < a0) ? 0 : b0 - a0 + 1;
+    r.pa = a1;
+    r.plen = (onone || b1 < a1) ? 0 : b1 - a1 + 1;
+    return r;
 }
 
 // The corners of block [x0, x1] x [y0, y1] under a point's map: min/max of the mapped coordinates.
@@ -191,7 +219,7 @@ __device__ __forceinline__ void block_extent(const SpanSlot &k, float x0, float 
         const float w = fmaf(k.A, x, fmaf(k.B, y, k.PQ));
         const float X = fmaf(k.C1, x, fmaf(k.C2, y, k.RS));
         const float Y = fmaf(k.D1, x, fmaf(k.D2, y, k.TU));
-        const float mx = X / w, my = Y / w;
+        const float rw = rcp_approx(w), mx = X * rw, my = Y * rw;  // the 0.25 px margin covers their error
         e.x = fminf(e.x, mx);
         e.y = fminf(e.y, my);
         e.z = fmaxf(e.z, mx);
@@ -248,6 +276,29 @@ __device__ __forceinline__ void issue_window(const SearchParams &p, const SpanSm
     }
 }
 
+// The G grid points from ordinal ord0: lane g decodes point g and writes its slot (the decode, the
+// homography and the FP64 guard of a point are a chain of about 5 K cycles: four at once).
+template <int COST, int G>
+__device__ __forceinline__ void span_points(const SearchParams &p, uint32_t ord0, SpanSlot *slots) {
+    const int lane = threadIdx.x & 31;
+    if (lane >= G) return;
+    const uint32_t o = ord0 + lane;
+    const bool gvalid = o < p.n;
+    int32_t ax[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    const uint32_t gidx = gvalid ? ordinal_to_index(p, o, ax) : 0u;
+    float q[8];
+    grid_values(p, ax, q);
+    const float2 cs = p.trig[min(ax[0], kMaxTrig - 1)];
+    const MapCoef kc = make_coef<COST>(q, cs, p);
+    FastMap fm;
+    RowTerms rt;
+    float gx, gy;
+    map_guard(kc, p, fm, rt, gx, gy);
+    const bool ok = gvalid && fm.li_x > 0.0f;
+    slots[lane] = SpanSlot{kc.A, rt.B, rt.PQ, kc.C1, rt.C2, rt.RS, kc.D1, rt.D2, rt.TU, kc.P, kc.Q, kc.R,
+                           kc.S, kc.T, kc.U, gx, gy, ok ? 1 : 0, gvalid ? 1 : 0, gidx};
+}
+
 // One task of the span path (ZNCC, one channel, quads staged): the G grid points of each warp
 // over every tile of the fixed image.  `wit` counts window stages used by this CTA (their
 // barrier phases).  Returns false if a bounded wait gave up.
@@ -268,34 +319,17 @@ __device__ __forceinline__ bool run_span_task(const SearchParams &p, uint32_t ta
     const int fpitch = p.fix.pitch;
 
     // ---- the warp's points: coefficients, guard, slots
-    const uint32_t ord0 = (task * NW + warp) * G;
-    float2 A2[GP], C12[GP], D12[GP];
     SpanSlot *my_slots = ss.slots + warp * G;
-#pragma unroll
-    for (int g = 0; g < G; g++) {
-        const uint32_t o = ord0 + g;
-        const bool gvalid = o < p.n;
-        int32_t ax[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-        const uint32_t gidx = gvalid ? ordinal_to_index(p, o, ax) : 0u;
-        float q[8];
-        grid_values(p, ax, q);
-        const float2 cs = p.trig[min(ax[0], kMaxTrig - 1)];
-        const MapCoef kc = make_coef<CGS_COST_ZNCC>(q, cs, p);
-        FastMap fm;
-        RowTerms rt;
-        float gx, gy;
-        map_guard(kc, p, fm, rt, gx, gy);
-        const bool ok = gvalid && fm.li_x > 0.0f;
-        if (lane == 0)
-            my_slots[g] = SpanSlot{kc.A, rt.B, rt.PQ, kc.C1, rt.C2, rt.RS, kc.D1, rt.D2, rt.TU, kc.P, kc.Q, kc.R,
-                                   kc.S, kc.T, kc.U, gx, gy, ok ? 1 : 0, gvalid ? 1 : 0, gidx};
-        if (g & 1) {
-            A2[g / 2].y = kc.A; C12[g / 2].y = kc.C1; D12[g / 2].y = kc.D1;
-        } else {
-            A2[g / 2].x = kc.A; C12[g / 2].x = kc.C1; D12[g / 2].x = kc.D1;
-        }
-    }
+    span_points<CGS_COST_ZNCC, G>(p, (task * NW + warp) * G, my_slots);
     __syncwarp();
+    float2 A2[GP], C12[GP], D12[GP];
+#pragma unroll
+    for (int h = 0; h < GP; h++) {
+        const SpanSlot &a = my_slots[2 * h], &b = my_slots[2 * h + 1];
+        A2[h] = make_float2(a.A, b.A);
+        C12[h] = make_float2(a.C1, b.C1);
+        D12[h] = make_float2(a.D1, b.D1);
+    }
     if (lane < GP) {
         const SpanSlot &a = my_slots[2 * lane], &b = my_slots[2 * lane + 1];
         ss.prow[warp * GP + lane] = PairRow{make_float2(a.B, b.B), make_float2(a.PQ, b.PQ), make_float2(a.C2, b.C2),
@@ -309,72 +343,67 @@ __device__ __forceinline__ bool run_span_task(const SearchParams &p, uint32_t ta
     const float fshift = p.shifts[0], mshift = p.shifts[1];
     __syncthreads();  // every point's slot is written
 
-    // ---- windows of every block of every tile: warp w takes tiles w, w + NW, ..; lanes take the
-    // task's points
+    // ---- windows of every block of every tile: warp w takes blocks w, w + NW, ..; lanes take the
+    // task's points; then one thread per tile lays its blocks out in the stage
     {
         constexpr int P = NW * G;
+        const float inf = __int_as_float(0x7f800000);
+        for (int i = warp; i < ntiles * TX; i += NW) {
+            const int t = i / TX, c = i - t * TX;
+            const int xc = (t % tiles_x) * TW + 32 * c, y0 = (t / tiles_x) * TH;
+            float4 e = make_float4(inf, inf, -inf, -inf);
+            if (xc < fw) {
+                const float fx0 = (float)xc, fx1 = (float)(min(xc + 32, fw) - 1);
+                const float fy0 = (float)y0, fy1 = (float)(min(y0 + TH, fh) - 1);
+                for (int k = lane; k < P; k += 32)
+                    if (ss.slots[k].ok) block_extent(ss.slots[k], fx0, fx1, fy0, fy1, e);
+                e.x = warp_fmin(e.x);
+                e.y = warp_fmin(e.y);
+                e.z = warp_fmax(e.z);
+                e.w = warp_fmax(e.w);
+            }
+            if (lane == 0) {  // the block's extent, in its window's place
+                float2 *d = reinterpret_cast<float2 *>(&ss.wins[i]);
+                d[0] = make_float2(e.x, e.y);
+                d[1] = make_float2(e.z, e.w);
+            }
+        }
+        __syncthreads();
         const int wcap = ss.cap - TH * TW / 4;  // quads of a stage after the fixed rows
-        for (int t = warp; t < ntiles; t += NW) {
-            const int x0 = (t % tiles_x) * TW, y0 = (t / tiles_x) * TH;
-            const float fy0 = (float)y0, fy1 = (float)(min(y0 + TH, fh) - 1);
-            float4 e[TX];
-#pragma unroll
-            for (int c = 0; c < TX; c++)
-                e[c] = make_float4(__int_as_float(0x7f800000), __int_as_float(0x7f800000),
-                                   -__int_as_float(0x7f800000), -__int_as_float(0x7f800000));
-            for (int k = lane; k < P; k += 32) {
-                const SpanSlot &sl = ss.slots[k];
-                if (sl.ok) {
-#pragma unroll
-                    for (int c = 0; c < TX; c++) {
-                        const int xc = x0 + 32 * c;
-                        if (xc < fw) block_extent(sl, (float)xc, (float)(min(xc + 32, fw) - 1), fy0, fy1, e[c]);
-                    }
-                }
-            }
-#pragma unroll
+        for (int t = threadIdx.x; t < ntiles; t += NW * 32) {
+            int used = 0;
+#pragma unroll 1
             for (int c = 0; c < TX; c++) {
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) {
-                    e[c].x = fminf(e[c].x, __shfl_xor_sync(0xffffffffu, e[c].x, o));
-                    e[c].y = fminf(e[c].y, __shfl_xor_sync(0xffffffffu, e[c].y, o));
-                    e[c].z = fmaxf(e[c].z, __shfl_xor_sync(0xffffffffu, e[c].z, o));
-                    e[c].w = fmaxf(e[c].w, __shfl_xor_sync(0xffffffffu, e[c].w, o));
-                }
-            }
-            if (lane == 0) {
-                int used = 0;
-#pragma unroll
-                for (int c = 0; c < TX; c++) {
-                    BlockWin bw{0, 0, 0, 0, 0, 0, 0u, 0.0f};
-                    // cells a fast sample can use: floor of its coordinate (within the guard, < 1/8 px,
-                    // of the real map, whose block image lies in the corners' hull), clipped to the image
-                    const float lx = fmaxf(e[c].x - 0.25f, -1.0f), ly = fmaxf(e[c].y - 0.25f, -1.0f);
-                    const float hx = fminf(e[c].z + 0.25f, mov_wf), hy = fminf(e[c].w + 0.25f, mov_hf);
-                    if (lx <= hx && ly <= hy) {
-                        const int cx0 = max(0, (int)floorf(lx)), cy0 = max(0, (int)floorf(ly));
-                        const int cx1 = min(p.mov.w - 1, (int)floorf(hx)), cy1 = min(p.mov.h - 1, (int)floorf(hy));
-                        if (cx0 <= cx1 && cy0 <= cy1) {
-                            const int w = cx1 - cx0 + 1, h = cy1 - cy0 + 1;
-                            const int pitch = w + ((p.win_pitch_mod - w) & 7);  // = win_pitch_mod (mod 8)
-                            bw.x0 = (int16_t)cx0;
-                            bw.y0 = (int16_t)cy0;
-                            bw.h = (int16_t)h;
-                            bw.pitch = pitch;
-                            if ((int64_t)pitch * h <= wcap - used) {
-                                bw.w = (int16_t)w;
-                                bw.off = used;
-                                bw.rel = 16u * ((uint32_t)used - (uint32_t)cx0 - (uint32_t)pitch * (uint32_t)cy0 -
-                                                (uint32_t)kMagicBits);
-                                bw.pitchf = -(float)pitch;
-                                used += pitch * h;
-                            } else {
-                                bw.w = -1;
-                            }
+                BlockWin bw{0, 0, 0, 0, 0, 0, 0u, 0.0f};
+                // cells a fast sample can use: floor of its coordinate (within the guard, < 1/8 px,
+                // of the real map, whose block image lies in the corners' hull), clipped to the image
+                const float2 *d = reinterpret_cast<const float2 *>(&ss.wins[t * TX + c]);
+                const float2 e0 = d[0], e1 = d[1];
+                const float lx = fmaxf(e0.x - 0.25f, -1.0f), ly = fmaxf(e0.y - 0.25f, -1.0f);
+                const float hx = fminf(e1.x + 0.25f, mov_wf), hy = fminf(e1.y + 0.25f, mov_hf);
+                if (lx <= hx && ly <= hy) {
+                    const int cx0 = max(0, (int)floorf(lx)), cy0 = max(0, (int)floorf(ly));
+                    const int cx1 = min(p.mov.w - 1, (int)floorf(hx)), cy1 = min(p.mov.h - 1, (int)floorf(hy));
+                    if (cx0 <= cx1 && cy0 <= cy1) {
+                        const int w = cx1 - cx0 + 1, h = cy1 - cy0 + 1;
+                        const int pitch = w + ((p.win_pitch_mod - w) & 7);  // = win_pitch_mod (mod 8)
+                        bw.x0 = (int16_t)cx0;
+                        bw.y0 = (int16_t)cy0;
+                        bw.h = (int16_t)h;
+                        bw.pitch = pitch;
+                        if ((int64_t)pitch * h <= wcap - used) {
+                            bw.w = (int16_t)w;
+                            bw.off = used;
+                            bw.rel = 16u * ((uint32_t)used - (uint32_t)cx0 - (uint32_t)pitch * (uint32_t)cy0 -
+                                            (uint32_t)kMagicBits);
+                            bw.pitchf = -(float)pitch;
+                            used += pitch * h;
+                        } else {
+                            bw.w = -1;
                         }
                     }
-                    ss.wins[t * TX + c] = bw;
                 }
+                ss.wins[t * TX + c] = bw;
             }
         }
     }
@@ -419,21 +448,9 @@ __device__ __forceinline__ bool run_span_task(const SearchParams &p, uint32_t ta
                     InnerSpan is{0, 0};
                     if (y < fh && sl.valid) {
                         const float yf = (float)y;
-                        int xa = 0, len = 0, pa = 0, plen = fw;  // ill-conditioned: every pixel exact
-                        if (sl.ok) {
-                            const float wm = fmaf(sl.A, 0.5f * (float)(fw - 1), fmaf(sl.B, yf, sl.PQ));
-                            const float s = wm > 0.0f ? 1.0f : -1.0f;
-                            row_span(sl, yf, s, fw, mov_wf, mov_hf, 1.5f * sl.gx, 1.5f * sl.gy, xa, len);
-                            row_span(sl, yf, s, fw, mov_wf, mov_hf, -1.5f * sl.gx, -1.5f * sl.gy, pa, plen);
-                            if (len > 0 && plen > 0) {  // the outer span holds the inner one
-                                const int lo = min(pa, xa), hi = max(pa + plen, xa + len);
-                                pa = lo;
-                                plen = hi - lo;
-                            } else if (len > 0) {
-                                pa = xa;
-                                plen = len;
-                            }
-                        }
+                        RowSpans sp{0, 0, 0, fw};  // ill-conditioned: every pixel exact
+                        if (sl.ok) sp = row_spans(sl, yf, fw, mov_wf, mov_hf);
+                        const int xa = sp.xa, len = sp.len, pa = sp.pa, plen = sp.plen;
                         is = InnerSpan{xa, len};
                         if (len > 0) {
                             const double2 *pr = p.fix_prefix + (int64_t)y * (fw + 1);
@@ -468,22 +485,29 @@ __device__ __forceinline__ bool run_span_task(const SearchParams &p, uint32_t ta
                     }
                     my_spans[g * TH + r] = is;
                 }
-                // sum over the TH lanes of each point (TH is 8, 16 or 32)
+                // sum over the TH lanes of each point (TH is 8, 16 or 32); the moving sums exist only
+                // where a band pixel was found inside, which is rare
+                const bool found = __any_sync(0xffffffffu, smm != 0.0 || sm != 0.0);
                 for (int o = 1; o < TH && o < 32; o <<= 1) {
                     s1 += __shfl_xor_sync(0xffffffffu, s1, o);
                     s2 += __shfl_xor_sync(0xffffffffu, s2, o);
-                    sm += __shfl_xor_sync(0xffffffffu, sm, o);
-                    smm += __shfl_xor_sync(0xffffffffu, smm, o);
-                    sfm += __shfl_xor_sync(0xffffffffu, sfm, o);
                     n += __shfl_xor_sync(0xffffffffu, n, o);
                 }
+                if (found)
+                    for (int o = 1; o < TH && o < 32; o <<= 1) {
+                        sm += __shfl_xor_sync(0xffffffffu, sm, o);
+                        smm += __shfl_xor_sync(0xffffffffu, smm, o);
+                        sfm += __shfl_xor_sync(0xffffffffu, sfm, o);
+                    }
                 if (act && r == 0) {
                     double *d = my_dtot + g * 5;
                     d[0] += s1;
-                    d[1] += sm;
                     d[2] += s2;
-                    d[3] += smm;
-                    d[4] += sfm;
+                    if (found) {
+                        d[1] += sm;
+                        d[3] += smm;
+                        d[4] += sfm;
+                    }
                     my_cnt[g] += n;
                 }
             }

@@ -108,36 +108,22 @@ __device__ __forceinline__ void run_span_mi_task(const SearchParams &p, uint32_t
     const float lmax = *reinterpret_cast<const float *>(p.span_rows_header);  // largest quad slope bound
 
     // ---- the warp's two points
-    const uint32_t ord0 = (task * NW + warp) * G;
-    float2 A2, C12, D12, sg2, gl2, hh2;
     SpanSlot *my_slots = ss.slots + warp * G;
+    span_points<CGS_COST_MI, G>(p, (task * NW + warp) * G, my_slots);
+    __syncwarp();
+    float2 A2, C12, D12, sg2, gl2, hh2;
 #pragma unroll
     for (int g = 0; g < G; g++) {
-        const uint32_t o = ord0 + g;
-        const bool gvalid = o < p.n;
-        int32_t ax[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-        const uint32_t gidx = gvalid ? ordinal_to_index(p, o, ax) : 0u;
-        float q[8];
-        grid_values(p, ax, q);
-        const float2 cs = p.trig[min(ax[0], kMaxTrig - 1)];
-        const MapCoef kc = make_coef<CGS_COST_MI>(q, cs, p);
-        FastMap fm;
-        RowTerms rt;
-        float gx, gy;
-        map_guard(kc, p, fm, rt, gx, gy);
-        const bool ok = gvalid && fm.li_x > 0.0f;
-        if (lane == 0)
-            my_slots[g] = SpanSlot{kc.A, rt.B, rt.PQ, kc.C1, rt.C2, rt.RS, kc.D1, rt.D2, rt.TU, kc.P, kc.Q, kc.R,
-                                   kc.S, kc.T, kc.U, gx, gy, ok ? 1 : 0, gvalid ? 1 : 0, gidx};
+        const SpanSlot &k = my_slots[g];
         // slope factor of the bin guard: |v_fast - v_exact| <= (3|c10| + |c01| + 2|c11|) max(gx, gy)
         // (in bin units with sB), the factor covering the roundings of the sum
-        const float sg = sB * fmaxf(gx, gy) * (1.0f + 0x1p-18f);
+        const float gm = fmaxf(k.gx, k.gy), sg = sB * gm * (1.0f + 0x1p-18f);
         const float gl = fmaf(lmax, sg, gv0);  // the bound near a cell edge
-        const float hh = 0.5f - fmaxf(gx, gy);  // fraction farther than this from 0.5: near a cell edge
+        const float hh = 0.5f - gm;            // fraction farther than this from 0.5: near a cell edge
         if (g == 0) {
-            A2.x = kc.A; C12.x = kc.C1; D12.x = kc.D1; sg2.x = sg; gl2.x = gl; hh2.x = hh;
+            A2.x = k.A; C12.x = k.C1; D12.x = k.D1; sg2.x = sg; gl2.x = gl; hh2.x = hh;
         } else {
-            A2.y = kc.A; C12.y = kc.C1; D12.y = kc.D1; sg2.y = sg; gl2.y = gl; hh2.y = hh;
+            A2.y = k.A; C12.y = k.C1; D12.y = k.D1; sg2.y = sg; gl2.y = gl; hh2.y = hh;
         }
     }
     __syncwarp();
@@ -205,21 +191,9 @@ __device__ __forceinline__ void run_span_mi_task(const SearchParams &p, uint32_t
                 InnerSpan is{0, 0};
                 if (y < fh && sl.valid) {
                     const float yf = (float)y;
-                    int xa = 0, len = 0, pa = 0, plen = fw;  // ill-conditioned: every pixel exact
-                    if (sl.ok) {
-                        const float wm = fmaf(sl.A, 0.5f * (float)(fw - 1), fmaf(sl.B, yf, sl.PQ));
-                        const float s = wm > 0.0f ? 1.0f : -1.0f;
-                        row_span(sl, yf, s, fw, mov_wf, mov_hf, 1.5f * sl.gx, 1.5f * sl.gy, xa, len);
-                        row_span(sl, yf, s, fw, mov_wf, mov_hf, -1.5f * sl.gx, -1.5f * sl.gy, pa, plen);
-                        if (len > 0 && plen > 0) {
-                            const int lo = min(pa, xa), hi = max(pa + plen, xa + len);
-                            pa = lo;
-                            plen = hi - lo;
-                        } else if (len > 0) {
-                            pa = xa;
-                            plen = len;
-                        }
-                    }
+                    RowSpans sp{0, 0, 0, fw};  // ill-conditioned: every pixel exact
+                    if (sl.ok) sp = row_spans(sl, yf, fw, mov_wf, mov_hf);
+                    const int xa = sp.xa, len = sp.len, pa = sp.pa, plen = sp.plen;
                     is = InnerSpan{xa, len};
                     n = len;
                     const int e0 = len > 0 ? xa : pa + plen, e1 = len > 0 ? xa + len : pa + plen;
