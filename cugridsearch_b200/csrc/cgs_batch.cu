@@ -227,7 +227,8 @@ static cgs_status enqueue_launch(const cgs_batch &b, cudaStream_t s) {
     // the multi-pair span kernel first: its pairs take the least time each, so running them
     // before the per-sample pairs lowers the pairs' completion times (the launch takes as long)
     if (b.g_n > 0) {
-        CGS_CUDA(launch_span_prep_batch(b.d_gprep, (int)b.g_n, b.g_prep_blocks, s), "span_prep_batch_kernel");
+        if (b.g_prep_blocks > 0)
+            CGS_CUDA(launch_span_prep_batch(b.d_gprep, (int)b.g_n, b.g_prep_blocks, s), "span_prep_batch_kernel");
         SpanBatchParams ga = b.g_args;
         void *gargs[] = {&ga};
         CGS_CUDA(cudaLaunchKernel(b.g_kfn, dim3(b.g_blocks), dim3(16 * 32), gargs, b.g_smem, s), "span_batch_kernel");
@@ -353,26 +354,23 @@ cgs_status cgs_batch_create(const cgs_pair *pairs, int32_t n, const cgs_batch_pl
     for (int32_t i = 0; i < n; i++) {
         const cgs_pair &q = pairs[i];
         Pending &pd = pend[i];
-        // ZNCC pairs that cgs_search runs on its span kernel share one multi-pair span launch
-        // (same kernel plan); other span-eligible pairs are searched by their own launches once
+        // pairs that cgs_search runs on a tiled span kernel share one multi-pair span launch (same
+        // kernel plan); MI pairs on its MI span kernel are searched by their own launches once
         // their grid fills the GPU by itself (a few tasks per SM), and stay in the persistent
         // kernel below that (a refinement level's local grids, balanced there many at once)
         uint32_t ppt = 0;
-        if ((q.options.cost == CGS_COST_ZNCC || q.options.cost == CGS_COST_MI) &&
-            span_route_bytes(q, &pd.span_bytes, &ppt)) {
-            SpanPlan zp;
-            const bool grouped = q.options.cost == CGS_COST_ZNCC && span_plan(q.moving, q.fixed, q.options, &zp) &&
-                                 kernel_span_zncc_batch(zp.G, zp.NW, zp.TX, zp.check) != nullptr &&
-                                 (!have_group || (zp.G == gplan.G && zp.NW == gplan.NW && zp.TX == gplan.TX &&
-                                                  zp.TH == gplan.TH && zp.pitch_mod == gplan.pitch_mod));
-            if (grouped) {
-                pd.route = 1;
-                pd.zp = zp;
-                if (!have_group) gplan = zp;
-                have_group = true;
-            } else if ((uint64_t)pd.p.n >= route_tasks * ppt) {
-                pd.route = 2;
-            }
+        SpanPlan zp;
+        if (span_plan(q.moving, q.fixed, q.options, &zp) &&
+            kernel_span_batch(zp.G, zp.NW, zp.TX, zp.check) != nullptr &&
+            (!have_group || (zp.G == gplan.G && zp.NW == gplan.NW && zp.TX == gplan.TX && zp.TH == gplan.TH &&
+                             zp.pitch_mod == gplan.pitch_mod))) {
+            pd.route = 1;
+            pd.zp = zp;
+            if (!have_group) gplan = zp;
+            have_group = true;
+        } else if ((q.options.cost == CGS_COST_ZNCC || q.options.cost == CGS_COST_MI) &&
+                   span_route_bytes(q, &pd.span_bytes, &ppt) && (uint64_t)pd.p.n >= route_tasks * ppt) {
+            pd.route = 2;
         }
         // ZNCC pairs of the persistent kernel on the fast sampling path read pre-gathered tap
         // quads, as single searches do
@@ -464,9 +462,9 @@ cgs_status cgs_batch_create(const cgs_pair *pairs, int32_t n, const cgs_batch_pl
     }
     for (uint32_t j = 0; j < b->n; j++) {
         Pending &pd = pend[b->order[j]];
-        if (pd.route != 1) continue;
-        pd.prefix_off = off;
         const cgs_pair &q = pairs[b->order[j]];
+        if (pd.route != 1 || !span_uses_prefix(q.options.cost)) continue;
+        pd.prefix_off = off;
         off = align_up(off + (size_t)q.fixed.height * (size_t)(q.fixed.width + 1) * sizeof(double2), 256);
     }
     off = align_up(off, (size_t)di.tex_align);
@@ -567,10 +565,12 @@ cgs_status cgs_batch_create(const cgs_pair *pairs, int32_t n, const cgs_batch_pl
         }
         p.mov_tex = b->tex[j];
         if (pd.route == 1) {
-            // as cgs_search sets up its span kernel: quads in the span form with the moving
-            // shift folded in, the fixed rows' prefix sums, tiles and the (common) window stage
-            preps[j].quad_form = 1;
-            double2 *prefix = reinterpret_cast<double2 *>(b->mem + pd.prefix_off);
+            // as cgs_search sets up its span kernels: quads in the cost's span form (ZNCC: with the
+            // moving shift folded in), the fixed rows' prefix sums, tiles and the (common) window stage
+            const int cost = q.options.cost;
+            preps[j].quad_form = span_quad_form(cost);
+            double2 *prefix =
+                span_uses_prefix(cost) ? reinterpret_cast<double2 *>(b->mem + pd.prefix_off) : nullptr;
             p.fix_prefix = prefix;
             p.tile_h = pd.zp.TH;
             p.tiles_x = pd.zp.tiles_x;
@@ -582,11 +582,11 @@ cgs_status cgs_batch_create(const cgs_pair *pairs, int32_t n, const cgs_batch_pl
             gpar.push_back(p);
             gtasks.push_back(p.num_tasks);
             gslot.push_back(j);
-            SpanPrepArgs ga;
             int blocks = 0;
-            span_prep_batch_args(fstage, pd.st.fpitch, q.fixed.width, q.fixed.height, prefix,
-                                 reinterpret_cast<float4 *>(org + pd.st.quad_off), pd.st.qplane, p.shifts, &ga,
-                                 &blocks);
+            const SpanPrepArgs ga =
+                span_prep_args(fstage, pd.st.fpitch, pd.st.fplane, 1, q.fixed.width, q.fixed.height, prefix,
+                               reinterpret_cast<float4 *>(org + pd.st.quad_off),
+                               cost == CGS_COST_ZNCC ? pd.st.qplane : 0, p.shifts, &blocks);
             gprep.push_back(ga);
             b->g_prep_blocks = std::max(b->g_prep_blocks, blocks);
         }
@@ -614,7 +614,7 @@ cgs_status cgs_batch_create(const cgs_pair *pairs, int32_t n, const cgs_batch_pl
         ga.tile_h = gplan.TH;
         ga.tiles = gtiles;
         ga.cap = gcap;
-        b->g_kfn = kernel_span_zncc_batch(gplan.G, gplan.NW, gplan.TX, gplan.check);
+        b->g_kfn = kernel_span_batch(gplan.G, gplan.NW, gplan.TX, gplan.check);
         b->g_smem = span_kernel_smem(gplan.G, gplan.NW, gplan.TH, gplan.TX, gtiles, gcap);
         e = cudaMemcpy(b->mem + gpar_off, gpar.data(), sizeof(SearchParams) * gn, cudaMemcpyHostToDevice);
         if (e == cudaSuccess) e = cudaMemcpy(b->mem + gtb_off, gtb.data(), 4 * gtb.size(), cudaMemcpyHostToDevice);

@@ -46,8 +46,9 @@ struct PrepParams {
     int32_t rowsf;
     float4 *quad_dst;    // moving-image tap quads (W x H per channel), or null
     int64_t qplane;
-    int32_t quad_form;   // 0: {P00, P10, P01 - P00, P11 - P10}; 1 (span kernel): {P00, P01 - P00, P10 - P00,
-                         // (P11 - P10) - (P01 - P00)}, P(dy, dx) the tap at (y + dy, x + dx)
+    int32_t quad_form;   // 0: {P00, P10, P01 - P00, P11 - P10}; 1 (ZNCC and MI span kernels): {P00, P01 - P00,
+                         // P10 - P00, (P11 - P10) - (P01 - P00)}; 2 (exact span kernel): {P00, P01, P10, P11};
+                         // P(dy, dx) the tap at (y + dy, x + dx)
 };
 
 // Staged layout of a moving/fixed image pair inside one scratch block.
@@ -96,14 +97,17 @@ const void *kernel_scan(int cost, int C);
 size_t scan_smem_bytes(int cost);
 
 // Span kernel of zero-mean NCC (cgs_span.cuh): G points per warp, NW warps, tiles of 32 TX
-// columns; `check` selects the self-checking build.  Its shared-memory size, the largest quad
-// plane it takes, and the launch of its own staging step (the fixed rows' FP64 prefix sums, the
-// moving shift folded into the quads) after prep_kernel.
+// columns; `check` selects the self-checking build.  The span kernel of the exact-sampling costs
+// (cgs_span_exact.cuh): 4 points per warp, 16 warps, C channels.  Their shared-memory size, the
+// largest quad plane they take, and the launch of their staging step after prep_kernel (the fixed
+// rows' FP64 prefix sums where `prefix` is given, the moving shift folded into `nquads` quads).
 const void *kernel_span_zncc(int G, int NW, int TX, bool check);
+const void *kernel_span_exact(int cost, int C, int TX, bool check);
 size_t span_kernel_smem(int G, int NW, int TH, int TX, int tiles, int cap);
 int64_t span_max_quads();
-cudaError_t launch_span_prep(const float *fix, int fpitch, int fw, int fh, double2 *prefix, float4 *quads,
-                             int64_t nquads, const float *shifts, cudaStream_t stream);
+SpanPrepArgs span_prep_args(const float *fix, int fpitch, int64_t fplane, int channels, int fw, int fh, double2 *prefix,
+                            float4 *quads, int64_t nquads, const float *shifts, int *blocks);
+cudaError_t launch_span_prep(const SpanPrepArgs &a, int blocks, cudaStream_t stream);
 constexpr unsigned int kStatusSpanBounds = 0x100u;  // result status bit of the self-checking span build
 constexpr int kWinStages = 1;                      // window stages of the ZNCC span kernel
 constexpr int kMinSpanCap = 1024;                   // smallest useful window stage (quads)
@@ -114,12 +118,16 @@ struct SpanPlan {
     size_t smem = 0;
     const void *kfn = nullptr;
 };
+// Whether cgs_search runs a request on a tiled span kernel (zero-mean NCC on fast samples, or a cost
+// of kernel_span_exact on exact ones), with its plan.
 bool span_plan(const cgs_image &mov, const cgs_image &fix, const cgs_options &o, SpanPlan *sp);
+// The staging form of the quads (PrepParams::quad_form) and whether the cost reads the fixed rows'
+// prefix sums.
+inline int span_quad_form(int cost) { return cost == CGS_COST_ZNCC || cost == CGS_COST_MI ? 1 : 2; }
+inline bool span_uses_prefix(int cost) { return cost != CGS_COST_SAD_AVG; }
 // The multi-pair span kernel of batches for a plan (null where not instantiated), and the
-// staging step of many pairs: per pair its arguments and block count, then one launch over all.
-const void *kernel_span_zncc_batch(int G, int NW, int TX, bool check);
-void span_prep_batch_args(const float *fix, int fpitch, int fw, int fh, double2 *prefix, float4 *quads,
-                          int64_t nquads, const float *shifts, SpanPrepArgs *a, int *blocks);
+// staging step of many pairs in one launch.
+const void *kernel_span_batch(int G, int NW, int TX, bool check);
 cudaError_t launch_span_prep_batch(const SpanPrepArgs *args, int n, int blocks, cudaStream_t stream);
 // Span kernel of MI (cgs_span_mi.cuh): 2 points per warp, NW warps, histograms of B <= 32 bins;
 // its shared-memory size and its staging step (the fixed bins times B + 1, int32; the quads'

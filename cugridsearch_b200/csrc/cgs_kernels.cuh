@@ -61,7 +61,8 @@ struct SearchParams {
     const float *shifts; // {fixed, moving} image means (staging kernel): the shifts of the ZNCC sums
     cudaTextureObject_t mov_tex;  // the staged moving planes as one (W+1) x C(H+1) texture
     const float4 *mov_quad;       // per channel, W x H taps {(y, x), (y+1, x), (y, x+1) - (y, x), (y+1, x+1) - (y+1, x)}
-                                  // (the span kernel's form: PrepParams::quad_form 1, less the moving shift)
+                                  // (the span kernels' forms: PrepParams::quad_form 1, for ZNCC less the
+                                  // moving shift, and 2)
     int32_t quad_pitch;           // quads per row
     int64_t quad_plane;           // quads per channel
     const float *row_table;       // calcMIAlt's row values (the float recurrence row += 1/(H_f-1))
@@ -86,6 +87,8 @@ struct SpanPrepArgs {
     int fpitch, fw, fh;
     double2 *prefix;
     int row_blocks;  // blocks [0, row_blocks) write the prefix sums, the others shift the quads
+    int channels;    // the sums run over the channels of a pixel (planes fplane floats apart)
+    int64_t fplane;
     float4 *quads;
     int64_t nquads;
     const float *shifts;
@@ -174,8 +177,8 @@ struct RowTerms {
 // corners).  The guard is twice that.  Beyond B_x the bound grows with slope
 // 7.2u M_w / w_lo + 4.1u, which must stay small for "clearly outside" to hold there.  A
 // point whose w may change sign over the image, or whose bound is not small, takes the
-// exact path everywhere.
-__device__ __forceinline__ void map_guard(const MapCoef &k, const SearchParams &p, FastMap &f, RowTerms &rt,
+// exact path everywhere.  Returns whether the bound holds (whatever the sampling mode).
+__device__ __forceinline__ bool map_guard(const MapCoef &k, const SearchParams &p, FastMap &f, RowTerms &rt,
                                           float &gx_out, float &gy_out) {
     f.A = k.A;
     f.C1 = k.C1;
@@ -213,6 +216,7 @@ __device__ __forceinline__ void map_guard(const MapCoef &k, const SearchParams &
     }
     gx_out = (float)gx;
     gy_out = (float)gy;
+    return ok;
 }
 
 // ---------------------------------------------------------------- costs

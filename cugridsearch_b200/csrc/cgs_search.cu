@@ -230,8 +230,8 @@ __device__ __forceinline__ void prep_body(const PrepParams &q, int64_t tid, int6
         // tap quads of the staged moving plane, the left column and the FP32 differences to the
         // right column: {P(y, x), P(y + 1, x), P(y, x + 1) - P(y, x), P(y + 1, x + 1) - P(y + 1, x)}
         // with P the padded plane (column W = the next row's pixel 0, row H = 0); the search
-        // kernel's bilinear step takes the differences as they are.  The span kernel's form holds
-        // the bilinear polynomial's coefficients instead (quad_form 1)
+        // kernel's bilinear step takes the differences as they are.  The span kernels' forms hold the
+        // bilinear polynomial's coefficients (quad_form 1) or the taps as they are (2)
         const int64_t qtot = q.qplane * q.c;
         auto P = [&](int c, int64_t y, int64_t x) -> float {
             if (y >= q.mh) return 0.0f;
@@ -242,9 +242,11 @@ __device__ __forceinline__ void prep_body(const PrepParams &q, int64_t tid, int6
             const int c = (int)(i / q.qplane);
             const int64_t e = i - (int64_t)c * q.qplane;
             const int64_t y = e / q.mw, x = e - y * q.mw;
-            const float v00 = P(c, y, x), v10 = P(c, y + 1, x);
-            const float d0 = P(c, y, x + 1) - v00, d1 = P(c, y + 1, x + 1) - v10;
-            q.quad_dst[i] = q.quad_form ? make_float4(v00, d0, v10 - v00, d1 - d0) : make_float4(v00, v10, d0, d1);
+            const float v00 = P(c, y, x), v10 = P(c, y + 1, x), v01 = P(c, y, x + 1), v11 = P(c, y + 1, x + 1);
+            const float d0 = v01 - v00, d1 = v11 - v10;
+            q.quad_dst[i] = q.quad_form == 2   ? make_float4(v00, v01, v10, v11)
+                            : q.quad_form == 1 ? make_float4(v00, d0, v10 - v00, d1 - d0)
+                                               : make_float4(v00, v10, d0, d1);
         }
     }
     if (q.row_table && tid == 0) {
@@ -684,31 +686,41 @@ static Plan choose_plan(int cost, const cgs_options &o, int mi_bins) {
     return pl;
 }
 
-// Launch plan of the span kernel: points per warp (the request's 2, else 4), 16 warps, tiles of
-// 32 TX columns by TH rows (256 x 16 unless the tuning variables CGS_SPAN_TX = 2 | 4 | 8 and
-// CGS_SPAN_TH = 8 | 16 | 32 say otherwise), the window stage filling the shared memory that is
-// left (at most CGS_SPAN_CAP 16-byte units when that is set; a stage holds the tile's fixed rows
-// and its blocks' windows) and window rows padded to CGS_SPAN_PITCH (mod 8) quads.
-// CGS_SPAN_CHECK=1 selects the self-checking build (every fast sample's quad address is checked
-// against its window; a miss sets status bit 0x100 and skips the sample).  False where the span
-// kernel does not apply: several channels, images of 32768 or more pixels a side, moving images
-// with (W + 8) H of 2^22 or more, or too many tiles for shared memory.
+// Launch plan of the tiled span kernels: points per warp (4; ZNCC: the request's 2), 16 warps, tiles
+// of 32 TX columns by TH rows, the window stage filling the shared memory that is left (at most
+// CGS_SPAN_CAP 16-byte units when that is set; it holds the tile's fixed rows and its blocks' windows,
+// of every channel) and window rows padded to CGS_SPAN_PITCH (mod 8) quads.  One channel: tiles of
+// 256 x 16 unless the tuning variables CGS_SPAN_TX = 2 | 4 | 8 (ZNCC) and CGS_SPAN_TH = 8 | 16 | 32 say
+// otherwise; three channels (exact samples): 64 x 16, whose 2 x 3 windows of about 1.1 K quads fit the
+// stage where eight would not.  CGS_SPAN_CHECK=1 selects the self-checking build (every sample's quad
+// address is checked against its window; a miss sets status bit 0x100 and skips the sample).
+//
+// The kernel runs zero-mean NCC on fast samples and SAD_AVG, SQD_REF and NCC_REF on exact ones, unless
+// the request asks for per-sample decisions or names a source of taps (a per-sample kernel's).
+// False where it does not apply: other channel counts, images of 32768 or more pixels a side, moving
+// images with (W + 8) H of 2^22 or more, or too many tiles for shared memory.
 static int env_int(const char *name, int dflt) {
     const char *v = std::getenv(name);
     return (v && *v) ? std::atoi(v) : dflt;
 }
 
 bool span_plan(const cgs_image &mov, const cgs_image &fix, const cgs_options &o, SpanPlan *sp) {
-    if (fix.channels != 1 || mov.width >= 32768 || mov.height >= 32768 || fix.width >= 32768 || fix.height >= 32768 ||
+    const int C = fix.channels;
+    const bool zncc = o.cost == CGS_COST_ZNCC && !exact_samples(o.cost, o.flags) && !(o.flags & CGS_FLAG_TEXTURE_TAPS);
+    const bool exact = (o.cost == CGS_COST_SAD_AVG || o.cost == CGS_COST_SQD_REF || o.cost == CGS_COST_NCC_REF) &&
+                       exact_samples(o.cost, o.flags) && !(o.flags & (CGS_FLAG_TEXTURE_TAPS | CGS_FLAG_QUAD_TAPS));
+    if (!(zncc || exact) || (o.flags & CGS_FLAG_PER_SAMPLE_DECISIONS)) return false;
+    if (!(C == 1 || (exact && C == 3))) return false;
+    if (mov.width >= 32768 || mov.height >= 32768 || fix.width >= 32768 || fix.height >= 32768 ||
         (int64_t)(mov.width + 8) * mov.height >= span_max_quads())
         return false;
-    sp->G = o.points_per_warp == 2 ? 2 : 4;
+    sp->G = zncc && o.points_per_warp == 2 ? 2 : 4;
     sp->NW = 16;
-    sp->TX = env_int("CGS_SPAN_TX", 8);
+    sp->TX = C == 3 ? 2 : zncc ? env_int("CGS_SPAN_TX", 8) : 8;
     sp->TH = env_int("CGS_SPAN_TH", 16);
     if (!(sp->TX == 2 || sp->TX == 4 || sp->TX == 8) || !(sp->TH == 8 || sp->TH == 16 || sp->TH == 32)) return false;
     sp->check = env_int("CGS_SPAN_CHECK", 0) != 0;
-    sp->kfn = kernel_span_zncc(sp->G, sp->NW, sp->TX, sp->check);
+    sp->kfn = zncc ? kernel_span_zncc(sp->G, sp->NW, sp->TX, sp->check) : kernel_span_exact(o.cost, C, sp->TX, sp->check);
     if (!sp->kfn) return false;
     sp->tiles_x = (fix.width + 32 * sp->TX - 1) / (32 * sp->TX);
     sp->tiles_y = (fix.height + sp->TH - 1) / sp->TH;
@@ -718,7 +730,7 @@ bool span_plan(const cgs_image &mov, const cgs_image &fix, const cgs_options &o,
     sp->cap = (int)((budget - fixed) / (16 * kWinStages));
     // CGS_SPAN_CAP (quads) lowers the stage size, e.g. to exercise the global-memory path
     sp->cap = std::max(kMinSpanCap, std::min(sp->cap, env_int("CGS_SPAN_CAP", sp->cap)));
-    sp->cap = std::max(sp->cap, kMinSpanCap + sp->TH * 32 * sp->TX / 4);  // room for the fixed rows
+    sp->cap = std::max(sp->cap, kMinSpanCap + C * sp->TH * 32 * sp->TX / 4);  // room for the fixed rows
     sp->pitch_mod = env_int("CGS_SPAN_PITCH", 0) & 7;
     sp->smem = span_kernel_smem(sp->G, sp->NW, sp->TH, sp->TX, tiles, sp->cap);
     return sp->smem <= budget;
@@ -968,16 +980,15 @@ static cgs_status search_core(const cgs_image *mov, const cgs_image *fix, const 
     // taps: pre-gathered quads where the fast sampling path runs (measured faster than texture
     // gathers there); texture gathers (MI: scalar loads) for exact sampling and for MI
     const bool fast_path = !exact_samples(cost, o.flags) && cost != CGS_COST_MI;
-    // zero-mean NCC and MI on the fast path: the span kernels (row decisions; ZNCC with
-    // shared-memory windows, MI with shared-memory histograms); both read span-form quads
+    // the span kernels (row decisions): single-channel ZNCC and the exact-sampling costs with
+    // shared-memory windows (span_plan), single-channel MI with shared-memory histograms
     SpanPlan sp;
-    const bool per_sample = (o.flags & CGS_FLAG_PER_SAMPLE_DECISIONS) != 0;
-    const bool span = cost == CGS_COST_ZNCC && fast_path && !(o.flags & CGS_FLAG_TEXTURE_TAPS) && !per_sample &&
-                      span_plan(*mov, *fix, o, &sp);
-    const bool span_mi = cost == CGS_COST_MI && !exact_samples(cost, o.flags) && !per_sample &&
-                         !(o.flags & (CGS_FLAG_TEXTURE_TAPS | CGS_FLAG_QUAD_TAPS)) &&
+    const bool span = span_plan(*mov, *fix, o, &sp);
+    const bool span_mi = cost == CGS_COST_MI && !exact_samples(cost, o.flags) &&
+                         !(o.flags & (CGS_FLAG_PER_SAMPLE_DECISIONS | CGS_FLAG_TEXTURE_TAPS | CGS_FLAG_QUAD_TAPS)) &&
                          span_mi_plan(*mov, *fix, o, mi_bins, &sp);
-    const bool quads = (o.flags & CGS_FLAG_QUAD_TAPS) || (fast_path && !(o.flags & CGS_FLAG_TEXTURE_TAPS)) || span_mi;
+    const bool quads = span || span_mi || (o.flags & CGS_FLAG_QUAD_TAPS) ||
+                       (fast_path && !(o.flags & CGS_FLAG_TEXTURE_TAPS));
     const void *kfn = (span || span_mi) ? sp.kfn : getter(C, pl.G, pl.NW, quads);
     if (!kfn) return fail(CGS_ERROR_UNSUPPORTED, "no kernel for this channel count / tuning");
     if (ext && !(span || span_mi)) return fail(CGS_ERROR_UNSUPPORTED, "caller scratch: span searches only");
@@ -1013,10 +1024,10 @@ static cgs_status search_core(const cgs_image *mov, const cgs_image *fix, const 
         p.win_pitch_mod = sp.pitch_mod;
     }
 
-    // the span kernels' tables follow the staging block: the ZNCC kernel's row prefix sums (W_f + 1
+    // the span kernels' tables follow the staging block: the tiled kernels' row prefix sums (W_f + 1
     // FP64 pairs per row), the MI kernel's fixed bins (int32, the fixed plane's pitch)
     const size_t prefix_off = (size_t)round_up((int64_t)(st.bytes - (size_t)di.tex_align), 256);
-    const size_t prefix_bytes = span      ? (size_t)fix->height * (size_t)(fix->width + 1) * sizeof(double2)
+    const size_t prefix_bytes = span      ? (span_uses_prefix(cost) ? 1 : 0) * (size_t)fix->height * (size_t)(fix->width + 1) * sizeof(double2)
                                 : span_mi ? (size_t)fix->height * (size_t)st.fpitch * sizeof(int32_t)
                                           : 0;
     const size_t main_bytes = st.bytes + (prefix_bytes ? prefix_bytes + 256 : 0);
@@ -1039,7 +1050,7 @@ static cgs_status search_core(const cgs_image *mov, const cgs_image *fix, const 
         if (!ext && ptr) cudaFreeAsync(ptr, stream);
     };
     char *sb = staging_origin(scratch, di.tex_align);
-    if (span) p.fix_prefix = reinterpret_cast<const double2 *>(sb + prefix_off);
+    if (span && span_uses_prefix(cost)) p.fix_prefix = reinterpret_cast<const double2 *>(sb + prefix_off);
     if (span_mi) {
         p.span_rows = reinterpret_cast<const float *>(sb + prefix_off);
         p.span_rows_header = reinterpret_cast<const float *>(sb + 32);  // zeroed with the header
@@ -1080,7 +1091,7 @@ static cgs_status search_core(const cgs_image *mov, const cgs_image *fix, const 
     if (quads) {
         q.quad_dst = reinterpret_cast<float4 *>(sb + st.quad_off);
         q.qplane = st.qplane;
-        q.quad_form = (span || span_mi) ? 1 : 0;
+        q.quad_form = (span || span_mi) ? span_quad_form(cost) : 0;
     }
     const int64_t prep_elems = (st.mplane + st.fplane) * C;
     const int prep_blocks = (int)std::min<int64_t>((prep_elems + 255) / 256, (int64_t)di.sms * 8);
@@ -1089,9 +1100,14 @@ static cgs_status search_core(const cgs_image *mov, const cgs_image *fix, const 
         prep_kernel<<<prep_blocks, 256, 0, stream>>>(q);
         e = cudaGetLastError();
     }
-    if (e == cudaSuccess && span)
-        e = launch_span_prep(fstage, st.fpitch, fix->width, fix->height, const_cast<double2 *>(p.fix_prefix),
-                             reinterpret_cast<float4 *>(sb + st.quad_off), st.qplane, p.shifts, stream);
+    if (e == cudaSuccess && span && p.fix_prefix) {
+        int blocks = 0;
+        const SpanPrepArgs a = span_prep_args(fstage, st.fpitch, st.fplane, C, fix->width, fix->height,
+                                              const_cast<double2 *>(p.fix_prefix),
+                                              reinterpret_cast<float4 *>(sb + st.quad_off),
+                                              cost == CGS_COST_ZNCC ? st.qplane : 0, p.shifts, &blocks);
+        e = launch_span_prep(a, blocks, stream);
+    }
     if (e == cudaSuccess && span_mi)
         e = launch_span_prep_mi(fstage, st.fpitch, fix->width, fix->height, mi_bins,
                                 reinterpret_cast<int32_t *>(sb + prefix_off),
@@ -1119,7 +1135,7 @@ static cgs_status search_core(const cgs_image *mov, const cgs_image *fix, const 
     }
     const uint32_t blocks = std::min<uint32_t>(p.num_tasks, (uint32_t)(di.sms * per_sm));
     void *args[] = {&p};
-    if (ext) {  // the span kernels read tap quads, no texture
+    if (span || span_mi) {  // these read tap quads, no texture
         p.mov_tex = 0;
         e = cudaLaunchKernel(kfn, dim3(blocks), dim3(threads), args, smem, stream);
     } else {

@@ -233,7 +233,7 @@ __device__ __forceinline__ void block_extent(const SpanSlot &k, float x0, float 
 
 // Thread 0: announce the bytes of tile t's copies on stage `st`'s barrier (its one arrival).  It
 // comes before the CTA barrier after which every warp issues its part (issue_window).
-template <int TX>
+template <int C, int TX>
 __device__ __forceinline__ void expect_window(const SearchParams &p, const SpanSmem &ss, int t, int st) {
     constexpr int TW = 32 * TX;
     const int x0 = (t % p.tiles_x) * TW, y0 = (t / p.tiles_x) * p.tile_h;
@@ -242,6 +242,7 @@ __device__ __forceinline__ void expect_window(const SearchParams &p, const SpanS
 #pragma unroll
     for (int c = 0; c < TX; c++)
         if (bw[c].h > 0 && bw[c].w > 0) bytes += (uint32_t)bw[c].w * (uint32_t)bw[c].h * 16u;
+    bytes *= C;
     mbar_arrive_expect_tx(&ss.bars[st], bytes);
 }
 
@@ -250,7 +251,7 @@ __device__ __forceinline__ void expect_window(const SearchParams &p, const SpanS
 // past the image's right edge are not copied) and the windows of its blocks (quads, after the
 // fixed tile).  A tile has about 220 row copies and a warp issues one in about 60 cycles, so one
 // warp would hold the others back for 14 K cycles per tile; shared by the CTA's warps it is 1 K.
-template <int NW, int TX>
+template <int C, int NW, int TX>
 __device__ __forceinline__ void issue_window(const SearchParams &p, const SpanSmem &ss, int t, int st) {
     constexpr int TW = 32 * TX;
     constexpr int WB = NW / TX;  // warps per block window
@@ -265,20 +266,57 @@ __device__ __forceinline__ void issue_window(const SearchParams &p, const SpanSm
         const uint32_t row_bytes = (uint32_t)((min(TW, p.fix.w - x0) * 4 + 15) & ~15);  // within the row pitch
         float *fdst = reinterpret_cast<float *>(ss.win + (size_t)st * ss.cap);
         for (int j = warp; j < rows; j += NW)
-            bulk_g2s(fdst + j * TW, p.fix.data + (int64_t)(y0 + j) * p.fix.pitch + x0, row_bytes, bar);
+#pragma unroll
+            for (int ch = 0; ch < C; ch++)
+                bulk_g2s(fdst + (ch * TH + j) * TW, p.fix.data + ch * p.fix.plane + (int64_t)(y0 + j) * p.fix.pitch + x0,
+                         row_bytes, bar);
     }
     const BlockWin b = ss.wins[t * TX + warp / WB];
     if (b.h > 0 && b.w > 0) {
-        float4 *wdst = ss.win + (size_t)st * ss.cap + TH * TW / 4 + b.off;
+        float4 *wdst = ss.win + (size_t)st * ss.cap + C * TH * TW / 4 + b.off;
         const float4 *src = p.mov_quad + (int64_t)b.y0 * p.quad_pitch + b.x0;
         for (int j = lane * WB + warp % WB; j < b.h; j += 32 * WB)
-            bulk_g2s(wdst + (size_t)j * b.pitch, src + (int64_t)j * p.quad_pitch, (uint32_t)b.w * 16u, bar);
+#pragma unroll
+            for (int ch = 0; ch < C; ch++)
+                bulk_g2s(wdst + (size_t)(ch * b.h + j) * b.pitch, src + ch * p.quad_plane + (int64_t)j * p.quad_pitch,
+                         (uint32_t)b.w * 16u, bar);
     }
 }
 
+// Correctly rounded quotients without a branch: x = X / w and y = Y / w of a pair of points from w,
+// -X and -Y (the caller forms the negatives by negating coefficients, which is exact).  The reciprocal
+// r of w is the approximate one and a Newton step; the quotient q0 = X r is corrected by its exact
+// residual, q = q0 + (X - w q0) r (P. Markstein, "Computation of elementary functions on the IBM RISC
+// System/6000 processor", IBM J. Res. Dev. 34, 1990).  Checked against IEEE division for every pair of
+// 24-bit mantissas (2^46 quotients): r and q are always the correctly rounded values, provided that no
+// step leaves the normal range (quot_range).  Eight packed operations and two reciprocals replace four
+// divisions of about ten instructions and a branch each.
+__device__ __forceinline__ void exact_quot2(float2 w, float2 nX, float2 nY, float2 &x, float2 &y) {
+    const float2 nr0 = make_float2(rcp_approx(-w.x), rcp_approx(-w.y));
+    const float2 e = __ffma2_rn(w, nr0, make_float2(1.0f, 1.0f));
+    const float2 nr = __ffma2_rn(e, nr0, nr0);
+    const float2 x0 = __fmul2_rn(nX, nr), y0 = __fmul2_rn(nY, nr);
+    x = __ffma2_rn(__ffma2_rn(w, x0, nX), nr, x0);
+    y = __ffma2_rn(__ffma2_rn(w, y0, nY), nr, y0);
+}
+
+// Whether exact_quot2 applies to every pixel of a fw x fh image: |w| in [2^-40, 2^40] at the corners
+// (w is linear and the guard keeps its sign), numerators below 2^60, and every numerator coefficient
+// zero or at least 2^-70, so that a numerator, a sum of multiples of 2^-93, is zero or at least that.
+__device__ __forceinline__ bool quot_range(const MapCoef &k, int fw, int fh) {
+    const float x1 = (float)(fw - 1), y1 = (float)(fh - 1), pq = k.P - k.Q;
+    const float w0 = fabsf(pq), w1 = fabsf(k.A * x1 + pq), w2 = fabsf(k.B * y1 + pq), w3 = fabsf(k.A * x1 + k.B * y1 + pq);
+    bool ok = fminf(fminf(w0, w1), fminf(w2, w3)) >= 0x1p-40f && fmaxf(fmaxf(w0, w1), fmaxf(w2, w3)) <= 0x1p40f;
+    const float c[8] = {k.C1, k.C2, k.R, k.S, k.D1, k.D2, k.T, k.U};
+#pragma unroll
+    for (int i = 0; i < 8; i++) ok = ok && (c[i] == 0.0f || (fabsf(c[i]) >= 0x1p-70f && fabsf(c[i]) <= 0x1p40f));
+    return ok;
+}
+
 // The G grid points from ordinal ord0: lane g decodes point g and writes its slot (the decode, the
-// homography and the FP64 guard of a point are a chain of about 5 K cycles: four at once).
-template <int COST, int G>
+// homography and the FP64 guard of a point are a chain of about 5 K cycles: four at once).  `ok`: the
+// guard holds and, for exact samples (EXACT), the point's quotients are in the range of exact_quot2.
+template <int COST, int G, bool EXACT = false>
 __device__ __forceinline__ void span_points(const SearchParams &p, uint32_t ord0, SpanSlot *slots) {
     const int lane = threadIdx.x & 31;
     if (lane >= G) return;
@@ -293,10 +331,81 @@ __device__ __forceinline__ void span_points(const SearchParams &p, uint32_t ord0
     FastMap fm;
     RowTerms rt;
     float gx, gy;
-    map_guard(kc, p, fm, rt, gx, gy);
-    const bool ok = gvalid && fm.li_x > 0.0f;
+    const bool guard = map_guard(kc, p, fm, rt, gx, gy);
+    const bool ok = gvalid && guard && (EXACT ? quot_range(kc, p.fix.w, p.fix.h) : fm.li_x > 0.0f);
     slots[lane] = SpanSlot{kc.A, rt.B, rt.PQ, kc.C1, rt.C2, rt.RS, kc.D1, rt.D2, rt.TU, kc.P, kc.Q, kc.R,
                            kc.S, kc.T, kc.U, gx, gy, ok ? 1 : 0, gvalid ? 1 : 0, gidx};
+}
+
+// The windows of every block of every tile, into ss.wins: warp w takes blocks w, w + NW, .. with the
+// task's points over its lanes, then one thread per tile lays its blocks out in the stage (C planes of
+// quads each, pitch x h apart).
+template <int C, int G, int NW, int TX>
+__device__ __forceinline__ void span_windows(const SearchParams &p, const SpanSmem &ss) {
+    constexpr int TW = 32 * TX;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int fw = p.fix.w, fh = p.fix.h, TH = p.tile_h, tiles_x = p.tiles_x, ntiles = p.tiles_x * p.tiles_y;
+    const float mov_wf = p.mov_wf, mov_hf = p.mov_hf;
+    constexpr int P = NW * G;
+    const float inf = __int_as_float(0x7f800000);
+    for (int i = warp; i < ntiles * TX; i += NW) {
+        const int t = i / TX, c = i - t * TX;
+        const int xc = (t % tiles_x) * TW + 32 * c, y0 = (t / tiles_x) * TH;
+        float4 e = make_float4(inf, inf, -inf, -inf);
+        if (xc < fw) {
+            const float fx0 = (float)xc, fx1 = (float)(min(xc + 32, fw) - 1);
+            const float fy0 = (float)y0, fy1 = (float)(min(y0 + TH, fh) - 1);
+            for (int k = lane; k < P; k += 32)
+                if (ss.slots[k].ok) block_extent(ss.slots[k], fx0, fx1, fy0, fy1, e);
+            e.x = warp_fmin(e.x);
+            e.y = warp_fmin(e.y);
+            e.z = warp_fmax(e.z);
+            e.w = warp_fmax(e.w);
+        }
+        if (lane == 0) {  // the block's extent, in its window's place
+            float2 *d = reinterpret_cast<float2 *>(&ss.wins[i]);
+            d[0] = make_float2(e.x, e.y);
+            d[1] = make_float2(e.z, e.w);
+        }
+    }
+    __syncthreads();
+    const int wcap = ss.cap - C * TH * TW / 4;  // quads of a stage after the fixed rows
+    for (int t = threadIdx.x; t < ntiles; t += NW * 32) {
+        int used = 0;
+#pragma unroll 1
+        for (int c = 0; c < TX; c++) {
+            BlockWin bw{0, 0, 0, 0, 0, 0, 0u, 0.0f};
+            // cells a fast sample can use: floor of its coordinate (within the guard, < 1/8 px,
+            // of the real map, whose block image lies in the corners' hull), clipped to the image
+            const float2 *d = reinterpret_cast<const float2 *>(&ss.wins[t * TX + c]);
+            const float2 e0 = d[0], e1 = d[1];
+            const float lx = fmaxf(e0.x - 0.25f, -1.0f), ly = fmaxf(e0.y - 0.25f, -1.0f);
+            const float hx = fminf(e1.x + 0.25f, mov_wf), hy = fminf(e1.y + 0.25f, mov_hf);
+            if (lx <= hx && ly <= hy) {
+                const int cx0 = max(0, (int)floorf(lx)), cy0 = max(0, (int)floorf(ly));
+                const int cx1 = min(p.mov.w - 1, (int)floorf(hx)), cy1 = min(p.mov.h - 1, (int)floorf(hy));
+                if (cx0 <= cx1 && cy0 <= cy1) {
+                    const int w = cx1 - cx0 + 1, h = cy1 - cy0 + 1;
+                    const int pitch = w + ((p.win_pitch_mod - w) & 7);  // = win_pitch_mod (mod 8)
+                    bw.x0 = (int16_t)cx0;
+                    bw.y0 = (int16_t)cy0;
+                    bw.h = (int16_t)h;
+                    bw.pitch = pitch;
+                    if ((int64_t)C * pitch * h <= wcap - used) {
+                        bw.w = (int16_t)w;
+                        bw.off = used;
+                        bw.rel = 16u * ((uint32_t)used - (uint32_t)cx0 - (uint32_t)pitch * (uint32_t)cy0 -
+                                        (uint32_t)kMagicBits);
+                        bw.pitchf = -(float)pitch;
+                        used += C * pitch * h;
+                    } else {
+                        bw.w = -1;
+                    }
+                }
+            }
+            ss.wins[t * TX + c] = bw;
+        }
+    }
 }
 
 // One task of the span path (ZNCC, one channel, quads staged): the G grid points of each warp
@@ -343,76 +452,13 @@ __device__ __forceinline__ bool run_span_task(const SearchParams &p, uint32_t ta
     const float fshift = p.shifts[0], mshift = p.shifts[1];
     __syncthreads();  // every point's slot is written
 
-    // ---- windows of every block of every tile: warp w takes blocks w, w + NW, ..; lanes take the
-    // task's points; then one thread per tile lays its blocks out in the stage
-    {
-        constexpr int P = NW * G;
-        const float inf = __int_as_float(0x7f800000);
-        for (int i = warp; i < ntiles * TX; i += NW) {
-            const int t = i / TX, c = i - t * TX;
-            const int xc = (t % tiles_x) * TW + 32 * c, y0 = (t / tiles_x) * TH;
-            float4 e = make_float4(inf, inf, -inf, -inf);
-            if (xc < fw) {
-                const float fx0 = (float)xc, fx1 = (float)(min(xc + 32, fw) - 1);
-                const float fy0 = (float)y0, fy1 = (float)(min(y0 + TH, fh) - 1);
-                for (int k = lane; k < P; k += 32)
-                    if (ss.slots[k].ok) block_extent(ss.slots[k], fx0, fx1, fy0, fy1, e);
-                e.x = warp_fmin(e.x);
-                e.y = warp_fmin(e.y);
-                e.z = warp_fmax(e.z);
-                e.w = warp_fmax(e.w);
-            }
-            if (lane == 0) {  // the block's extent, in its window's place
-                float2 *d = reinterpret_cast<float2 *>(&ss.wins[i]);
-                d[0] = make_float2(e.x, e.y);
-                d[1] = make_float2(e.z, e.w);
-            }
-        }
-        __syncthreads();
-        const int wcap = ss.cap - TH * TW / 4;  // quads of a stage after the fixed rows
-        for (int t = threadIdx.x; t < ntiles; t += NW * 32) {
-            int used = 0;
-#pragma unroll 1
-            for (int c = 0; c < TX; c++) {
-                BlockWin bw{0, 0, 0, 0, 0, 0, 0u, 0.0f};
-                // cells a fast sample can use: floor of its coordinate (within the guard, < 1/8 px,
-                // of the real map, whose block image lies in the corners' hull), clipped to the image
-                const float2 *d = reinterpret_cast<const float2 *>(&ss.wins[t * TX + c]);
-                const float2 e0 = d[0], e1 = d[1];
-                const float lx = fmaxf(e0.x - 0.25f, -1.0f), ly = fmaxf(e0.y - 0.25f, -1.0f);
-                const float hx = fminf(e1.x + 0.25f, mov_wf), hy = fminf(e1.y + 0.25f, mov_hf);
-                if (lx <= hx && ly <= hy) {
-                    const int cx0 = max(0, (int)floorf(lx)), cy0 = max(0, (int)floorf(ly));
-                    const int cx1 = min(p.mov.w - 1, (int)floorf(hx)), cy1 = min(p.mov.h - 1, (int)floorf(hy));
-                    if (cx0 <= cx1 && cy0 <= cy1) {
-                        const int w = cx1 - cx0 + 1, h = cy1 - cy0 + 1;
-                        const int pitch = w + ((p.win_pitch_mod - w) & 7);  // = win_pitch_mod (mod 8)
-                        bw.x0 = (int16_t)cx0;
-                        bw.y0 = (int16_t)cy0;
-                        bw.h = (int16_t)h;
-                        bw.pitch = pitch;
-                        if ((int64_t)pitch * h <= wcap - used) {
-                            bw.w = (int16_t)w;
-                            bw.off = used;
-                            bw.rel = 16u * ((uint32_t)used - (uint32_t)cx0 - (uint32_t)pitch * (uint32_t)cy0 -
-                                            (uint32_t)kMagicBits);
-                            bw.pitchf = -(float)pitch;
-                            used += pitch * h;
-                        } else {
-                            bw.w = -1;
-                        }
-                    }
-                }
-                ss.wins[t * TX + c] = bw;
-            }
-        }
-    }
+    span_windows<1, G, NW, TX>(p, ss);
     __syncthreads();
     if (threadIdx.x == 0)
-        for (int t = 0; t < kWinStages && t < ntiles; t++) expect_window<TX>(p, ss, t, (int)((wit + t) % kWinStages));
+        for (int t = 0; t < kWinStages && t < ntiles; t++) expect_window<1, TX>(p, ss, t, (int)((wit + t) % kWinStages));
     __syncthreads();
     for (int t = 0; t < kWinStages && t < ntiles; t++)
-        issue_window<NW, TX>(p, ss, t, (int)((wit + t) % kWinStages));
+        issue_window<1, NW, TX>(p, ss, t, (int)((wit + t) % kWinStages));
 
     // ---- sweep
     float2 part[GP][3];  // {sum m', sum m'^2, sum f'm'} of each pair of points
@@ -714,7 +760,7 @@ __device__ __forceinline__ bool run_span_task(const SearchParams &p, uint32_t ta
                 }
         }
         const bool more = t + kWinStages < ntiles;
-        if (threadIdx.x == 0 && more) expect_window<TX>(p, ss, t + kWinStages, st);
+        if (threadIdx.x == 0 && more) expect_window<1, TX>(p, ss, t + kWinStages, st);
         __syncthreads();  // every warp is done with this stage
         if (*ss.abort_flag) {
             // a wait gave up: let this stage's copies and the next stage's (already issued) land,
@@ -726,7 +772,7 @@ __device__ __forceinline__ bool run_span_task(const SearchParams &p, uint32_t ta
             }
             return false;
         }
-        if (more) issue_window<NW, TX>(p, ss, t + kWinStages, st);
+        if (more) issue_window<1, NW, TX>(p, ss, t + kWinStages, st);
     }
 
     // ---- per grid point: finalise, dump, argmin key (as the pixel-loop kernel)
@@ -786,7 +832,7 @@ __global__ void __launch_bounds__(NW * 32, 1) span_kernel(const __grid_constant_
 }
 
 // Blocks [0, row_blocks) write the FP64 prefix sums of each staged fixed row, prefix[y (W + 1) +
-// x] = {sum f, sum f^2} of pixels 0 .. x - 1 of row y (channel 0; one warp per row, a warp scan
+// x] = {sum f, sum f^2} of pixels 0 .. x - 1 of row y (over the channels; one warp per row, a warp scan
 // per 32 pixels carried in order, so the sums are the same in every run); the other blocks of
 // the `nblocks` subtract the moving image's shift from every quad's constant term, so that the
 // sweep's bilinear values are shifted already.
@@ -807,8 +853,12 @@ __device__ __forceinline__ void span_prep_body(const SpanPrepArgs &a, int block,
     double c1 = 0.0, c2 = 0.0;
     for (int x0 = 0; x0 < fw; x0 += 32) {
         const int x = x0 + lane;
-        double v = x < fw ? (double)src[x] : 0.0;
-        double v2 = v * v;
+        double v = 0.0, v2 = 0.0;
+        for (int ch = 0; x < fw && ch < a.channels; ch++) {
+            const double u = (double)src[ch * a.fplane + x];
+            v += u;
+            v2 += u * u;
+        }
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
             const double t1 = __shfl_up_sync(0xffffffffu, v, o), t2 = __shfl_up_sync(0xffffffffu, v2, o);
@@ -831,64 +881,6 @@ static __global__ void __launch_bounds__(256) span_prep_kernel(const SpanPrepArg
 // exceeds every pair's row_blocks).
 static __global__ void __launch_bounds__(256) span_prep_batch_kernel(const SpanPrepArgs *__restrict__ args) {
     span_prep_body(args[blockIdx.y], (int)blockIdx.x, (int)gridDim.x);
-}
-
-// ---------------------------------------------------------------- the multi-pair span kernel
-//
-// Batches: the tasks of many ZNCC pairs (each with its own staged planes, prefix sums, tiles
-// and grid) from one counter, so that pairs too small to fill the GPU alone share it.  A
-// task's pair is found in the prefix of task counts; its parameters are read from global
-// memory.  Shared memory is carved once for the largest tile count of the pairs and one window
-// stage size (`cap`) for all of them; each pair's results are those of span_kernel on that pair.
-template <int G, int NW, int TX, bool CHECK>
-__global__ void __launch_bounds__(NW * 32, 1) span_batch_kernel(const __grid_constant__ SpanBatchParams b) {
-    extern __shared__ __align__(128) unsigned char smem[];
-    const SpanSmem ss = carve_span<G, NW>(smem, b.tile_h, TX, b.tiles, b.cap);
-    // the task word sits in the carve's head, after the flags (no static shared memory: the
-    // dynamic carve may take all 227 KB)
-    volatile uint32_t &s_task = *reinterpret_cast<volatile uint32_t *>(ss.bounds_flag + 1);
-    if (threadIdx.x == 0) {
-        for (int s = 0; s < kWinStages; s++) mbar_init(&ss.bars[s], 1);
-        fence_mbar_init();
-        *ss.abort_flag = 0;
-        *ss.bounds_flag = 0;
-    }
-    uint32_t wit = 0;
-    for (;;) {
-        __syncthreads();  // the previous task is done with s_task
-        if (threadIdx.x == 0) s_task = atomicAdd(b.next_task, 1u);
-        __syncthreads();
-        const uint32_t t = s_task;
-        if (t >= b.total_tasks) return;
-        uint32_t lo = 0, hi = b.n_pairs;  // task_begin[lo] <= t < task_begin[hi]
-        while (hi - lo > 1) {
-            const uint32_t mid = (lo + hi) >> 1;
-            if (__ldg(b.task_begin + mid) <= t) lo = mid;
-            else hi = mid;
-        }
-        const SearchParams &p = b.pairs[lo];
-        const uint32_t slot = __ldg(b.slot + lo);
-        if (threadIdx.x == 0 && b.t_start) atomicMin(b.t_start + slot, (unsigned long long)global_ns());
-        if (!run_span_task<G, NW, TX, CHECK>(p, t - __ldg(b.task_begin + lo), ss, wit)) {
-            if (threadIdx.x == 0) {
-                // retire this task and every task not yet taken, with the timeout status
-                retire_tasks(p, ~0ull, 1u, true);
-                for (;;) {
-                    const uint32_t u = atomicAdd(b.next_task, 1u);
-                    if (u >= b.total_tasks) break;
-                    uint32_t l2 = 0, h2 = b.n_pairs;
-                    while (h2 - l2 > 1) {
-                        const uint32_t mid = (l2 + h2) >> 1;
-                        if (__ldg(b.task_begin + mid) <= u) l2 = mid;
-                        else h2 = mid;
-                    }
-                    retire_tasks(b.pairs[l2], ~0ull, 1u, true);
-                }
-            }
-            return;
-        }
-        if (threadIdx.x == 0 && b.t_end) atomicMax(b.t_end + slot, (unsigned long long)global_ns());
-    }
 }
 
 }  // namespace cgs

@@ -1,0 +1,480 @@
+// cgs_span_exact.cuh -- the span kernel for the reference functors that sample exactly:
+// averageAbsoluteDifference (SAD_AVG), calcSQD (SQD_REF) and calcNCC (NCC_REF), one or three
+// channels.  Every sample is formed by the reference's operation sequence, bit for bit, as the
+// per-sample kernel does; what changes is around it: the in/out decisions are taken per image row,
+// the taps come from shared-memory windows and the quotients need no branch.
+//
+// Decisions, tiles, windows, stages: as in the zero-mean NCC span kernel (cgs_span.cuh).  A point's
+// inner span lies at least 1.5 guard bands inside the moving image, and the guard bounds the distance
+// between the real and the reference's coordinates, so every pixel of the inner span is inside for the
+// reference; band pixels are decided and sampled in the span pass.  A point without a guard, or whose
+// quotients could leave exact_quot2's range, has no spans: the whole warp samples all of its pixels
+// with IEEE divisions (no_span_rows).
+//
+// Sweep.  Two points per FP32x2 operation.  The map keeps the reference's order
+// w = ((A x + B y) + P) - Q with each operation rounded; packed operations round each component as
+// the scalar ones.  X and Y are formed with negated coefficients (the same bits, sign flipped), which
+// the quotient step wants.  Floors and fractions are exact operations.  The quads hold the raw taps
+// {v00, v01, v10, v11}.  For the two NCC-like costs the row weights carry a factor 2^-8, so samples
+// come out scaled by it (a power of two: the same bits) and the sums of squares have the headroom of
+// the reference's v / 255 without its division; the factor leaves in FP64 at the end.
+//
+// What bounds it: the FP32 pipe.  A pair of points takes 29 packed operations (two pipe cycles each)
+// and about 21 scalar ones per pixel and channel: 40 cycles of a scheduler's FP32 pipe per 32
+// evaluations, 10 per SM, or 8.9e11 evaluations/s; the per-sample kernel needed two IEEE divisions
+// (about 20 instructions and two branches), the in/out decisions and a texture gather per evaluation.
+//
+// Sums.  Per lane and band of TH rows in FP32, then a warp sum into FP64 totals; the fixed image's
+// sum of squares comes from the row prefix sums.  The cost is formed in FP32 from the rounded totals
+// (finalize), so its special cases are the per-sample kernel's.  Costs do not depend on the order of
+// the points or on how many share a launch.
+#pragma once
+#include "cgs_span.cuh"
+
+namespace cgs {
+
+// FP32 sums of a pair of points in the sweep: SAD {sum |d|}; SQD {sum d^2, sum m^2}; NCC {sum m^2, sum f m}.
+template <int COST> struct SpanSums { static constexpr int value = COST == CGS_COST_SAD_AVG ? 1 : 2; };
+
+// Scale of the samples and fixed values in the sums (see above).
+template <int COST> struct SpanScale { static constexpr float value = COST == CGS_COST_SAD_AVG ? 1.0f : 0x1p-8f; };
+
+// One (fixed f, moving m) sample, both scaled, into FP64 sums.
+template <int COST>
+__device__ __forceinline__ void accumulate64(double *a, float f, float m) {
+    const float d = m - f;
+    if constexpr (COST == CGS_COST_SAD_AVG) {
+        a[0] += (double)fabsf(d);
+    } else if constexpr (COST == CGS_COST_SQD_REF) {
+        a[0] += (double)d * (double)d;
+        a[1] += (double)m * (double)m;
+    } else {
+        a[0] += (double)m * (double)m;
+        a[1] += (double)f * (double)m;
+    }
+}
+
+template <int COST, int C, int G, int NW, int TX, bool CHECK>
+__device__ __forceinline__ bool run_span_exact_task(const SearchParams &p, uint32_t task, const SpanSmem &ss,
+                                                    uint32_t &wit) {
+    static_assert(G % 2 == 0, "the span path pairs grid points");
+    constexpr int GP = G / 2;
+    constexpr int TW = 32 * TX;
+    constexpr int NS = SpanSums<COST>::value;
+    constexpr float kS = SpanScale<COST>::value;
+    constexpr bool kFix = COST != CGS_COST_SAD_AVG;  // the cost needs sum f^2
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int fw = p.fix.w, fh = p.fix.h;
+    const int TH = p.tile_h;
+    const int tiles_x = p.tiles_x, ntiles = p.tiles_x * p.tiles_y;
+    const float mov_wf = p.mov_wf, mov_hf = p.mov_hf;
+
+    // ---- the warp's points
+    SpanSlot *my_slots = ss.slots + warp * G;
+    span_points<COST, G, true>(p, (task * NW + warp) * G, my_slots);
+    __syncwarp();
+    // w = ((A x + By) + P) + nQ, -X = ((nC1 x + nC2 y) + nR) + S, -Y alike
+    float2 A2[GP], P2[GP], nQ2[GP], nC12[GP], nR2[GP], S2[GP], nD12[GP], nT2[GP], U2[GP];
+    bool nospan = false;  // some point of the warp has no spans
+#pragma unroll
+    for (int h = 0; h < GP; h++) {
+        const SpanSlot &a = my_slots[2 * h], &b = my_slots[2 * h + 1];
+        A2[h] = make_float2(a.A, b.A);
+        P2[h] = make_float2(a.P, b.P);
+        nQ2[h] = make_float2(-a.Q, -b.Q);
+        nC12[h] = make_float2(-a.C1, -b.C1);
+        nR2[h] = make_float2(-a.R, -b.R);
+        S2[h] = make_float2(a.S, b.S);
+        nD12[h] = make_float2(-a.D1, -b.D1);
+        nT2[h] = make_float2(-a.T, -b.T);
+        U2[h] = make_float2(a.U, b.U);
+        nospan |= (a.valid && !a.ok) || (b.valid && !b.ok);
+    }
+    if (lane < GP) {
+        const SpanSlot &a = my_slots[2 * lane], &b = my_slots[2 * lane + 1];
+        PairRow pr{};
+        pr.B = make_float2(a.B, b.B);
+        pr.C2 = make_float2(-a.C2, -b.C2);
+        pr.D2 = make_float2(-a.D2, -b.D2);
+        ss.prow[warp * GP + lane] = pr;
+    }
+    double *my_dtot = ss.dtot + warp * G * 5;  // {sum f^2, the sweep's NS sums} per point, stride 5
+    int *my_cnt = ss.cnt + warp * G;
+    for (int i = lane; i < G * 5; i += 32) my_dtot[i] = 0.0;
+    if (lane < G) my_cnt[lane] = 0;
+    __syncthreads();  // every point's slot is written
+
+    span_windows<C, G, NW, TX>(p, ss);
+    __syncthreads();
+    if (threadIdx.x == 0)
+        for (int t = 0; t < kWinStages && t < ntiles; t++) expect_window<C, TX>(p, ss, t, (int)((wit + t) % kWinStages));
+    __syncthreads();
+    for (int t = 0; t < kWinStages && t < ntiles; t++)
+        issue_window<C, NW, TX>(p, ss, t, (int)((wit + t) % kWinStages));
+
+    // one sample of point g at (x, y) by the reference's sequence, into a (and f^2 into s2) if inside
+    auto exact_sample = [&](const SpanSlot &sl, int x, int y, double *a, double &s2) -> int {
+        const MapCoef kc{sl.A, sl.B, sl.P, sl.Q, sl.C1, sl.C2, sl.R, sl.S, sl.D1, sl.D2, sl.T, sl.U};
+        float ex, ey;
+        exact_map(kc, (float)x, (float)y, ex, ey);
+        if (!in_image(ey, ex, mov_wf, mov_hf)) return 0;
+#pragma unroll
+        for (int ch = 0; ch < C; ch++) {
+            const float m = bilinear_in(p.mov.data + ch * p.mov.plane, p.mov.pitch, ey, ex);
+            const float f = p.fix.data[ch * p.fix.plane + (int64_t)y * p.fix.pitch + x];
+            accumulate64<COST>(a, f * kS, m * kS);
+            if constexpr (kFix) s2 += (double)f * (double)f;
+        }
+        return 1;
+    };
+    // adds the lanes' FP64 sums of point g (lanes of one group of `width`) into its totals
+    auto add_totals = [&](int g, bool leader, int width, double *a, double s2, int n, bool moving) {
+        for (int o = 1; o < width; o <<= 1) {
+            if constexpr (kFix) s2 += __shfl_xor_sync(0xffffffffu, s2, o);
+            n += __shfl_xor_sync(0xffffffffu, n, o);
+        }
+        if (moving)
+            for (int o = 1; o < width; o <<= 1)
+#pragma unroll
+                for (int j = 0; j < NS; j++) a[j] += __shfl_xor_sync(0xffffffffu, a[j], o);
+        if (leader) {
+            double *d = my_dtot + g * 5;
+            if constexpr (kFix) d[0] += s2;
+            if (moving)
+#pragma unroll
+                for (int j = 0; j < NS; j++) d[1 + j] += a[j];
+            my_cnt[g] += n;
+        }
+    };
+    // every pixel of the band's rows for the points without spans, all lanes over the columns
+    auto no_span_rows = [&](int y0, int y1) {
+        for (int g = 0; g < G; g++) {
+            const SpanSlot &sl = my_slots[g];
+            if (!sl.valid || sl.ok) continue;
+            double a[NS] = {}, s2 = 0.0;
+            int n = 0;
+            for (int y = y0; y < y1; y++)
+                for (int x = lane; x < fw; x += 32) n += exact_sample(sl, x, y, a, s2);
+            add_totals(g, lane == 0, 32, a, s2, n, true);
+            __syncwarp();
+        }
+    };
+
+    // ---- sweep
+    float2 part[GP][NS];
+#pragma unroll
+    for (int h = 0; h < GP; h++)
+#pragma unroll
+        for (int j = 0; j < NS; j++) part[h][j] = make_float2(0.0f, 0.0f);
+    InnerSpan *my_spans = ss.spans + warp * G * TH;
+    RowRun *my_runs = ss.runs + warp * TH;
+    const float2 magic2 = make_float2(kMagic, kMagic), minus1 = make_float2(-1.0f, -1.0f);
+    const float2 one2 = make_float2(1.0f, 1.0f), s2c = make_float2(kS, kS);
+    // -0, not known to the compiler: a product is a multiply-add of -0 (the same bits), because the
+    // assembler contracts a packed multiplication into the packed addition that consumes it, rounding
+    // modifiers notwithstanding (seen on CUDA 12.9; scalar ones are left alone)
+    const float nzero = __uint_as_float(0x80000000u | ((uint32_t)p.dims >> 8));
+    const float2 nzero2 = make_float2(nzero, nzero);
+    const float2 nsc = make_float2(-kS, -kS), smagic2 = make_float2(kS * kMagic, kS * kMagic);
+    const uint64_t mqbase = reinterpret_cast<uint64_t>(p.mov_quad) - 16ull * (uint64_t)(uint32_t)kMagicBits;
+    const float qpitch = -(float)p.quad_pitch * (1.0f / kS);
+    const uint64_t qplane = 16ull * (uint64_t)p.quad_plane;
+
+    for (int t = 0; t < ntiles; t++, wit++) {
+        const int tx = t % tiles_x, ty = t / tiles_x;
+        const int x0 = tx * TW, y0 = ty * TH;
+        const int x1 = min(x0 + TW, fw) - 1;
+        if (tx == 0) {
+            // the band's rows: spans, the fixed sums of the inner ones, the band pixels
+            for (int k = 0; 32 * k < G * TH; k++) {
+                const int i = lane + 32 * k;
+                const bool act = i < G * TH;
+                const int g = act ? i / TH : 0, r = i - g * TH;
+                double a[NS] = {}, s2 = 0.0;
+                int n = 0;
+                bool found = false;
+                if (act) {
+                    const SpanSlot &sl = my_slots[g];
+                    const int y = y0 + r;
+                    InnerSpan is{0, 0};
+                    if (y < fh && sl.valid && sl.ok) {
+                        const RowSpans sp = row_spans(sl, (float)y, fw, mov_wf, mov_hf);
+                        const int xa = sp.xa, len = sp.len, pa = sp.pa, plen = sp.plen;
+                        is = InnerSpan{xa, len};
+                        if (len > 0) {
+                            if constexpr (kFix) {
+                                const double2 *pr = p.fix_prefix + (int64_t)y * (fw + 1);
+                                s2 = pr[xa + len].y - pr[xa].y;
+                            }
+                            n = len;
+                        }
+                        // band pixels: the outer span outside the inner one, [pa, e0) and [e1, pa + plen)
+                        const int e0 = len > 0 ? xa : pa + plen, e1 = len > 0 ? xa + len : pa + plen;
+                        int nb = 0;
+                        for (int x = pa; x < e0; x++) nb += exact_sample(sl, x, y, a, s2);
+                        for (int x = e1; x < pa + plen; x++) nb += exact_sample(sl, x, y, a, s2);
+                        n += nb;
+                        found = nb > 0;
+                    }
+                    my_spans[g * TH + r] = is;
+                }
+                add_totals(g, act && r == 0, TH, a, s2, n, __any_sync(0xffffffffu, found));
+            }
+            __syncwarp();
+            if (lane < TH) {  // the rows' common inner run and the hull of the inner spans
+                int ia = 0, ib = fw - 1, ua = 1 << 30, ub = -1;
+#pragma unroll
+                for (int g = 0; g < G; g++) {
+                    const InnerSpan is = my_spans[g * TH + lane];
+                    if (is.len > 0) {
+                        ia = max(ia, is.xa);
+                        ib = min(ib, is.xa + is.len - 1);
+                        ua = min(ua, is.xa);
+                        ub = max(ub, is.xa + is.len - 1);
+                    } else {
+                        ib = -1;
+                    }
+                }
+                my_runs[lane] = RowRun{ia, ib, ua, ub};
+            }
+            __syncwarp();
+            if (nospan) no_span_rows(y0, min(y0 + TH, fh));
+        }
+        const int st = (int)(wit % kWinStages);
+        if (!mbar_wait_bounded(&ss.bars[st], (wit / kWinStages) & 1u, kWaitLimitNs)) *ss.abort_flag = 1;
+        const BlockWin *twin = ss.wins + t * TX;
+        const float *sfix = reinterpret_cast<const float *>(ss.win + (size_t)st * ss.cap);  // C x TH x TW
+        const uint32_t wbase = smem_addr(ss.win + (size_t)st * ss.cap + C * TH * TW / 4);
+        const uint32_t szero = smem_addr(ss.win);
+
+        for (int r = 0; r < TH; r++) {
+            if (y0 + r >= fh) break;
+            const RowRun run = my_runs[r];
+            if (run.ua > x1 || run.ub < x0) continue;  // no point samples this row of the tile
+            const float yf = (float)(y0 + r);
+            const float2 yf2 = make_float2(yf, yf);
+            float2 byw[GP], byx[GP], byy[GP];
+#pragma unroll
+            for (int h = 0; h < GP; h++) {
+                const PairRow &pr = ss.prow[warp * GP + h];
+                byw[h] = __ffma2_rn(pr.B, yf2, nzero2);
+                byx[h] = __ffma2_rn(pr.C2, yf2, nzero2);
+                byy[h] = __ffma2_rn(pr.D2, yf2, nzero2);
+            }
+            const float *frow = sfix + r * TW;
+            // one block of 32 columns; EDGE: some column may lie outside a point's inner span;
+            // SMEM: the block's window is in the stage
+            auto column = [&](int c, auto edge_tag, auto smem_tag) {
+                constexpr bool EDGE = decltype(edge_tag)::value;
+                constexpr bool SMEM = decltype(smem_tag)::value;
+                uint32_t sbase = 0u, wplane = 0u;
+                float pitch = qpitch;
+                if constexpr (SMEM) {
+                    const uint2 rp = *reinterpret_cast<const uint2 *>(&twin[c].rel);
+                    sbase = wbase + rp.x;
+                    pitch = __uint_as_float(rp.y) * (1.0f / kS);
+                    if constexpr (C > 1) wplane = 16u * (uint32_t)(twin[c].pitch * twin[c].h);
+                }
+                const float2 pitch2 = make_float2(pitch, pitch);
+                const int x = x0 + 32 * c + lane;
+                float f[C];
+#pragma unroll
+                for (int ch = 0; ch < C; ch++) f[ch] = frow[ch * TH * TW + 32 * c + lane] * kS;
+                const float xf = (float)x;
+                const float2 xf2 = make_float2(xf, xf);
+#pragma unroll
+                for (int h = 0; h < GP; h++) {
+                    const float2 w = __fadd2_rn(__fadd2_rn(__fadd2_rn(__ffma2_rn(A2[h], xf2, nzero2), byw[h]), P2[h]), nQ2[h]);
+                    const float2 nX = __fadd2_rn(__fadd2_rn(__fadd2_rn(__ffma2_rn(nC12[h], xf2, nzero2), byx[h]), nR2[h]), S2[h]);
+                    const float2 nY = __fadd2_rn(__fadd2_rn(__fadd2_rn(__ffma2_rn(nD12[h], xf2, nzero2), byy[h]), nT2[h]), U2[h]);
+                    float2 ex, ey;
+                    exact_quot2(w, nX, nY, ex, ey);
+                    // floor (round-down add of 1.5 * 2^23 leaves it in the mantissa), fractions a and 1 - a
+                    // (exact, and rounded as the reference's 1 - a), the y weights scaled by kS
+                    const float2 tx2 = __fadd2_rd(ex, magic2), ty2 = __fadd2_rd(ey, magic2);
+                    const float2 nfx2 = __ffma2_rn(tx2, minus1, magic2), nfy2 = __ffma2_rn(ty2, nsc, smagic2);
+                    const float2 ax = __fadd2_rn(ex, nfx2), ay = __ffma2_rn(ey, s2c, nfy2);
+                    const float2 ox = __ffma2_rn(ax, minus1, one2), oy = __ffma2_rn(ay, minus1, s2c);
+                    const float2 qi = __ffma2_rn(nfy2, pitch2, tx2);
+                    bool in0 = true, in1 = true;
+                    if constexpr (EDGE) {
+                        const InnerSpan a = my_spans[2 * h * TH + r], b = my_spans[(2 * h + 1) * TH + r];
+                        in0 = (unsigned)(x - a.xa) < (unsigned)a.len;
+                        in1 = (unsigned)(x - b.xa) < (unsigned)b.len;
+                    }
+                    uint32_t q0b = __float_as_uint(qi.x), q1b = __float_as_uint(qi.y);
+                    if constexpr (EDGE) {
+                        q0b = in0 ? q0b : (uint32_t)kMagicBits;
+                        q1b = in1 ? q1b : (uint32_t)kMagicBits;
+                    }
+                    uint32_t a0 = 0u, a1 = 0u;
+                    if constexpr (SMEM) {
+                        a0 = sbase + (q0b << 4);
+                        a1 = sbase + (q1b << 4);
+                        if constexpr (EDGE) {
+                            a0 = in0 ? a0 : szero;
+                            a1 = in1 ? a1 : szero;
+                        }
+                    }
+                    if constexpr (CHECK) {  // inside the block's window or the image, else recorded and skipped
+                        const BlockWin bw = twin[c];
+                        const int wx = SMEM ? bw.x0 : 0, wy = SMEM ? bw.y0 : 0;
+                        const unsigned ww = SMEM ? bw.w : p.mov.w, wh = SMEM ? bw.h : p.mov.h;
+                        const int ix0 = (int)(__float_as_uint(tx2.x) - (uint32_t)kMagicBits) - wx;
+                        const int iy0 = (int)(__float_as_uint(ty2.x) - (uint32_t)kMagicBits) - wy;
+                        const int ix1 = (int)(__float_as_uint(tx2.y) - (uint32_t)kMagicBits) - wx;
+                        const int iy1 = (int)(__float_as_uint(ty2.y) - (uint32_t)kMagicBits) - wy;
+                        const bool b0 = in0 && ((unsigned)ix0 >= ww || (unsigned)iy0 >= wh);
+                        const bool b1 = in1 && ((unsigned)ix1 >= ww || (unsigned)iy1 >= wh);
+                        if (b0 | b1) *ss.bounds_flag = 1;
+                        a0 = b0 ? szero : a0;
+                        a1 = b1 ? szero : a1;
+                        q0b = b0 ? (uint32_t)kMagicBits : q0b;
+                        q1b = b1 ? (uint32_t)kMagicBits : q1b;
+                    }
+#pragma unroll
+                    for (int ch = 0; ch < C; ch++) {
+                        float4 q0, q1;
+                        if constexpr (SMEM) {
+                            // a masked or skipped sample reads the stage's start, whatever the plane
+                            const uint32_t b0 = (EDGE || CHECK) && C > 1 ? (a0 == szero ? szero : a0 + ch * wplane)
+                                                                         : a0 + ch * wplane;
+                            const uint32_t b1 = (EDGE || CHECK) && C > 1 ? (a1 == szero ? szero : a1 + ch * wplane)
+                                                                         : a1 + ch * wplane;
+                            asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                                         : "=f"(q0.x), "=f"(q0.y), "=f"(q0.z), "=f"(q0.w) : "r"(b0));
+                            asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                                         : "=f"(q1.x), "=f"(q1.y), "=f"(q1.z), "=f"(q1.w) : "r"(b1));
+                        } else {
+                            q0 = __ldg(reinterpret_cast<const float4 *>(mqbase + ch * qplane + 16ull * q0b));
+                            q1 = __ldg(reinterpret_cast<const float4 *>(mqbase + ch * qplane + 16ull * q1b));
+                        }
+                        // valueAt_bilinear's order: (1 - ay)((1 - ax) v00 + ax v01) + ay((1 - ax) v10 + ax v11)
+                        const float t0 = xa(xm(ox.x, q0.x), xm(ax.x, q0.y)), b0v = xa(xm(ox.x, q0.z), xm(ax.x, q0.w));
+                        const float t1 = xa(xm(ox.y, q1.x), xm(ax.y, q1.y)), b1v = xa(xm(ox.y, q1.z), xm(ax.y, q1.w));
+                        float2 m = make_float2(xa(xm(oy.x, t0), xm(ay.x, b0v)), xa(xm(oy.y, t1), xm(ay.y, b1v)));
+                        float2 fm = make_float2(f[ch], f[ch]);
+                        if constexpr (EDGE) {  // by selection: a NaN outside the overlap stays out of the sums
+                            m = make_float2(in0 ? m.x : 0.0f, in1 ? m.y : 0.0f);
+                            fm = make_float2(in0 ? f[ch] : 0.0f, in1 ? f[ch] : 0.0f);
+                        }
+                        if constexpr (COST == CGS_COST_SAD_AVG) {
+                            part[h][0].x += fabsf(m.x - fm.x);
+                            part[h][0].y += fabsf(m.y - fm.y);
+                        } else if constexpr (COST == CGS_COST_SQD_REF) {
+                            const float2 d = __ffma2_rn(fm, minus1, m);
+                            part[h][0] = __ffma2_rn(d, d, part[h][0]);
+                            part[h][1] = __ffma2_rn(m, m, part[h][1]);
+                        } else {
+                            part[h][0] = __ffma2_rn(m, m, part[h][0]);
+                            part[h][1] = __ffma2_rn(fm, m, part[h][1]);
+                        }
+                    }
+                }
+            };
+            auto block = [&](int c, auto edge_tag) {
+                if (twin[c].w > 0) column(c, edge_tag, std::true_type{});
+                else column(c, edge_tag, std::false_type{});
+            };
+            // blocks with any inner span: [cu0, cu1]; those inside every point's, [cf0, cf1], unmasked
+            const int cu0 = max(0, (run.ua - x0) >> 5), cu1 = min(TX - 1, (run.ub - x0) >> 5);
+            int cf0 = cu1 + 1, cf1 = cu1;
+            if (run.ia <= run.ib) {
+                const int a = max(cu0, (run.ia - x0 + 31) >> 5), b = min(cu1, ((run.ib - x0 + 1) >> 5) - 1);
+                if (a <= b) {
+                    cf0 = a;
+                    cf1 = b;
+                }
+            }
+#pragma unroll 1
+            for (int c = cu0; c <= cu1; c++) {
+                if (c >= cf0 && c <= cf1) block(c, std::false_type{});
+                else block(c, std::true_type{});
+            }
+        }
+        // end of a band of tiles: the band's warp sums into the FP64 totals
+        if (tx == tiles_x - 1) {
+#pragma unroll
+            for (int h = 0; h < GP; h++)
+#pragma unroll
+                for (int j = 0; j < NS; j++) {
+                    const float s0 = warp_sum(part[h][j].x), s1 = warp_sum(part[h][j].y);
+                    if (lane == 0) {
+                        my_dtot[(2 * h) * 5 + 1 + j] += (double)s0;
+                        my_dtot[(2 * h + 1) * 5 + 1 + j] += (double)s1;
+                    }
+                    part[h][j] = make_float2(0.0f, 0.0f);
+                }
+        }
+        const bool more = t + kWinStages < ntiles;
+        if (threadIdx.x == 0 && more) expect_window<C, TX>(p, ss, t + kWinStages, st);
+        __syncthreads();  // every warp is done with this stage
+        if (*ss.abort_flag) {
+            if (threadIdx.x == 0) mbar_wait_bounded(&ss.bars[st], (wit / kWinStages) & 1u, kWaitLimitNs);
+            return false;
+        }
+        if (more) issue_window<C, NW, TX>(p, ss, t + kWinStages, st);
+    }
+
+    // ---- per grid point: the cost from the totals, dump, argmin key
+    __syncwarp();
+    unsigned long long kk = ~0ull;
+    if (lane < G) {
+        const SpanSlot &sl = my_slots[lane];
+        const int n = my_cnt[lane] * C;
+        const double *d = my_dtot + lane * 5;
+        constexpr double k2 = (256.0 / 255.0) * (256.0 / 255.0);
+        float a[3] = {0.0f, 0.0f, 0.0f};
+        if constexpr (COST == CGS_COST_SAD_AVG) {
+            a[0] = (float)d[1];
+        } else if constexpr (COST == CGS_COST_SQD_REF) {
+            a[0] = (float)(d[1] * k2);
+            a[1] = (float)(d[2] * k2);
+            a[2] = (float)(d[0] * (1.0 / 65025.0));
+        } else {
+            a[0] = (float)(d[0] * (1.0 / 65025.0));
+            a[1] = (float)(d[1] * k2);
+            a[2] = (float)(d[2] * k2);
+        }
+        const float cost = finalize<COST>(a, n, p);
+        if (sl.valid) {
+            if (p.costs) p.costs[sl.index] = cost;
+            kk = make_key(cost, sl.index);
+        }
+    }
+    kk = warp_min_u64(kk);
+    if (lane == 0) ss.wbest[warp] = kk;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        unsigned long long b = ~0ull;
+        for (int w = 0; w < NW; w++) b = ss.wbest[w] < b ? ss.wbest[w] : b;
+        if (CHECK && *ss.bounds_flag) atomicOr(p.status, kStatusSpanBounds);
+        retire_tasks(p, b, 1u, false);
+    }
+    return true;
+}
+
+// The single-pair kernel: persistent CTAs, tasks dealt round-robin.
+template <int COST, int C, int G, int NW, int TX, bool CHECK>
+__global__ void __launch_bounds__(NW * 32, 1) span_exact_kernel(const __grid_constant__ SearchParams p) {
+    extern __shared__ __align__(128) unsigned char smem[];
+    const SpanSmem ss = carve_span<G, NW>(smem, p.tile_h, TX, p.tiles_x * p.tiles_y, p.win_cap);
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < kWinStages; s++) mbar_init(&ss.bars[s], 1);
+        fence_mbar_init();
+        *ss.abort_flag = 0;
+        *ss.bounds_flag = 0;
+    }
+    __syncthreads();
+    const uint32_t my_tasks =
+        (p.num_tasks > blockIdx.x) ? (p.num_tasks - blockIdx.x + gridDim.x - 1) / gridDim.x : 0u;
+    uint32_t wit = 0;
+    for (uint32_t k = 0; k < my_tasks; k++) {
+        if (!run_span_exact_task<COST, C, G, NW, TX, CHECK>(p, blockIdx.x + k * gridDim.x, ss, wit)) {
+            if (threadIdx.x == 0) retire_tasks(p, ~0ull, my_tasks - k, true);
+            return;
+        }
+    }
+}
+
+}  // namespace cgs

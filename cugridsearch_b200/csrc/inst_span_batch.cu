@@ -1,0 +1,12 @@
+// The multi-pair span kernel of batches: 16 warps of 4 points, tiles of 256 columns.
+#include "cgs_internal.h"
+#include "cgs_span_batch.cuh"
+
+namespace cgs {
+
+const void *kernel_span_batch(int G, int NW, int TX, bool check) {
+    if (G == 4 && NW == 16 && TX == 8 && !check) return (const void *)span_batch_kernel<4, 16, 8, false>;
+    return nullptr;
+}
+
+}  // namespace cgs

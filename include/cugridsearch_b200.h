@@ -103,11 +103,14 @@ typedef struct cgs_options {
  * only speed and scratch size differ. */
 #define CGS_FLAG_QUAD_TAPS 8
 #define CGS_FLAG_TEXTURE_TAPS 16
-/* Zero-mean NCC and MI on the fast path run span kernels by default (single channel; MI with
- * at most 32 bins and neither taps flag): in/out decisions per image row; ZNCC reads its taps
- * from per-block moving-image windows in shared memory, MI keeps its histograms there.  This
- * flag selects the per-sample decision kernel instead.  Both make the same decisions and form
- * the same bins: ZNCC costs agree within FP32 summation order, MI costs are bit-identical. */
+/* Span kernels (the default where they apply): in/out decisions per image row instead of per
+ * sample.  They run zero-mean NCC (single channel) and MI (single channel, at most 32 bins) on fast
+ * samples, and SAD_AVG, SQD_REF and NCC_REF (1 or 3 channels) on exact ones, unless a taps flag is
+ * set (ZNCC: the texture flag).  ZNCC and the exact costs read their taps from per-block
+ * moving-image windows in shared memory, MI keeps its histograms there.  They ignore
+ * warps_per_block, and points_per_warp other than ZNCC's 2.  This flag selects the per-sample
+ * decision kernel instead.  Both make the same decisions and form the same samples (exact) and bins
+ * (MI): costs agree within FP32 summation order, MI costs are bit-identical. */
 #define CGS_FLAG_PER_SAMPLE_DECISIONS 32
 /* Skip the FP64 verification pass (see cgs_argmin).  Without the pass the verification fields
  * read verified = 0, index_fp64 = -1, cost_fp64 = NaN. */
@@ -276,8 +279,8 @@ cgs_status cgs_quantize_image(cgs_image *img, float mod, cgs_stream_t stream);
 /* ---------------------------------------------------------------- batched search
  *
  * Many image pairs of uneven sizes, each with its own grid and cost, evaluated by one recorded
- * launch sequence (a persistent kernel over the per-sample pairs, one multi-pair span kernel over
- * the ZNCC pairs).  The reference searches one pair per call and its callers loop
+ * launch sequence (one multi-pair span kernel over the ZNCC, SAD, SQD and NCC pairs, a persistent
+ * kernel over the per-sample pairs).  The reference searches one pair per call and its callers loop
  * over pairs and refinement levels (src/gpu/cudaGridSearch_main_mi.cu:312-363, one
  * search_by_value + find_extrema per pass); a batch replaces that loop.  Each pair's costs and
  * argmin equal those of cgs_search on the same pair: bit for bit with block_split = 0, within
@@ -320,9 +323,10 @@ typedef struct cgs_batch cgs_batch; /* opaque handle */
 
 /* Creates a batch: validates every pair, lays out device scratch for all of them (one block
  * from the library's pool, held until cgs_batch_destroy), orders the pairs by estimated work
- * (cheapest first) and records one CUDA graph: clear scratch, stage every pair; the ZNCC pairs
- * that cgs_search runs on its span kernel (fast sampling, no per-sample flag) in one multi-pair
- * span launch, with cgs_search's costs and argmins bit for bit; the other pairs in the
+ * (cheapest first) and records one CUDA graph: clear scratch, stage every pair; the pairs that
+ * cgs_search runs on a span kernel with windows (ZNCC on fast samples, SAD_AVG, SQD_REF and NCC_REF
+ * on exact ones, no per-sample or taps flag) in one multi-pair span launch, with cgs_search's costs
+ * and argmins bit for bit; the other pairs in the
  * persistent batch kernel, for the plan (NULL: 4 points per warp, 16 warps, warp-private
  * histograms; 2 points per warp, then block-shared histograms, where those do not fit); then,
  * pair after pair, cgs_search's own launches for MI pairs that it runs on its MI span kernel and

@@ -1,0 +1,89 @@
+"""The span kernel of the exact-sampling costs (cgs_span_exact.cuh: SAD_AVG, SQD_REF and NCC_REF with
+one or three channels) at the edges of its tiles, blocks and bands, against the FP64 oracle:
+
+* fixed images one pixel around a 32-column block, a 256-column (three channels: 64-column) tile and a
+  16-row band, moving images of another size;
+* the self-checking build (CGS_SPAN_CHECK=1, one channel) finds every sample's quad in its window, and
+  windows that do not fit the stage (CGS_SPAN_CAP) give the same bits from global memory;
+* grids whose perspective lets w change sign (points without spans);
+* a 1 x 1 fixed image, whose SAD is one sample: bit for bit the oracle's, so that coordinates, quotients
+  and interpolation round as the reference's.
+"""
+import numpy as np
+import pytest
+
+import oracle as O
+from conftest import close_costs
+from cugridsearch_b200 import synthetic as S
+from test_span_gpu import _env, _run
+
+pytestmark = pytest.mark.gpu
+COSTS = ["SAD_AVG", "SQD_REF", "NCC_REF"]
+
+
+def _pair(seed, cost, h, w, mh, mw, channels, count=2, u8=False):
+    size = max(h, w, mh, mw, 16)
+    p = S.small_pair(seed, size=size, count=count, cost=cost, channels=channels, u8=u8)
+    p.fixed = np.ascontiguousarray(p.fixed[:h, :w])
+    p.moving = np.ascontiguousarray(p.moving[:mh, :mw])
+    span = 0.1 * min(h, w, mh, mw)
+    p.lo[4:6], p.hi[4:6] = -span, span
+    return p
+
+
+def _oracle_agrees(pair, cost, c):
+    g = O.make_grid(*pair.grid_args())
+    c32, c64 = O.search(cost, g, O.Image(pair.moving), O.Image(pair.fixed))
+    bad = close_costs(c, c32, c64, cost)
+    assert not bad.any(), (int(bad.sum()), c[bad][:4], c32[bad][:4], c64[bad][:4])
+
+
+@pytest.mark.parametrize("cost", COSTS)
+@pytest.mark.parametrize("h,w,mh,mw,channels", [(15, 31, 20, 33, 1), (16, 32, 16, 32, 1), (17, 33, 14, 40, 1),
+                                                (33, 257, 37, 250, 1), (1, 256, 3, 256, 1), (48, 5, 48, 5, 1),
+                                                (17, 65, 19, 61, 3), (16, 64, 16, 64, 3), (31, 129, 33, 140, 3)])
+def test_edges_match_oracle(cuda, lib, cost, h, w, mh, mw, channels):
+    pair = _pair(500 + h + w, cost, h, w, mh, mw, channels, u8=channels == 3)
+    with _env(**({"CGS_SPAN_CHECK": 1} if channels == 1 else {})):
+        _, c = _run(cuda, pair, cost)
+    _oracle_agrees(pair, cost, c)
+
+
+@pytest.mark.parametrize("cost", COSTS)
+def test_plain_checked_and_global_taps_agree(cuda, lib, cost):
+    pair = _pair(7, cost, 70, 130, 75, 120, 1, count=3)
+    _, c0 = _run(cuda, pair, cost)
+    with _env(CGS_SPAN_CHECK=1):
+        _, c1 = _run(cuda, pair, cost)
+    with _env(CGS_SPAN_CAP=1024):
+        _, c2 = _run(cuda, pair, cost)
+    np.testing.assert_array_equal(c1.view(np.uint32), c0.view(np.uint32))
+    np.testing.assert_array_equal(c2.view(np.uint32), c0.view(np.uint32))
+    pair.fixed, pair.moving = np.repeat(pair.fixed, 3, 2), np.repeat(pair.moving, 3, 2)
+    _, c3 = _run(cuda, pair, cost)
+    with _env(CGS_SPAN_CAP=1024):
+        _, c4 = _run(cuda, pair, cost)
+    np.testing.assert_array_equal(c4.view(np.uint32), c3.view(np.uint32))
+    _oracle_agrees(pair, cost, c3)
+
+
+@pytest.mark.parametrize("channels", [1, 3])
+@pytest.mark.parametrize("cost", COSTS)
+def test_points_without_spans(cuda, lib, cost, channels):
+    pair = _pair(11, cost, 24, 40, 24, 40, channels, count=3)
+    pair.lo[6:8], pair.hi[6:8] = -0.06, 0.06  # w changes sign inside the image at the outer values
+    _, c = _run(cuda, pair, cost)
+    _oracle_agrees(pair, cost, c)
+
+
+def test_one_sample_is_the_references_bit_for_bit(cuda, lib):
+    pair = _pair(13, "SAD_AVG", 1, 1, 64, 64, 1, count=4)
+    pair.fixed[:] = 0.0
+    pair.lo[4:6], pair.hi[4:6] = -60.3, 3.7
+    pair.moving = np.random.default_rng(3).uniform(0, 255, pair.moving.shape).astype(np.float32)
+    _, c = _run(cuda, pair, "SAD_AVG")
+    g = O.make_grid(*pair.grid_args())
+    c32, _ = O.search("SAD_AVG", g, O.Image(pair.moving), O.Image(pair.fixed))
+    assert np.isfinite(c32).sum() > 1000
+    np.testing.assert_array_equal(c[np.isfinite(c32)].view(np.uint32), c32[np.isfinite(c32)].view(np.uint32))
+    np.testing.assert_array_equal(np.isfinite(c), np.isfinite(c32))
