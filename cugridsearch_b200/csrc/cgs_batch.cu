@@ -360,7 +360,7 @@ cgs_status cgs_batch_create(const cgs_pair *pairs, int32_t n, const cgs_batch_pl
         // kernel below that (a refinement level's local grids, balanced there many at once)
         uint32_t ppt = 0;
         SpanPlan zp;
-        if (span_plan(q.moving, q.fixed, q.options, &zp) &&
+        if (span_plan(q.moving, q.fixed, q.options, pd.mi_bins, &zp) &&
             kernel_span_batch(zp.G, zp.NW, zp.TX, zp.check) != nullptr &&
             (!have_group || (zp.G == gplan.G && zp.NW == gplan.NW && zp.TX == gplan.TX && zp.TH == gplan.TH &&
                              zp.pitch_mod == gplan.pitch_mod))) {
@@ -438,10 +438,10 @@ cgs_status cgs_batch_create(const cgs_pair *pairs, int32_t n, const cgs_batch_pl
     int gcap = 0;
     if (gn > 0) {
         const size_t budget = 227 * 1024;
-        const size_t fixed = span_kernel_smem(gplan.G, gplan.NW, gplan.TH, gplan.TX, gtiles, 0);
+        const size_t fixed = span_kernel_smem(gplan.G, gplan.NW, gplan.TH, gplan.TX, gtiles, 0, true, 0);
         gcap = fixed + (size_t)kMinSpanCap * 16 * kWinStages > budget ? 0 : (int)((budget - fixed) / (16 * kWinStages));
         gcap = std::max(gcap, kMinSpanCap + gplan.TH * 32 * gplan.TX / 4);
-        const size_t gsm = span_kernel_smem(gplan.G, gplan.NW, gplan.TH, gplan.TX, gtiles, gcap);
+        const size_t gsm = span_kernel_smem(gplan.G, gplan.NW, gplan.TH, gplan.TX, gtiles, gcap, true, 0);
         if (fixed + (size_t)kMinSpanCap * 16 * kWinStages > budget || gsm > budget) {
             for (int32_t i = 0; i < n; i++) pend[i].route = pend[i].route == 1 ? 0 : pend[i].route;
             gn = 0;  // cannot happen for the sizes span_plan admits; the pairs go to the persistent kernel
@@ -568,7 +568,7 @@ cgs_status cgs_batch_create(const cgs_pair *pairs, int32_t n, const cgs_batch_pl
             // as cgs_search sets up its span kernels: quads in the cost's span form (ZNCC: with the
             // moving shift folded in), the fixed rows' prefix sums, tiles and the (common) window stage
             const int cost = q.options.cost;
-            preps[j].quad_form = span_quad_form(cost);
+            preps[j].quad_form = span_quad_form(cost, 1);
             double2 *prefix =
                 span_uses_prefix(cost) ? reinterpret_cast<double2 *>(b->mem + pd.prefix_off) : nullptr;
             p.fix_prefix = prefix;
@@ -615,7 +615,7 @@ cgs_status cgs_batch_create(const cgs_pair *pairs, int32_t n, const cgs_batch_pl
         ga.tiles = gtiles;
         ga.cap = gcap;
         b->g_kfn = kernel_span_batch(gplan.G, gplan.NW, gplan.TX, gplan.check);
-        b->g_smem = span_kernel_smem(gplan.G, gplan.NW, gplan.TH, gplan.TX, gtiles, gcap);
+        b->g_smem = span_kernel_smem(gplan.G, gplan.NW, gplan.TH, gplan.TX, gtiles, gcap, true, 0);
         e = cudaMemcpy(b->mem + gpar_off, gpar.data(), sizeof(SearchParams) * gn, cudaMemcpyHostToDevice);
         if (e == cudaSuccess) e = cudaMemcpy(b->mem + gtb_off, gtb.data(), 4 * gtb.size(), cudaMemcpyHostToDevice);
         if (e == cudaSuccess) e = cudaMemcpy(b->mem + gslot_off, gslot.data(), 4 * gn, cudaMemcpyHostToDevice);

@@ -46,9 +46,13 @@ struct PrepParams {
     int32_t rowsf;
     float4 *quad_dst;    // moving-image tap quads (W x H per channel), or null
     int64_t qplane;
-    int32_t quad_form;   // 0: {P00, P10, P01 - P00, P11 - P10}; 1 (ZNCC and MI span kernels): {P00, P01 - P00,
+    int32_t quad_form;   // 0: {P00, P10, P01 - P00, P11 - P10}; 1 (ZNCC and one-channel MI span kernels): {P00, P01 - P00,
                          // P10 - P00, (P11 - P10) - (P01 - P00)}; 2 (exact span kernel): {P00, P01, P10, P11};
                          // P(dy, dx) the tap at (y + dy, x + dx)
+    float quad_scale;    // form 1: a power of two on the quads (one-channel MI: bins / 256), or 0 (none)
+    int32_t *bin_dst;    // the fixed image's bins times 4 (bins + 1) (the histogram row's byte offset), laid
+                         // out as the fixed planes, or null
+    int32_t bins;
 };
 
 // Staged layout of a moving/fixed image pair inside one scratch block.
@@ -97,13 +101,13 @@ const void *kernel_scan(int cost, int C);
 size_t scan_smem_bytes(int cost);
 
 // Span kernel of zero-mean NCC (cgs_span.cuh): G points per warp, NW warps, tiles of 32 TX
-// columns; `check` selects the self-checking build.  The span kernel of the exact-sampling costs
-// (cgs_span_exact.cuh): 4 points per warp, 16 warps, C channels.  Their shared-memory size, the
-// largest quad plane they take, and the launch of their staging step after prep_kernel (the fixed
+// columns; `check` selects the self-checking build.  The span kernel of the exact-sampling costs and MI
+// (cgs_span_exact.cuh): 16 warps, C channels.  Their shared-memory size (`exact`: the latter's, with
+// histograms of mi_bins bins for MI, else 0), the largest quad plane they take, and the launch of their staging step after prep_kernel (the fixed
 // rows' FP64 prefix sums where `prefix` is given, the moving shift folded into `nquads` quads).
 const void *kernel_span_zncc(int G, int NW, int TX, bool check);
-const void *kernel_span_exact(int cost, int C, int TX, bool check);
-size_t span_kernel_smem(int G, int NW, int TH, int TX, int tiles, int cap);
+const void *kernel_span_exact(int cost, int C, int G, int TX, bool check);
+size_t span_kernel_smem(int G, int NW, int TH, int TX, int tiles, int cap, bool exact, int mi_bins);
 int64_t span_max_quads();
 SpanPrepArgs span_prep_args(const float *fix, int fpitch, int64_t fplane, int channels, int fw, int fh, double2 *prefix,
                             float4 *quads, int64_t nquads, const float *shifts, int *blocks);
@@ -114,23 +118,28 @@ constexpr int kMinSpanCap = 1024;                   // smallest useful window st
 struct SpanPlan {
     int G = 4, NW = 16, TX = 2, TH = 16;
     int tiles_x = 0, tiles_y = 0, cap = 0, pitch_mod = 0;
+    bool exact = false;  // cgs_span_exact.cuh
+    int mi_bins = 0;     // MI: histogram bins
     bool check = false;
     size_t smem = 0;
     const void *kfn = nullptr;
 };
-// Whether cgs_search runs a request on a tiled span kernel (zero-mean NCC on fast samples, or a cost
-// of kernel_span_exact on exact ones), with its plan.
-bool span_plan(const cgs_image &mov, const cgs_image &fix, const cgs_options &o, SpanPlan *sp);
+// Whether cgs_search runs a request on a span kernel with windows (zero-mean NCC and three-channel MI in
+// their default sampling mode, SAD_AVG, SQD_REF and NCC_REF on exact samples), with its plan.
+bool span_plan(const cgs_image &mov, const cgs_image &fix, const cgs_options &o, int mi_bins, SpanPlan *sp);
 // The staging form of the quads (PrepParams::quad_form) and whether the cost reads the fixed rows'
 // prefix sums.
-inline int span_quad_form(int cost) { return cost == CGS_COST_ZNCC || cost == CGS_COST_MI ? 1 : 2; }
-inline bool span_uses_prefix(int cost) { return cost != CGS_COST_SAD_AVG; }
+inline int span_quad_form(int cost, int channels) {
+    return cost == CGS_COST_ZNCC || (cost == CGS_COST_MI && channels == 1) ? 1 : 2;
+}
+inline bool span_uses_prefix(int cost) { return cost != CGS_COST_SAD_AVG && cost != CGS_COST_MI; }
 // The multi-pair span kernel of batches for a plan (null where not instantiated), and the
 // staging step of many pairs in one launch.
 const void *kernel_span_batch(int G, int NW, int TX, bool check);
 cudaError_t launch_span_prep_batch(const SpanPrepArgs *args, int n, int blocks, cudaStream_t stream);
-// Span kernel of MI (cgs_span_mi.cuh): 2 points per warp, NW warps, histograms of B <= 32 bins;
-// its shared-memory size and its staging step (the fixed bins times B + 1, int32; the quads'
+
+// Span kernel of single-channel MI (cgs_span_mi.cuh): 2 points per warp, NW warps, histograms of B <= 32
+// bins; its shared-memory size and its staging step (the fixed bins times B + 1, int32; the quads'
 // largest slope bound into a header word).
 const void *kernel_span_mi(int NW, bool check);
 size_t span_mi_kernel_smem(int NW, int TH, int B);

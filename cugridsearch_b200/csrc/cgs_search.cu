@@ -225,6 +225,10 @@ __device__ __forceinline__ void prep_body(const PrepParams &q, int64_t tid, int6
         else if (q.fix_alias && y + 1 < q.fh && x == q.fw)
             v = load_pix(q.fix_src, q.fix_pix, ((y + 1) * q.fw) * q.c + c);
         q.fix_dst[i] = v;
+        if (q.bin_dst) {
+            const int b = (int)floorf(v * ((float)q.bins * (1.0f / 256.0f)));
+            q.bin_dst[i] = min(max(b, 0), q.bins - 1) * (4 * (q.bins + 1));
+        }
     }
     if (q.quad_dst) {
         // tap quads of the staged moving plane, the left column and the FP32 differences to the
@@ -247,6 +251,10 @@ __device__ __forceinline__ void prep_body(const PrepParams &q, int64_t tid, int6
             q.quad_dst[i] = q.quad_form == 2   ? make_float4(v00, v01, v10, v11)
                             : q.quad_form == 1 ? make_float4(v00, d0, v10 - v00, d1 - d0)
                                                : make_float4(v00, v10, d0, d1);
+            if (q.quad_scale != 0.0f) {
+                float4 &o = q.quad_dst[i];
+                o = make_float4(o.x * q.quad_scale, o.y * q.quad_scale, o.z * q.quad_scale, o.w * q.quad_scale);
+            }
         }
     }
     if (q.row_table && tid == 0) {
@@ -686,53 +694,62 @@ static Plan choose_plan(int cost, const cgs_options &o, int mi_bins) {
     return pl;
 }
 
-// Launch plan of the tiled span kernels: points per warp (4; ZNCC: the request's 2), 16 warps, tiles
-// of 32 TX columns by TH rows, the window stage filling the shared memory that is left (at most
-// CGS_SPAN_CAP 16-byte units when that is set; it holds the tile's fixed rows and its blocks' windows,
-// of every channel) and window rows padded to CGS_SPAN_PITCH (mod 8) quads.  One channel: tiles of
-// 256 x 16 unless the tuning variables CGS_SPAN_TX = 2 | 4 | 8 (ZNCC) and CGS_SPAN_TH = 8 | 16 | 32 say
-// otherwise; three channels (exact samples): 64 x 16, whose 2 x 3 windows of about 1.1 K quads fit the
-// stage where eight would not.  CGS_SPAN_CHECK=1 selects the self-checking build (every sample's quad
-// address is checked against its window; a miss sets status bit 0x100 and skips the sample).
+// Launch plan of the span kernels: points per warp (4; ZNCC: the request's 2; MI: 2, whose histograms
+// of 32 bins take 139 KB of shared memory), 16 warps, tiles of 32 TX columns by TH rows, the window
+// stage filling the shared memory that is left (at most CGS_SPAN_CAP 16-byte units when that is set; it
+// holds the tile's fixed rows and its blocks' windows, of every channel) and window rows padded to
+// CGS_SPAN_PITCH (mod 8) quads.  Tiles are as wide as the windows fit (a 32 x 16 block's takes about
+// 1.1 K quads per channel): 256 columns, MI 128 (4.8 K quads of stage), three channels 64; TH = 16.  The
+// tuning variables CGS_SPAN_TX = 2 | 4 | 8 (ZNCC) and CGS_SPAN_TH = 8 | 16 | 32 say otherwise.
+// CGS_SPAN_CHECK=1 selects the self-checking build (every sample's quad address is checked against its
+// window; a miss sets status bit 0x100 and skips the sample).
 //
-// The kernel runs zero-mean NCC on fast samples and SAD_AVG, SQD_REF and NCC_REF on exact ones, unless
-// the request asks for per-sample decisions or names a source of taps (a per-sample kernel's).
-// False where it does not apply: other channel counts, images of 32768 or more pixels a side, moving
-// images with (W + 8) H of 2^22 or more, or too many tiles for shared memory.
+// The kernels run zero-mean NCC and MI in their default sampling mode, SAD_AVG, SQD_REF and NCC_REF on
+// exact samples, unless the request asks for per-sample decisions or names a source of taps (a
+// per-sample kernel's; ZNCC reads quads either way).  False where they do not apply: other channel
+// counts, MI with more than 32 bins, images of 32768 or more pixels a side, moving images with
+// (W + 8) H of 2^22 or more, or too many tiles for shared memory.
 static int env_int(const char *name, int dflt) {
     const char *v = std::getenv(name);
     return (v && *v) ? std::atoi(v) : dflt;
 }
 
-bool span_plan(const cgs_image &mov, const cgs_image &fix, const cgs_options &o, SpanPlan *sp) {
+bool span_plan(const cgs_image &mov, const cgs_image &fix, const cgs_options &o, int mi_bins, SpanPlan *sp) {
     const int C = fix.channels;
-    const bool zncc = o.cost == CGS_COST_ZNCC && !exact_samples(o.cost, o.flags) && !(o.flags & CGS_FLAG_TEXTURE_TAPS);
+    const bool exact_mode = exact_samples(o.cost, o.flags);
+    const bool taps = (o.flags & (CGS_FLAG_TEXTURE_TAPS | CGS_FLAG_QUAD_TAPS)) != 0;
+    const bool zncc = o.cost == CGS_COST_ZNCC && !exact_mode && !(o.flags & CGS_FLAG_TEXTURE_TAPS);
+    const bool mi = o.cost == CGS_COST_MI && !exact_mode && !taps && mi_bins <= 32;
     const bool exact = (o.cost == CGS_COST_SAD_AVG || o.cost == CGS_COST_SQD_REF || o.cost == CGS_COST_NCC_REF) &&
-                       exact_samples(o.cost, o.flags) && !(o.flags & (CGS_FLAG_TEXTURE_TAPS | CGS_FLAG_QUAD_TAPS));
-    if (!(zncc || exact) || (o.flags & CGS_FLAG_PER_SAMPLE_DECISIONS)) return false;
-    if (!(C == 1 || (exact && C == 3))) return false;
+                       exact_mode && !taps;
+    if (!(zncc || mi || exact) || (o.flags & CGS_FLAG_PER_SAMPLE_DECISIONS)) return false;
+    if (!(C == 3 ? !zncc : C == 1 && !mi)) return false;
     if (mov.width >= 32768 || mov.height >= 32768 || fix.width >= 32768 || fix.height >= 32768 ||
         (int64_t)(mov.width + 8) * mov.height >= span_max_quads())
         return false;
-    sp->G = zncc && o.points_per_warp == 2 ? 2 : 4;
+    sp->exact = !zncc;
+    sp->mi_bins = mi ? mi_bins : 0;
+    sp->G = mi || (zncc && o.points_per_warp == 2) ? 2 : 4;
     sp->NW = 16;
-    sp->TX = C == 3 ? 2 : zncc ? env_int("CGS_SPAN_TX", 8) : 8;
+    sp->TX = zncc ? env_int("CGS_SPAN_TX", 8) : C == 3 ? 2 : mi ? 4 : 8;
     sp->TH = env_int("CGS_SPAN_TH", 16);
     if (!(sp->TX == 2 || sp->TX == 4 || sp->TX == 8) || !(sp->TH == 8 || sp->TH == 16 || sp->TH == 32)) return false;
     sp->check = env_int("CGS_SPAN_CHECK", 0) != 0;
-    sp->kfn = zncc ? kernel_span_zncc(sp->G, sp->NW, sp->TX, sp->check) : kernel_span_exact(o.cost, C, sp->TX, sp->check);
+    sp->kfn = zncc ? kernel_span_zncc(sp->G, sp->NW, sp->TX, sp->check)
+                   : kernel_span_exact(o.cost, C, sp->G, sp->TX, sp->check);
     if (!sp->kfn) return false;
     sp->tiles_x = (fix.width + 32 * sp->TX - 1) / (32 * sp->TX);
     sp->tiles_y = (fix.height + sp->TH - 1) / sp->TH;
     const int tiles = sp->tiles_x * sp->tiles_y;
-    const size_t budget = 227 * 1024, fixed = span_kernel_smem(sp->G, sp->NW, sp->TH, sp->TX, tiles, 0);
+    const size_t budget = 227 * 1024;
+    const size_t fixed = span_kernel_smem(sp->G, sp->NW, sp->TH, sp->TX, tiles, 0, sp->exact, sp->mi_bins);
     if (fixed + (size_t)kMinSpanCap * 16 * kWinStages > budget) return false;
     sp->cap = (int)((budget - fixed) / (16 * kWinStages));
     // CGS_SPAN_CAP (quads) lowers the stage size, e.g. to exercise the global-memory path
     sp->cap = std::max(kMinSpanCap, std::min(sp->cap, env_int("CGS_SPAN_CAP", sp->cap)));
     sp->cap = std::max(sp->cap, kMinSpanCap + C * sp->TH * 32 * sp->TX / 4);  // room for the fixed rows
     sp->pitch_mod = env_int("CGS_SPAN_PITCH", 0) & 7;
-    sp->smem = span_kernel_smem(sp->G, sp->NW, sp->TH, sp->TX, tiles, sp->cap);
+    sp->smem = span_kernel_smem(sp->G, sp->NW, sp->TH, sp->TX, tiles, sp->cap, sp->exact, sp->mi_bins);
     return sp->smem <= budget;
 }
 
@@ -980,18 +997,16 @@ static cgs_status search_core(const cgs_image *mov, const cgs_image *fix, const 
     // taps: pre-gathered quads where the fast sampling path runs (measured faster than texture
     // gathers there); texture gathers (MI: scalar loads) for exact sampling and for MI
     const bool fast_path = !exact_samples(cost, o.flags) && cost != CGS_COST_MI;
-    // the span kernels (row decisions): single-channel ZNCC and the exact-sampling costs with
-    // shared-memory windows (span_plan), single-channel MI with shared-memory histograms
-    SpanPlan sp;
-    const bool span = span_plan(*mov, *fix, o, &sp);
-    const bool span_mi = cost == CGS_COST_MI && !exact_samples(cost, o.flags) &&
+    SpanPlan sp;  // the span kernels (decisions per image row)
+    const bool span = span_plan(*mov, *fix, o, mi_bins, &sp);
+    const bool span_mi = !span && cost == CGS_COST_MI && !exact_samples(cost, o.flags) &&
                          !(o.flags & (CGS_FLAG_PER_SAMPLE_DECISIONS | CGS_FLAG_TEXTURE_TAPS | CGS_FLAG_QUAD_TAPS)) &&
                          span_mi_plan(*mov, *fix, o, mi_bins, &sp);
-    const bool quads = span || span_mi || (o.flags & CGS_FLAG_QUAD_TAPS) ||
-                       (fast_path && !(o.flags & CGS_FLAG_TEXTURE_TAPS));
-    const void *kfn = (span || span_mi) ? sp.kfn : getter(C, pl.G, pl.NW, quads);
+    const bool spans = span || span_mi;
+    const bool quads = spans || (o.flags & CGS_FLAG_QUAD_TAPS) || (fast_path && !(o.flags & CGS_FLAG_TEXTURE_TAPS));
+    const void *kfn = spans ? sp.kfn : getter(C, pl.G, pl.NW, quads);
     if (!kfn) return fail(CGS_ERROR_UNSUPPORTED, "no kernel for this channel count / tuning");
-    if (ext && !(span || span_mi)) return fail(CGS_ERROR_UNSUPPORTED, "caller scratch: span searches only");
+    if (ext && !spans) return fail(CGS_ERROR_UNSUPPORTED, "caller scratch: span searches only");
 
     DeviceInfo di;
     if ((s = device_info(&di)) != CGS_SUCCESS) return s;
@@ -1012,11 +1027,11 @@ static cgs_status search_core(const cgs_image *mov, const cgs_image *fix, const 
     // staged layout
     const Staging st = staging_layout(*mov, *fix, di.tex_align, di.tex_pitch_align, false, false, quads);
     const int64_t stage_bytes = set_chunks(&p, st, C, fix->height);
-    const size_t smem = (span || span_mi) ? sp.smem
-                                          : cta_smem_bytes(pl.G, pl.NW, (size_t)stage_bytes,
-                                                           acc_bytes(cost, pl.G, pl.NW, false, mi_bins));
+    const size_t smem = spans ? sp.smem
+                              : cta_smem_bytes(pl.G, pl.NW, (size_t)stage_bytes,
+                                              acc_bytes(cost, pl.G, pl.NW, false, mi_bins));
     if (smem > 227 * 1024) return fail(CGS_ERROR_UNSUPPORTED, "shared-memory plan exceeds 227 KB");
-    if (span || span_mi) {
+    if (spans) {
         p.tile_h = sp.TH;
         p.tiles_x = sp.tiles_x;
         p.tiles_y = sp.tiles_y;
@@ -1024,12 +1039,13 @@ static cgs_status search_core(const cgs_image *mov, const cgs_image *fix, const 
         p.win_pitch_mod = sp.pitch_mod;
     }
 
-    // the span kernels' tables follow the staging block: the tiled kernels' row prefix sums (W_f + 1
-    // FP64 pairs per row), the MI kernel's fixed bins (int32, the fixed plane's pitch)
+    // the span kernels' tables follow the staging block: the fixed rows' prefix sums (W_f + 1 FP64 pairs
+    // per row), or MI's plane of fixed bins (int32, laid out as the fixed planes)
     const size_t prefix_off = (size_t)round_up((int64_t)(st.bytes - (size_t)di.tex_align), 256);
-    const size_t prefix_bytes = span      ? (span_uses_prefix(cost) ? 1 : 0) * (size_t)fix->height * (size_t)(fix->width + 1) * sizeof(double2)
-                                : span_mi ? (size_t)fix->height * (size_t)st.fpitch * sizeof(int32_t)
-                                          : 0;
+    const bool mi_rows = spans && cost == CGS_COST_MI;
+    const size_t prefix_bytes = mi_rows                          ? (size_t)C * (size_t)st.fplane * sizeof(int32_t)
+                                : span && span_uses_prefix(cost) ? (size_t)fix->height * (size_t)(fix->width + 1) * sizeof(double2)
+                                                                 : 0;
     const size_t main_bytes = st.bytes + (prefix_bytes ? prefix_bytes + 256 : 0);
     const bool verify = !(o.flags & CGS_FLAG_NO_VERIFY) && verify_supported(cost);
     const size_t vbytes = verify ? verify_scratch_bytes() + (costs ? 0 : (size_t)p.n * 4) : 0;
@@ -1051,10 +1067,8 @@ static cgs_status search_core(const cgs_image *mov, const cgs_image *fix, const 
     };
     char *sb = staging_origin(scratch, di.tex_align);
     if (span && span_uses_prefix(cost)) p.fix_prefix = reinterpret_cast<const double2 *>(sb + prefix_off);
-    if (span_mi) {
-        p.span_rows = reinterpret_cast<const float *>(sb + prefix_off);
-        p.span_rows_header = reinterpret_cast<const float *>(sb + 32);  // zeroed with the header
-    }
+    if (mi_rows) p.span_rows = reinterpret_cast<const float *>(sb + prefix_off);
+    if (span_mi) p.span_rows_header = reinterpret_cast<const float *>(sb + 32);  // zeroed with the header
     p.key = reinterpret_cast<unsigned long long *>(sb);
     p.done = reinterpret_cast<unsigned int *>(sb + 8);
     p.status = reinterpret_cast<unsigned int *>(sb + 12);
@@ -1091,7 +1105,12 @@ static cgs_status search_core(const cgs_image *mov, const cgs_image *fix, const 
     if (quads) {
         q.quad_dst = reinterpret_cast<float4 *>(sb + st.quad_off);
         q.qplane = st.qplane;
-        q.quad_form = (span || span_mi) ? span_quad_form(cost) : 0;
+        q.quad_form = spans ? span_quad_form(cost, C) : 0;
+        if (span_mi) q.quad_scale = (float)mi_bins * (1.0f / 256.0f);
+    }
+    if (mi_rows && !span_mi) {
+        q.bin_dst = reinterpret_cast<int32_t *>(sb + prefix_off);
+        q.bins = mi_bins;
     }
     const int64_t prep_elems = (st.mplane + st.fplane) * C;
     const int prep_blocks = (int)std::min<int64_t>((prep_elems + 255) / 256, (int64_t)di.sms * 8);
@@ -1119,11 +1138,11 @@ static cgs_status search_core(const cgs_image *mov, const cgs_image *fix, const 
         return cuda_fail(e, "prep_kernel");
     }
 
-    const int threads = ((span || span_mi) ? sp.NW : pl.NW) * 32;
-    const uint32_t per_task = (span || span_mi) ? (uint32_t)(sp.NW * sp.G) : (uint32_t)(pl.NW * pl.G);
+    const int threads = (spans ? sp.NW : pl.NW) * 32;
+    const uint32_t per_task = spans ? (uint32_t)(sp.NW * sp.G) : (uint32_t)(pl.NW * pl.G);
     p.num_tasks = (p.n + per_task - 1) / per_task;
     e = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e == cudaSuccess && !span && !span_mi)
+    if (e == cudaSuccess && !spans)
         e = cudaFuncSetAttribute(kfn, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxL1);
     int per_sm = 0;
     if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kfn, threads, smem);
@@ -1135,7 +1154,7 @@ static cgs_status search_core(const cgs_image *mov, const cgs_image *fix, const 
     }
     const uint32_t blocks = std::min<uint32_t>(p.num_tasks, (uint32_t)(di.sms * per_sm));
     void *args[] = {&p};
-    if (span || span_mi) {  // these read tap quads, no texture
+    if (spans) {  // these read tap quads, no texture
         p.mov_tex = 0;
         e = cudaLaunchKernel(kfn, dim3(blocks), dim3(threads), args, smem, stream);
     } else {

@@ -111,7 +111,7 @@ __host__ __device__ constexpr size_t span_smem_bytes(int G, int NW, int TH, int 
     return span_head_bytes(NW) + (size_t)NW * G * sizeof(SpanSlot) + (size_t)NW * (G / 2) * sizeof(PairRow) +
            (size_t)tiles * TX * sizeof(BlockWin) + (size_t)NW * G * TH * sizeof(InnerSpan) +
            (size_t)NW * TH * sizeof(RowRun) + (size_t)NW * G * (5 * sizeof(double) + sizeof(int)) +
-           (size_t)kWinStages * cap * 16 + 128;
+           (size_t)kWinStages * cap * 16 + 144;
 }
 
 struct SpanSmem {
@@ -128,10 +128,14 @@ struct SpanSmem {
     int *cnt;          // [NW][G] overlap counts of the warps' points
     float4 *win;       // [kWinStages][cap]
     int cap;
+    float2 *rowtab;    // exact span kernel: [NW][TH][G / 2][3] products of the rows
+    uint32_t *hist;    // exact span kernel, MI: [NW * G][(B + 1)^2]
 };
 
+// `exact`: the exact span kernel's row products, and histograms of mi_bins bins (0: none), before the stage.
 template <int G, int NW>
-__device__ __forceinline__ SpanSmem carve_span(unsigned char *smem, int TH, int TX, int tiles, int cap) {
+__device__ __forceinline__ SpanSmem carve_span(unsigned char *smem, int TH, int TX, int tiles, int cap,
+                                               bool exact = false, int mi_bins = 0) {
     SpanSmem s;
     s.bars = reinterpret_cast<uint64_t *>(smem);
     s.wbest = reinterpret_cast<unsigned long long *>(smem + 64);
@@ -152,6 +156,13 @@ __device__ __forceinline__ SpanSmem carve_span(unsigned char *smem, int TH, int 
     q += (size_t)NW * G * 5 * sizeof(double);
     s.cnt = reinterpret_cast<int *>(q);
     q += (size_t)NW * G * sizeof(int);
+    s.rowtab = reinterpret_cast<float2 *>(smem + (((size_t)(q - smem) + 15) & ~(size_t)15));
+    s.hist = nullptr;
+    if (exact) {
+        q = reinterpret_cast<unsigned char *>(s.rowtab) + (((size_t)NW * TH * (G / 2) * 24 + 15) & ~(size_t)15);
+        s.hist = reinterpret_cast<uint32_t *>(q);
+        if (mi_bins > 0) q += ((size_t)NW * G * (mi_bins + 1) * (mi_bins + 1) * 4 + 15) & ~(size_t)15;
+    }
     // aligned by offset from the shared base (an integer round trip of the pointer would lose
     // its shared-memory provenance and turn every window read into a generic load)
     const size_t off = ((size_t)(q - smem) + 127) & ~(size_t)127;
@@ -231,6 +242,15 @@ __device__ __forceinline__ void block_extent(const SpanSlot &k, float x0, float 
     one(x1, y1);
 }
 
+// One count into a shared-memory histogram.  No compiler memory clobber: the counts are read only
+// after a __syncwarp or __syncthreads, and the loads of the next samples may move ahead of it.
+__device__ __forceinline__ void red_shared_add1(uint32_t addr) {
+    asm volatile("red.shared.add.u32 [%0], 1;" ::"r"(addr));
+}
+
+// The reference's bin of value v: min(max(floor(v B / 256), 0), B - 1).
+__device__ __forceinline__ int mi_bin(float v, float sB, int B) { return min(max((int)floorf(v * sB), 0), B - 1); }
+
 // Thread 0: announce the bytes of tile t's copies on stage `st`'s barrier (its one arrival).  It
 // comes before the CTA barrier after which every warp issues its part (issue_window).
 template <int C, int TX>
@@ -247,12 +267,13 @@ __device__ __forceinline__ void expect_window(const SearchParams &p, const SpanS
 }
 
 // Issue (every warp its part) the copies of tile t into stage `st`, completing on that stage's
-// barrier: the tile's rows of the staged fixed image (TH x TW floats at the stage's start; columns
+// barrier: the tile's rows of the fixed plane(s) fsrc, of p.fix's pitch (TH x TW floats at the stage's start; columns
 // past the image's right edge are not copied) and the windows of its blocks (quads, after the
 // fixed tile).  A tile has about 220 row copies and a warp issues one in about 60 cycles, so one
 // warp would hold the others back for 14 K cycles per tile; shared by the CTA's warps it is 1 K.
 template <int C, int NW, int TX>
-__device__ __forceinline__ void issue_window(const SearchParams &p, const SpanSmem &ss, int t, int st) {
+__device__ __forceinline__ void issue_window(const SearchParams &p, const SpanSmem &ss, const float *fsrc, int t,
+                                             int st) {
     constexpr int TW = 32 * TX;
     constexpr int WB = NW / TX;  // warps per block window
     static_assert(NW % TX == 0, "whole warps per block window");
@@ -268,7 +289,7 @@ __device__ __forceinline__ void issue_window(const SearchParams &p, const SpanSm
         for (int j = warp; j < rows; j += NW)
 #pragma unroll
             for (int ch = 0; ch < C; ch++)
-                bulk_g2s(fdst + (ch * TH + j) * TW, p.fix.data + ch * p.fix.plane + (int64_t)(y0 + j) * p.fix.pitch + x0,
+                bulk_g2s(fdst + (ch * TH + j) * TW, fsrc + ch * p.fix.plane + (int64_t)(y0 + j) * p.fix.pitch + x0,
                          row_bytes, bar);
     }
     const BlockWin b = ss.wins[t * TX + warp / WB];
@@ -458,7 +479,7 @@ __device__ __forceinline__ bool run_span_task(const SearchParams &p, uint32_t ta
         for (int t = 0; t < kWinStages && t < ntiles; t++) expect_window<1, TX>(p, ss, t, (int)((wit + t) % kWinStages));
     __syncthreads();
     for (int t = 0; t < kWinStages && t < ntiles; t++)
-        issue_window<1, NW, TX>(p, ss, t, (int)((wit + t) % kWinStages));
+        issue_window<1, NW, TX>(p, ss, p.fix.data, t, (int)((wit + t) % kWinStages));
 
     // ---- sweep
     float2 part[GP][3];  // {sum m', sum m'^2, sum f'm'} of each pair of points
@@ -772,7 +793,7 @@ __device__ __forceinline__ bool run_span_task(const SearchParams &p, uint32_t ta
             }
             return false;
         }
-        if (more) issue_window<1, NW, TX>(p, ss, t + kWinStages, st);
+        if (more) issue_window<1, NW, TX>(p, ss, p.fix.data, t + kWinStages, st);
     }
 
     // ---- per grid point: finalise, dump, argmin key (as the pixel-loop kernel)

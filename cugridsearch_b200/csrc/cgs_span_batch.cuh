@@ -26,7 +26,7 @@ __device__ __forceinline__ bool run_pair_task(const SearchParams &p, uint32_t ta
 template <int G, int NW, int TX, bool CHECK>
 __global__ void __launch_bounds__(NW * 32, 1) span_batch_kernel(const __grid_constant__ SpanBatchParams b) {
     extern __shared__ __align__(128) unsigned char smem[];
-    const SpanSmem ss = carve_span<G, NW>(smem, b.tile_h, TX, b.tiles, b.cap);
+    const SpanSmem ss = carve_span<G, NW>(smem, b.tile_h, TX, b.tiles, b.cap, true);
     // the task word sits in the carve's head, after the flags (no static shared memory: the
     // dynamic carve may take all 227 KB)
     volatile uint32_t &s_task = *reinterpret_cast<volatile uint32_t *>(ss.bounds_flag + 1);

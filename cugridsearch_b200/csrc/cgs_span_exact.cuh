@@ -1,43 +1,63 @@
-// cgs_span_exact.cuh -- the span kernel for the reference functors that sample exactly:
-// averageAbsoluteDifference (SAD_AVG), calcSQD (SQD_REF) and calcNCC (NCC_REF), one or three
-// channels.  Every sample is formed by the reference's operation sequence, bit for bit, as the
-// per-sample kernel does; what changes is around it: the in/out decisions are taken per image row,
-// the taps come from shared-memory windows and the quotients need no branch.
+// cgs_span_exact.cuh -- the span kernel of the costs that need the reference's samples bit for bit:
+// averageAbsoluteDifference (SAD_AVG), calcSQD (SQD_REF), calcNCC (NCC_REF) and the joint-histogram MI,
+// one or three channels.  Every sample is formed by the reference's operation sequence, as the
+// per-sample kernel does; what changes is around it: the in/out decisions are taken per image row, the
+// taps come from shared-memory windows and the quotients need no branch.
 //
-// Decisions, tiles, windows, stages: as in the zero-mean NCC span kernel (cgs_span.cuh).  A point's
+// Decisions, tiles, windows, stage: as in the zero-mean NCC span kernel (cgs_span.cuh).  A point's
 // inner span lies at least 1.5 guard bands inside the moving image, and the guard bounds the distance
 // between the real and the reference's coordinates, so every pixel of the inner span is inside for the
 // reference; band pixels are decided and sampled in the span pass.  A point without a guard, or whose
 // quotients could leave exact_quot2's range, has no spans: the whole warp samples all of its pixels
 // with IEEE divisions (no_span_rows).
 //
-// Sweep.  Two points per FP32x2 operation.  The map keeps the reference's order
-// w = ((A x + B y) + P) - Q with each operation rounded; packed operations round each component as
-// the scalar ones.  X and Y are formed with negated coefficients (the same bits, sign flipped), which
-// the quotient step wants.  Floors and fractions are exact operations.  The quads hold the raw taps
-// {v00, v01, v10, v11}.  For the two NCC-like costs the row weights carry a factor 2^-8, so samples
-// come out scaled by it (a power of two: the same bits) and the sums of squares have the headroom of
-// the reference's v / 255 without its division; the factor leaves in FP64 at the end.
+// Sweep.  Lane l takes the columns x0 + 32 c + l of a tile, block c after block c and in each block
+// the rows that have samples there (two ballots per block sort the rows into full, masked and none).
+// A block's products A x, C1 x, D1 x are formed once for its rows and the rows' B y, C2 y, D2 y once per
+// band (shared memory): three of 29 packed operations per sample and pair saved.  Two points per
+// FP32x2 operation; with one pair per warp two rows run at once.  The map keeps the reference's order
+// w = ((A x + B y) + P) - Q with each operation rounded; X and Y are formed with negated coefficients
+// (the same bits, sign flipped), which the quotient step wants.  Floors and fractions are exact
+// operations.  The quads hold the raw taps {v00, v01, v10, v11}.  The row weights carry a power of two,
+// so samples come out scaled by it, the same bits: 2^-8 for the NCC-like costs, whose sums of squares
+// then have the headroom of the reference's v / 255 without its division (the factor leaves in FP64 at
+// the end), and B / 256 for MI, whose sample is then its bin after a clamp and a floor.
 //
-// What bounds it: the FP32 pipe.  A pair of points takes 29 packed operations (two pipe cycles each)
-// and about 21 scalar ones per pixel and channel: 40 cycles of a scheduler's FP32 pipe per 32
-// evaluations, 10 per SM, or 8.9e11 evaluations/s; the per-sample kernel needed two IEEE divisions
-// (about 20 instructions and two branches), the in/out decisions and a texture gather per evaluation.
+// What bounds it: the FP32 pipe.  A pair of points takes 26 packed operations (two pipe cycles each)
+// and about 20 scalar ones per pixel and channel; the heavier of the two FP32 pipes is active on 72 % of
+// cycles (SAD, 256 x 256).  39 instructions per 32 evaluations, of which 5 are register moves.  SAD
+// 64 x 64, 4^8: 604 us against 842 on the per-sample kernel; calcNCC 203 x 157: 3.82 ms against 6.1.  Row
+// after row instead of block after block: 659 us and 4.2 ms.
 //
-// Sums.  Per lane and band of TH rows in FP32, then a warp sum into FP64 totals; the fixed image's
-// sum of squares comes from the row prefix sums.  The cost is formed in FP32 from the rounded totals
-// (finalize), so its special cases are the per-sample kernel's.  Costs do not depend on the order of
-// the points or on how many share a launch.
+// Three-channel MI runs here too (2.8 ms against 4.7 on the per-sample kernel for 301 x 211, 3^8); with
+// one channel the guarded fast samples of cgs_span_mi.cuh are faster.
+//
+// MI counts.  Each warp keeps its points' (B + 1) x (B + 1) u32 histograms in shared memory (row = fixed
+// bin, the last row and column for the marginals), filled with shared-memory atomics; the tile's fixed
+// rows are the fixed image's bins times the row stride, in bytes.  The cost is formed by mi_from_hist,
+// as in the per-sample kernel: equal counts give equal bits.
+//
+// Sums of the other costs.  Per lane and band of TH rows in FP32, then a warp sum into FP64 totals; the
+// fixed image's sum of squares comes from the row prefix sums.  SAD is formed in FP64, the NCC-like
+// costs in FP32 from the rounded totals (finalize), so their special cases are the per-sample kernel's.  Costs do not depend on
+// the order of the points or on how many share a launch.
 #pragma once
 #include "cgs_span.cuh"
 
 namespace cgs {
 
 // FP32 sums of a pair of points in the sweep: SAD {sum |d|}; SQD {sum d^2, sum m^2}; NCC {sum m^2, sum f m}.
-template <int COST> struct SpanSums { static constexpr int value = COST == CGS_COST_SAD_AVG ? 1 : 2; };
+template <int COST> struct SpanSums {
+    static constexpr int value = COST == CGS_COST_SAD_AVG || COST == CGS_COST_MI ? 1 : 2;
+};
 
-// Scale of the samples and fixed values in the sums (see above).
-template <int COST> struct SpanScale { static constexpr float value = COST == CGS_COST_SAD_AVG ? 1.0f : 0x1p-8f; };
+// Shared memory of the exact span kernel: the span kernels' (carve_span), the rows' products B y, -C2 y,
+// -D2 y of the warps' pairs, [NW][TH][G / 2], and the MI histograms, [NW * G][(B + 1)^2], before the
+// window stage.
+__host__ __device__ constexpr size_t span_exact_extra(int G, int NW, int TH, int mi_bins) {
+    return (((size_t)NW * TH * (G / 2) * 24 + 15) & ~(size_t)15) +
+           (mi_bins > 0 ? (((size_t)NW * G * (mi_bins + 1) * (mi_bins + 1) * 4 + 15) & ~(size_t)15) : 0);
+}
 
 // One (fixed f, moving m) sample, both scaled, into FP64 sums.
 template <int COST>
@@ -45,6 +65,7 @@ __device__ __forceinline__ void accumulate64(double *a, float f, float m) {
     const float d = m - f;
     if constexpr (COST == CGS_COST_SAD_AVG) {
         a[0] += (double)fabsf(d);
+    } else if constexpr (COST == CGS_COST_MI) {
     } else if constexpr (COST == CGS_COST_SQD_REF) {
         a[0] += (double)d * (double)d;
         a[1] += (double)m * (double)m;
@@ -59,61 +80,64 @@ __device__ __forceinline__ bool run_span_exact_task(const SearchParams &p, uint3
                                                     uint32_t &wit) {
     static_assert(G % 2 == 0, "the span path pairs grid points");
     constexpr int GP = G / 2;
+    constexpr int NB = GP == 1 ? 2 : 1;  // full rows at once
     constexpr int TW = 32 * TX;
     constexpr int NS = SpanSums<COST>::value;
-    constexpr float kS = SpanScale<COST>::value;
-    constexpr bool kFix = COST != CGS_COST_SAD_AVG;  // the cost needs sum f^2
+    constexpr bool kMI = COST == CGS_COST_MI;
+    constexpr bool kFix = COST == CGS_COST_SQD_REF || COST == CGS_COST_NCC_REF;  // the cost needs sum f^2
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int fw = p.fix.w, fh = p.fix.h;
     const int TH = p.tile_h;
     const int tiles_x = p.tiles_x, ntiles = p.tiles_x * p.tiles_y;
     const float mov_wf = p.mov_wf, mov_hf = p.mov_hf;
+    const int B = p.mi_bins, hstride = B + 1, hsize = hstride * hstride;
+    // the samples' scale (a power of two)
+    const float kS = kMI ? (float)B * (1.0f / 256.0f) : COST == CGS_COST_SAD_AVG ? 1.0f : 0x1p-8f;
 
     // ---- the warp's points
     SpanSlot *my_slots = ss.slots + warp * G;
     span_points<COST, G, true>(p, (task * NW + warp) * G, my_slots);
     __syncwarp();
     // w = ((A x + By) + P) + nQ, -X = ((nC1 x + nC2 y) + nR) + S, -Y alike
-    float2 A2[GP], P2[GP], nQ2[GP], nC12[GP], nR2[GP], S2[GP], nD12[GP], nT2[GP], U2[GP];
+    float2 P2[GP], nQ2[GP], nR2[GP], S2[GP], nT2[GP], U2[GP];
     bool nospan = false;  // some point of the warp has no spans
 #pragma unroll
     for (int h = 0; h < GP; h++) {
         const SpanSlot &a = my_slots[2 * h], &b = my_slots[2 * h + 1];
-        A2[h] = make_float2(a.A, b.A);
         P2[h] = make_float2(a.P, b.P);
         nQ2[h] = make_float2(-a.Q, -b.Q);
-        nC12[h] = make_float2(-a.C1, -b.C1);
         nR2[h] = make_float2(-a.R, -b.R);
         S2[h] = make_float2(a.S, b.S);
-        nD12[h] = make_float2(-a.D1, -b.D1);
         nT2[h] = make_float2(-a.T, -b.T);
         U2[h] = make_float2(a.U, b.U);
         nospan |= (a.valid && !a.ok) || (b.valid && !b.ok);
     }
-    if (lane < GP) {
-        const SpanSlot &a = my_slots[2 * lane], &b = my_slots[2 * lane + 1];
-        PairRow pr{};
-        pr.B = make_float2(a.B, b.B);
-        pr.C2 = make_float2(-a.C2, -b.C2);
-        pr.D2 = make_float2(-a.D2, -b.D2);
-        ss.prow[warp * GP + lane] = pr;
-    }
+    float2 *my_rows = ss.rowtab + (size_t)warp * TH * GP * 3;  // [TH][GP]{B y, -C2 y, -D2 y}
+    uint32_t *my_hist = ss.hist + (size_t)warp * G * hsize;
     double *my_dtot = ss.dtot + warp * G * 5;  // {sum f^2, the sweep's NS sums} per point, stride 5
     int *my_cnt = ss.cnt + warp * G;
-    for (int i = lane; i < G * 5; i += 32) my_dtot[i] = 0.0;
+    if constexpr (kMI) {
+        for (int i = lane; i < G * hsize; i += 32) my_hist[i] = 0u;
+    } else {
+        for (int i = lane; i < G * 5; i += 32) my_dtot[i] = 0.0;
+    }
     if (lane < G) my_cnt[lane] = 0;
     __syncthreads();  // every point's slot is written
 
+    // the tile's fixed rows: the staged image, or MI's plane of bins
+    const float *fsrc = kMI ? p.span_rows : p.fix.data;
     span_windows<C, G, NW, TX>(p, ss);
     __syncthreads();
     if (threadIdx.x == 0)
         for (int t = 0; t < kWinStages && t < ntiles; t++) expect_window<C, TX>(p, ss, t, (int)((wit + t) % kWinStages));
     __syncthreads();
     for (int t = 0; t < kWinStages && t < ntiles; t++)
-        issue_window<C, NW, TX>(p, ss, t, (int)((wit + t) % kWinStages));
+        issue_window<C, NW, TX>(p, ss, fsrc, t, (int)((wit + t) % kWinStages));
 
-    // one sample of point g at (x, y) by the reference's sequence, into a (and f^2 into s2) if inside
-    auto exact_sample = [&](const SpanSlot &sl, int x, int y, double *a, double &s2) -> int {
+    // one sample of point g at (x, y) by the reference's sequence, into a (and f^2 into s2) or the
+    // histogram if inside
+    auto exact_sample = [&](int g, int x, int y, double *a, double &s2) -> int {
+        const SpanSlot &sl = my_slots[g];
         const MapCoef kc{sl.A, sl.B, sl.P, sl.Q, sl.C1, sl.C2, sl.R, sl.S, sl.D1, sl.D2, sl.T, sl.U};
         float ex, ey;
         exact_map(kc, (float)x, (float)y, ex, ey);
@@ -122,7 +146,10 @@ __device__ __forceinline__ bool run_span_exact_task(const SearchParams &p, uint3
         for (int ch = 0; ch < C; ch++) {
             const float m = bilinear_in(p.mov.data + ch * p.mov.plane, p.mov.pitch, ey, ex);
             const float f = p.fix.data[ch * p.fix.plane + (int64_t)y * p.fix.pitch + x];
-            accumulate64<COST>(a, f * kS, m * kS);
+            if constexpr (kMI)
+                red_shared_add1(smem_addr(my_hist + g * hsize + mi_bin(f, kS, B) * hstride + mi_bin(m, kS, B)));
+            else
+                accumulate64<COST>(a, f * kS, m * kS);
             if constexpr (kFix) s2 += (double)f * (double)f;
         }
         return 1;
@@ -133,14 +160,14 @@ __device__ __forceinline__ bool run_span_exact_task(const SearchParams &p, uint3
             if constexpr (kFix) s2 += __shfl_xor_sync(0xffffffffu, s2, o);
             n += __shfl_xor_sync(0xffffffffu, n, o);
         }
-        if (moving)
+        if (!kMI && moving)
             for (int o = 1; o < width; o <<= 1)
 #pragma unroll
                 for (int j = 0; j < NS; j++) a[j] += __shfl_xor_sync(0xffffffffu, a[j], o);
         if (leader) {
             double *d = my_dtot + g * 5;
             if constexpr (kFix) d[0] += s2;
-            if (moving)
+            if (!kMI && moving)
 #pragma unroll
                 for (int j = 0; j < NS; j++) d[1 + j] += a[j];
             my_cnt[g] += n;
@@ -154,7 +181,7 @@ __device__ __forceinline__ bool run_span_exact_task(const SearchParams &p, uint3
             double a[NS] = {}, s2 = 0.0;
             int n = 0;
             for (int y = y0; y < y1; y++)
-                for (int x = lane; x < fw; x += 32) n += exact_sample(sl, x, y, a, s2);
+                for (int x = lane; x < fw; x += 32) n += exact_sample(g, x, y, a, s2);
             add_totals(g, lane == 0, 32, a, s2, n, true);
             __syncwarp();
         }
@@ -177,8 +204,11 @@ __device__ __forceinline__ bool run_span_exact_task(const SearchParams &p, uint3
     const float2 nzero2 = make_float2(nzero, nzero);
     const float2 nsc = make_float2(-kS, -kS), smagic2 = make_float2(kS * kMagic, kS * kMagic);
     const uint64_t mqbase = reinterpret_cast<uint64_t>(p.mov_quad) - 16ull * (uint64_t)(uint32_t)kMagicBits;
-    const float qpitch = -(float)p.quad_pitch * (1.0f / kS);
+    const float ikS = 1.0f / kS;  // exact
     const uint64_t qplane = 16ull * (uint64_t)p.quad_plane;
+    // MI: histogram address of (fixed bin, moving bin bits): 4 bits + the fixed bin's byte offset + hbase
+    const uint32_t hbase = smem_addr(my_hist) - 4u * (uint32_t)kMagicBits, hpoint = 4u * (uint32_t)hsize;
+    const float bin_max = (float)(B - 1);
 
     for (int t = 0; t < ntiles; t++, wit++) {
         const int tx = t % tiles_x, ty = t / tiles_x;
@@ -211,8 +241,8 @@ __device__ __forceinline__ bool run_span_exact_task(const SearchParams &p, uint3
                         // band pixels: the outer span outside the inner one, [pa, e0) and [e1, pa + plen)
                         const int e0 = len > 0 ? xa : pa + plen, e1 = len > 0 ? xa + len : pa + plen;
                         int nb = 0;
-                        for (int x = pa; x < e0; x++) nb += exact_sample(sl, x, y, a, s2);
-                        for (int x = e1; x < pa + plen; x++) nb += exact_sample(sl, x, y, a, s2);
+                        for (int x = pa; x < e0; x++) nb += exact_sample(g, x, y, a, s2);
+                        for (int x = e1; x < pa + plen; x++) nb += exact_sample(g, x, y, a, s2);
                         n += nb;
                         found = nb > 0;
                     }
@@ -237,6 +267,15 @@ __device__ __forceinline__ bool run_span_exact_task(const SearchParams &p, uint3
                 }
                 my_runs[lane] = RowRun{ia, ib, ua, ub};
             }
+            for (int i = lane; i < TH * GP; i += 32) {  // the rows' products
+                const int r = i / GP, h = i - r * GP;
+                const SpanSlot &a = my_slots[2 * h], &b = my_slots[2 * h + 1];
+                const float yf = (float)(y0 + r);
+                float2 *d = my_rows + i * 3;
+                d[0] = make_float2(xm(a.B, yf), xm(b.B, yf));
+                d[1] = make_float2(-xm(a.C2, yf), -xm(b.C2, yf));
+                d[2] = make_float2(-xm(a.D2, yf), -xm(b.D2, yf));
+            }
             __syncwarp();
             if (nospan) no_span_rows(y0, min(y0 + TH, fh));
         }
@@ -247,46 +286,61 @@ __device__ __forceinline__ bool run_span_exact_task(const SearchParams &p, uint3
         const uint32_t wbase = smem_addr(ss.win + (size_t)st * ss.cap + C * TH * TW / 4);
         const uint32_t szero = smem_addr(ss.win);
 
-        for (int r = 0; r < TH; r++) {
-            if (y0 + r >= fh) break;
-            const RowRun run = my_runs[r];
-            if (run.ua > x1 || run.ub < x0) continue;  // no point samples this row of the tile
-            const float yf = (float)(y0 + r);
-            const float2 yf2 = make_float2(yf, yf);
-            float2 byw[GP], byx[GP], byy[GP];
+        // this lane's row of the band (lanes past it: none)
+        const RowRun lrun = lane < TH && y0 + lane < fh ? my_runs[lane] : RowRun{1, 0, 1 << 30, -1};
+#pragma unroll 1
+        for (int c = 0; c < TX; c++) {
+            const int xb = x0 + 32 * c;
+            // the rows with samples in the block, and those where the block lies in every point's inner span
+            uint32_t any = __ballot_sync(0xffffffffu, lrun.ua <= xb + 31 && lrun.ub >= xb);
+            const uint32_t full = __ballot_sync(0xffffffffu, lrun.ia <= xb && lrun.ib >= xb + 31);
+            if (any == 0u) continue;
+            const bool in_stage = twin[c].w > 0;
+            const int x = xb + lane;
+            const float xf = (float)x;
+            const float2 xf2 = make_float2(xf, xf);
+            float2 ax0[GP], cx0[GP], dx0[GP];  // A x, -C1 x, -D1 x
 #pragma unroll
             for (int h = 0; h < GP; h++) {
-                const PairRow &pr = ss.prow[warp * GP + h];
-                byw[h] = __ffma2_rn(pr.B, yf2, nzero2);
-                byx[h] = __ffma2_rn(pr.C2, yf2, nzero2);
-                byy[h] = __ffma2_rn(pr.D2, yf2, nzero2);
+                const SpanSlot &a = my_slots[2 * h], &b = my_slots[2 * h + 1];
+                ax0[h] = __ffma2_rn(make_float2(a.A, b.A), xf2, nzero2);
+                cx0[h] = __ffma2_rn(make_float2(-a.C1, -b.C1), xf2, nzero2);
+                dx0[h] = __ffma2_rn(make_float2(-a.D1, -b.D1), xf2, nzero2);
             }
-            const float *frow = sfix + r * TW;
-            // one block of 32 columns; EDGE: some column may lie outside a point's inner span;
-            // SMEM: the block's window is in the stage
-            auto column = [&](int c, auto edge_tag, auto smem_tag) {
+            uint32_t sbase = 0u, wplane = 0u;
+            float pitch;
+            if (in_stage) {
+                // shared address of window quad (ix, iy): wbase + 16 (off + (ix - x0) + pitch (iy - y0))
+                sbase = wbase + twin[c].rel;
+                pitch = twin[c].pitchf * ikS;
+                wplane = 16u * (uint32_t)(twin[c].pitch * twin[c].h);
+            } else {
+                pitch = -(float)p.quad_pitch * ikS;
+            }
+            const float2 pitch2 = make_float2(pitch, pitch);
+            const float *fcol = sfix + 32 * c + lane;
+
+            // NR rows from row r; EDGE: some column may lie outside a point's inner span; SMEM: the
+            // block's window is in the stage
+            auto rows = [&](int r, auto nr_tag, auto edge_tag, auto smem_tag) {
+                constexpr int NR = decltype(nr_tag)::value;
                 constexpr bool EDGE = decltype(edge_tag)::value;
                 constexpr bool SMEM = decltype(smem_tag)::value;
-                uint32_t sbase = 0u, wplane = 0u;
-                float pitch = qpitch;
-                if constexpr (SMEM) {
-                    const uint2 rp = *reinterpret_cast<const uint2 *>(&twin[c].rel);
-                    sbase = wbase + rp.x;
-                    pitch = __uint_as_float(rp.y) * (1.0f / kS);
-                    if constexpr (C > 1) wplane = 16u * (uint32_t)(twin[c].pitch * twin[c].h);
-                }
-                const float2 pitch2 = make_float2(pitch, pitch);
-                const int x = x0 + 32 * c + lane;
-                float f[C];
+                float f[NR][C];
 #pragma unroll
-                for (int ch = 0; ch < C; ch++) f[ch] = frow[ch * TH * TW + 32 * c + lane] * kS;
-                const float xf = (float)x;
-                const float2 xf2 = make_float2(xf, xf);
+                for (int k = 0; k < NR; k++)
 #pragma unroll
-                for (int h = 0; h < GP; h++) {
-                    const float2 w = __fadd2_rn(__fadd2_rn(__fadd2_rn(__ffma2_rn(A2[h], xf2, nzero2), byw[h]), P2[h]), nQ2[h]);
-                    const float2 nX = __fadd2_rn(__fadd2_rn(__fadd2_rn(__ffma2_rn(nC12[h], xf2, nzero2), byx[h]), nR2[h]), S2[h]);
-                    const float2 nY = __fadd2_rn(__fadd2_rn(__fadd2_rn(__ffma2_rn(nD12[h], xf2, nzero2), byy[h]), nT2[h]), U2[h]);
+                    for (int ch = 0; ch < C; ch++) {
+                        f[k][ch] = fcol[(ch * TH + r + k) * TW];
+                        if constexpr (kFix) f[k][ch] *= 0x1p-8f;
+                    }
+#pragma unroll
+                for (int kh = 0; kh < NR * GP; kh++) {
+                    const int k = kh / GP, h = kh - k * GP;
+                    const float2 *rt = my_rows + ((r + k) * GP + h) * 3;
+                    const float2 w = __fadd2_rn(__fadd2_rn(__fadd2_rn(ax0[h], rt[0]), P2[h]), nQ2[h]);
+                    const float2 nX = __fadd2_rn(__fadd2_rn(__fadd2_rn(cx0[h], rt[1]), nR2[h]), S2[h]);
+                    const float2 nY = __fadd2_rn(__fadd2_rn(__fadd2_rn(dx0[h], rt[2]), nT2[h]), U2[h]);
                     float2 ex, ey;
                     exact_quot2(w, nX, nY, ex, ey);
                     // floor (round-down add of 1.5 * 2^23 leaves it in the mantissa), fractions a and 1 - a
@@ -298,7 +352,7 @@ __device__ __forceinline__ bool run_span_exact_task(const SearchParams &p, uint3
                     const float2 qi = __ffma2_rn(nfy2, pitch2, tx2);
                     bool in0 = true, in1 = true;
                     if constexpr (EDGE) {
-                        const InnerSpan a = my_spans[2 * h * TH + r], b = my_spans[(2 * h + 1) * TH + r];
+                        const InnerSpan a = my_spans[2 * h * TH + r + k], b = my_spans[(2 * h + 1) * TH + r + k];
                         in0 = (unsigned)(x - a.xa) < (unsigned)a.len;
                         in1 = (unsigned)(x - b.xa) < (unsigned)b.len;
                     }
@@ -337,10 +391,9 @@ __device__ __forceinline__ bool run_span_exact_task(const SearchParams &p, uint3
                         float4 q0, q1;
                         if constexpr (SMEM) {
                             // a masked or skipped sample reads the stage's start, whatever the plane
-                            const uint32_t b0 = (EDGE || CHECK) && C > 1 ? (a0 == szero ? szero : a0 + ch * wplane)
-                                                                         : a0 + ch * wplane;
-                            const uint32_t b1 = (EDGE || CHECK) && C > 1 ? (a1 == szero ? szero : a1 + ch * wplane)
-                                                                         : a1 + ch * wplane;
+                            const uint32_t o = ch * wplane;
+                            const uint32_t b0 = (EDGE || CHECK) && C > 1 && a0 == szero ? szero : a0 + o;
+                            const uint32_t b1 = (EDGE || CHECK) && C > 1 && a1 == szero ? szero : a1 + o;
                             asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
                                          : "=f"(q0.x), "=f"(q0.y), "=f"(q0.z), "=f"(q0.w) : "r"(b0));
                             asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
@@ -353,47 +406,58 @@ __device__ __forceinline__ bool run_span_exact_task(const SearchParams &p, uint3
                         const float t0 = xa(xm(ox.x, q0.x), xm(ax.x, q0.y)), b0v = xa(xm(ox.x, q0.z), xm(ax.x, q0.w));
                         const float t1 = xa(xm(ox.y, q1.x), xm(ax.y, q1.y)), b1v = xa(xm(ox.y, q1.z), xm(ax.y, q1.w));
                         float2 m = make_float2(xa(xm(oy.x, t0), xm(ay.x, b0v)), xa(xm(oy.y, t1), xm(ay.y, b1v)));
-                        float2 fm = make_float2(f[ch], f[ch]);
-                        if constexpr (EDGE) {  // by selection: a NaN outside the overlap stays out of the sums
-                            m = make_float2(in0 ? m.x : 0.0f, in1 ? m.y : 0.0f);
-                            fm = make_float2(in0 ? f[ch] : 0.0f, in1 ? f[ch] : 0.0f);
-                        }
-                        if constexpr (COST == CGS_COST_SAD_AVG) {
-                            part[h][0].x += fabsf(m.x - fm.x);
-                            part[h][0].y += fabsf(m.y - fm.y);
-                        } else if constexpr (COST == CGS_COST_SQD_REF) {
-                            const float2 d = __ffma2_rn(fm, minus1, m);
-                            part[h][0] = __ffma2_rn(d, d, part[h][0]);
-                            part[h][1] = __ffma2_rn(m, m, part[h][1]);
+                        if constexpr (kMI) {
+                            // m = v B / 256: clamped to [0, B - 1] and floored, the reference's bin
+                            m = make_float2(fminf(fmaxf(m.x, 0.0f), bin_max), fminf(fmaxf(m.y, 0.0f), bin_max));
+                            const float2 b2 = __fadd2_rd(m, magic2);
+                            const uint32_t hf = hbase + __float_as_uint(f[k][ch]);
+                            if (in0) red_shared_add1(hf + (2 * h) * hpoint + 4u * __float_as_uint(b2.x));
+                            if (in1) red_shared_add1(hf + (2 * h + 1) * hpoint + 4u * __float_as_uint(b2.y));
                         } else {
-                            part[h][0] = __ffma2_rn(m, m, part[h][0]);
-                            part[h][1] = __ffma2_rn(fm, m, part[h][1]);
+                            float2 fm = make_float2(f[k][ch], f[k][ch]);
+                            if constexpr (EDGE) {  // by selection: a NaN outside the overlap stays out of the sums
+                                m = make_float2(in0 ? m.x : 0.0f, in1 ? m.y : 0.0f);
+                                fm = make_float2(in0 ? fm.x : 0.0f, in1 ? fm.y : 0.0f);
+                            }
+                            if constexpr (COST == CGS_COST_SAD_AVG) {
+                                const float2 d = __ffma2_rn(fm, minus1, m);
+                                part[h][0].x += fabsf(d.x);
+                                part[h][0].y += fabsf(d.y);
+                            } else if constexpr (COST == CGS_COST_SQD_REF) {
+                                const float2 d = __ffma2_rn(fm, minus1, m);
+                                part[h][0] = __ffma2_rn(d, d, part[h][0]);
+                                part[h][1] = __ffma2_rn(m, m, part[h][1]);
+                            } else {
+                                part[h][0] = __ffma2_rn(m, m, part[h][0]);
+                                part[h][1] = __ffma2_rn(fm, m, part[h][1]);
+                            }
                         }
                     }
                 }
             };
-            auto block = [&](int c, auto edge_tag) {
-                if (twin[c].w > 0) column(c, edge_tag, std::true_type{});
-                else column(c, edge_tag, std::false_type{});
-            };
-            // blocks with any inner span: [cu0, cu1]; those inside every point's, [cf0, cf1], unmasked
-            const int cu0 = max(0, (run.ua - x0) >> 5), cu1 = min(TX - 1, (run.ub - x0) >> 5);
-            int cf0 = cu1 + 1, cf1 = cu1;
-            if (run.ia <= run.ib) {
-                const int a = max(cu0, (run.ia - x0 + 31) >> 5), b = min(cu1, ((run.ib - x0 + 1) >> 5) - 1);
-                if (a <= b) {
-                    cf0 = a;
-                    cf1 = b;
-                }
-            }
+            auto block = [&](auto smem_tag) {
+                using One = std::integral_constant<int, 1>;
+                using Many = std::integral_constant<int, NB>;
 #pragma unroll 1
-            for (int c = cu0; c <= cu1; c++) {
-                if (c >= cf0 && c <= cf1) block(c, std::false_type{});
-                else block(c, std::true_type{});
-            }
+                while (any) {
+                    const int r = __ffs(any) - 1;
+                    if constexpr (NB == 2) {
+                        if (((full >> r) & 3u) == 3u) {
+                            rows(r, Many{}, std::false_type{}, smem_tag);
+                            any &= ~(3u << r);
+                            continue;
+                        }
+                    }
+                    if ((full >> r) & 1u) rows(r, One{}, std::false_type{}, smem_tag);
+                    else rows(r, One{}, std::true_type{}, smem_tag);
+                    any &= any - 1u;
+                }
+            };
+            if (in_stage) block(std::true_type{});
+            else block(std::false_type{});
         }
         // end of a band of tiles: the band's warp sums into the FP64 totals
-        if (tx == tiles_x - 1) {
+        if (!kMI && tx == tiles_x - 1) {
 #pragma unroll
             for (int h = 0; h < GP; h++)
 #pragma unroll
@@ -413,21 +477,26 @@ __device__ __forceinline__ bool run_span_exact_task(const SearchParams &p, uint3
             if (threadIdx.x == 0) mbar_wait_bounded(&ss.bars[st], (wit / kWinStages) & 1u, kWaitLimitNs);
             return false;
         }
-        if (more) issue_window<C, NW, TX>(p, ss, t + kWinStages, st);
+        if (more) issue_window<C, NW, TX>(p, ss, fsrc, t + kWinStages, st);
     }
 
-    // ---- per grid point: the cost from the totals, dump, argmin key
+    // ---- per grid point: the cost from the totals or the counts, dump, argmin key
     __syncwarp();
     unsigned long long kk = ~0ull;
-    if (lane < G) {
-        const SpanSlot &sl = my_slots[lane];
+    float cost = 0.0f;
+    if constexpr (kMI) {
+#pragma unroll
+        for (int g = 0; g < G; g++) {
+            const float c = mi_from_hist(my_hist + g * hsize, my_cnt[g] * C, B, hstride, p);
+            if (lane == g) cost = c;
+            __syncwarp();
+        }
+    } else if (lane < G) {
         const int n = my_cnt[lane] * C;
         const double *d = my_dtot + lane * 5;
         constexpr double k2 = (256.0 / 255.0) * (256.0 / 255.0);
         float a[3] = {0.0f, 0.0f, 0.0f};
-        if constexpr (COST == CGS_COST_SAD_AVG) {
-            a[0] = (float)d[1];
-        } else if constexpr (COST == CGS_COST_SQD_REF) {
+        if constexpr (COST == CGS_COST_SQD_REF) {
             a[0] = (float)(d[1] * k2);
             a[1] = (float)(d[2] * k2);
             a[2] = (float)(d[0] * (1.0 / 65025.0));
@@ -436,7 +505,11 @@ __device__ __forceinline__ bool run_span_exact_task(const SearchParams &p, uint3
             a[1] = (float)(d[1] * k2);
             a[2] = (float)(d[2] * k2);
         }
-        const float cost = finalize<COST>(a, n, p);
+        // 0 / 0 is NaN, as in the reference
+        cost = COST == CGS_COST_SAD_AVG ? (float)(d[1] / (double)n) : finalize<COST>(a, n, p);
+    }
+    if (lane < G) {
+        const SpanSlot &sl = my_slots[lane];
         if (sl.valid) {
             if (p.costs) p.costs[sl.index] = cost;
             kk = make_key(cost, sl.index);
@@ -458,7 +531,8 @@ __device__ __forceinline__ bool run_span_exact_task(const SearchParams &p, uint3
 template <int COST, int C, int G, int NW, int TX, bool CHECK>
 __global__ void __launch_bounds__(NW * 32, 1) span_exact_kernel(const __grid_constant__ SearchParams p) {
     extern __shared__ __align__(128) unsigned char smem[];
-    const SpanSmem ss = carve_span<G, NW>(smem, p.tile_h, TX, p.tiles_x * p.tiles_y, p.win_cap);
+    const SpanSmem ss = carve_span<G, NW>(smem, p.tile_h, TX, p.tiles_x * p.tiles_y, p.win_cap, true,
+                                          COST == CGS_COST_MI ? p.mi_bins : 0);
     if (threadIdx.x == 0) {
         for (int s = 0; s < kWinStages; s++) mbar_init(&ss.bars[s], 1);
         fence_mbar_init();

@@ -20,11 +20,21 @@
 //
 // Layout.  Each warp keeps two grid points (one FP32x2 pair) and their (B + 1) x (B + 1) u32
 // histograms in shared memory (row = fixed bin, the last row and column for the marginals),
-// filled with shared-memory atomics.  The fixed image's bins, premultiplied by the row stride,
-// come from a plane written by span_prep_mi_kernel; the taps come from the quad plane in
-// global memory through L1 (the histograms take the shared memory that windows would need).
-// The warps of a CTA meet at a barrier per band of rows, so that their points (neighbours in the
-// locality order) read the same region of the quad plane while it is in L1.
+// filled with shared-memory atomics of the constant 1 (which aggregate equal addresses of a warp;
+// packing two points' counts into one word, with an atomic of 65536, had 24 times the conflicts).
+// The fixed image's bins, premultiplied by the row stride, come from a plane written by
+// span_prep_mi_kernel; the taps come from the quad plane, scaled to bins, in global memory
+// through L1 (the histograms take the shared memory that windows would need).  The warps of a CTA
+// meet at a barrier per band of rows, so that their points (neighbours in the locality order)
+// read the same region of the quad plane while it is in L1.  In a band a warp sweeps block after
+// block of 32 columns, two full rows at once.
+//
+// What bounds it: instruction issue and the latency of quads that miss L1.  40 instructions per 32
+// evaluations; 512 x 512, 5^8: 182 ms against 207 ms with 47 (clamping the sample before the guard
+// makes the ends' outer edges no edges and the floor exact, which removed two range tests, a
+// conversion and an integer clamp; samples that do not count go to an unused cell instead of around
+// a branch; one vote per two rows).  Sampling exactly instead of guarding the bins
+// (cgs_span_exact.cuh) took 211 ms with windows and 237 without.
 #pragma once
 #include "cgs_span.cuh"
 
@@ -76,15 +86,6 @@ __device__ __forceinline__ SpanMiSmem carve_span_mi(unsigned char *smem, int TH,
     return s;
 }
 
-// One count into a shared-memory histogram.  No compiler memory clobber: the counts are read only
-// after a __syncwarp or __syncthreads, and the loads of the next samples may move ahead of it.
-__device__ __forceinline__ void red_shared_add1(uint32_t addr) {
-    asm volatile("red.shared.add.u32 [%0], 1;" ::"r"(addr));
-}
-
-// The reference's bin of value v: min(max(floor(v B / 256), 0), B - 1).
-__device__ __forceinline__ int mi_bin(float v, float sB, int B) { return min(max((int)floorf(v * sB), 0), B - 1); }
-
 // One task: the two grid points of each warp over every row of the fixed image.
 template <int NW, bool CHECK>
 __device__ __forceinline__ void run_span_mi_task(const SearchParams &p, uint32_t task, const SpanMiSmem &ss) {
@@ -115,9 +116,9 @@ __device__ __forceinline__ void run_span_mi_task(const SearchParams &p, uint32_t
 #pragma unroll
     for (int g = 0; g < G; g++) {
         const SpanSlot &k = my_slots[g];
-        // slope factor of the bin guard: |v_fast - v_exact| <= (3|c10| + |c01| + 2|c11|) max(gx, gy)
-        // (in bin units with sB), the factor covering the roundings of the sum
-        const float gm = fmaxf(k.gx, k.gy), sg = sB * gm * (1.0f + 0x1p-18f);
+        // slope factor of the bin guard: |v_fast - v_exact| <= (3|c10| + |c01| + 2|c11|) max(gx, gy) (in
+        // bins, as the quads are), the factor covering the roundings of the sum
+        const float gm = fmaxf(k.gx, k.gy), sg = gm * (1.0f + 0x1p-18f);
         const float gl = fmaf(lmax, sg, gv0);  // the bound near a cell edge
         const float hh = 0.5f - gm;            // fraction farther than this from 0.5: near a cell edge
         if (g == 0) {
@@ -171,10 +172,13 @@ __device__ __forceinline__ void run_span_mi_task(const SearchParams &p, uint32_t
 
     InnerSpan *my_spans = ss.spans + warp * G * TH;
     RowRun *my_runs = ss.runs + warp * TH;
-    const float2 magic2 = make_float2(kMagic, kMagic), nmagic2 = make_float2(-kMagic, -kMagic);
+    const float2 magic2 = make_float2(kMagic, kMagic), one2 = make_float2(1.0f, 1.0f), gv2 = make_float2(gv0, gv0);
+    // histogram addresses: 4 (bits of the floored bin + the fixed bin's row) + hbin; the unused cell (B, B)
+    const uint32_t hbin = hist_s - 4u * (uint32_t)kMagicBits, hpoint = 4u * (uint32_t)hsize;
+    const uint32_t hdump = hist_s + 4u * (uint32_t)(hsize - 1);
     const float2 minus1 = make_float2(-1.0f, -1.0f), mhalf2 = make_float2(-0.5f, -0.5f);
     const uint64_t mqbase = reinterpret_cast<uint64_t>(p.mov_quad) - 16ull * (uint64_t)(uint32_t)kMagicBits;
-    const float2 qpitch2 = make_float2((float)p.quad_pitch, (float)p.quad_pitch);
+    const float2 qpitch2 = make_float2(-(float)p.quad_pitch, -(float)p.quad_pitch);
     const int nblocks = (fw + 31) >> 5;
 
     for (int y0 = 0; y0 < fh; y0 += TH) {
@@ -224,49 +228,54 @@ __device__ __forceinline__ void run_span_mi_task(const SearchParams &p, uint32_t
         }
         __syncwarp();
 
-        // ---- the band's rows
-        for (int r = 0; r < TH && y0 + r < fh; r++) {
-            const RowRun run = my_runs[r];
-            if (run.ua > run.ub) continue;
-            const int y = y0 + r;
-            const float2 yf2 = make_float2((float)y, (float)y);
-            const PairRow pr = ss.prow[warp];
-            const float2 byw = __ffma2_rn(pr.B, yf2, pr.PQ);
-            const float2 byx = __ffma2_rn(pr.C2, yf2, pr.RS);
-            const float2 byy = __ffma2_rn(pr.D2, yf2, pr.TU);
-            const int32_t *brow = fbins + (int64_t)y * fpitch;
-            // NB consecutive blocks of 32 columns from block c (the lane's columns 32 c + lane + 32 k);
-            // EDGE: some column may lie outside a point's inner span
-            auto column = [&](int c, auto edge_tag, auto nb_tag) {
+        // ---- the band's blocks of 32 columns, and in each the rows with samples there
+        const RowRun lrun = lane < TH && y0 + lane < fh ? my_runs[lane] : RowRun{1, 0, 1 << 30, -1};
+        const int32_t *bband = fbins + (int64_t)y0 * fpitch;
+        const PairRow pr = ss.prow[warp];
+#pragma unroll 1
+        for (int c = 0; c < nblocks; c++) {
+            const int xb = 32 * c;
+            uint32_t any = __ballot_sync(0xffffffffu, lrun.ua <= xb + 31 && lrun.ub >= xb);
+            uint32_t full = __ballot_sync(0xffffffffu, lrun.ia <= xb && lrun.ib >= xb + 31);
+            if (any == 0u) continue;
+            const int x = xb + lane;
+            const float xf = (float)x;
+            const float2 xf2 = make_float2(xf, xf);
+            const float2 bxw = __ffma2_rn(A2, xf2, pr.PQ);
+            const float2 bxx = __ffma2_rn(C12, xf2, pr.RS);
+            const float2 bxy = __ffma2_rn(D12, xf2, pr.TU);
+            const int32_t *bcol = bband + min(x, fw - 1);
+            // NB rows from row r; EDGE: some column may lie outside a point's inner span
+            auto rows = [&](int r, auto edge_tag, auto nb_tag) {
                 constexpr bool EDGE = decltype(edge_tag)::value;
                 constexpr int NB = decltype(nb_tag)::value;
-                int x[NB], fb[NB];
+                int fb[NB];
                 bool in0[NB], in1[NB], amb0[NB], amb1[NB];
 #pragma unroll
                 for (int k = 0; k < NB; k++) {
-                    x[k] = 32 * (c + k) + lane;
                     in0[k] = true;
                     in1[k] = true;
                     if constexpr (EDGE) {
-                        const InnerSpan a = my_spans[r], b = my_spans[TH + r];
-                        in0[k] = (unsigned)(x[k] - a.xa) < (unsigned)a.len;
-                        in1[k] = (unsigned)(x[k] - b.xa) < (unsigned)b.len;
+                        const InnerSpan a = my_spans[r + k], b = my_spans[TH + r + k];
+                        in0[k] = (unsigned)(x - a.xa) < (unsigned)a.len;
+                        in1[k] = (unsigned)(x - b.xa) < (unsigned)b.len;
                     }
-                    fb[k] = __ldg(brow + min(x[k], fw - 1));  // fixed bin x (B + 1)
+                    fb[k] = __ldg(bcol + (r + k) * fpitch);  // fixed bin x (B + 1)
                 }
 #pragma unroll
                 for (int k = 0; k < NB; k++) {
-                    const float xf = (float)x[k];
-                    const float2 xf2 = make_float2(xf, xf);
-                    const float2 w = __ffma2_rn(A2, xf2, byw);
-                    const float2 X = __ffma2_rn(C12, xf2, byx);
-                    const float2 Y = __ffma2_rn(D12, xf2, byy);
+                    const float yf = (float)(y0 + r + k);
+                    const float2 yf2 = make_float2(yf, yf);
+                    const float2 w = __ffma2_rn(pr.B, yf2, bxw);
+                    const float2 X = __ffma2_rn(pr.C2, yf2, bxx);
+                    const float2 Y = __ffma2_rn(pr.D2, yf2, bxy);
                     const float2 rw = make_float2(rcp_approx(w.x), rcp_approx(w.y));
-                    const float2 mx = __fmul2_rn(X, rw), my = __fmul2_rn(Y, rw);
-                    const float2 tx2 = __fadd2_rd(mx, magic2), ty2 = __fadd2_rd(my, magic2);
-                    const float2 fx2 = __fadd2_rn(tx2, nmagic2), fy2 = __fadd2_rn(ty2, nmagic2);
-                    const float2 ax2 = __ffma2_rn(fx2, minus1, mx), ay2 = __ffma2_rn(fy2, minus1, my);
-                    const float2 qi = __ffma2_rn(fy2, qpitch2, tx2);
+                    // floor of X / w from the unrounded product, its negative, fraction, quad index (as in
+                    // the ZNCC span kernel)
+                    const float2 tx2 = __ffma2_rd(X, rw, magic2), ty2 = __ffma2_rd(Y, rw, magic2);
+                    const float2 nfx2 = __ffma2_rn(tx2, minus1, magic2), nfy2 = __ffma2_rn(ty2, minus1, magic2);
+                    const float2 ax2 = __ffma2_rn(X, rw, nfx2), ay2 = __ffma2_rn(Y, rw, nfy2);
+                    const float2 qi = __ffma2_rn(nfy2, qpitch2, tx2);
                     uint32_t q0b = __float_as_uint(qi.x), q1b = __float_as_uint(qi.y);
                     if constexpr (EDGE) {
                         q0b = in0[k] ? q0b : (uint32_t)kMagicBits;
@@ -287,30 +296,36 @@ __device__ __forceinline__ void run_span_mi_task(const SearchParams &p, uint32_t
                     }
                     const float4 q0 = __ldg(reinterpret_cast<const float4 *>(mqbase + 16ull * q0b));
                     const float4 q1 = __ldg(reinterpret_cast<const float4 *>(mqbase + 16ull * q1b));
-                    // values: quad = {c00, c10, c01, c11}, m = (c00 + ax c10) + ay (c01 + ax c11)
+                    // values in bins: quad = {c00, c10, c01, c11} B / 256, t = (c00 + ax c10) + ay (c01 + ax c11)
                     const float v0 = fmaf(ay2.x, fmaf(ax2.x, q0.w, q0.z), fmaf(ax2.x, q0.y, q0.x));
                     const float v1 = fmaf(ay2.y, fmaf(ax2.y, q1.w, q1.z), fmaf(ax2.y, q1.y, q1.x));
-                    const float2 t = __fmul2_rn(make_float2(v0, v1), make_float2(sB, sB));
-                    const float2 tb = __fadd2_rd(t, magic2);  // floor(t) in the mantissa (|t| < 2^22)
-                    const float2 fr = __ffma2_rn(__fadd2_rn(tb, nmagic2), minus1, t);
+                    // clamped to [0.5, B - 0.5]: the bins at the ends take everything beyond, and their outer
+                    // edges, where the bin is clamped, are no edges for the guard
+                    const float2 t = make_float2(fminf(fmaxf(v0, 0.5f), Bh), fminf(fmaxf(v1, 0.5f), Bh));
+                    const float2 tb = __ffma2_rd(t, one2, magic2);  // the bin, in the mantissa
+                    const float2 dfr = __fadd2_rn(__ffma2_rn(t, one2, __ffma2_rn(tb, minus1, magic2)), mhalf2);
                     // bin-edge guard: the sample's distance to the nearer edge against the bound
                     const float s0 = fmaf(2.0f, fabsf(q0.w), fmaf(3.0f, fabsf(q0.y), fabsf(q0.z)));
                     const float s1 = fmaf(2.0f, fabsf(q1.w), fmaf(3.0f, fabsf(q1.y), fabsf(q1.z)));
-                    float2 gb = __ffma2_rn(make_float2(s0, s1), sg2, make_float2(gv0, gv0));
-                    const float2 dfr = __fadd2_rn(fr, mhalf2);
+                    float2 gb = __ffma2_rn(make_float2(s0, s1), sg2, gv2);
                     const float2 dax = __fadd2_rn(ax2, mhalf2), day = __fadd2_rn(ay2, mhalf2);
                     // within the guard of a cell edge: the image's largest slope bounds the difference
-                    if (fmaxf(fabsf(dax.x), fabsf(day.x)) > hh2.x) gb.x = fmaxf(gb.x, gl2.x);
-                    if (fmaxf(fabsf(dax.y), fabsf(day.y)) > hh2.y) gb.y = fmaxf(gb.y, gl2.y);
-                    // an edge at 0 or B is no edge: the bin is clamped there
-                    amb0[k] = in0[k] && (fabsf(dfr.x) > 0.5f - gb.x) && (t.x > 0.5f) && (t.x < Bh);
-                    amb1[k] = in1[k] && (fabsf(dfr.y) > 0.5f - gb.y) && (t.y > 0.5f) && (t.y < Bh);
-                    const int bm0 = min(max(__float2int_rd(t.x), 0), B - 1);
-                    const int bm1 = min(max(__float2int_rd(t.y), 0), B - 1);
-                    if (in0[k] && !amb0[k]) red_shared_add1(hist_s + 4u * (uint32_t)(fb[k] + bm0));
-                    if (in1[k] && !amb1[k]) red_shared_add1(hist_s + 4u * (uint32_t)(hsize + fb[k] + bm1));
+                    gb.x = fmaxf(fabsf(dax.x), fabsf(day.x)) > hh2.x ? gl2.x : gb.x;
+                    gb.y = fmaxf(fabsf(dax.y), fabsf(day.y)) > hh2.y ? gl2.y : gb.y;
+                    // a NaN bound (a NaN tap) decides nothing
+                    amb0[k] = in0[k] && !(fabsf(dfr.x) + gb.x <= 0.5f);
+                    amb1[k] = in1[k] && !(fabsf(dfr.y) + gb.y <= 0.5f);
+                    // a sample that does not count (yet) goes to the unused cell (B, B): no branch
+                    const uint32_t hb = hbin + 4u * (uint32_t)fb[k];
+                    const uint32_t h0 = hb + 4u * __float_as_uint(tb.x), h1 = hb + hpoint + 4u * __float_as_uint(tb.y);
+                    red_shared_add1((EDGE ? in0[k] && !amb0[k] : !amb0[k]) ? h0 : hdump);
+                    red_shared_add1((EDGE ? in1[k] && !amb1[k] : !amb1[k]) ? h1 : hdump);
                 }
                 // undecided samples: queued for the exact sequence
+                bool undecided = false;
+#pragma unroll
+                for (int k = 0; k < NB; k++) undecided = undecided || amb0[k] || amb1[k];
+                if (!__any_sync(0xffffffffu, undecided)) return;
 #pragma unroll
                 for (int k = 0; k < NB; k++) {
                     const unsigned m0 = __ballot_sync(0xffffffffu, amb0[k]), m1 = __ballot_sync(0xffffffffu, amb1[k]);
@@ -318,7 +333,7 @@ __device__ __forceinline__ void run_span_mi_task(const SearchParams &p, uint32_t
                         const unsigned lt = (1u << lane) - 1u;
                         const int base = *my_qcnt;
                         const int c0 = __popc(m0);
-                        const uint32_t enc = (uint32_t)x[k] | ((uint32_t)y << 15);
+                        const uint32_t enc = (uint32_t)x | ((uint32_t)(y0 + r + k) << 15);
                         if (amb0[k]) my_queue[base + __popc(m0 & lt)] = enc;
                         if (amb1[k]) my_queue[base + c0 + __popc(m1 & lt)] = enc | (1u << 30);
                         __syncwarp();
@@ -328,25 +343,21 @@ __device__ __forceinline__ void run_span_mi_task(const SearchParams &p, uint32_t
                     }
                 }
             };
-            const int cu0 = max(0, run.ua >> 5), cu1 = min(nblocks - 1, run.ub >> 5);
-            int cf0 = cu1 + 1, cf1 = cu1;
-            if (run.ia <= run.ib) {
-                const int a = max(cu0, (run.ia + 31) >> 5), b = min(cu1, ((run.ib + 1) >> 5) - 1);
-                if (a <= b) {
-                    cf0 = a;
-                    cf1 = b;
-                }
-            }
             using One = std::integral_constant<int, 1>;
             using Two = std::integral_constant<int, 2>;
 #pragma unroll 1
-            for (int c = cu0; c < cf0; c++) column(c, std::true_type{}, One{});
-            int c = cf0;
-#pragma unroll 1
-            for (; c + 1 <= cf1; c += 2) column(c, std::false_type{}, Two{});  // two blocks in flight
-            if (c <= cf1) column(c, std::false_type{}, One{});
-#pragma unroll 1
-            for (int c2 = cf1 + 1; c2 <= cu1; c2++) column(c2, std::true_type{}, One{});
+            for (int r = 0; r < TH; r++, any >>= 1, full >>= 1) {
+                if ((full & 3u) == 3u) {  // two full rows in flight
+                    rows(r, std::false_type{}, Two{});
+                    r++;
+                    any >>= 1;
+                    full >>= 1;
+                } else if (full & 1u) {
+                    rows(r, std::false_type{}, One{});
+                } else if (any & 1u) {
+                    rows(r, std::true_type{}, One{});
+                }
+            }
         }
         drain();
     }

@@ -28,10 +28,6 @@ const void *kernel_span_zncc(int G, int NW, int TX, bool check) {
     return nullptr;
 }
 
-size_t span_kernel_smem(int G, int NW, int TH, int TX, int tiles, int cap) {
-    return span_smem_bytes(G, NW, TH, TX, tiles, cap);
-}
-
 int64_t span_max_quads() { return kSpanMaxQuads; }
 
 static int span_prep_row_blocks(int fh) { return (int)(((int64_t)fh * 32 + 255) / 256); }

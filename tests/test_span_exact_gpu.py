@@ -87,3 +87,24 @@ def test_one_sample_is_the_references_bit_for_bit(cuda, lib):
     assert np.isfinite(c32).sum() > 1000
     np.testing.assert_array_equal(c[np.isfinite(c32)].view(np.uint32), c32[np.isfinite(c32)].view(np.uint32))
     np.testing.assert_array_equal(np.isfinite(c), np.isfinite(c32))
+
+
+@pytest.mark.parametrize("h,w,mh,mw", [(17, 65, 19, 61), (16, 64, 16, 64), (31, 129, 33, 140)])
+@pytest.mark.parametrize("bins", [8, 32])
+def test_three_channel_mi_is_the_per_sample_kernels(cuda, lib, h, w, mh, mw, bins):
+    """Equal counts and the same cost function: the same bits, at the edges of blocks and bands."""
+    pair = _pair(700 + w, "MI", h, w, mh, mw, 3, u8=True)
+    _, c = _run(cuda, pair, "MI", mi_bins=bins)
+    _, c0 = _run(cuda, pair, "MI", mi_bins=bins, per_sample_decisions=True)
+    np.testing.assert_array_equal(c.view(np.uint32), c0.view(np.uint32))
+
+
+@pytest.mark.parametrize("h,w", [(15, 31), (17, 33), (33, 257), (2, 64)])
+def test_one_channel_mi_is_the_per_sample_kernels(cuda, lib, h, w):
+    """The guarded fast samples at the same edges, with values beyond both ends of the bins."""
+    pair = _pair(800 + w, "MI", h, w, h + 3, w - 2, 1)
+    pair.moving = pair.moving * 1.5 - 40.0
+    with _env(CGS_SPAN_CHECK=1):
+        _, c = _run(cuda, pair, "MI")
+    _, c0 = _run(cuda, pair, "MI", per_sample_decisions=True)
+    np.testing.assert_array_equal(c.view(np.uint32), c0.view(np.uint32))
