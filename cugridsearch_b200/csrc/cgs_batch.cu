@@ -572,6 +572,7 @@ cgs_status cgs_batch_create(const cgs_pair *pairs, int32_t n, const cgs_batch_pl
             double2 *prefix =
                 span_uses_prefix(cost) ? reinterpret_cast<double2 *>(b->mem + pd.prefix_off) : nullptr;
             p.fix_prefix = prefix;
+            p.splits = 1;
             p.tile_h = pd.zp.TH;
             p.tiles_x = pd.zp.tiles_x;
             p.tiles_y = pd.zp.tiles_y;

@@ -49,6 +49,8 @@ struct PrepParams {
     int32_t quad_form;   // 0: {P00, P10, P01 - P00, P11 - P10}; 1 (ZNCC and one-channel MI span kernels): {P00, P01 - P00,
                          // P10 - P00, (P11 - P10) - (P01 - P00)}; 2 (exact span kernel): {P00, P01, P10, P11};
                          // P(dy, dx) the tap at (y + dy, x + dx)
+    unsigned int *zero_dst;  // zeroed words (the span kernels' counts of done parts), or null
+    int64_t zero_n;
     float quad_scale;    // form 1: a power of two on the quads (one-channel MI: bins / 256), or 0 (none)
     int32_t *bin_dst;    // the fixed image's bins times 4 (bins + 1) (the histogram row's byte offset), laid
                          // out as the fixed planes, or null

@@ -72,6 +72,12 @@ struct SearchParams {
     // (the tile's fixed rows, then its window), window row pitch modulo 8
     int32_t tile_h, tiles_x, tiles_y, win_cap, win_pitch_mod;
     const double2 *fix_prefix;    // span kernel: FP64 {sum f, sum f^2} prefix sums of each fixed row, W + 1 per row
+    // span kernels with windows: a task's bands of rows split over `splits` CTAs (1: whole tasks), the bands'
+    // FP64 totals [task][band][point][5], the parts' counts [task][part][point], the parts done [task]
+    int32_t splits;
+    double *split_tot;
+    int *split_cnt;
+    unsigned int *split_done;
     const float *span_rows;       // span kernels, MI: the fixed bins (int32, laid out as the fixed planes) times the
                                   // histogram's row stride: B + 1 counts (one channel), in bytes (PrepParams::bin_dst)
     const float *span_rows_header;  // one-channel MI: the quads' largest slope bound (written by its staging step)

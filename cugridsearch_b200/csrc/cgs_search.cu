@@ -257,6 +257,7 @@ __device__ __forceinline__ void prep_body(const PrepParams &q, int64_t tid, int6
             }
         }
     }
+    for (int64_t i = tid; i < q.zero_n; i += nthr) q.zero_dst[i] = 0u;
     if (q.row_table && tid == 0) {
         // calcMIAlt's rows: row = -0.5; while (row < 0.5) row += 1 / (float)(rowsf - 1)
         // (cudaErrorFunction_mi.cuh:164), the same float additions as the reference
@@ -753,6 +754,22 @@ bool span_plan(const cgs_image &mov, const cgs_image &fix, const cgs_options &o,
     return sp->smem <= budget;
 }
 
+// Parts that a windowed span search's tasks are split into (see the span kernel): the number, at most one
+// per band and 16, with the least waves x (sweep share + setup), a part's setup (decode, windows, the
+// first copies) being about 12 K cycles and a task's sweep 8 (ZNCC) or 15 cycles per 32 evaluations.
+// Whole tasks unless that saves 3 %, or where the bands' totals would take over 64 MB.
+static int span_splits(const SpanPlan &sp, int cost, uint32_t tasks, const cgs_image &fix, int sms) {
+    const double points = (double)sp.G * sp.NW;
+    if (cost == CGS_COST_MI || (double)tasks * sp.tiles_y * points * 40.0 > 64e6) return 1;
+    const double sweep = (double)fix.width * fix.height * fix.channels * points / 32.0 * (cost == CGS_COST_ZNCC ? 8.0 : 15.0);
+    const double setup = 12000.0 / sweep;
+    auto waves = [&](int k) { return (double)(((uint64_t)tasks * k + sms - 1) / sms) * (1.0 / k + setup); };
+    int best = 1;
+    for (int k = 2; k <= std::min(sp.tiles_y, 16); k++)
+        if (waves(k) < 0.97 * waves(1) && waves(k) < waves(best)) best = k;
+    return best;
+}
+
 // Launch plan of the MI span kernel: 16 warps of 2 points, bands of TH = 16 rows (CGS_SPAN_TH
 // = 8 | 16 | 32), self-checking with CGS_SPAN_CHECK=1.  False where it does not apply: several
 // channels, more than 32 bins (the histograms of 32 points must fit shared memory), images of
@@ -1046,7 +1063,17 @@ static cgs_status search_core(const cgs_image *mov, const cgs_image *fix, const 
     const size_t prefix_bytes = mi_rows                          ? (size_t)C * (size_t)st.fplane * sizeof(int32_t)
                                 : span && span_uses_prefix(cost) ? (size_t)fix->height * (size_t)(fix->width + 1) * sizeof(double2)
                                                                  : 0;
-    const size_t main_bytes = st.bytes + (prefix_bytes ? prefix_bytes + 256 : 0);
+    const uint32_t per_task = spans ? (uint32_t)(sp.NW * sp.G) : (uint32_t)(pl.NW * pl.G);
+    p.num_tasks = (p.n + per_task - 1) / per_task;
+    // split tasks: the bands' totals, the parts' counts, the parts done
+    p.splits = span ? span_splits(sp, cost, p.num_tasks, *fix, di.sms) : 1;
+    const size_t tot_off = (size_t)round_up((int64_t)(prefix_off + prefix_bytes), 256);
+    const size_t tot_bytes = (size_t)p.num_tasks * sp.tiles_y * per_task * 5 * sizeof(double);
+    const size_t cnt_bytes = (size_t)round_up((int64_t)p.num_tasks * p.splits * per_task * (int64_t)sizeof(int), 256);
+    const size_t split_bytes = p.splits > 1 ? tot_bytes + cnt_bytes + (size_t)p.num_tasks * sizeof(unsigned int) : 0;
+    const size_t main_bytes = split_bytes      ? tot_off + split_bytes + (size_t)di.tex_align + 256
+                              : prefix_bytes ? st.bytes + prefix_bytes + 256
+                                             : st.bytes;
     const bool verify = !(o.flags & CGS_FLAG_NO_VERIFY) && verify_supported(cost);
     const size_t vbytes = verify ? verify_scratch_bytes() + (costs ? 0 : (size_t)p.n * 4) : 0;
     const size_t ext_bytes = (size_t)round_up((int64_t)main_bytes, 256) + vbytes;
@@ -1108,6 +1135,13 @@ static cgs_status search_core(const cgs_image *mov, const cgs_image *fix, const 
         q.quad_form = spans ? span_quad_form(cost, C) : 0;
         if (span_mi) q.quad_scale = (float)mi_bins * (1.0f / 256.0f);
     }
+    if (split_bytes) {
+        p.split_tot = reinterpret_cast<double *>(sb + tot_off);
+        p.split_cnt = reinterpret_cast<int *>(sb + tot_off + tot_bytes);
+        p.split_done = reinterpret_cast<unsigned int *>(sb + tot_off + tot_bytes + cnt_bytes);
+        q.zero_dst = p.split_done;
+        q.zero_n = p.num_tasks;
+    }
     if (mi_rows && !span_mi) {
         q.bin_dst = reinterpret_cast<int32_t *>(sb + prefix_off);
         q.bins = mi_bins;
@@ -1139,8 +1173,6 @@ static cgs_status search_core(const cgs_image *mov, const cgs_image *fix, const 
     }
 
     const int threads = (spans ? sp.NW : pl.NW) * 32;
-    const uint32_t per_task = spans ? (uint32_t)(sp.NW * sp.G) : (uint32_t)(pl.NW * pl.G);
-    p.num_tasks = (p.n + per_task - 1) / per_task;
     e = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e == cudaSuccess && !spans)
         e = cudaFuncSetAttribute(kfn, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxL1);
@@ -1152,7 +1184,7 @@ static cgs_status search_core(const cgs_image *mov, const cgs_image *fix, const 
         return e != cudaSuccess ? cuda_fail(e, "search kernel setup")
                                 : fail(CGS_ERROR_UNSUPPORTED, "search kernel does not fit on an SM");
     }
-    const uint32_t blocks = std::min<uint32_t>(p.num_tasks, (uint32_t)(di.sms * per_sm));
+    const uint32_t blocks = std::min<uint32_t>(p.num_tasks * (uint32_t)p.splits, (uint32_t)(di.sms * per_sm));
     void *args[] = {&p};
     if (spans) {  // these read tap quads, no texture
         p.mov_tex = 0;

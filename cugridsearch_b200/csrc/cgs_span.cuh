@@ -110,7 +110,7 @@ __host__ __device__ constexpr size_t span_head_bytes(int NW) { return 256 + 8 * 
 __host__ __device__ constexpr size_t span_smem_bytes(int G, int NW, int TH, int TX, int tiles, int cap) {
     return span_head_bytes(NW) + (size_t)NW * G * sizeof(SpanSlot) + (size_t)NW * (G / 2) * sizeof(PairRow) +
            (size_t)tiles * TX * sizeof(BlockWin) + (size_t)NW * G * TH * sizeof(InnerSpan) +
-           (size_t)NW * TH * sizeof(RowRun) + (size_t)NW * G * (5 * sizeof(double) + sizeof(int)) +
+           (size_t)NW * TH * sizeof(RowRun) + (size_t)NW * G * (10 * sizeof(double) + sizeof(int)) +
            (size_t)kWinStages * cap * 16 + 144;
 }
 
@@ -125,6 +125,7 @@ struct SpanSmem {
     InnerSpan *spans;  // [NW][G][TH]
     RowRun *runs;      // [NW][TH]
     double *dtot;      // [NW][G * 5] FP64 task totals {sum f, sum m', sum f^2, sum m'^2, sum f'm'}
+    double *dband;     // [NW][G * 5] the same sums of the current band
     int *cnt;          // [NW][G] overlap counts of the warps' points
     float4 *win;       // [kWinStages][cap]
     int cap;
@@ -153,6 +154,8 @@ __device__ __forceinline__ SpanSmem carve_span(unsigned char *smem, int TH, int 
     s.runs = reinterpret_cast<RowRun *>(q);
     q += (size_t)NW * TH * sizeof(RowRun);
     s.dtot = reinterpret_cast<double *>(q);
+    q += (size_t)NW * G * 5 * sizeof(double);
+    s.dband = reinterpret_cast<double *>(q);
     q += (size_t)NW * G * 5 * sizeof(double);
     s.cnt = reinterpret_cast<int *>(q);
     q += (size_t)NW * G * sizeof(int);
@@ -358,18 +361,18 @@ __device__ __forceinline__ void span_points(const SearchParams &p, uint32_t ord0
                            kc.S, kc.T, kc.U, gx, gy, ok ? 1 : 0, gvalid ? 1 : 0, gidx};
 }
 
-// The windows of every block of every tile, into ss.wins: warp w takes blocks w, w + NW, .. with the
+// The windows of every block of tiles t0 .. t1 - 1, into ss.wins: warp w takes blocks w, w + NW, .. with the
 // task's points over its lanes, then one thread per tile lays its blocks out in the stage (C planes of
 // quads each, pitch x h apart).
 template <int C, int G, int NW, int TX>
-__device__ __forceinline__ void span_windows(const SearchParams &p, const SpanSmem &ss) {
+__device__ __forceinline__ void span_windows(const SearchParams &p, const SpanSmem &ss, int t0, int t1) {
     constexpr int TW = 32 * TX;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int fw = p.fix.w, fh = p.fix.h, TH = p.tile_h, tiles_x = p.tiles_x, ntiles = p.tiles_x * p.tiles_y;
+    const int fw = p.fix.w, fh = p.fix.h, TH = p.tile_h, tiles_x = p.tiles_x;
     const float mov_wf = p.mov_wf, mov_hf = p.mov_hf;
     constexpr int P = NW * G;
     const float inf = __int_as_float(0x7f800000);
-    for (int i = warp; i < ntiles * TX; i += NW) {
+    for (int i = t0 * TX + warp; i < t1 * TX; i += NW) {
         const int t = i / TX, c = i - t * TX;
         const int xc = (t % tiles_x) * TW + 32 * c, y0 = (t / tiles_x) * TH;
         float4 e = make_float4(inf, inf, -inf, -inf);
@@ -391,7 +394,7 @@ __device__ __forceinline__ void span_windows(const SearchParams &p, const SpanSm
     }
     __syncthreads();
     const int wcap = ss.cap - C * TH * TW / 4;  // quads of a stage after the fixed rows
-    for (int t = threadIdx.x; t < ntiles; t += NW * 32) {
+    for (int t = t0 + threadIdx.x; t < t1; t += NW * 32) {
         int used = 0;
 #pragma unroll 1
         for (int c = 0; c < TX; c++) {
@@ -429,11 +432,75 @@ __device__ __forceinline__ void span_windows(const SearchParams &p, const SpanSm
     }
 }
 
-// One task of the span path (ZNCC, one channel, quads staged): the G grid points of each warp
-// over every tile of the fixed image.  `wit` counts window stages used by this CTA (their
+// Split tasks.  With fewer tasks than a few per SM the last wave leaves SMs idle (324 tasks on 148 SMs
+// take three waves for the work of 2.2), so the host splits every task's bands of rows into `splits`
+// parts, one per CTA at a time (span_splits).  The totals of each band go to global memory, and the CTA
+// that completes a task's parts adds them in band order: the sums, and their order, are those of an
+// unsplit task.
+
+// The band's sums of a warp's points (my_band, cleared) into the task totals, or to global memory.
+template <int G, int NW>
+__device__ __forceinline__ void fold_band(const SearchParams &p, uint32_t task, int band, double *my_dtot, double *my_band) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    __syncwarp();
+    for (int i = lane; i < G * 5; i += 32) {
+        const double v = my_band[i];
+        my_band[i] = 0.0;
+        if (p.splits > 1) p.split_tot[(((size_t)task * p.tiles_y + band) * NW + warp) * (G * 5) + i] = v;
+        else my_dtot[i] += v;
+    }
+    __syncwarp();
+}
+
+// After a part's bands: whether this CTA completed the task, whose totals and counts it then holds.
+template <int G, int NW>
+__device__ __forceinline__ bool join_parts(const SearchParams &p, uint32_t task, int part, const SpanSmem &ss, double *my_dtot,
+                                           int *my_cnt) {
+    if (p.splits <= 1) return true;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    int *cnt = p.split_cnt + (size_t)task * p.splits * (NW * G) + warp * G;
+    if (lane < G) cnt[part * (NW * G) + lane] = my_cnt[lane];
+    __threadfence();
+    __syncthreads();
+    volatile int &s_last = *(ss.bounds_flag + 2);
+    if (threadIdx.x == 0) s_last = atomicAdd(p.split_done + task, 1u) + 1u == (unsigned)p.splits;
+    __syncthreads();
+    if (!s_last) return false;
+    __threadfence();
+    for (int i = lane; i < G * 5; i += 32) {
+        const double *t = p.split_tot + ((size_t)task * p.tiles_y * NW + warp) * (G * 5) + i;
+        double d = 0.0;
+        for (int b = 0; b < p.tiles_y; b++) d += __ldcg(t + (size_t)b * (NW * G * 5));
+        my_dtot[i] = d;
+    }
+    if (lane < G) {
+        int n = 0;
+        for (int k = 0; k < p.splits; k++) n += __ldcg(cnt + k * (NW * G) + lane);
+        my_cnt[lane] = n;
+    }
+    __syncwarp();
+    return true;
+}
+
+// Thread 0 of a CTA that stops: the parts it will not run count as done, and a task whose parts are all
+// done is retired with the timeout status.
+__device__ __forceinline__ void retire_parts(const SearchParams &p, uint32_t unit, uint32_t step, uint32_t units) {
+    for (uint32_t u = unit; u < units; u += step) {
+        if (p.splits <= 1) {
+            retire_tasks(p, ~0ull, 1u, true);
+            continue;
+        }
+        atomicOr(p.status, (unsigned)CGS_ERROR_DEVICE_TIMEOUT);
+        __threadfence();
+        if (atomicAdd(p.split_done + u / p.splits, 1u) + 1u == (unsigned)p.splits) retire_tasks(p, ~0ull, 1u, true);
+    }
+}
+
+// One task, or part of a task, of the span path (ZNCC, one channel, quads staged): the G grid points of
+// each warp over the part's tiles of the fixed image.  `wit` counts window stages used by this CTA (their
 // barrier phases).  Returns false if a bounded wait gave up.
 template <int G, int NW, int TX, bool CHECK>
-__device__ __forceinline__ bool run_span_task(const SearchParams &p, uint32_t task, const SpanSmem &ss,
+__device__ __forceinline__ bool run_span_task(const SearchParams &p, uint32_t unit, const SpanSmem &ss,
                                               uint32_t &wit) {
     static_assert(G % 2 == 0, "the span path pairs grid points");
     constexpr int GP = G / 2;
@@ -441,7 +508,10 @@ __device__ __forceinline__ bool run_span_task(const SearchParams &p, uint32_t ta
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int fw = p.fix.w, fh = p.fix.h;
     const int TH = p.tile_h;
-    const int tiles_x = p.tiles_x, ntiles = p.tiles_x * p.tiles_y;
+    const int tiles_x = p.tiles_x;
+    const uint32_t task = unit / (uint32_t)p.splits;
+    const int part = (int)(unit - task * (uint32_t)p.splits);
+    const int t0 = part * p.tiles_y / p.splits * tiles_x, t1 = (part + 1) * p.tiles_y / p.splits * tiles_x;  // its tiles
     const float mov_wf = p.mov_wf, mov_hf = p.mov_hf;
     const float *__restrict__ mdata = p.mov.data;
     const int mpitch = p.mov.pitch;
@@ -468,25 +538,26 @@ __device__ __forceinline__ bool run_span_task(const SearchParams &p, uint32_t ta
     // FP64 task totals and overlap counts of the warp's points (shared memory)
     double *my_dtot = ss.dtot + warp * G * 5;
     int *my_cnt = ss.cnt + warp * G;
-    for (int i = lane; i < G * 5; i += 32) my_dtot[i] = 0.0;
+    double *my_band = ss.dband + warp * G * 5;
+    for (int i = lane; i < G * 5; i += 32) my_dtot[i] = my_band[i] = 0.0;
     if (lane < G) my_cnt[lane] = 0;
     const float fshift = p.shifts[0], mshift = p.shifts[1];
     __syncthreads();  // every point's slot is written
 
-    span_windows<1, G, NW, TX>(p, ss);
+    span_windows<1, G, NW, TX>(p, ss, t0, t1);
     __syncthreads();
     if (threadIdx.x == 0)
-        for (int t = 0; t < kWinStages && t < ntiles; t++) expect_window<1, TX>(p, ss, t, (int)((wit + t) % kWinStages));
+        for (int t = 0; t < kWinStages && t0 + t < t1; t++) expect_window<1, TX>(p, ss, t0 + t, (int)((wit + t) % kWinStages));
     __syncthreads();
-    for (int t = 0; t < kWinStages && t < ntiles; t++)
-        issue_window<1, NW, TX>(p, ss, p.fix.data, t, (int)((wit + t) % kWinStages));
+    for (int t = 0; t < kWinStages && t0 + t < t1; t++)
+        issue_window<1, NW, TX>(p, ss, p.fix.data, t0 + t, (int)((wit + t) % kWinStages));
 
     // ---- sweep
-    float2 part[GP][3];  // {sum m', sum m'^2, sum f'm'} of each pair of points
+    float2 part_sum[GP][3];  // {sum m', sum m'^2, sum f'm'} of each pair of points
 #pragma unroll
     for (int h = 0; h < GP; h++)
 #pragma unroll
-        for (int j = 0; j < 3; j++) part[h][j] = make_float2(0.0f, 0.0f);
+        for (int j = 0; j < 3; j++) part_sum[h][j] = make_float2(0.0f, 0.0f);
     InnerSpan *my_spans = ss.spans + warp * G * TH;
     RowRun *my_runs = ss.runs + warp * TH;
     const float2 magic2 = make_float2(kMagic, kMagic), minus1 = make_float2(-1.0f, -1.0f);
@@ -495,7 +566,7 @@ __device__ __forceinline__ bool run_span_task(const SearchParams &p, uint32_t ta
     const uint64_t mqbase = reinterpret_cast<uint64_t>(p.mov_quad) - 16ull * (uint64_t)(uint32_t)kMagicBits;
     const float2 qpitch2 = make_float2(-(float)p.quad_pitch, -(float)p.quad_pitch);
 
-    for (int t = 0; t < ntiles; t++, wit++) {
+    for (int t = t0; t < t1; t++, wit++) {
         const int tx = t % tiles_x, ty = t / tiles_x;
         const int x0 = tx * TW, y0 = ty * TH;
         const int x1 = min(x0 + TW, fw) - 1;
@@ -567,7 +638,7 @@ __device__ __forceinline__ bool run_span_task(const SearchParams &p, uint32_t ta
                         sfm += __shfl_xor_sync(0xffffffffu, sfm, o);
                     }
                 if (act && r == 0) {
-                    double *d = my_dtot + g * 5;
+                    double *d = my_band + g * 5;
                     d[0] += s1;
                     d[2] += s2;
                     if (found) {
@@ -718,9 +789,9 @@ __device__ __forceinline__ bool run_span_task(const SearchParams &p, uint32_t ta
                         ms = make_float2(in0 ? ms.x : 0.0f, in1 ? ms.y : 0.0f);
                         fm = make_float2(in0 ? fs : 0.0f, in1 ? fs : 0.0f);
                     }
-                    part[h][0] = __fadd2_rn(part[h][0], ms);
-                    part[h][1] = __ffma2_rn(ms, ms, part[h][1]);
-                    part[h][2] = __ffma2_rn(fm, ms, part[h][2]);
+                    part_sum[h][0] = __fadd2_rn(part_sum[h][0], ms);
+                    part_sum[h][1] = __ffma2_rn(ms, ms, part_sum[h][1]);
+                    part_sum[h][2] = __ffma2_rn(fm, ms, part_sum[h][2]);
                 }
             };
             auto block = [&](int c, auto edge_tag) {
@@ -772,15 +843,16 @@ __device__ __forceinline__ bool run_span_task(const SearchParams &p, uint32_t ta
 #pragma unroll
                 for (int j = 0; j < 3; j++) {
                     const int slot = j == 0 ? 1 : (j == 1 ? 3 : 4);  // sum m', sum m'^2, sum f'm'
-                    const float s0 = warp_sum(part[h][j].x), s1 = warp_sum(part[h][j].y);
+                    const float s0 = warp_sum(part_sum[h][j].x), s1 = warp_sum(part_sum[h][j].y);
                     if (lane == 0) {
-                        my_dtot[(2 * h) * 5 + slot] += (double)s0;
-                        my_dtot[(2 * h + 1) * 5 + slot] += (double)s1;
+                        my_band[(2 * h) * 5 + slot] += (double)s0;
+                        my_band[(2 * h + 1) * 5 + slot] += (double)s1;
                     }
-                    part[h][j] = make_float2(0.0f, 0.0f);
+                    part_sum[h][j] = make_float2(0.0f, 0.0f);
                 }
+            fold_band<G, NW>(p, task, ty, my_dtot, my_band);
         }
-        const bool more = t + kWinStages < ntiles;
+        const bool more = t + kWinStages < t1;
         if (threadIdx.x == 0 && more) expect_window<1, TX>(p, ss, t + kWinStages, st);
         __syncthreads();  // every warp is done with this stage
         if (*ss.abort_flag) {
@@ -788,13 +860,15 @@ __device__ __forceinline__ bool run_span_task(const SearchParams &p, uint32_t ta
             // within the same bound, before the CTA stops
             if (threadIdx.x == 0) {
                 mbar_wait_bounded(&ss.bars[st], (wit / kWinStages) & 1u, kWaitLimitNs);
-                if (kWinStages > 1 && t + 1 < ntiles)
+                if (kWinStages > 1 && t + 1 < t1)
                     mbar_wait_bounded(&ss.bars[(wit + 1) % kWinStages], ((wit + 1) / kWinStages) & 1u, kWaitLimitNs);
             }
             return false;
         }
         if (more) issue_window<1, NW, TX>(p, ss, p.fix.data, t + kWinStages, st);
     }
+
+    if (!join_parts<G, NW>(p, task, part, ss, my_dtot, my_cnt)) return true;
 
     // ---- per grid point: finalise, dump, argmin key (as the pixel-loop kernel)
     __syncwarp();
@@ -829,7 +903,7 @@ __device__ __forceinline__ bool run_span_task(const SearchParams &p, uint32_t ta
     return true;
 }
 
-// The single-pair span kernel: persistent CTAs, tasks dealt round-robin.
+// The single-pair span kernel: persistent CTAs, tasks (or their parts) dealt round-robin.
 template <int G, int NW, int TX, bool CHECK>
 __global__ void __launch_bounds__(NW * 32, 1) span_kernel(const __grid_constant__ SearchParams p) {
     extern __shared__ __align__(128) unsigned char smem[];
@@ -841,12 +915,11 @@ __global__ void __launch_bounds__(NW * 32, 1) span_kernel(const __grid_constant_
         *ss.bounds_flag = 0;
     }
     __syncthreads();
-    const uint32_t my_tasks =
-        (p.num_tasks > blockIdx.x) ? (p.num_tasks - blockIdx.x + gridDim.x - 1) / gridDim.x : 0u;
+    const uint32_t units = p.num_tasks * (uint32_t)p.splits;
     uint32_t wit = 0;
-    for (uint32_t k = 0; k < my_tasks; k++) {
-        if (!run_span_task<G, NW, TX, CHECK>(p, blockIdx.x + k * gridDim.x, ss, wit)) {
-            if (threadIdx.x == 0) retire_tasks(p, ~0ull, my_tasks - k, true);
+    for (uint32_t u = blockIdx.x; u < units; u += gridDim.x) {
+        if (!run_span_task<G, NW, TX, CHECK>(p, u, ss, wit)) {
+            if (threadIdx.x == 0) retire_parts(p, u, gridDim.x, units);
             return;
         }
     }

@@ -76,7 +76,7 @@ __device__ __forceinline__ void accumulate64(double *a, float f, float m) {
 }
 
 template <int COST, int C, int G, int NW, int TX, bool CHECK>
-__device__ __forceinline__ bool run_span_exact_task(const SearchParams &p, uint32_t task, const SpanSmem &ss,
+__device__ __forceinline__ bool run_span_exact_task(const SearchParams &p, uint32_t unit, const SpanSmem &ss,
                                                     uint32_t &wit) {
     static_assert(G % 2 == 0, "the span path pairs grid points");
     constexpr int GP = G / 2;
@@ -88,7 +88,10 @@ __device__ __forceinline__ bool run_span_exact_task(const SearchParams &p, uint3
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int fw = p.fix.w, fh = p.fix.h;
     const int TH = p.tile_h;
-    const int tiles_x = p.tiles_x, ntiles = p.tiles_x * p.tiles_y;
+    const int tiles_x = p.tiles_x;
+    const uint32_t task = unit / (uint32_t)p.splits;
+    const int part = (int)(unit - task * (uint32_t)p.splits);
+    const int t0 = part * p.tiles_y / p.splits * tiles_x, t1 = (part + 1) * p.tiles_y / p.splits * tiles_x;  // its tiles
     const float mov_wf = p.mov_wf, mov_hf = p.mov_hf;
     const int B = p.mi_bins, hstride = B + 1, hsize = hstride * hstride;
     // the samples' scale (a power of two)
@@ -115,24 +118,26 @@ __device__ __forceinline__ bool run_span_exact_task(const SearchParams &p, uint3
     float2 *my_rows = ss.rowtab + (size_t)warp * TH * GP * 3;  // [TH][GP]{B y, -C2 y, -D2 y}
     uint32_t *my_hist = ss.hist + (size_t)warp * G * hsize;
     double *my_dtot = ss.dtot + warp * G * 5;  // {sum f^2, the sweep's NS sums} per point, stride 5
+    double *my_band = ss.dband + warp * G * 5;  // of the current band
     int *my_cnt = ss.cnt + warp * G;
     if constexpr (kMI) {
         for (int i = lane; i < G * hsize; i += 32) my_hist[i] = 0u;
     } else {
-        for (int i = lane; i < G * 5; i += 32) my_dtot[i] = 0.0;
+        for (int i = lane; i < G * 5; i += 32) my_dtot[i] = my_band[i] = 0.0;
     }
     if (lane < G) my_cnt[lane] = 0;
     __syncthreads();  // every point's slot is written
 
     // the tile's fixed rows: the staged image, or MI's plane of bins
     const float *fsrc = kMI ? p.span_rows : p.fix.data;
-    span_windows<C, G, NW, TX>(p, ss);
+    span_windows<C, G, NW, TX>(p, ss, t0, t1);
     __syncthreads();
     if (threadIdx.x == 0)
-        for (int t = 0; t < kWinStages && t < ntiles; t++) expect_window<C, TX>(p, ss, t, (int)((wit + t) % kWinStages));
+        for (int t = 0; t < kWinStages && t0 + t < t1; t++)
+            expect_window<C, TX>(p, ss, t0 + t, (int)((wit + t) % kWinStages));
     __syncthreads();
-    for (int t = 0; t < kWinStages && t < ntiles; t++)
-        issue_window<C, NW, TX>(p, ss, fsrc, t, (int)((wit + t) % kWinStages));
+    for (int t = 0; t < kWinStages && t0 + t < t1; t++)
+        issue_window<C, NW, TX>(p, ss, fsrc, t0 + t, (int)((wit + t) % kWinStages));
 
     // one sample of point g at (x, y) by the reference's sequence, into a (and f^2 into s2) or the
     // histogram if inside
@@ -165,7 +170,7 @@ __device__ __forceinline__ bool run_span_exact_task(const SearchParams &p, uint3
 #pragma unroll
                 for (int j = 0; j < NS; j++) a[j] += __shfl_xor_sync(0xffffffffu, a[j], o);
         if (leader) {
-            double *d = my_dtot + g * 5;
+            double *d = my_band + g * 5;
             if constexpr (kFix) d[0] += s2;
             if (!kMI && moving)
 #pragma unroll
@@ -188,11 +193,11 @@ __device__ __forceinline__ bool run_span_exact_task(const SearchParams &p, uint3
     };
 
     // ---- sweep
-    float2 part[GP][NS];
+    float2 acc[GP][NS];
 #pragma unroll
     for (int h = 0; h < GP; h++)
 #pragma unroll
-        for (int j = 0; j < NS; j++) part[h][j] = make_float2(0.0f, 0.0f);
+        for (int j = 0; j < NS; j++) acc[h][j] = make_float2(0.0f, 0.0f);
     InnerSpan *my_spans = ss.spans + warp * G * TH;
     RowRun *my_runs = ss.runs + warp * TH;
     const float2 magic2 = make_float2(kMagic, kMagic), minus1 = make_float2(-1.0f, -1.0f);
@@ -210,7 +215,7 @@ __device__ __forceinline__ bool run_span_exact_task(const SearchParams &p, uint3
     const uint32_t hbase = smem_addr(my_hist) - 4u * (uint32_t)kMagicBits, hpoint = 4u * (uint32_t)hsize;
     const float bin_max = (float)(B - 1);
 
-    for (int t = 0; t < ntiles; t++, wit++) {
+    for (int t = t0; t < t1; t++, wit++) {
         const int tx = t % tiles_x, ty = t / tiles_x;
         const int x0 = tx * TW, y0 = ty * TH;
         const int x1 = min(x0 + TW, fw) - 1;
@@ -421,15 +426,15 @@ __device__ __forceinline__ bool run_span_exact_task(const SearchParams &p, uint3
                             }
                             if constexpr (COST == CGS_COST_SAD_AVG) {
                                 const float2 d = __ffma2_rn(fm, minus1, m);
-                                part[h][0].x += fabsf(d.x);
-                                part[h][0].y += fabsf(d.y);
+                                acc[h][0].x += fabsf(d.x);
+                                acc[h][0].y += fabsf(d.y);
                             } else if constexpr (COST == CGS_COST_SQD_REF) {
                                 const float2 d = __ffma2_rn(fm, minus1, m);
-                                part[h][0] = __ffma2_rn(d, d, part[h][0]);
-                                part[h][1] = __ffma2_rn(m, m, part[h][1]);
+                                acc[h][0] = __ffma2_rn(d, d, acc[h][0]);
+                                acc[h][1] = __ffma2_rn(m, m, acc[h][1]);
                             } else {
-                                part[h][0] = __ffma2_rn(m, m, part[h][0]);
-                                part[h][1] = __ffma2_rn(fm, m, part[h][1]);
+                                acc[h][0] = __ffma2_rn(m, m, acc[h][0]);
+                                acc[h][1] = __ffma2_rn(fm, m, acc[h][1]);
                             }
                         }
                     }
@@ -462,15 +467,16 @@ __device__ __forceinline__ bool run_span_exact_task(const SearchParams &p, uint3
             for (int h = 0; h < GP; h++)
 #pragma unroll
                 for (int j = 0; j < NS; j++) {
-                    const float s0 = warp_sum(part[h][j].x), s1 = warp_sum(part[h][j].y);
+                    const float s0 = warp_sum(acc[h][j].x), s1 = warp_sum(acc[h][j].y);
                     if (lane == 0) {
-                        my_dtot[(2 * h) * 5 + 1 + j] += (double)s0;
-                        my_dtot[(2 * h + 1) * 5 + 1 + j] += (double)s1;
+                        my_band[(2 * h) * 5 + 1 + j] += (double)s0;
+                        my_band[(2 * h + 1) * 5 + 1 + j] += (double)s1;
                     }
-                    part[h][j] = make_float2(0.0f, 0.0f);
+                    acc[h][j] = make_float2(0.0f, 0.0f);
                 }
+            fold_band<G, NW>(p, task, ty, my_dtot, my_band);
         }
-        const bool more = t + kWinStages < ntiles;
+        const bool more = t + kWinStages < t1;
         if (threadIdx.x == 0 && more) expect_window<C, TX>(p, ss, t + kWinStages, st);
         __syncthreads();  // every warp is done with this stage
         if (*ss.abort_flag) {
@@ -479,6 +485,8 @@ __device__ __forceinline__ bool run_span_exact_task(const SearchParams &p, uint3
         }
         if (more) issue_window<C, NW, TX>(p, ss, fsrc, t + kWinStages, st);
     }
+
+    if (!kMI && !join_parts<G, NW>(p, task, part, ss, my_dtot, my_cnt)) return true;
 
     // ---- per grid point: the cost from the totals or the counts, dump, argmin key
     __syncwarp();
@@ -527,7 +535,7 @@ __device__ __forceinline__ bool run_span_exact_task(const SearchParams &p, uint3
     return true;
 }
 
-// The single-pair kernel: persistent CTAs, tasks dealt round-robin.
+// The single-pair kernel: persistent CTAs, tasks (or their parts) dealt round-robin.
 template <int COST, int C, int G, int NW, int TX, bool CHECK>
 __global__ void __launch_bounds__(NW * 32, 1) span_exact_kernel(const __grid_constant__ SearchParams p) {
     extern __shared__ __align__(128) unsigned char smem[];
@@ -540,12 +548,11 @@ __global__ void __launch_bounds__(NW * 32, 1) span_exact_kernel(const __grid_con
         *ss.bounds_flag = 0;
     }
     __syncthreads();
-    const uint32_t my_tasks =
-        (p.num_tasks > blockIdx.x) ? (p.num_tasks - blockIdx.x + gridDim.x - 1) / gridDim.x : 0u;
+    const uint32_t units = p.num_tasks * (uint32_t)p.splits;
     uint32_t wit = 0;
-    for (uint32_t k = 0; k < my_tasks; k++) {
-        if (!run_span_exact_task<COST, C, G, NW, TX, CHECK>(p, blockIdx.x + k * gridDim.x, ss, wit)) {
-            if (threadIdx.x == 0) retire_tasks(p, ~0ull, my_tasks - k, true);
+    for (uint32_t u = blockIdx.x; u < units; u += gridDim.x) {
+        if (!run_span_exact_task<COST, C, G, NW, TX, CHECK>(p, u, ss, wit)) {
+            if (threadIdx.x == 0) retire_parts(p, u, gridDim.x, units);
             return;
         }
     }

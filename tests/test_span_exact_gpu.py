@@ -108,3 +108,22 @@ def test_one_channel_mi_is_the_per_sample_kernels(cuda, lib, h, w):
         _, c = _run(cuda, pair, "MI")
     _, c0 = _run(cuda, pair, "MI", per_sample_decisions=True)
     np.testing.assert_array_equal(c.view(np.uint32), c0.view(np.uint32))
+
+
+@pytest.mark.parametrize("cost", COSTS + ["ZNCC"])
+def test_split_tasks_equal_whole_ones(cuda, lib, cost):
+    """256 points of a 200 x 180 image are four tasks, split over their 13 bands in a single search and
+    whole in a batch: the same bits."""
+    import torch
+    import cugridsearch_b200 as cgs
+    pair = _pair(21, cost, 200, 180, 190, 200, 1)
+    res, c = _run(cuda, pair, cost)
+    mov, fix = (cgs.CudaImage(torch.from_numpy(x).to(cuda)) for x in (pair.moving, pair.fixed))
+    grid = cgs.CudaGrid.from_ranges(*pair.grid_args())
+    costs, out = torch.empty(grid.numElements(), device=cuda), cgs.result_buffer(cuda)
+    with cgs.Batch([cgs.BatchPair(cost, mov, fix, grid, out, costs)]) as b:
+        b.launch()
+        torch.cuda.synchronize()
+    np.testing.assert_array_equal(costs.cpu().numpy().view(np.uint32), c.view(np.uint32))
+    assert cgs.read_result(out).index == res.index
+    _oracle_agrees(pair, cost, c)
