@@ -223,7 +223,7 @@ static cgs_status enqueue_launch(const cgs_batch &b, cudaStream_t s) {
     const unsigned px = (unsigned)std::max<int64_t>(1, std::min<int64_t>(64, (b.max_stage_elems + 255) / 256));
     const PrepParams *qs = b.d_prep;
     void *pargs[] = {&qs};
-    CGS_CUDA(cudaLaunchKernel(batch_prep_kernel_fn(), dim3(px, b.n), dim3(256), pargs, 0, s), "batch_prep_kernel");
+    CGS_CUDA(cudaLaunchKernel(batch_prep_kernel_fn(), dim3(px + 1, b.n), dim3(256), pargs, 0, s), "batch_prep_kernel");
     // the multi-pair span kernel first: its pairs take the least time each, so running them
     // before the per-sample pairs lowers the pairs' completion times (the launch takes as long)
     if (b.g_n > 0) {
@@ -536,6 +536,7 @@ cgs_status cgs_batch_create(const cgs_pair *pairs, int32_t n, const cgs_batch_pl
         p.costs = q.costs;
         p.result = q.result;
         preps[j] = make_prep(&q.moving, &q.fixed, pd.st, sb, mstage, fstage);
+        if (q.options.cost != CGS_COST_ZNCC) preps[j].shifts = nullptr;
         if (pd.quads) {
             p.mov_quad = reinterpret_cast<const float4 *>(org + pd.st.quad_off);
             p.quad_pitch = q.moving.width;
@@ -708,7 +709,7 @@ cgs_status cgs_batch_autotune(cgs_batch *b, int32_t sample_points, cgs_tune_entr
         const unsigned px = (unsigned)std::max<int64_t>(1, std::min<int64_t>(64, (b->max_stage_elems + 255) / 256));
         const PrepParams *qs = b->d_prep;
         void *pargs[] = {&qs};
-        CGS_CUDA(cudaLaunchKernel(batch_prep_kernel_fn(), dim3(px, b->n), dim3(256), pargs, 0, st),
+        CGS_CUDA(cudaLaunchKernel(batch_prep_kernel_fn(), dim3(px + 1, b->n), dim3(256), pargs, 0, st),
                  "batch_prep_kernel");
     }
     // the tuning copy of the parameters: the first `cap` points of every grid, no cost dump,

@@ -49,6 +49,7 @@ struct PrepParams {
     int32_t quad_form;   // 0: {P00, P10, P01 - P00, P11 - P10}; 1 (ZNCC and one-channel MI span kernels): {P00, P01 - P00,
                          // P10 - P00, (P11 - P10) - (P01 - P00)}; 2 (exact span kernel): {P00, P01, P10, P11};
                          // P(dy, dx) the tap at (y + dy, x + dx)
+    unsigned int *verify_hdr;  // the verification pass's band count and ticket, zeroed; or null
     unsigned int *zero_dst;  // zeroed words (the span kernels' counts of done parts), or null
     int64_t zero_n;
     float quad_scale;    // form 1: a power of two on the quads (one-channel MI: bins / 256), or 0 (none)

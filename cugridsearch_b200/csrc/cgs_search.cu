@@ -195,6 +195,7 @@ __device__ __forceinline__ float load_pix(const void *src, int pix, int64_t i) {
 // 16-byte row pitch so rows can be bulk-copied.
 __device__ __forceinline__ void prep_body(const PrepParams &q, int64_t tid, int64_t nthr) {
     if (tid == 0) {
+        if (q.verify_hdr) q.verify_hdr[0] = q.verify_hdr[1] = 0u;
         *q.key = ~0ull;
         *q.done = 0u;
         *q.status = 0u;
@@ -273,8 +274,25 @@ __device__ __forceinline__ void prep_body(const PrepParams &q, int64_t tid, int6
 
 // The images' means for the ZNCC shifts, over a fixed subsample (at most kShiftSamples evenly
 // strided elements of each HWC image), summed in FP64 in a fixed order by one block of 256
-// threads: the same bits on every call.  shifts = {fixed mean, moving mean}.
+// threads: the same bits on every call.  shifts = {fixed mean, moving mean}.  A thread's 16 samples
+// are loaded at once (one after the other they took 8 of the staging kernel's 10 us).
 constexpr int64_t kShiftSamples = 4096;
+
+template <class T>
+__device__ __forceinline__ double strided_sum(const void *src, int64_t stride, int count) {
+    constexpr int N = (int)(kShiftSamples / 256);
+    const T *v = static_cast<const T *>(src);
+    float f[N];
+#pragma unroll
+    for (int k = 0; k < N; k++) {
+        const int i = (int)threadIdx.x + 256 * k;
+        f[k] = i < count ? (float)v[i * stride] : 0.0f;
+    }
+    double s = 0.0;
+#pragma unroll
+    for (int k = 0; k < N; k++) s += (double)f[k];
+    return s;
+}
 
 __device__ void staging_means(const PrepParams &q) {
     __shared__ double part[2][8];
@@ -285,9 +303,11 @@ __device__ void staging_means(const PrepParams &q) {
         const int pix = k == 0 ? q.fix_pix : q.mov_pix;
         const int64_t total = k == 0 ? (int64_t)q.fh * q.fw * q.c : (int64_t)q.mh * q.mw * q.c;
         const int64_t stride = total > kShiftSamples ? total / kShiftSamples : 1;
-        const int64_t count = total > kShiftSamples ? kShiftSamples : total;
-        double s = 0.0;
-        for (int64_t i = t; i < count; i += 256) s += (double)load_pix(src, pix, i * stride);
+        const int count = (int)(total > kShiftSamples ? kShiftSamples : total);
+        double s = pix == CGS_PIXEL_U8    ? strided_sum<uint8_t>(src, stride, count)
+                   : pix == CGS_PIXEL_F64 ? strided_sum<double>(src, stride, count)
+                   : pix == CGS_PIXEL_U16 ? strided_sum<uint16_t>(src, stride, count)
+                                          : strided_sum<float>(src, stride, count);
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
         if ((t & 31) == 0) part[k][t >> 5] = s;
@@ -303,16 +323,21 @@ __device__ void staging_means(const PrepParams &q) {
     }
 }
 
-__global__ void __launch_bounds__(256) prep_kernel(const PrepParams q) {
-    if (blockIdx.x == 0 && q.shifts) staging_means(q);
-    prep_body(q, blockIdx.x * (int64_t)blockDim.x + threadIdx.x, (int64_t)gridDim.x * blockDim.x);
+// The last block takes the means (where the pair needs them), the others the planes.
+__device__ __forceinline__ void prep_block(const PrepParams &q) {
+    const int blocks = (int)gridDim.x - 1;
+    if ((int)blockIdx.x == blocks) {
+        if (q.shifts) staging_means(q);
+        return;
+    }
+    prep_body(q, blockIdx.x * (int64_t)blockDim.x + threadIdx.x, (int64_t)blocks * blockDim.x);
 }
+
+__global__ void __launch_bounds__(256) prep_kernel(const PrepParams q) { prep_block(q); }
 
 // Staging of a batch: blockIdx.y selects the pair, the x blocks stride over its elements.
 __global__ void __launch_bounds__(256) batch_prep_kernel(const PrepParams *__restrict__ qs) {
-    const PrepParams &q = qs[blockIdx.y];
-    if (blockIdx.x == 0 && q.shifts) staging_means(q);
-    prep_body(q, blockIdx.x * (int64_t)blockDim.x + threadIdx.x, (int64_t)gridDim.x * blockDim.x);
+    prep_block(qs[blockIdx.y]);
 }
 
 const void *batch_prep_kernel_fn() { return (const void *)batch_prep_kernel; }
@@ -886,7 +911,7 @@ static cgs_status search_scanline(const cgs_image *mov, const cgs_image *fix, co
     cudaError_t e = cudaMemsetAsync(sb, 0, 256, stream);
     if (e == cudaSuccess) {
         const int64_t prep_elems = (st.mplane + st.fplane) * C;
-        prep_kernel<<<(int)std::min<int64_t>((prep_elems + 255) / 256, (int64_t)di.sms * 8), 256, 0, stream>>>(q);
+        prep_kernel<<<(int)std::min<int64_t>((prep_elems + 255) / 256, (int64_t)di.sms * 8) + 1, 256, 0, stream>>>(q);
         e = cudaGetLastError();
     }
     const size_t smem = scan_smem_bytes(cost);
@@ -1129,12 +1154,14 @@ static cgs_status search_core(const cgs_image *mov, const cgs_image *fix, const 
     }
 
     PrepParams q = make_prep(mov, fix, st, sb, mstage, fstage);
+    if (cost != CGS_COST_ZNCC) q.shifts = nullptr;  // no other cost reads the means
     if (quads) {
         q.quad_dst = reinterpret_cast<float4 *>(sb + st.quad_off);
         q.qplane = st.qplane;
         q.quad_form = spans ? span_quad_form(cost, C) : 0;
         if (span_mi) q.quad_scale = (float)mi_bins * (1.0f / 256.0f);
     }
+    q.verify_hdr = static_cast<unsigned int *>(vblock);
     if (split_bytes) {
         p.split_tot = reinterpret_cast<double *>(sb + tot_off);
         p.split_cnt = reinterpret_cast<int *>(sb + tot_off + tot_bytes);
@@ -1150,7 +1177,7 @@ static cgs_status search_core(const cgs_image *mov, const cgs_image *fix, const 
     const int prep_blocks = (int)std::min<int64_t>((prep_elems + 255) / 256, (int64_t)di.sms * 8);
     cudaError_t e = cudaMemsetAsync(sb, 0, 256, stream);
     if (e == cudaSuccess) {
-        prep_kernel<<<prep_blocks, 256, 0, stream>>>(q);
+        prep_kernel<<<prep_blocks + 1, 256, 0, stream>>>(q);
         e = cudaGetLastError();
     }
     if (e == cudaSuccess && span && p.fix_prefix) {
@@ -1199,10 +1226,7 @@ static cgs_status search_core(const cgs_image *mov, const cgs_image *fix, const 
             if (e == cudaSuccess) e = cudaEventRecord(te->last, stream);
         }
     }
-    if (s == CGS_SUCCESS && e == cudaSuccess && verify) {
-        e = cudaMemsetAsync(vblock, 0, 8, stream);  // band count and CTA ticket
-        if (e == cudaSuccess) s = launch_verify(p, vblock, stream, di.sms);
-    }
+    if (s == CGS_SUCCESS && e == cudaSuccess && verify) s = launch_verify(p, vblock, stream, di.sms);
     release(vblock);
     release(scratch);
     if (s != CGS_SUCCESS) return s;
@@ -1398,7 +1422,7 @@ cgs_status cgs_search_noalloc(const cgs_image *mov, const cgs_image *fix, const 
     cudaError_t e = cudaMemsetAsync(sb, 0, 256, stream);
     if (e == cudaSuccess) {
         const int64_t prep_elems = (st.mplane + st.fplane) * C;
-        prep_kernel<<<(int)std::min<int64_t>((prep_elems + 255) / 256, (int64_t)di.sms * 8), 256, 0, stream>>>(q);
+        prep_kernel<<<(int)std::min<int64_t>((prep_elems + 255) / 256, (int64_t)di.sms * 8) + 1, 256, 0, stream>>>(q);
         e = cudaGetLastError();
     }
     if (e != cudaSuccess) return cuda_fail(e, "prep_kernel");
@@ -1453,7 +1477,7 @@ cgs_status cgs_mi_histogram(const cgs_image *mov, const cgs_image *fix, const fl
     if (e == cudaSuccess) e = cudaMemsetAsync(hist, 0, (size_t)bins * bins * 4, stream);
     const int64_t prep_elems = (st.mplane + st.fplane) * C;
     if (e == cudaSuccess) {
-        prep_kernel<<<(int)std::min<int64_t>((prep_elems + 255) / 256, (int64_t)di.sms * 8), 256, 0, stream>>>(q);
+        prep_kernel<<<(int)std::min<int64_t>((prep_elems + 255) / 256, (int64_t)di.sms * 8) + 1, 256, 0, stream>>>(q);
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) {
