@@ -52,6 +52,7 @@ struct PrepParams {
     unsigned int *verify_hdr;  // the verification pass's band count and ticket, zeroed; or null
     unsigned int *zero_dst;  // zeroed words (the span kernels' counts of done parts), or null
     int64_t zero_n;
+    float2 *pair_dst;    // fixed-image pairs (W x H per channel; fix_alias), or null
     float quad_scale;    // form 1: a power of two on the quads (one-channel MI: bins / 256), or 0 (none)
     int32_t *bin_dst;    // the fixed image's bins times 4 (bins + 1) (the histogram row's byte offset), laid
                          // out as the fixed planes, or null

@@ -65,6 +65,8 @@ struct SearchParams {
                                   // moving shift, and 2)
     int32_t quad_pitch;           // quads per row
     int64_t quad_plane;           // quads per channel
+    const float2 *fix_pair;       // scanline sums: per channel, W x H {(y, x), (y, x+1) - (y, x)} of the fixed image
+    int64_t pair_plane;           // pairs per channel
     const float *row_table;       // calcMIAlt's row values (the float recurrence row += 1/(H_f-1))
     int32_t n_rows;
     cgs_argmin *result;

@@ -12,8 +12,9 @@
 // Work layout: one warp per grid point (persistent over grid points in the locality order of
 // the pixel kernel).  For each block of 32 rows every lane sets up one row (the exact
 // intersection, ~100 correctly rounded operations), the warp then walks the rows, lanes
-// taking every 32nd lambda.  Both images are read through L1 from the staged planes, whose
-// extra column and zero row make the reference's flat-index neighbours explicit.
+// taking every 32nd lambda.  calcMIAlt (scan_kernel) reads both images through L1 from the staged
+// planes, whose extra column and zero row make the reference's flat-index neighbours explicit;
+// calcNCCAlt and calcSQDAlt (scan_sum_kernel) read tap quads and pairs made from them.
 #pragma once
 #include "cgs_kernels.cuh"
 #include "cgs_seq.cuh"
@@ -41,7 +42,6 @@ __device__ __forceinline__ Homog h_norm(const float *q, float c, float s, int mw
 struct RowInfo {
     float ls, le;        // first lambda, exclusive lambda limit (min of the reference's two bounds)
     float vx, vy, p0x, p0y;
-    float mag;           // |v| (calcNCCAlt/calcSQDAlt mov_area increment)
     float rowv;          // fixed-image row coordinate of the samples
     uint32_t n;          // number of lambda samples (0 when the row misses the moving image)
     int nseg;            // lambda segments; -1: more than kMaxSegs (lanes step explicitly)
@@ -161,24 +161,248 @@ __device__ __forceinline__ float value_exact(const float *pl, int pitch, float w
     return in_image(y, x, wf, hf) ? bilinear_in(pl, pitch, y, x) : 0.0f;
 }
 
-// The same value with fused interpolation (for sums, where only FP32 accuracy matters).
-__device__ __forceinline__ float value_fast(const float *pl, int pitch, float wf, float hf, float y, float x) {
-    if (!in_image(y, x, wf, hf)) return 0.0f;
-    const float fy = floorf(y), fx = floorf(x);
-    const float *q = pl + (int)fx + pitch * (int)fy;
-    const float v00 = __ldg(q), v01 = __ldg(q + 1), v10 = __ldg(q + pitch), v11 = __ldg(q + pitch + 1);
-    const float ax = x - fx, ay = y - fy;
-    const float top = fmaf(ax, v01 - v00, v00), bot = fmaf(ax, v11 - v10, v10);
-    return fmaf(ay, bot - top, top);
-}
-
 constexpr int kScanRows = 32;  // rows set up per block (one per lane)
 constexpr int kScanWarps = 8;  // warps per CTA (one grid point each)
 
-template <int COST, int C, int NW>
-__global__ void __launch_bounds__(NW * 32, 1) scan_kernel(const __grid_constant__ SearchParams p) {
-    constexpr bool kMI = (COST == CGS_COST_MI_ALT);
+// The CTA's best key into the search's, and the result by the last CTA (one thread).
+__device__ __forceinline__ void scan_finish(const SearchParams &p, const unsigned long long *wbest) {
+    unsigned long long b = ~0ull;
+    for (int w = 0; w < kScanWarps; w++) b = wbest[w] < b ? wbest[w] : b;
+    if (b != ~0ull) atomicMin(p.key, b);
+    __threadfence();
+    const unsigned int ticket = atomicAdd(p.done, 1u);
+    if (ticket == gridDim.x - 1) {
+        __threadfence();
+        write_result(p);
+    }
+}
+
+// x_0 = x, x_1 = fl(x + 1), ... below limit, as runs of exact unit steps: seq_segments for an
+// increment of 1, where every binade's ulp divides the step (0 <= x, limit < 2^23) and no run stalls.
+// segs: {first index, its value's bits} per run.
+constexpr int kMaxUnitSegs = 16;  // lambda up to 2^14; more runs: lanes step explicitly
+__device__ __forceinline__ uint32_t unit_segments(float x, float limit, uint2 *segs, int &nseg) {
+    nseg = 0;
+    uint32_t k = 0;
+    while (x < limit) {
+        if (nseg < kMaxUnitSegs) segs[nseg] = make_uint2(k, __float_as_uint(x));
+        nseg++;
+        if (x >= 1.0f) {  // below 1 a step always leaves the binade
+            const float end = __uint_as_float(__float_as_uint(x) | 0x7fffffu);  // the binade's last value
+            const float n_in = floorf(end - x);                                 // exact: multiples of one ulp
+            const double n_lim = ceil((double)limit - (double)x) - 1.0;         // exact: at most 48 bits
+            if (n_lim < (double)n_in) return k + (uint32_t)n_lim + 1u;
+            k += (uint32_t)n_in;
+            x += n_in;
+        }
+        x = xa(x, 1.0f);
+        k++;
+    }
+    return k;
+}
+
+struct SumRow {
+    float vx, vy, p0x, p0y;
+    float ls, mag;   // first lambda; |v| (the reference's mov_area increment)
+    uint32_t n;      // number of lambda samples (0 when the row misses the moving image)
+    int nseg;        // runs; above kMaxUnitSegs: lanes step explicitly
+};
+
+// One lambda sample of the sums.  The moving image comes as tap quads {v00, v10, v01 - v00, v11 - v10},
+// the fixed one, sampled on a whole row where the lower taps' weight is 0, as pairs {v0, v1 - v0}: one
+// load per channel and image (eight scalar ones took 36.9 warp instructions per 32 samples of a
+// channel), and the same roundings as interpolating the taps.
+template <int C>
+struct SumSample {
+    float4 m[C];
+    float2 f[C];
+    float ax, ay, af;
+    bool inside;
+    __device__ __forceinline__ void load(const SearchParams &p, const SumRow &r, float2 nzero2, float lam,
+                                         uint32_t frow) {
+        constexpr float kMagic = 8388608.0f;      // 2^23: rounding down onto the integers
+        constexpr uint32_t kBits = 0x4b000000u;
+        const float2 pos = __fadd2_rn(__ffma2_rn(make_float2(lam, lam), make_float2(r.vx, r.vy), nzero2),
+                                      make_float2(r.p0x, r.p0y));
+        const float tx = __fadd_rd(pos.x, kMagic), ty = __fadd_rd(pos.y, kMagic), tl = __fadd_rd(lam, kMagic);
+        const uint32_t ux = __float_as_uint(tx) - kBits, uy = __float_as_uint(ty) - kBits;
+        // 0 <= floor < size as unsigned integers: false for negative, huge and NaN positions too
+        inside = ux < (uint32_t)p.mov.w && uy < (uint32_t)p.mov.h;
+        const uint32_t i = inside ? uy * (uint32_t)p.mov.w + ux : 0u;
+        ax = pos.x - (tx - kMagic);
+        ay = pos.y - (ty - kMagic);
+        af = lam - (tl - kMagic);
+        const uint32_t j = frow + (__float_as_uint(tl) - kBits);
+#pragma unroll
+        for (int c = 0; c < C; c++) {
+            m[c] = __ldg(p.mov_quad + c * p.quad_plane + i);
+            f[c] = __ldg(p.fix_pair + c * p.pair_plane + j);
+        }
+    }
+    template <int COST>
+    __device__ __forceinline__ void add(float &out, float2 &i12) const {
+        const float2 s2 = make_float2(1.0f / 255.0f, 1.0f / 255.0f);
+#pragma unroll
+        for (int c = 0; c < C; c++) {
+            const float2 tb = __ffma2_rn(make_float2(ax, ax), make_float2(m[c].z, m[c].w), make_float2(m[c].x, m[c].y));
+            const float v = fmaf(ay, tb.y - tb.x, tb.x);
+            const float2 w = __fmul2_rn(make_float2(inside ? v : 0.0f, fmaf(af, f[c].y, f[c].x)), s2);
+            if constexpr (COST == CGS_COST_NCC_ALT) {
+                out = fmaf(w.x, w.y, out);
+            } else {
+                const float d = w.x - w.y;
+                out = fmaf(d, d, out);
+            }
+            i12 = __ffma2_rn(w, w, i12);
+        }
+    }
+};
+
+// calcNCCAlt and calcSQDAlt.  6,561 points on a 320 x 240 RGB pair take 1.73 ms (19 % of the L1's load
+// instructions, 53 % of its wavefronts -- a quad load is four of them at best -- and 53 % of the issue
+// slots; the rest is latency and the last points' tail).  Eight scalar taps a sample and channel, runs
+// looked up for every sample and one CTA of 8 warps on an SM (84 KB of runs) took 7.95 ms.  Three CTAs fit
+// here; two samples a lane are in flight, added in the lambda order.
+template <int COST, int C>
+__global__ void __launch_bounds__(kScanWarps * 32, 3) scan_sum_kernel(const __grid_constant__ SearchParams p) {
     constexpr bool kNCC = (COST == CGS_COST_NCC_ALT);
+    constexpr int kStride = kMaxUnitSegs + 1;  // odd: the lanes' rows start in different banks
+    __shared__ unsigned long long wbest[kScanWarps];
+    __shared__ SumRow rows_all[kScanWarps][kScanRows];
+    __shared__ uint2 segs_all[kScanWarps][kScanRows * kStride];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    SumRow *rows = rows_all[warp];
+    uint2 *segs = segs_all[warp];
+    const int fw = p.fix.w, fh = p.fix.h, mw = p.mov.w, mh = p.mov.h;
+    const float fwf = (float)fw;
+    // -0 the compiler cannot see: a product with it stays apart from the sum that follows
+    const float nzero = __uint_as_float(0x80000000u | ((uint32_t)p.dims >> 8));
+    const float2 nzero2 = make_float2(nzero, nzero);
+
+    unsigned long long best = ~0ull;
+    const uint32_t total_warps = gridDim.x * kScanWarps;
+    for (uint32_t o = blockIdx.x * kScanWarps + warp; o < p.n; o += total_warps) {
+        int32_t ax[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+        const uint32_t gidx = ordinal_to_index(p, o, ax);
+        float q[8];
+        grid_values(p, ax, q);
+        const float2 cs = p.trig[min(ax[0], kMaxTrig - 1)];
+        const Homog H = h_centred(q, cs.x, cs.y, p.cx, p.cy);
+
+        float out = 0.0f;                          // lane partial sums
+        float2 i12 = make_float2(0.0f, 0.0f);
+        double mov_area_d = 0.0;                   // sum n_r * mag_r
+        uint32_t steps = 0;                        // lambda steps over all rows
+        for (int rb = 0; rb < fh; rb += kScanRows) {
+            const int nb = min(kScanRows, fh - rb);
+            __syncwarp();
+            if (lane < nb) {
+                SumRow r;
+                float le = fwf;
+                r.ls = r.vx = r.vy = r.p0x = r.p0y = 0.0f;
+                bool in = false;
+                assign_values(H, mw, mh, fw, fh, rb + lane, r.ls, le, r.vx, r.vy, r.p0x, r.p0y, in);
+                r.mag = __fsqrt_rn(xa(xm(r.vx, r.vx), xm(r.vy, r.vy)));
+                r.nseg = 0;
+                r.n = in ? unit_segments(r.ls, fminf(le, fwf), segs + lane * kStride, r.nseg) : 0u;
+                rows[lane] = r;
+            }
+            __syncwarp();
+            for (int rr = 0; rr < nb; rr++) {
+                const SumRow r = rows[rr];
+                if (r.n == 0) continue;
+                steps += r.n;
+                mov_area_d += (double)r.n * (double)r.mag;
+                const uint32_t frow = (uint32_t)(rb + rr) * (uint32_t)fw;
+                if (r.nseg > kMaxUnitSegs) {
+                    float lam = r.ls;
+                    if (lane < (int)r.n) seq_advance(lam, 1.0, (uint32_t)lane);
+                    for (uint32_t k = lane; k < r.n; k += 32) {
+                        SumSample<C> s;
+                        s.load(p, r, nzero2, lam, frow);
+                        s.template add<COST>(out, i12);
+                        if (k + 32 < r.n) seq_advance(lam, 1.0, 32);
+                    }
+                    continue;
+                }
+                const uint2 *next = segs + rr * kStride, *last = next + r.nseg;
+                uint2 cur = make_uint2(0u, 0u);
+                uint32_t knext = 0u;  // index where the run after the current one begins
+                float lam = 0.0f;     // lambda of sample k
+                auto seek = [&](uint32_t k) {  // lam of sample k, from the one 32 before it within a run
+                    lam += 32.0f;
+                    if (k >= knext) {
+                        do {
+                            cur = *next++;
+                            knext = next < last ? next->x : 0xffffffffu;
+                        } while (k >= knext);
+                        lam = __uint_as_float(cur.y) + (float)(k - cur.x);
+                    }
+                };
+                uint32_t k = lane;
+                for (; k - lane + 64 <= r.n; k += 64) {  // uniform: two full warps of samples
+                    SumSample<C> s0, s1;
+                    seek(k);
+                    s0.load(p, r, nzero2, lam, frow);
+                    seek(k + 32);
+                    s1.load(p, r, nzero2, lam, frow);
+                    s0.template add<COST>(out, i12);
+                    s1.template add<COST>(out, i12);
+                }
+                for (; k < r.n; k += 32) {
+                    SumSample<C> s;
+                    seek(k);
+                    s.load(p, r, nzero2, lam, frow);
+                    s.template add<COST>(out, i12);
+                }
+            }
+        }
+
+        out = warp_sum(out);
+        const float i1 = warp_sum(i12.x), i2 = warp_sum(i12.y);
+        // gates (cudaErrorFunctions.cuh:296, 372): fix_area counts lambda steps exactly;
+        // mov_area is a float running sum, decided from its double value unless that is
+        // within the float sum's error bound of the threshold, then replayed exactly
+        const float fix_area = (float)steps;
+        const float den_m = xm((float)(p.mov.w * p.mov.h), q[2]);
+        const bool gate_fix = (double)xd(fix_area, (float)(fw * fh)) > 0.35;
+        bool gate_mov = false;
+        if (lane == 0) {
+            const double ratio = mov_area_d / (double)den_m;
+            const double margin = ((double)steps + 4.0) * 5.9604644775390625e-8 * fabs(ratio) + 1e-12;
+            if (fabs(ratio - 0.25) > margin) {
+                gate_mov = ratio > 0.25;
+            } else {
+                // exact replay of the reference's sequential float sum
+                float mov_area = 0.0f;
+                for (int r = 0; r < fh; r++) {
+                    float ls = 0.0f, le = fwf, vx = 0, vy = 0, p0x = 0, p0y = 0;
+                    bool in = false;
+                    assign_values(H, mw, mh, fw, fh, r, ls, le, vx, vy, p0x, p0y, in);
+                    if (!in) continue;
+                    bool st;
+                    const uint32_t n = seq_count_below(ls, 1.0, fminf(le, fwf), st);
+                    const float mag = __fsqrt_rn(xa(xm(vx, vx), xm(vy, vy)));
+                    seq_advance(mov_area, (double)mag, n);
+                }
+                gate_mov = (double)xd(mov_area, den_m) > 0.25;
+            }
+            const float cost = gate_mov && gate_fix ? xd(kNCC ? -out : out, __fsqrt_rn(xm(i1, i2))) : 123123.0f;
+            if (p.costs) p.costs[gidx] = cost;
+            const unsigned long long kk = make_key(cost, gidx);
+            best = kk < best ? kk : best;
+        }
+    }
+
+    if (lane == 0) wbest[warp] = best;
+    __syncthreads();
+    if (threadIdx.x == 0) scan_finish(p, wbest);
+}
+
+// calcMIAlt.
+template <int C>
+__global__ void __launch_bounds__(kScanWarps * 32, 1) scan_kernel(const __grid_constant__ SearchParams p) {
+    constexpr int NW = kScanWarps;
     constexpr int BN = 64;                 // calcMIAlt's bins
     constexpr int HS = BN + 1;             // padded row stride; row / column BN hold the marginals
     extern __shared__ __align__(128) unsigned char smem[];
@@ -193,9 +417,8 @@ __global__ void __launch_bounds__(NW * 32, 1) scan_kernel(const __grid_constant_
     uint32_t *hist = hist_all + (size_t)warp * HS * HS;
     const int fw = p.fix.w, fh = p.fix.h, mw = p.mov.w, mh = p.mov.h;
     const float fwf = (float)fw, fhf = (float)fh, mwf = p.mov_wf, mhf = p.mov_hf;
-    const int nrows = kMI ? p.n_rows : fh;
-    const double lam_inc = kMI ? (double)(1.0f / (float)(fw - 1)) : 1.0;
-    const float lam_cap = kMI ? 1.0f : fwf;
+    const int nrows = p.n_rows;
+    const double lam_inc = (double)(1.0f / (float)(fw - 1));
 
     unsigned long long best = ~0ull;
     const uint32_t total_warps = gridDim.x * NW;
@@ -205,15 +428,11 @@ __global__ void __launch_bounds__(NW * 32, 1) scan_kernel(const __grid_constant_
         float q[8];
         grid_values(p, ax, q);
         const float2 cs = p.trig[min(ax[0], kMaxTrig - 1)];
-        const Homog H = kMI ? h_norm(q, cs.x, cs.y, mw, mh, fw, fh) : h_centred(q, cs.x, cs.y, p.cx, p.cy);
+        const Homog H = h_norm(q, cs.x, cs.y, mw, mh, fw, fh);
 
-        float out = 0.0f, i1 = 0.0f, i2 = 0.0f;  // lane partial sums (NCC/SQD)
-        double mov_area_d = 0.0;                 // sum n_r * mag_r (lane 0)
-        uint32_t steps = 0;                      // lambda steps over all rows (uniform)
+        uint32_t steps = 0;  // lambda steps over all rows (uniform)
         bool stalled = false;
-        if constexpr (kMI) {
-            for (int i = lane; i < HS * HS; i += 32) hist[i] = 0u;
-        }
+        for (int i = lane; i < HS * HS; i += 32) hist[i] = 0u;
         __syncwarp();
 
         for (int rb = 0; rb < nrows; rb += kScanRows) {
@@ -221,28 +440,21 @@ __global__ void __launch_bounds__(NW * 32, 1) scan_kernel(const __grid_constant_
             if (lane < nb) {
                 RowInfo ri;
                 ri.ls = 0.0f;
-                ri.le = kMI ? 1.0f : fwf;
+                ri.le = 1.0f;
                 ri.vx = ri.vy = ri.p0x = ri.p0y = 0.0f;
                 bool in = false;
-                if constexpr (kMI) {
-                    const float rv = p.row_table[rb + lane];
-                    assign_values_norm(H, rv, ri.ls, ri.le, ri.vx, ri.vy, ri.p0x, ri.p0y, in);
-                    ri.rowv = __double2float_rn(((double)rv + 0.5) * (double)(fh - 1));
-                    ri.mag = 0.0f;
-                } else {
-                    assign_values(H, mw, mh, fw, fh, rb + lane, ri.ls, ri.le, ri.vx, ri.vy, ri.p0x, ri.p0y, in);
-                    ri.rowv = (float)(rb + lane);
-                    ri.mag = __fsqrt_rn(xa(xm(ri.vx, ri.vx), xm(ri.vy, ri.vy)));
-                }
+                const float rv = p.row_table[rb + lane];
+                assign_values_norm(H, rv, ri.ls, ri.le, ri.vx, ri.vy, ri.p0x, ri.p0y, in);
+                ri.rowv = __double2float_rn(((double)rv + 0.5) * (double)(fh - 1));
                 bool st = false, ovf = false;
                 ri.nseg = 0;
-                ri.n = in ? seq_segments(ri.ls, lam_inc, fminf(ri.le, lam_cap), segs + lane * kMaxSegs, kMaxSegs,
+                ri.n = in ? seq_segments(ri.ls, lam_inc, fminf(ri.le, 1.0f), segs + lane * kMaxSegs, kMaxSegs,
                                          ri.nseg, ovf, st)
                           : 0u;
                 if (ovf) ri.nseg = -1;
                 // a row has at most about W_f / step samples; anything else is a stalled
                 // recurrence the reference would never leave
-                const double max_n = (double)(kMI ? fw : fw) / fmin(lam_inc, 1.0) + 8.0;
+                const double max_n = (double)fw / fmin(lam_inc, 1.0) + 8.0;
                 if ((double)ri.n > max_n) st = true;
                 if (st) ri.n = 0u;
                 rows[lane] = ri;
@@ -253,7 +465,6 @@ __global__ void __launch_bounds__(NW * 32, 1) scan_kernel(const __grid_constant_
                 const RowInfo ri = rows[rr];
                 if (ri.n == 0) continue;
                 steps += ri.n;
-                if (lane == 0 && !kMI) mov_area_d += (double)ri.n * (double)ri.mag;
                 const Seg *rs = segs + rr * kMaxSegs;
                 int cur = 0;
                 float lam = ri.ls;
@@ -267,29 +478,16 @@ __global__ void __launch_bounds__(NW * 32, 1) scan_kernel(const __grid_constant_
                     for (int c = 0; c < C; c++) {
                         const float *mpl = p.mov.data + c * p.mov.plane;
                         const float *fpl = p.fix.data + c * p.fix.plane;
-                        if constexpr (kMI) {
-                            const float nx = __double2float_rn(((double)nx0 + 0.5) * (double)mw);
-                            const float ny = __double2float_rn(((double)ny0 + 0.5) * (double)mh);
-                            const float lamIdx = xm(lam, (float)(fw - 1));
-                            const float vf = value_exact(fpl, p.fix.pitch, fwf, fhf, ri.rowv, lamIdx);
-                            const float vm = value_exact(mpl, p.mov.pitch, mwf, mhf, ny, nx);
-                            int bf = (int)floorf(xm(64.0f, xd(vf, 256.0f)));
-                            int bm = (int)floorf(xm(64.0f, xd(vm, 256.0f)));
-                            bf = min(max(bf, 0), BN - 1);
-                            bm = min(max(bm, 0), BN - 1);
-                            atomicAdd(&hist[bf * HS + bm], 1u);
-                        } else {
-                            const float vm = value_fast(mpl, p.mov.pitch, mwf, mhf, ny0, nx0) * (1.0f / 255.0f);
-                            const float vf = value_fast(fpl, p.fix.pitch, fwf, fhf, ri.rowv, lam) * (1.0f / 255.0f);
-                            if constexpr (kNCC) {
-                                out = fmaf(vm, vf, out);
-                            } else {
-                                const float d = vm - vf;
-                                out = fmaf(d, d, out);
-                            }
-                            i1 = fmaf(vm, vm, i1);
-                            i2 = fmaf(vf, vf, i2);
-                        }
+                        const float nx = __double2float_rn(((double)nx0 + 0.5) * (double)mw);
+                        const float ny = __double2float_rn(((double)ny0 + 0.5) * (double)mh);
+                        const float lamIdx = xm(lam, (float)(fw - 1));
+                        const float vf = value_exact(fpl, p.fix.pitch, fwf, fhf, ri.rowv, lamIdx);
+                        const float vm = value_exact(mpl, p.mov.pitch, mwf, mhf, ny, nx);
+                        int bf = (int)floorf(xm(64.0f, xd(vf, 256.0f)));
+                        int bm = (int)floorf(xm(64.0f, xd(vm, 256.0f)));
+                        bf = min(max(bf, 0), BN - 1);
+                        bm = min(max(bm, 0), BN - 1);
+                        atomicAdd(&hist[bf * HS + bm], 1u);
                     }
                     if (ri.nseg < 0 && k + 32 < ri.n) ok &= seq_advance(lam, lam_inc, 32);
                 }
@@ -299,80 +497,38 @@ __global__ void __launch_bounds__(NW * 32, 1) scan_kernel(const __grid_constant_
         }
 
         // ---- cost of this grid point
-        float cost;
-        if constexpr (kMI) {
-            __syncwarp();
-            // marginals: fixed (rows) into column BN, moving (columns) into row BN
-            for (int i = lane; i < BN; i += 32) {
-                uint32_t rs = 0, csum = 0;
-                for (int j = 0; j < BN; j++) {
-                    rs += hist[i * HS + j];
-                    csum += hist[j * HS + i];
-                }
-                hist[i * HS + BN] = rs;
-                hist[BN * HS + i] = csum;
+        // marginals: fixed (rows) into column BN, moving (columns) into row BN
+        for (int i = lane; i < BN; i += 32) {
+            uint32_t rs = 0, csum = 0;
+            for (int j = 0; j < BN; j++) {
+                rs += hist[i * HS + j];
+                csum += hist[j * HS + i];
             }
-            __syncwarp();
-            uint32_t cnt = 0;
-            for (int i = lane; i < BN; i += 32) cnt += hist[i * HS + BN];
-            cnt = (uint32_t)warp_sum_i((int)cnt);
-            // the reference's float formula: P = n_xy / count, sum P (log2 P - (log2 Px + log2 Py))
-            const float countf = (float)cnt;
-            float s = 0.0f;
-            for (int b = lane; b < BN * BN; b += 32) {
-                const int i = b / BN, j = b - i * BN;
-                const uint32_t v = hist[i * HS + j];
-                if (v) {
-                    const float P = (float)v / countf;
-                    const float Px = (float)hist[i * HS + BN] / countf;
-                    const float Py = (float)hist[BN * HS + j] / countf;
-                    s += P * (log2f(P) - (log2f(Px) + log2f(Py)));
-                }
-            }
-            s = warp_sum(s);
-            // fix_area: one 1/(W_f H_f) per lambda step, accumulated as the reference does
-            float fix_area = 0.0f;
-            seq_advance(fix_area, 1.0 / (double)((int64_t)fw * fh), steps);
-            cost = (-1.0f * s) * fix_area;
-        } else {
-            out = warp_sum(out);
-            i1 = warp_sum(i1);
-            i2 = warp_sum(i2);
-            // gates (cudaErrorFunctions.cuh:296, 372): fix_area counts lambda steps exactly;
-            // mov_area is a float running sum, decided from its double value unless that is
-            // within the float sum's error bound of the threshold, then replayed exactly
-            const float fix_area = (float)steps;
-            const float den_m = xm((float)(p.mov.w * p.mov.h), q[2]);
-            bool gate_fix = (double)xd(fix_area, (float)(fw * fh)) > 0.35;
-            bool gate_mov = false;
-            if (lane == 0) {
-                const double ratio = mov_area_d / (double)den_m;
-                const double margin = ((double)steps + 4.0) * 5.9604644775390625e-8 * fabs(ratio) + 1e-12;
-                if (fabs(ratio - 0.25) > margin) {
-                    gate_mov = ratio > 0.25;
-                } else {
-                    // exact replay of the reference's sequential float sum
-                    float mov_area = 0.0f;
-                    for (int r = 0; r < fh; r++) {
-                        float ls = 0.0f, le = fwf, vx = 0, vy = 0, p0x = 0, p0y = 0;
-                        bool in = false;
-                        assign_values(H, mw, mh, fw, fh, r, ls, le, vx, vy, p0x, p0y, in);
-                        if (!in) continue;
-                        bool st;
-                        const uint32_t n = seq_count_below(ls, 1.0, fminf(le, fwf), st);
-                        const float mag = __fsqrt_rn(xa(xm(vx, vx), xm(vy, vy)));
-                        seq_advance(mov_area, (double)mag, n);
-                    }
-                    gate_mov = (double)xd(mov_area, den_m) > 0.25;
-                }
-            }
-            gate_mov = __shfl_sync(0xffffffffu, gate_mov, 0);
-            if (gate_mov && gate_fix) {
-                cost = kNCC ? xd(-out, __fsqrt_rn(xm(i1, i2))) : xd(out, __fsqrt_rn(xm(i1, i2)));
-            } else {
-                cost = 123123.0f;
+            hist[i * HS + BN] = rs;
+            hist[BN * HS + i] = csum;
+        }
+        __syncwarp();
+        uint32_t cnt = 0;
+        for (int i = lane; i < BN; i += 32) cnt += hist[i * HS + BN];
+        cnt = (uint32_t)warp_sum_i((int)cnt);
+        // the reference's float formula: P = n_xy / count, sum P (log2 P - (log2 Px + log2 Py))
+        const float countf = (float)cnt;
+        float s = 0.0f;
+        for (int b = lane; b < BN * BN; b += 32) {
+            const int i = b / BN, j = b - i * BN;
+            const uint32_t v = hist[i * HS + j];
+            if (v) {
+                const float P = (float)v / countf;
+                const float Px = (float)hist[i * HS + BN] / countf;
+                const float Py = (float)hist[BN * HS + j] / countf;
+                s += P * (log2f(P) - (log2f(Px) + log2f(Py)));
             }
         }
+        s = warp_sum(s);
+        // fix_area: one 1/(W_f H_f) per lambda step, accumulated as the reference does
+        float fix_area = 0.0f;
+        seq_advance(fix_area, 1.0 / (double)((int64_t)fw * fh), steps);
+        const float cost = (-1.0f * s) * fix_area;
         stalled = __any_sync(0xffffffffu, stalled);
         if (lane == 0) {
             if (stalled) atomicOr(p.status, (unsigned)CGS_ERROR_UNSUPPORTED);
@@ -385,17 +541,7 @@ __global__ void __launch_bounds__(NW * 32, 1) scan_kernel(const __grid_constant_
 
     if (lane == 0) wbest[warp] = best;
     __syncthreads();
-    if (threadIdx.x == 0) {
-        unsigned long long b = ~0ull;
-        for (int w = 0; w < NW; w++) b = wbest[w] < b ? wbest[w] : b;
-        if (b != ~0ull) atomicMin(p.key, b);
-        __threadfence();
-        const unsigned int ticket = atomicAdd(p.done, 1u);
-        if (ticket == gridDim.x - 1) {
-            __threadfence();
-            write_result(p);
-        }
-    }
+    if (threadIdx.x == 0) scan_finish(p, wbest);
 }
 
 }  // namespace cgs

@@ -258,6 +258,24 @@ __device__ __forceinline__ void prep_body(const PrepParams &q, int64_t tid, int6
             }
         }
     }
+    if (q.pair_dst) {
+        // the fixed image's {P(y, x), P(y, x + 1) - P(y, x)}, P its padded plane.  A sample on row y reads
+        // row y + 1 with weight 0, which shows only where the rows' difference is not finite
+        const int64_t plane = (int64_t)q.fh * q.fw;
+        auto P = [&](int c, int64_t y, int64_t x) -> float {
+            const int64_t e = y * q.fw + x;  // column W: the next row's pixel 0
+            return e < plane ? load_pix(q.fix_src, q.fix_pix, e * q.c + c) : 0.0f;
+        };
+        for (int64_t i = tid; i < plane * q.c; i += nthr) {
+            const int c = (int)(i / plane);
+            const int64_t e = i - (int64_t)c * plane;
+            const int64_t y = e / q.fw, x = e - y * q.fw;
+            const float v0 = P(c, y, x), v1 = P(c, y, x + 1);
+            const float below = fabsf(P(c, y + 1, x) - v0) + fabsf(P(c, y + 1, x + 1) - v1);
+            const bool finite = below < __int_as_float(0x7f800000);
+            q.pair_dst[i] = make_float2(finite ? v0 : __int_as_float(0x7fffffff), v1 - v0);
+        }
+    }
     for (int64_t i = tid; i < q.zero_n; i += nthr) q.zero_dst[i] = 0u;
     if (q.row_table && tid == 0) {
         // calcMIAlt's rows: row = -0.5; while (row < 0.5) row += 1 / (float)(rowsf - 1)
@@ -867,12 +885,13 @@ static cgs_status search_scanline(const cgs_image *mov, const cgs_image *fix, co
     const bool mi = cost == CGS_COST_MI_ALT;
     p.n_rows = mi ? mi_alt_rows(fix->height) : fix->height;
 
-    const Staging st = staging_layout(*mov, *fix, di.tex_align, di.tex_pitch_align, true, mi);
+    const Staging st = staging_layout(*mov, *fix, di.tex_align, di.tex_pitch_align, true, mi, !mi);
+    const size_t pair_bytes = mi ? 0 : (size_t)fix->width * fix->height * C * 8;
     cgs_status s;
     cudaMemPool_t pool;
     if ((s = get_pool(di.dev, &pool)) != CGS_SUCCESS) return s;
     void *scratch = nullptr;
-    CGS_CUDA(cudaMallocFromPoolAsync(&scratch, st.bytes, pool, stream), "cudaMallocFromPoolAsync");
+    CGS_CUDA(cudaMallocFromPoolAsync(&scratch, st.bytes + pair_bytes + 256, pool, stream), "cudaMallocFromPoolAsync");
     char *sb = staging_origin(scratch, di.tex_align);
     p.key = reinterpret_cast<unsigned long long *>(sb);
     p.done = reinterpret_cast<unsigned int *>(sb + 8);
@@ -885,6 +904,13 @@ static cgs_status search_scanline(const cgs_image *mov, const cgs_image *fix, co
     p.mov = Plane{mstage, mov->height, mov->width, C, st.mpitch, st.mplane};
     p.fix = Plane{fstage, fix->height, fix->width, C, st.fpitch, st.fplane};
     p.row_table = rtab;
+    if (!mi) {
+        const size_t pair_off = (size_t)round_up((int64_t)(st.quad_off + (size_t)st.qplane * C * 16), 256);
+        p.mov_quad = reinterpret_cast<const float4 *>(sb + st.quad_off);
+        p.quad_plane = st.qplane;
+        p.fix_pair = reinterpret_cast<const float2 *>(sb + pair_off);
+        p.pair_plane = (int64_t)fix->width * fix->height;
+    }
     p.costs = costs;
     p.result = result;
 
@@ -907,6 +933,9 @@ static cgs_status search_scanline(const cgs_image *mov, const cgs_image *fix, co
     q.vmax = reinterpret_cast<float *>(sb + 16);
     q.fix_alias = 1;
     q.row_table = rtab;
+    q.quad_dst = const_cast<float4 *>(p.mov_quad);
+    q.qplane = p.quad_plane;
+    q.pair_dst = const_cast<float2 *>(p.fix_pair);
     q.rowsf = fix->height;
     cudaError_t e = cudaMemsetAsync(sb, 0, 256, stream);
     if (e == cudaSuccess) {
