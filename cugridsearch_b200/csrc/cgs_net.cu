@@ -205,27 +205,33 @@ __global__ void __launch_bounds__(kThreads) conv_fwd_kernel(const bf16 *__restri
 //
 // The forward convolution as an implicit GEMM on the 5th-generation tensor cores: D[m][co] =
 // sum_k A[m][k] B[co][k], m = (b, ho, wo) output pixels, k = (tap, ci).  A (gathered, im2col)
-// and B (the BF16 weights, [Cout][Kp]) are staged in shared memory by the CTA's 512 threads
-// with cp.async; one thread issues tcgen05.mma (kind::f16, BF16 x BF16 -> FP32, M = 128, N =
+// and B (the BF16 weights, [Cout][Kp]) come to shared memory through the registers of the CTA's 256
+// threads; one thread issues tcgen05.mma (kind::f16, BF16 x BF16 -> FP32, M = 128, N =
 // the CTA's channels, Cout or 64, K = 16 per instruction) into a TMEM accumulator of N columns,
-// completion tracked by tcgen05.commit on an mbarrier per stage (two stages: the next K slice is
-// gathered while the tensor cores work on the current one).  The epilogue reads the accumulator
-// back with tcgen05.ld (warp w owns TMEM lanes 32 (w % 4) .. + 31, i.e. output rows, and every
-// fourth group of 32 columns from w / 4), adds the bias, applies ReLU and stores BF16.
+// completion tracked by tcgen05.commit on an mbarrier per stage (three stages).  The epilogue reads the
+// accumulator back with tcgen05.ld (warp w owns TMEM lanes 32 (w % 4) .. + 31, i.e. output rows, and every
+// second group of 8 columns from w / 4), adds the bias, applies ReLU and stores BF16.
 //
 // Shared-memory operands use the UMMA K-major layout without swizzle: 16-byte chunks of 8
-// consecutive k of one row, chunk (row, kc) at 16 (kc * ROWS + row) bytes, so 8 consecutive
+// consecutive k of one row, chunk (row, kc) at 16 (kc * (ROWS + 1) + row) bytes, so 8 consecutive
 // rows of a chunk column form one 128-byte core matrix; descriptor strides: between row
 // groups of 8 (SBO) 128 bytes, between the two 8-k halves of a K = 16 instruction (LBO)
-// 16 ROWS bytes.
+// 16 (ROWS + 1) bytes.  The odd column stride lets 8 neighbouring lanes copy the 128 contiguous bytes of
+// one row's slice into 8 different bank groups.
+//
+// A CTA takes many row tiles; a slice is stored one step, and loaded two steps, before its instructions,
+// across tile boundaries, so that loads are in flight during the epilogue.  Plain loads, because the
+// asynchronous copies of 16 bytes (cp.async) ran at 37 cycles a warp instruction on an SM whatever their
+// order, depth or number of CTAs: at batch 256 layer 0's forward took 94 us with them and 40 us this way, those
+// of layers 1, 3 and 4 53 and 32 on average, the data gradient into layer 0's output 160 and 90 (with one CTA per tile, and
+// 16 bytes of 32 different pixels a warp instruction: 237).  Bound now by the latency of the chain of loads,
+// barriers and MMAs, and where a tile has one or two slices by the epilogue's row stores.
 constexpr int kUmmaM = 128, kUmmaBK = 64;  // rows per tile, k per stage (up to four K = 16 instructions)
-constexpr int kUmmaT = 512;                 // threads per CTA: 4 per output row for the gathers
-
-// 16-byte global -> shared copy (cp.async, L2 only); bytes = 0 fills the 16 bytes with zeros.
-__device__ __forceinline__ void cp_async16(void *dst, const void *src, uint32_t bytes) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_addr(dst)), "l"(src), "r"(bytes)
-                 : "memory");
-}
+constexpr int kUmmaT = 512;                 // threads per CTA of the weight gradient
+constexpr int kUmmaS = 3;                   // its operand stages
+constexpr int kConvT = 256;                 // threads per CTA of the forward and the data gradient
+constexpr int kConvS = 3;                   // their operand stages
+constexpr int kConvCtas = 3;                // their CTAs per SM
 
 // Shared-memory matrix descriptor: start address, leading and stride byte offsets (16-byte
 // units), descriptor version 1, no swizzle.
@@ -243,39 +249,39 @@ __host__ __device__ constexpr uint32_t umma_idesc_bf16(int M, int N) {
 // BWD = true: the data gradient, x = the output gradient dy [n][Ho][Ho][Cout], w = the transposed
 // weights [Cin][9 Cout], mask = the previous layer's output (ReLU mask), y = dx [n][H][H][Cin].
 // With stride 2 an input pixel (hi, wi) receives only the taps ky = hi + 1 (mod 2), kx = wi + 1
-// (mod 2), so the rows are split by parity class (py, px) = (hi, wi) mod 2 (blockIdx.z, the four-tap
+// (mod 2), so the rows are split by parity class (py, px) = (hi, wi) mod 2 (units of their own, the four-tap
 // class first): a class's rows are the pixels (2i + py, 2j + px) and its K = (1 + py)(1 + px) Cout,
 // k = (t, co) over the class's taps t = (ty, tx), ky = py ? 2 ty : 1, kx = px ? 2 tx : 1, which
 // read dy at (i + py (1 - ty), j + px (1 - tx)) where that is inside the output.
 template <int N, bool BWD>
-__global__ void __launch_bounds__(kUmmaT) conv_umma_kernel(const bf16 *__restrict__ x, const bf16 *__restrict__ w,
-                                                           const float *__restrict__ bias,
-                                                           const bf16 *__restrict__ mask, bf16 *__restrict__ y,
-                                                           const ConvGeom g, unsigned int *__restrict__ status) {
+__global__ void __launch_bounds__(kConvT, N >= 256 ? 1 : N >= 128 ? 2 : kConvCtas)
+conv_umma_kernel(const bf16 *__restrict__ x, const bf16 *__restrict__ w, const float *__restrict__ bias,
+                 const bf16 *__restrict__ mask, bf16 *__restrict__ y, const ConvGeom g, int tiles, int units,
+                 unsigned int *__restrict__ status) {
     static_assert(N % 16 == 0 && N >= 32 && N <= 256 && (N & (N - 1)) == 0, "TMEM columns: a power of two, 32..256");
-    constexpr int kA = kUmmaM * kUmmaBK * 2, kB = N * kUmmaBK * 2;  // bytes per stage
+    constexpr int S = kConvS, R = kUmmaM * 8 / kConvT, RB = N * 8 / kConvT;  // stages; chunks of A, B per thread and slice
+    constexpr uint32_t kColA = 16 * (kUmmaM + 1), kColB = 16 * (N + 1);    // bytes between chunk columns
+    constexpr uint32_t kA = kColA * (kUmmaBK / 8), kB = kColB * (kUmmaBK / 8);  // bytes per stage
     extern __shared__ __align__(1024) unsigned char smem[];
-    unsigned char *sA[2] = {smem, smem + kA};
-    unsigned char *sB[2] = {smem + 2 * kA, smem + 2 * kA + kB};
-    uint64_t *bars = reinterpret_cast<uint64_t *>(smem + 2 * kA + 2 * kB);
-    uint32_t *tslot = reinterpret_cast<uint32_t *>(bars + 2);
+    unsigned char *sB = smem + S * kA;
+    uint64_t *bars = reinterpret_cast<uint64_t *>(smem + S * (kA + kB));
+    uint32_t *tslot = reinterpret_cast<uint32_t *>(bars + S);
     volatile int *gave_up = reinterpret_cast<volatile int *>(tslot + 1);  // a bounded wait gave up
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int side = BWD ? g.H >> 1 : g.Ho;  // rows: output pixels, or one parity class of input pixels
-    const int M = g.n * side * side;
-    const int ph = BWD ? 3 - (int)blockIdx.z : 0, py = ph >> 1, px = ph & 1, ntx = 1 + px;
-    const int KT = BWD ? (1 + py) * ntx * g.Cout : g.Kp;  // GEMM K (a multiple of 32; of 64 for BWD)
-    const int wstride = BWD ? 9 * g.Cout : g.Kp;           // B row stride
-    const int CO = BWD ? g.Cin : g.Cout;                   // GEMM N: the output's channels
-    const int m0 = blockIdx.x * kUmmaM, co0 = blockIdx.y * N;  // this CTA: rows m0.., channels co0 .. co0 + N
+    // sizes are powers of two (launch_conv_umma checks)
+    const int lside = 31 - __clz(g.Ho);  // rows: output pixels, or one parity class of input pixels (H = 2 Ho)
+    const int lch = 31 - __clz(BWD ? g.Cout : g.Cin);  // channels of x
+    const int side = g.Ho, M = g.n << (2 * lside);
+    const int CO = BWD ? g.Cin : g.Cout;  // GEMM N: the output's channels
+    const int wstride = BWD ? 9 * g.Cout : g.Kp;
+    const int co0 = blockIdx.y * N;
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(tslot)),
                      "r"(N));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
     if (threadIdx.x == 0) {
-        mbar_init(&bars[0], 1);
-        mbar_init(&bars[1], 1);
+        for (int i = 0; i < S; i++) mbar_init(&bars[i], 1);
         fence_mbar_init();
         *gave_up = 0;
     }
@@ -283,213 +289,241 @@ __global__ void __launch_bounds__(kUmmaT) conv_umma_kernel(const bf16 *__restric
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tacc = *tslot;
-    const int nk = (KT + kUmmaBK - 1) / kUmmaBK;  // KT is a multiple of 32: the last slice may be half
     constexpr uint32_t idesc = umma_idesc_bf16(kUmmaM, N);
-    // this thread's output row (its im2col row), decoded once; its chunks kc = part + 4 j
-    const int row = threadIdx.x & (kUmmaM - 1), part = threadIdx.x >> 7, m = m0 + row;
-    const bool mvalid = m < M;
-    int b = 0, ho = 0, wo = 0;
-    if (mvalid) {
-        b = m / (side * side);
-        const int r = m - b * side * side;
-        ho = r / side;  // (i, j) of the parity class for the data gradient
-        wo = r - ho * side;
-    }
-    // one K slice into stage st2: A chunks by cp.async (16 bytes of one tap's channels; zero
-    // fill outside the image and past K), or gathered through registers where 8 consecutive k
-    // span taps (Cin = 2: four taps of two channels; other Cin not a multiple of 8: element by
-    // element); B chunks by cp.async
-    auto load_slice = [&](int kb2, int st2) {
-        const int k0 = kb2 * kUmmaBK;
-        const int kchunks = min(kUmmaBK, KT - k0) >> 3;
-        int woff = 0;  // BWD: a slice lies inside one tap t (64 divides Cout); B reads wt's block of tap(t)
-        if constexpr (BWD) {
-            const int t = k0 / g.Cout, ty = t / ntx, tx = t - ty * ntx;
-            woff = (3 * (py ? 2 * ty : 1) + (px ? 2 * tx : 1) - t) * g.Cout;
-        }
+    // GEMM K of a unit's parity class (a multiple of 32; of 64 for BWD)
+    auto unit_k = [&](int ph) { return BWD ? (1 + (ph >> 1)) * (1 + (ph & 1)) * g.Cout : g.Kp; };
+    auto unit_class = [&](int u) { return BWD ? 3 - (u >= tiles) - (u >= 2 * tiles) - (u >= 3 * tiles) : 0; };
+    auto unit_row = [&](int u, int ph) { return (BWD ? u - (3 - ph) * tiles : u) * kUmmaM; };
+
+    // ---- the loads' cursor: unit pu, slice pkb; this thread's chunk column and rows (Cin = 2, one slice of
+    // four columns: one row, columns kc and kc + 2, uniform in a warp)
+    const bool pairs = !BWD && g.Cin == 2;
+    const int kc = pairs ? threadIdx.x >> 7 : threadIdx.x & 7;
+    const int row0 = pairs ? threadIdx.x & 127 : threadIdx.x >> 3;
+    int pu = blockIdx.x, pkb = 0, pph = 0;
+    int base[R];        // the rows' pixels of x (their middle taps)
+    uint32_t edge = 0;  // bits 4 r, 4 r + 1: row r's pixel on the low (BWD: high) edge in y, x; 4 r + 2: no row
+    auto set_unit = [&]() {
+        if (pu >= units) return;
+        pph = unit_class(pu);
+        const int m0 = unit_row(pu, pph);
+        edge = 0;
 #pragma unroll
-        for (int j = 0; j < kUmmaBK / 8 / (kUmmaT / kUmmaM); j++) {
-            const int kc = part + (kUmmaT / kUmmaM) * j;
-            unsigned char *dst = sA[st2] + 16 * (kc * kUmmaM + row);
-            const int k8 = k0 + kc * 8;
-            if constexpr (BWD) {
-                // 8 consecutive k = 8 output channels of one tap (Cout is a multiple of 8)
-                const bf16 *src = x;
-                uint32_t bytes = 0;
-                if (mvalid && kc < kchunks) {
-                    const int t = k8 / g.Cout, co = k8 - t * g.Cout, ty = t / ntx, tx = t - ty * ntx;
-                    const int ho2 = ho + py * (1 - ty), wo2 = wo + px * (1 - tx);
-                    if (ho2 < g.Ho && wo2 < g.Ho) {
-                        src = x + (((int64_t)b * g.Ho + ho2) * g.Ho + wo2) * g.Cout + co;
-                        bytes = 16;
-                    }
-                }
-                cp_async16(dst, src, bytes);
-            } else if ((g.Cin & 7) == 0) {
-                const bf16 *src = x;
-                uint32_t bytes = 0;
-                if (mvalid && kc < kchunks && k8 < g.K) {
-                    const int tap = k8 / g.Cin, ci = k8 - tap * g.Cin;
-                    const int hi = 2 * ho + tap / 3 - 1, wi = 2 * wo + tap % 3 - 1;
-                    if (hi >= 0 && hi < g.H && wi >= 0 && wi < g.H) {
-                        src = x + (((int64_t)b * g.H + hi) * g.H + wi) * g.Cin + ci;
-                        bytes = 16;
-                    }
-                }
-                cp_async16(dst, src, bytes);
-            } else if (g.Cin == 2) {
-                // 8 consecutive k = 4 taps x 2 channels: four 4-byte loads
-                uint32_t v[4] = {0u, 0u, 0u, 0u};
-                if (mvalid && kc < kchunks) {
-#pragma unroll
-                    for (int t = 0; t < 4; t++) {
-                        const int tap = (k8 >> 1) + t;
-                        if (2 * tap < g.K) {
-                            const int hi = 2 * ho + tap / 3 - 1, wi = 2 * wo + tap % 3 - 1;
-                            if (hi >= 0 && hi < g.H && wi >= 0 && wi < g.H)
-                                v[t] = *reinterpret_cast<const uint32_t *>(x + (((int64_t)b * g.H + hi) * g.H + wi) * 2);
-                        }
-                    }
-                }
-                *reinterpret_cast<uint4 *>(dst) = make_uint4(v[0], v[1], v[2], v[3]);
-            } else {
-                uint4 va = make_uint4(0, 0, 0, 0);
-                if (mvalid && kc < kchunks) va = im2col8(x, g, b, ho, wo, k8);
-                *reinterpret_cast<uint4 *>(dst) = va;
-            }
+        for (int r = 0; r < R; r++) {
+            const int m = m0 + row0 + kConvT / 8 * r;
+            const int b = m >> (2 * lside), i = (m >> lside) & (side - 1), j = m & (side - 1);
+            const int e = BWD ? side - 1 : 0;
+            base[r] = BWD ? m : (b * g.H + 2 * i) * g.H + 2 * j;
+            edge |= ((i == e ? 1u : 0u) | (j == e ? 2u : 0u) | (m >= M ? 4u : 0u)) << (4 * r);
         }
-        for (int c = threadIdx.x; c < N * (kUmmaBK / 8); c += kUmmaT) {
-            const int co = c % N, kc = c / N;
-            const bool v = kc < kchunks;
-            cp_async16(sB[st2] + 16 * (kc * N + co),
-                       v ? w + (int64_t)(co0 + co) * wstride + woff + k0 + kc * 8 : w, v ? 16u : 0u);
-        }
-        asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    load_slice(0, 0);
-    for (int kb = 0; kb < nk; kb++) {
-        const int st = kb & 1;
-        const int kchunks = min(kUmmaBK, KT - kb * kUmmaBK) >> 3;
-        if (kb + 1 < nk) {
-            // stage (kb + 1) & 1 is free once the MMAs of slice kb - 1 are done
-            if (kb >= 1 && !*gave_up &&
-                !mbar_wait_bounded(&bars[(kb + 1) & 1], (uint32_t)((kb - 1) >> 1) & 1u, kWaitLimitNs))
-                *gave_up = 1;
-            load_slice(kb + 1, (kb + 1) & 1);
-            asm volatile("cp.async.wait_group 1;" ::: "memory");  // slice kb has landed
-        } else {
-            asm volatile("cp.async.wait_group 0;" ::: "memory");
-        }
-        fence_proxy_async_smem();  // this thread's copies and stores, before the tensor cores read them
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        __syncthreads();
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        if (threadIdx.x == 0 && !*gave_up) {
+    // the cursor's slice into registers, zeros outside the image and past K; the cursor moves on
+    uint4 va[R], vb[RB];
+    const int bc = threadIdx.x & 7, brow = threadIdx.x >> 3;
+    auto fetch = [&]() {
+        if (pu >= units) return;
+        const int k0 = pkb * kUmmaBK, KT = unit_k(pph), k8 = k0 + 8 * kc;
+        int woff = 0;
+        if (pairs) {
+            // 8 consecutive k = 4 taps x 2 channels: four 4-byte loads
 #pragma unroll
-            for (int j = 0; j < kUmmaBK / 16; j++) {
-                if (2 * j >= kchunks) break;  // a half slice: two instructions
-                const uint64_t da = umma_smem_desc(smem_addr(sA[st]) + j * 2 * 16 * kUmmaM, 16 * kUmmaM, 128);
-                const uint64_t db = umma_smem_desc(smem_addr(sB[st]) + j * 2 * 16 * N, 16 * N, 128);
-                const uint32_t acc = (kb > 0 || j > 0) ? 1u : 0u;
-                asm volatile(
-                    "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                    "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tacc),
-                    "l"(da), "l"(db), "r"(idesc), "r"(acc)
-                    : "memory");
+            for (int h = 0; h < 2; h++) {
+                uint32_t v[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+                for (int t = 0; t < 4; t++) {
+                    const int tap = 4 * (kc + 2 * h) + t, ky = tap / 3, kx = tap - 3 * ky;
+                    const uint32_t out = (ky == 0 ? 1u : 0u) | (kx == 0 ? 2u : 0u) | 4u;
+                    if (tap < 9 && !(edge & out))
+                        v[t] = __ldg(reinterpret_cast<const uint32_t *>(x + 2 * (int64_t)(base[0] + (ky - 1) * g.H + kx - 1)));
+                }
+                va[h] = make_uint4(v[0], v[1], v[2], v[3]);
             }
-            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                             smem_addr(&bars[st]))
-                         : "memory");
+        } else {
+            // 8 consecutive k = 8 channels of one tap
+            const int tap = k8 >> lch, ch = k8 & ((1 << lch) - 1);
+            int off;
+            uint32_t out;  // the tap leaves the image for rows on these edges
+            if constexpr (BWD) {
+                const int py = pph >> 1, px = pph & 1, ty = tap >> px, tx = tap & px;
+                const int dy = py & ~ty, dx = px & ~tx;  // py (1 - ty), px (1 - tx)
+                off = dy * side + dx;
+                out = (uint32_t)(dy | dx << 1) | 4u;
+                const int t0 = k0 >> lch, ty0 = t0 >> px, tx0 = t0 & px;  // a slice lies inside one tap
+                woff = (3 * (py ? 2 * ty0 : 1) + (px ? 2 * tx0 : 1) - t0) * g.Cout;
+            } else {
+                const int ky = tap / 3, kx = tap - 3 * ky;
+                off = (ky - 1) * g.H + kx - 1;
+                out = (ky == 0 ? 1u : 0u) | (kx == 0 ? 2u : 0u) | 4u;
+            }
+#pragma unroll
+            for (int r = 0; r < R; r++) {
+                va[r] = make_uint4(0u, 0u, 0u, 0u);
+                if (k8 < KT && !((edge >> (4 * r)) & out))
+                    va[r] = __ldg(reinterpret_cast<const uint4 *>(x + ((int64_t)(base[r] + off) << lch) + ch));
+            }
         }
-    }
-    // the last commit tracks every MMA issued before it
-    const int last = nk - 1;
-    if (!*gave_up && !mbar_wait_bounded(&bars[last & 1], (uint32_t)(last >> 1) & 1u, kWaitLimitNs)) *gave_up = 1;
-    const bool ok = __syncthreads_and(*gave_up == 0) != 0;  // the same decision in every warp
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    if (!ok) {
-        // a wait gave up: the tensor cores may still be writing the accumulator; give the last
-        // commit one more bounded wait before the columns are freed
-        if (threadIdx.x == 0) {
-            atomicOr(status, 1u);
-            mbar_wait_bounded(&bars[last & 1], (uint32_t)(last >> 1) & 1u, kWaitLimitNs);
+        const bf16 *wp = w + (int64_t)(co0 + brow) * wstride + woff + k0 + 8 * bc;
+#pragma unroll
+        for (int r = 0; r < RB; r++) {
+            vb[r] = make_uint4(0u, 0u, 0u, 0u);
+            if (k0 + 8 * bc < KT) vb[r] = __ldg(reinterpret_cast<const uint4 *>(wp + (int64_t)(kConvT / 8) * r * wstride));
         }
-    } else {
-        // warp w reads TMEM lanes 32 (w % 4) .. + 31 (its output rows) and every (T / 128)-th group
-        // of 32 columns from group w / 4
+        if ((++pkb) * kUmmaBK >= KT) {
+            pkb = 0;
+            pu += gridDim.x;
+            set_unit();
+        }
+    };
+    // the fetched slice into stage st2
+    auto put = [&](int st2) {
+        unsigned char *dst = smem + st2 * kA + kColA * kc + 16 * row0;
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+            if (!pairs) *reinterpret_cast<uint4 *>(dst + 16 * (kConvT / 8) * r) = va[r];
+            else if (r < 2) *reinterpret_cast<uint4 *>(dst + 2 * kColA * r) = va[r];
+        }
+#pragma unroll
+        for (int r = 0; r < RB; r++)
+            *reinterpret_cast<uint4 *>(sB + st2 * kB + kColB * bc + 16 * (brow + kConvT / 8 * r)) = vb[r];
+    };
+    set_unit();
+    fetch();
+    put(0);
+    fetch();
+    int st = 0, par = 0;      // stage and barrier parity of the current slice
+    int pst = 0, pp = 0;      // of the slice before it
+    int lst = 1, lpar = 1;    // stage of the fetched slice, parity of the slice that was in it
+    bool reused = false;      // the stages hold earlier slices
+    for (int u = blockIdx.x; u < units; u += gridDim.x) {
+        const int ph = unit_class(u), KT = unit_k(ph);
+        const int m0 = unit_row(u, ph);
+        for (int k0 = 0; k0 < KT; k0 += kUmmaBK) {
+            // the stage is free once the MMAs of the slice that was in it are done
+            if (reused && !*gave_up && !mbar_wait_bounded(&bars[lst], (uint32_t)lpar, kWaitLimitNs)) *gave_up = 1;
+            put(lst);
+            if (++lst == S) {
+                lst = 0;
+                lpar ^= 1;
+                reused = true;
+            }
+            fence_proxy_async_smem();  // this thread's stores, before the tensor cores read them
+            fetch();
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncthreads();
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            if (threadIdx.x == 0 && !*gave_up) {
+                const uint32_t a0 = smem_addr(smem + st * kA), b0 = smem_addr(sB + st * kB);
+#pragma unroll
+                for (int j = 0; j < kUmmaBK / 16; j++) {
+                    if (k0 + 16 * j >= KT) break;  // a half slice: two instructions
+                    const uint64_t da = umma_smem_desc(a0 + 2 * j * kColA, kColA, 128);
+                    const uint64_t db = umma_smem_desc(b0 + 2 * j * kColB, kColB, 128);
+                    const uint32_t acc = (k0 > 0 || j > 0) ? 1u : 0u;
+                    asm volatile(
+                        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+                        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tacc),
+                        "l"(da), "l"(db), "r"(idesc), "r"(acc)
+                        : "memory");
+                }
+                asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
+                                 smem_addr(&bars[st]))
+                             : "memory");
+            }
+            pst = st;
+            pp = par;
+            if (++st == S) {
+                st = 0;
+                par ^= 1;
+            }
+        }
+        // warp w reads TMEM lanes 32 (w % 4) .. + 31 (its output rows) and every second group of 8 columns
+        // from group w / 4
         const int mr = m0 + 32 * (warp & 3) + lane;  // the row; its pixel mo
         int mo = mr;
         if constexpr (BWD) {
-            const int bb = mr / (side * side), r = mr - bb * side * side, i = r / side, j = r - i * side;
-            mo = (bb * g.H + 2 * i + py) * g.H + 2 * j + px;
+            const int bb = mr >> (2 * lside), i = (mr >> lside) & (side - 1), j = mr & (side - 1);
+            mo = (bb * g.H + 2 * i + (ph >> 1)) * g.H + 2 * j + (ph & 1);
         }
-#pragma unroll 1
-        for (int c0 = 32 * (warp >> 2); c0 < N; c0 += 32 * (kUmmaT / kUmmaM)) {
-            uint32_t r[32];
-            asm volatile(
-                "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, "
-                "%14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-                  "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]),
-                  "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]),
-                  "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]),
-                  "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-                : "r"(tacc + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)c0));
+        constexpr int E = N / (kConvT / kUmmaM * 8);  // groups of a warp
+        constexpr int EP = BWD && E <= 4 ? E : 1;     // the previous layer's ReLU mask of up to 4 groups, ahead
+        uint4 pv[EP];
+        if (BWD && E <= 4 && mr < M) {
+#pragma unroll
+            for (int e = 0; e < EP; e++)
+                pv[e] = *reinterpret_cast<const uint4 *>(mask + (int64_t)mo * CO + co0 + 8 * (warp >> 2) + 16 * e);
+        }
+        // the unit's last commit tracks every MMA issued before it
+        if (!*gave_up && !mbar_wait_bounded(&bars[pst], (uint32_t)pp, kWaitLimitNs)) *gave_up = 1;
+        const bool ok = __syncthreads_and(*gave_up == 0) != 0;  // the same decision in every warp
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        if (!ok) {
+            // a wait gave up: the tensor cores may still be writing the accumulator; give the last
+            // commit one more bounded wait before the columns are freed
+            if (threadIdx.x == 0) {
+                atomicOr(status, 1u);
+                mbar_wait_bounded(&bars[pst], (uint32_t)pp, kWaitLimitNs);
+            }
+            break;
+        }
+#pragma unroll
+        for (int e = 0; e < E; e++) {
+            const int c0 = 8 * (warp >> 2) + 16 * e;
+            const int64_t o0 = (int64_t)mo * CO + co0 + c0;
+            if (BWD && E > 4 && mr < M) pv[0] = *reinterpret_cast<const uint4 *>(mask + o0);
+            uint32_t r[8];
+            asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                         : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
+                           "=r"(r[7])
+                         : "r"(tacc + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)c0));
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
             if (mr < M) {
-#pragma unroll
-                for (int q = 0; q < 4; q++) {
-                    const int64_t o0 = (int64_t)mo * CO + co0 + c0 + 8 * q;
-                    __nv_bfloat162 o[4];
-                    if constexpr (BWD) {  // the previous layer's ReLU mask
-                        const uint4 pv = *reinterpret_cast<const uint4 *>(mask + o0);
-                        const __nv_bfloat162 *pm = reinterpret_cast<const __nv_bfloat162 *>(&pv);
-#pragma unroll
-                        for (int i = 0; i < 4; i++) {
-                            const float2 pf = __bfloat1622float2(pm[i]);
-                            const int c = 8 * q + 2 * i;
-                            o[i] = __floats2bfloat162_rn(pf.x > 0.0f ? __uint_as_float(r[c]) : 0.0f,
-                                                         pf.y > 0.0f ? __uint_as_float(r[c + 1]) : 0.0f);
-                        }
-                    } else {
-#pragma unroll
-                        for (int i = 0; i < 4; i++) {
-                            const int c = 8 * q + 2 * i;
-                            o[i] = __floats2bfloat162_rn(fmaxf(__uint_as_float(r[c]) + bias[co0 + c0 + c], 0.0f),
-                                                         fmaxf(__uint_as_float(r[c + 1]) + bias[co0 + c0 + c + 1], 0.0f));
-                        }
-                    }
-                    *reinterpret_cast<uint4 *>(y + o0) = *reinterpret_cast<const uint4 *>(o);
+                __nv_bfloat162 o[4];
+                const __nv_bfloat162 *pm = reinterpret_cast<const __nv_bfloat162 *>(&pv[E <= 4 && BWD ? e : 0]);
+                float4 bv[2] = {};
+                if (!BWD) {
+                    bv[0] = __ldg(reinterpret_cast<const float4 *>(bias + co0 + c0));
+                    bv[1] = __ldg(reinterpret_cast<const float4 *>(bias + co0 + c0) + 1);
                 }
+                const float *bc = reinterpret_cast<const float *>(bv);
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    const float r0 = __uint_as_float(r[2 * i]), r1 = __uint_as_float(r[2 * i + 1]);
+                    if constexpr (BWD) {
+                        const float2 pf = __bfloat1622float2(pm[i]);
+                        o[i] = __floats2bfloat162_rn(pf.x > 0.0f ? r0 : 0.0f, pf.y > 0.0f ? r1 : 0.0f);
+                    } else {
+                        o[i] = __floats2bfloat162_rn(fmaxf(r0 + bc[2 * i], 0.0f), fmaxf(r1 + bc[2 * i + 1], 0.0f));
+                    }
+                }
+                *reinterpret_cast<uint4 *>(y + o0) = *reinterpret_cast<const uint4 *>(o);
             }
         }
+        // the next unit's first MMA, after its slice's barrier, overwrites the accumulator read here
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tacc), "r"(N));
 }
 
-// Dynamic shared memory of conv_umma_kernel<N, BWD>: two stages of A and B, the barriers and the
-// TMEM address, rounded up where needed so that at most 512 / N CTAs share an SM (the TMEM
-// columns of all resident CTAs then fit; no allocation waits).  At 512 threads per CTA at most 4
-// CTAs are resident anyway.
+// Dynamic shared memory of conv_umma_kernel<N, BWD>: the stages of A and B, the barriers and the TMEM
+// address.  All resident CTAs' TMEM columns fit by shared memory: at most three CTAs up to N = 64, two of
+// N = 128, one of N = 256 (no allocation waits).
 static size_t umma_fwd_smem(int N) {
-    const size_t need = 2 * (size_t)(kUmmaM + N) * kUmmaBK * 2 + 64;
-    const size_t per_sm = 228 * 1024, cap = (size_t)(512 / N);
-    if (cap >= (size_t)(2048 / kUmmaT)) return need;
-    const size_t floor_for_cap = per_sm / (cap + 1) + 1024;
-    return std::max(need, std::min(floor_for_cap, (size_t)227 * 1024));
+    return kConvS * (size_t)(kUmmaM + 1 + N + 1) * kUmmaBK * 2 + 8 * kConvS + 16;
 }
 
 template <int N, bool BWD>
 static cudaError_t launch_umma_n(const bf16 *x, const bf16 *w, const float *bias, const bf16 *mask, bf16 *y,
-                                 const ConvGeom &g, int blocks, int channels, unsigned int *status, cudaStream_t s) {
+                                 const ConvGeom &g, int blocks, int channels, unsigned int *status, cudaStream_t s,
+                                 int sms) {
     const size_t smem = umma_fwd_smem(N);
     cudaError_t e = cudaFuncSetAttribute(conv_umma_kernel<N, BWD>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)smem);
     if (e != cudaSuccess) return e;
-    conv_umma_kernel<N, BWD><<<dim3(blocks, channels / N, BWD ? 4 : 1), kUmmaT, smem, s>>>(x, w, bias, mask, y, g,
-                                                                                           status);
+    const int units = blocks * (BWD ? 4 : 1), ny = channels / N;
+    const int resident = sms * (N >= 256 ? 1 : N >= 128 ? 2 : kConvCtas);
+    const int grid = std::max(1, std::min(units, resident / ny));
+    conv_umma_kernel<N, BWD><<<dim3(grid, ny), kConvT, smem, s>>>(x, w, bias, mask, y, g, blocks, units, status);
     return cudaGetLastError();
 }
 
@@ -499,24 +533,26 @@ static cudaError_t launch_umma_n(const bf16 *x, const bf16 *w, const float *bias
 // of 64 (the A tile is then gathered once per channel tile).
 static cudaError_t launch_conv_umma(bool bwd, const bf16 *x, const bf16 *w, const float *bias, const bf16 *mask,
                                     bf16 *y, const ConvGeom &g, unsigned int *status, cudaStream_t s, int sms) {
-    // the data gradient runs the four parity classes of input pixels as grid.z (stride 2, H even)
-    if (bwd && ((g.H & 1) || g.Ho != g.H / 2 || (g.Cout & 63))) return cudaErrorInvalidValue;
+    // the data gradient runs the four parity classes of input pixels as units of their own (stride 2, H even)
+    auto pow2 = [](int v) { return v > 0 && (v & (v - 1)) == 0; };
+    if ((g.H & 1) || g.Ho != g.H / 2 || !pow2(g.Ho) || !pow2(g.Cin) || !pow2(g.Cout)) return cudaErrorInvalidValue;
+    if (bwd ? (g.Cout & 63) != 0 : g.Cin != 2 && (g.Cin & 31)) return cudaErrorInvalidValue;
     const int side = bwd ? g.H / 2 : g.Ho, channels = bwd ? g.Cin : g.Cout;
     const int blocks = (g.n * side * side + kUmmaM - 1) / kUmmaM;
     const int nt = (channels > 64 && blocks * (bwd ? 4 : 1) < 2 * sms) ? 64 : channels;
     if (bwd) {
         switch (nt) {
-            case 32: return launch_umma_n<32, true>(x, w, bias, mask, y, g, blocks, channels, status, s);
-            case 64: return launch_umma_n<64, true>(x, w, bias, mask, y, g, blocks, channels, status, s);
-            case 128: return launch_umma_n<128, true>(x, w, bias, mask, y, g, blocks, channels, status, s);
+            case 32: return launch_umma_n<32, true>(x, w, bias, mask, y, g, blocks, channels, status, s, sms);
+            case 64: return launch_umma_n<64, true>(x, w, bias, mask, y, g, blocks, channels, status, s, sms);
+            case 128: return launch_umma_n<128, true>(x, w, bias, mask, y, g, blocks, channels, status, s, sms);
             default: return cudaErrorInvalidValue;
         }
     }
     switch (nt) {
-        case 32: return launch_umma_n<32, false>(x, w, bias, mask, y, g, blocks, channels, status, s);
-        case 64: return launch_umma_n<64, false>(x, w, bias, mask, y, g, blocks, channels, status, s);
-        case 128: return launch_umma_n<128, false>(x, w, bias, mask, y, g, blocks, channels, status, s);
-        case 256: return launch_umma_n<256, false>(x, w, bias, mask, y, g, blocks, channels, status, s);
+        case 32: return launch_umma_n<32, false>(x, w, bias, mask, y, g, blocks, channels, status, s, sms);
+        case 64: return launch_umma_n<64, false>(x, w, bias, mask, y, g, blocks, channels, status, s, sms);
+        case 128: return launch_umma_n<128, false>(x, w, bias, mask, y, g, blocks, channels, status, s, sms);
+        case 256: return launch_umma_n<256, false>(x, w, bias, mask, y, g, blocks, channels, status, s, sms);
         default: return cudaErrorInvalidValue;
     }
 }
@@ -528,22 +564,23 @@ static cudaError_t launch_conv_umma(bool bwd, const bf16 *x, const bf16 *w, cons
 // for K <= k < Kp, and 1 for k = Kp, so that accumulator row Kp is the bias gradient.  Both
 // operands are MN-major in shared memory: the natural 16-byte chunk (8 consecutive k, or 8
 // channels, of one pixel) is one row of a core matrix, chunk (pixel p, chunk column c) at
-// 1024 c + 16 p bytes; descriptor strides: between pixel groups of 8 (LBO, the K direction) 128
-// bytes, between chunk columns (SBO, the M / N direction) 1024 bytes.  The epilogue writes
+// 1040 c + 16 p bytes; descriptor strides: between pixel groups of 8 (LBO, the K direction) 128
+// bytes, between chunk columns (SBO, the M / N direction) 1040 bytes, so that 8 neighbouring lanes copy
+// 128 contiguous bytes of one pixel into 8 different bank groups.  Slices pass through registers as in the forward.  The epilogue writes
 // part[z][co][k] (k < Kp) and partb[z][co] (k = Kp), summed over splits in a fixed order after.
 template <int N>
-__global__ void __launch_bounds__(kUmmaT) conv_wgrad_umma_kernel(const bf16 *__restrict__ dy,
+__global__ void __launch_bounds__(kUmmaT, 2) conv_wgrad_umma_kernel(const bf16 *__restrict__ dy,
                                                                  const bf16 *__restrict__ x, float *__restrict__ part,
                                                                  float *__restrict__ partb, const ConvGeom g,
                                                                  int slices_per_split,
                                                                  unsigned int *__restrict__ status) {
     static_assert(N >= 32 && N <= 256 && (N & (N - 1)) == 0, "TMEM columns: a power of two, 32..256");
-    constexpr int kA = kUmmaM * 64 * 2, kB = N * 64 * 2;  // bytes per stage: 128 rows k / N channels x 64 pixels
+    constexpr int S = kUmmaS, kCol = 16 * 65;                   // stages, bytes between chunk columns
+    constexpr int kA = kUmmaM / 8 * kCol, kB = N / 8 * kCol;  // per stage: 128 rows k / N channels x 64 pixels
     extern __shared__ __align__(1024) unsigned char smem[];
-    unsigned char *sA[2] = {smem, smem + kA};
-    unsigned char *sB[2] = {smem + 2 * kA, smem + 2 * kA + kB};
-    uint64_t *bars = reinterpret_cast<uint64_t *>(smem + 2 * kA + 2 * kB);
-    uint32_t *tslot = reinterpret_cast<uint32_t *>(bars + 2);
+    unsigned char *sB = smem + S * kA;
+    uint64_t *bars = reinterpret_cast<uint64_t *>(smem + S * (kA + kB));
+    uint32_t *tslot = reinterpret_cast<uint32_t *>(bars + S);
     volatile int *gave_up = reinterpret_cast<volatile int *>(tslot + 1);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int P = g.n * g.Ho * g.Ho, k0 = blockIdx.x * kUmmaM;
@@ -555,13 +592,15 @@ __global__ void __launch_bounds__(kUmmaT) conv_wgrad_umma_kernel(const bf16 *__r
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
     if (threadIdx.x == 0) {
-        mbar_init(&bars[0], 1);
-        mbar_init(&bars[1], 1);
+        for (int i = 0; i < S; i++) mbar_init(&bars[i], 1);
         fence_mbar_init();
         *gave_up = 0;
     }
     // chunk columns of A past K hold the same values for every pixel: zeros, and the 1 of row Kp
-    const int pl = threadIdx.x & 63, cg = threadIdx.x >> 6;  // this thread's pixel in a slice, first chunk column
+    // this thread's pixel in a slice and first chunk column (Cin = 2, three columns: uniform in a warp)
+    const bool pairs = g.Cin == 2;
+    const int pl = pairs ? threadIdx.x & 63 : threadIdx.x >> 3, cg = pairs ? threadIdx.x >> 6 : threadIdx.x & 7;
+    const int lside = 31 - __clz(g.Ho), lch = 31 - __clz(g.Cin);  // powers of two, as in the forward
     const int kreal = (g.K - k0 + 7) >> 3;                    // chunk columns with im2col values (may be <= 0)
 #pragma unroll
     for (int j = 0; j < 2; j++) {
@@ -577,8 +616,7 @@ __global__ void __launch_bounds__(kUmmaT) conv_wgrad_umma_kernel(const bf16 *__r
                 else if (word == 2) v.z = one;
                 else v.w = one;
             }
-            *reinterpret_cast<uint4 *>(sA[0] + 1024 * c + 16 * pl) = v;
-            *reinterpret_cast<uint4 *>(sA[1] + 1024 * c + 16 * pl) = v;
+            for (int i = 0; i < S; i++) *reinterpret_cast<uint4 *>(smem + i * kA + kCol * c + 16 * pl) = v;
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -586,82 +624,80 @@ __global__ void __launch_bounds__(kUmmaT) conv_wgrad_umma_kernel(const bf16 *__r
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tacc = *tslot;
     constexpr uint32_t idesc = umma_idesc_bf16(kUmmaM, N) | (1u << 15) | (1u << 16);  // A and B MN-major
-    // one slice of 64 pixels into stage st2: A's im2col chunks and B's dy chunks by cp.async
-    // (zero fill outside the image and past the last pixel), Cin = 2 through registers
-    auto load_slice = [&](int si, int st2) {
+    // slice si (64 pixels) into registers: A's im2col chunks and B's dy chunks, zeros outside the image and
+    // past the last pixel
+    constexpr int RB = (N * 8 + kUmmaT - 1) / kUmmaT;
+    uint4 va[2], vb[RB];
+    auto fetch = [&](int si) {
+        if (si >= ns) return;
         const int p = (s_begin + si) * 64 + pl;
         const bool pv = p < P;
-        int b = 0, ho = 0, wo = 0;
-        if (pv) {
-            b = p / (g.Ho * g.Ho);
-            const int r = p - b * g.Ho * g.Ho;
-            ho = r / g.Ho;
-            wo = r - ho * g.Ho;
-        }
+        const int b = p >> (2 * lside), ho = (p >> lside) & (g.Ho - 1), wo = p & (g.Ho - 1);
+        const int base = (b * g.H + 2 * ho) * g.H + 2 * wo;
 #pragma unroll
         for (int j = 0; j < 2; j++) {
-            const int c = cg + 8 * j;
-            if (c < kreal) {
-                unsigned char *dst = sA[st2] + 1024 * c + 16 * pl;
-                const int k8 = k0 + 8 * c;
-                if ((g.Cin & 7) == 0) {
-                    const bf16 *src = x;
-                    uint32_t bytes = 0;
-                    if (pv) {
-                        const int tap = k8 / g.Cin, ci = k8 - tap * g.Cin;
-                        const int hi = 2 * ho + tap / 3 - 1, wi = 2 * wo + tap % 3 - 1;
-                        if (hi >= 0 && hi < g.H && wi >= 0 && wi < g.H) {
-                            src = x + (((int64_t)b * g.H + hi) * g.H + wi) * g.Cin + ci;
-                            bytes = 16;
-                        }
-                    }
-                    cp_async16(dst, src, bytes);
-                } else if (g.Cin == 2) {
-                    uint32_t v[4] = {0u, 0u, 0u, 0u};
-                    if (pv) {
+            const int c = cg + 8 * j, k8 = k0 + 8 * c;
+            if (c >= kreal) continue;
+            if (pairs) {
+                uint32_t v[4] = {0u, 0u, 0u, 0u};
 #pragma unroll
-                        for (int t = 0; t < 4; t++) {
-                            const int tap = (k8 >> 1) + t;
-                            if (2 * tap < g.K) {
-                                const int hi = 2 * ho + tap / 3 - 1, wi = 2 * wo + tap % 3 - 1;
-                                if (hi >= 0 && hi < g.H && wi >= 0 && wi < g.H)
-                                    v[t] = *reinterpret_cast<const uint32_t *>(
-                                        x + (((int64_t)b * g.H + hi) * g.H + wi) * 2);
-                            }
-                        }
-                    }
-                    *reinterpret_cast<uint4 *>(dst) = make_uint4(v[0], v[1], v[2], v[3]);
-                } else {
-                    *reinterpret_cast<uint4 *>(dst) = pv ? im2col8(x, g, b, ho, wo, k8) : make_uint4(0, 0, 0, 0);
+                for (int t = 0; t < 4; t++) {
+                    const int tap = (k8 >> 1) + t, ky = tap / 3, kx = tap - 3 * ky;
+                    if (pv && tap < 9 && (ky > 0 || ho > 0) && (kx > 0 || wo > 0))
+                        v[t] = __ldg(reinterpret_cast<const uint32_t *>(x + 2 * (int64_t)(base + (ky - 1) * g.H + kx - 1)));
                 }
+                va[j] = make_uint4(v[0], v[1], v[2], v[3]);
+            } else {
+                const int tap = k8 >> lch, ci = k8 & (g.Cin - 1), ky = tap / 3, kx = tap - 3 * ky;
+                va[j] = make_uint4(0u, 0u, 0u, 0u);
+                if (pv && (ky > 0 || ho > 0) && (kx > 0 || wo > 0))
+                    va[j] = __ldg(reinterpret_cast<const uint4 *>(
+                        x + ((int64_t)(base + (ky - 1) * g.H + kx - 1) << lch) + ci));
             }
         }
-        for (int c = cg; c < N / 8; c += 8)
-            cp_async16(sB[st2] + 1024 * c + 16 * pl, pv ? dy + (int64_t)p * g.Cout + 8 * c : dy, pv ? 16u : 0u);
-        asm volatile("cp.async.commit_group;" ::: "memory");
+#pragma unroll
+        for (int r = 0; r < RB; r++) {
+            const int i = threadIdx.x + kUmmaT * r, c = i % (N / 8), pg = (s_begin + si) * 64 + i / (N / 8);
+            vb[r] = make_uint4(0u, 0u, 0u, 0u);
+            if (i < N * 8 && pg < P) vb[r] = __ldg(reinterpret_cast<const uint4 *>(dy + (int64_t)pg * g.Cout + 8 * c));
+        }
     };
-    load_slice(0, 0);
+    // the fetched slice into stage st2
+    auto put = [&](int st2) {
+#pragma unroll
+        for (int j = 0; j < 2; j++)
+            if (cg + 8 * j < kreal) *reinterpret_cast<uint4 *>(smem + st2 * kA + kCol * (cg + 8 * j) + 16 * pl) = va[j];
+#pragma unroll
+        for (int r = 0; r < RB; r++) {
+            const int i = threadIdx.x + kUmmaT * r;
+            if (i < N * 8) *reinterpret_cast<uint4 *>(sB + st2 * kB + kCol * (i % (N / 8)) + 16 * (i / (N / 8))) = vb[r];
+        }
+    };
+    fetch(0);
+    put(0);
+    fetch(1);
+    int st = 0, par = 0, pst = 0, pp = 0;  // stage and parity of this slice, of the one before it
+    int lst = 1, lpar = 1;  // stage of the fetched slice, parity of the slice that was in it
+    bool reused = false;    // the stages hold earlier slices
     for (int si = 0; si < ns; si++) {
-        const int st = si & 1;
-        if (si + 1 < ns) {
-            // stage (si + 1) & 1 is free once the MMAs of slice si - 1 are done
-            if (si >= 1 && !*gave_up &&
-                !mbar_wait_bounded(&bars[(si + 1) & 1], (uint32_t)((si - 1) >> 1) & 1u, kWaitLimitNs))
-                *gave_up = 1;
-            load_slice(si + 1, (si + 1) & 1);
-            asm volatile("cp.async.wait_group 1;" ::: "memory");
-        } else {
-            asm volatile("cp.async.wait_group 0;" ::: "memory");
+        // the stage is free once the MMAs of the slice that was in it are done
+        if (reused && !*gave_up && !mbar_wait_bounded(&bars[lst], (uint32_t)lpar, kWaitLimitNs)) *gave_up = 1;
+        if (si + 1 < ns) put(lst);
+        if (++lst == S) {
+            lst = 0;
+            lpar ^= 1;
+            reused = true;
         }
         fence_proxy_async_smem();
+        fetch(si + 2);
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         __syncthreads();
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         if (threadIdx.x == 0 && !*gave_up) {
 #pragma unroll
             for (int j = 0; j < 4; j++) {  // K = 16 pixels per instruction: pixel groups 2 j, 2 j + 1
-                const uint64_t da = umma_smem_desc(smem_addr(sA[st]) + 256 * j, 128, 1024);
-                const uint64_t db = umma_smem_desc(smem_addr(sB[st]) + 256 * j, 128, 1024);
+                const uint64_t da = umma_smem_desc(smem_addr(smem + st * kA) + 256 * j, 128, kCol);
+                const uint64_t db = umma_smem_desc(smem_addr(sB + st * kB) + 256 * j, 128, kCol);
                 const uint32_t acc = (si > 0 || j > 0) ? 1u : 0u;
                 asm volatile(
                     "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
@@ -673,15 +709,20 @@ __global__ void __launch_bounds__(kUmmaT) conv_wgrad_umma_kernel(const bf16 *__r
                              smem_addr(&bars[st]))
                          : "memory");
         }
+        pst = st;
+        pp = par;
+        if (++st == S) {
+            st = 0;
+            par ^= 1;
+        }
     }
-    const int last = ns - 1;
-    if (!*gave_up && !mbar_wait_bounded(&bars[last & 1], (uint32_t)(last >> 1) & 1u, kWaitLimitNs)) *gave_up = 1;
+    if (!*gave_up && !mbar_wait_bounded(&bars[pst], (uint32_t)pp, kWaitLimitNs)) *gave_up = 1;
     const bool ok = __syncthreads_and(*gave_up == 0) != 0;
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     if (!ok) {
         if (threadIdx.x == 0) {
             atomicOr(status, 1u);
-            mbar_wait_bounded(&bars[last & 1], (uint32_t)(last >> 1) & 1u, kWaitLimitNs);
+            mbar_wait_bounded(&bars[pst], (uint32_t)pp, kWaitLimitNs);
         }
     } else {
         const int k = k0 + 32 * (warp & 3) + lane;  // this thread's accumulator row
@@ -725,7 +766,7 @@ static int wgrad_umma_splits(const ConvGeom &g, int sms, int *slices_per_split) 
 template <int N>
 static cudaError_t launch_wgrad_n(const bf16 *dy, const bf16 *x, float *part, float *partb, const ConvGeom &g,
                                   int splits, int sps, unsigned int *status, cudaStream_t s) {
-    const size_t smem = umma_fwd_smem(N);
+    const size_t smem = kUmmaS * (size_t)(kUmmaM + N) / 8 * 16 * 65 + 8 * kUmmaS + 16;
     cudaError_t e = cudaFuncSetAttribute(conv_wgrad_umma_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)smem);
     if (e != cudaSuccess) return e;
