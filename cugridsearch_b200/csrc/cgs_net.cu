@@ -25,6 +25,7 @@
 #include <cstring>
 #include <random>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "cgs_internal.h"
@@ -904,19 +905,32 @@ __global__ void __launch_bounds__(kThreads) conv_bwd_weight_kernel(const bf16 *_
 }
 
 // dst[i] = sum_z part[z][i] in split order (deterministic).
+__device__ __forceinline__ void sum_splits(const float *__restrict__ part, int splits, int64_t n,
+                                           float *__restrict__ dst, int64_t i) {
+    float s = 0.0f;
+    int z = 0;
+    for (; z + 8 <= splits; z += 8) {  // eight loads in flight, added in split order
+        float v[8];
+#pragma unroll
+        for (int u = 0; u < 8; u++) v[u] = part[(int64_t)(z + u) * n + i];
+#pragma unroll
+        for (int u = 0; u < 8; u++) s += v[u];
+    }
+    for (; z < splits; z++) s += part[(int64_t)z * n + i];
+    dst[i] = s;
+}
+
 __global__ void sum_splits_kernel(const float *__restrict__ part, int splits, int64_t n, float *__restrict__ dst) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        float s = 0.0f;
-        int z = 0;
-        for (; z + 8 <= splits; z += 8) {  // eight loads in flight, added in split order
-            float v[8];
-#pragma unroll
-            for (int u = 0; u < 8; u++) v[u] = part[(int64_t)(z + u) * n + i];
-#pragma unroll
-            for (int u = 0; u < 8; u++) s += v[u];
-        }
-        for (; z < splits; z++) s += part[(int64_t)z * n + i];
-        dst[i] = s;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+        sum_splits(part, splits, n, dst, i);
+}
+
+// A layer's weight and bias gradients in one launch.
+__global__ void sum_splits2_kernel(const float *__restrict__ part, const float *__restrict__ partb, int splits,
+                                   int64_t n, int nb, float *__restrict__ dst, float *__restrict__ dstb) {
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n + nb; i += (int64_t)gridDim.x * blockDim.x) {
+        if (i < n) sum_splits(part, splits, n, dst, i);
+        else sum_splits(partb, splits, nb, dstb, i - n);
     }
 }
 
@@ -965,13 +979,28 @@ __global__ void gap_kernel(const bf16 *__restrict__ y5, int n, float *__restrict
 }
 
 // out[b][j] = act(sum_i w[j][i] in[b][i] + bias[j]); act = ReLU when relu != 0.
+// One output per thread, its products added in order; 16 products' operands are loaded at once (one by one,
+// a strided load of w each, 256 x 256 -> 128 took 25 us).  nin is a multiple of 16.
 __global__ void fc_kernel(const float *__restrict__ in, const float *__restrict__ w, const float *__restrict__ bias,
                           int n, int nin, int nout, int relu, float *__restrict__ out) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n * nout) return;
     const int b = i / nout, j = i - b * nout;
     float s = bias[j];
-    for (int k = 0; k < nin; k++) s = fmaf(w[(int64_t)j * nin + k], in[(int64_t)b * nin + k], s);
+    const float4 *w4 = reinterpret_cast<const float4 *>(w + (int64_t)j * nin);
+    const float4 *in4 = reinterpret_cast<const float4 *>(in + (int64_t)b * nin);
+#pragma unroll 2
+    for (int k = 0; k < nin / 4; k += 4) {
+        float4 u[4], v[4];
+#pragma unroll
+        for (int t = 0; t < 4; t++) {
+            u[t] = w4[k + t];
+            v[t] = in4[k + t];
+        }
+#pragma unroll
+        for (int t = 0; t < 4; t++)
+            s = fmaf(u[t].w, v[t].w, fmaf(u[t].z, v[t].z, fmaf(u[t].y, v[t].y, fmaf(u[t].x, v[t].x, s))));
+    }
     out[i] = relu ? fmaxf(s, 0.0f) : s;
 }
 
@@ -1015,35 +1044,29 @@ __global__ void fc_bwd_weight_kernel(const float *__restrict__ dout, const float
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= nout * (nin + 1)) return;
     const int j = i / (nin + 1), k = i - j * (nin + 1);
-    // summed over the batch in order; the loads of 8 batch rows are issued before their 8
-    // multiply-adds, so the loop waits on memory once per 8 rows instead of once per row
+    // summed over the batch in order; the loads of 32 (8) batch rows are issued before their
+    // multiply-adds, so the loop waits on memory once per 32 rows
     float s = 0.0f;
-    if (k < nin) {
-        int b = 0;
-        for (; b + 8 <= n; b += 8) {
-            float u[8], v[8];
+    int b = 0;
+    const bool bias = k == nin;
+    auto rows = [&](auto count) {
+        constexpr int N = decltype(count)::value;
+        for (; b + N <= n; b += N) {
+            float u[N], v[N];
 #pragma unroll
-            for (int t = 0; t < 8; t++) {
+            for (int t = 0; t < N; t++) {
                 u[t] = dout[(int64_t)(b + t) * nout + j];
-                v[t] = in[(int64_t)(b + t) * nin + k];
+                v[t] = bias ? 1.0f : in[(int64_t)(b + t) * nin + k];
             }
 #pragma unroll
-            for (int t = 0; t < 8; t++) s = fmaf(u[t], v[t], s);
+            for (int t = 0; t < N; t++) s = fmaf(u[t], v[t], s);  // bias: u + s, exactly
         }
-        for (; b < n; b++) s = fmaf(dout[(int64_t)b * nout + j], in[(int64_t)b * nin + k], s);
-        dw[(int64_t)j * nin + k] = s;
-    } else {
-        int b = 0;
-        for (; b + 8 <= n; b += 8) {
-            float u[8];
-#pragma unroll
-            for (int t = 0; t < 8; t++) u[t] = dout[(int64_t)(b + t) * nout + j];
-#pragma unroll
-            for (int t = 0; t < 8; t++) s += u[t];
-        }
-        for (; b < n; b++) s += dout[(int64_t)b * nout + j];
-        db[j] = s;
-    }
+    };
+    rows(std::integral_constant<int, 32>());
+    rows(std::integral_constant<int, 8>());
+    rows(std::integral_constant<int, 1>());
+    if (bias) db[j] = s;
+    else dw[(int64_t)j * nin + k] = s;
 }
 
 // Pooling backward through layer 5's ReLU: dy5[b][p][c] = (y5 > 0) dfeat[b][c] / 16.
@@ -1334,9 +1357,9 @@ cgs_status cgs_net_forward(cgs_net *nt, const float *fixed, const float *moving,
         if (e != cudaSuccess) return cuda_fail(e, "conv_umma_kernel (forward)");
     }
     gap_kernel<<<(n * kFeat + 255) / 256, 256, 0, s>>>(nt->act[kLayers], n, nt->feat);
-    fc_kernel<<<(n * kHid + 255) / 256, 256, 0, s>>>(nt->feat, nt->params + nt->L.fc1w, nt->params + nt->L.fc1b, n,
+    fc_kernel<<<(n * kHid + 63) / 64, 64, 0, s>>>(nt->feat, nt->params + nt->L.fc1w, nt->params + nt->L.fc1b, n,
                                                      kFeat, kHid, 1, nt->hid);
-    fc_kernel<<<(n * kOut + 255) / 256, 256, 0, s>>>(nt->hid, nt->params + nt->L.fc2w, nt->params + nt->L.fc2b, n,
+    fc_kernel<<<(n * kOut + 63) / 64, 64, 0, s>>>(nt->hid, nt->params + nt->L.fc2w, nt->params + nt->L.fc2b, n,
                                                      kHid, kOut, 0, nt->out);
     CGS_CUDA(cudaGetLastError(), "network forward");
     if (out) CGS_CUDA(cudaMemcpyAsync(out, nt->out, (size_t)n * kOut * 4, cudaMemcpyDeviceToDevice, s), "cudaMemcpyAsync");
@@ -1351,11 +1374,11 @@ cgs_status cgs_net_backward(cgs_net *nt, const float *labels, float *loss, cgs_s
     float *G = nt->grads;
     loss_kernel<<<(n + 127) / 128, 128, 0, s>>>(nt->out, labels, n, nt->dout, nt->lossp);
     // fc2, fc1
-    fc_bwd_weight_kernel<<<(kOut * (kHid + 1) + 255) / 256, 256, 0, s>>>(nt->dout, nt->hid, n, kHid, kOut,
+    fc_bwd_weight_kernel<<<(kOut * (kHid + 1) + 127) / 128, 128, 0, s>>>(nt->dout, nt->hid, n, kHid, kOut,
                                                                          G + nt->L.fc2w, G + nt->L.fc2b);
     fc_bwd_input_kernel<<<(n * kHid + 255) / 256, 256, 0, s>>>(nt->dout, nt->params + nt->L.fc2w, nt->hid, n, kHid,
                                                                kOut, 1, nt->dhid);
-    fc_bwd_weight_kernel<<<(kHid * (kFeat + 1) + 255) / 256, 256, 0, s>>>(nt->dhid, nt->feat, n, kFeat, kHid,
+    fc_bwd_weight_kernel<<<(kHid * (kFeat + 1) + 127) / 128, 128, 0, s>>>(nt->dhid, nt->feat, n, kFeat, kHid,
                                                                           G + nt->L.fc1w, G + nt->L.fc1b);
     fc_bwd_input_kernel<<<(n * kFeat + 255) / 256, 256, 0, s>>>(nt->dhid, nt->params + nt->L.fc1w, nt->feat, n,
                                                                 kFeat, kHid, 0, nt->dfeat);
@@ -1380,9 +1403,8 @@ cgs_status cgs_net_backward(cgs_net *nt, const float *labels, float *loss, cgs_s
             float *partb = nt->ws + (int64_t)splits * wn;
             cudaError_t e = launch_conv_wgrad_umma(dy, nt->act[l], nt->ws, partb, g, splits, sps, nt->status, s);
             if (e != cudaSuccess) return cuda_fail(e, "conv_wgrad_umma_kernel");
-            sum_splits_kernel<<<(int)std::min<int64_t>((wn + 255) / 256, 1024), 256, 0, s>>>(nt->ws, splits, wn,
-                                                                                              G + nt->L.w[l]);
-            sum_splits_kernel<<<(g.Cout + 255) / 256, 256, 0, s>>>(partb, splits, g.Cout, G + nt->L.b[l]);
+            sum_splits2_kernel<<<(int)std::min<int64_t>((wn + g.Cout + 127) / 128, 2048), 128, 0, s>>>(
+                nt->ws, partb, splits, wn, g.Cout, G + nt->L.w[l], G + nt->L.b[l]);
         }
         if (l > 0) {
             const int Min = n * g.H * g.H;
