@@ -243,7 +243,7 @@ def search(cost: str, moving: CudaImage, fixed: CudaImage, grid: CudaGrid, costs
     returns the :class:`Argmin`.  ``exact_samples``: None = the cost's default (exact for
     the reference functors, fast for ZNCC / MI), True / False force a mode.  ``quad_taps``:
     None = the library's choice, True = pre-gathered 16-byte quads, False = texture gathers.
-    ``per_sample_decisions``: run single-channel ZNCC and MI on the per-sample decision kernel
+    ``per_sample_decisions``: run ZNCC, MI, SAD, SQD and NCC on the per-sample decision kernel
     instead of the span kernels (CGS_FLAG_PER_SAMPLE_DECISIONS).  ``verify``: run the FP64 verification pass
     (the Argmin's *_fp64 fields); False sets CGS_FLAG_NO_VERIFY."""
     opt = _options(cost, mi_bins, overlap_gate, points_per_warp, warps_per_block, natural_order, exact_samples,
@@ -447,7 +447,7 @@ class BatchPair:
 
 class Batch:
     """Many pairs in one recorded launch sequence (cgs_batch_*): a persistent kernel over the
-    pairs' tasks, then the span-kernel searches of the ZNCC and MI pairs that :func:`search`
+    pairs' tasks, then the span-kernel searches of the pairs that :func:`search`
     runs on span kernels; the pairs' images, dumps and results are bound at creation;
     :meth:`launch` replays the recorded CUDA graph."""
 

@@ -1,8 +1,8 @@
 // cgs_batch.cu -- C ABI of the batched search: a handle that stages many image pairs, orders
 // their tasks, holds a CUDA graph of one launch sequence -- clear, stage, the persistent batch
-// kernel over the per-sample pairs, the multi-pair span kernel over the ZNCC pairs that
-// cgs_search runs on its span kernel, and cgs_search's own launches for large MI pairs that it
-// runs on the MI span kernel -- replays it, and tunes the persistent kernel's plan by timing
+// kernel over the per-sample pairs and small MI pairs, the multi-pair span kernel over the ZNCC, SAD, SQD
+// and NCC pairs that cgs_search runs on its span kernels with windows, and cgs_search's own launches for
+// large MI pairs that it runs on the MI span kernel -- replays it, and tunes the persistent kernel's plan by timing
 // candidates on a sample of every pair's grid.
 #include <algorithm>
 #include <cmath>

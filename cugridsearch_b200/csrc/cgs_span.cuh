@@ -33,7 +33,8 @@
 // two stages of half the size sent a third of the blocks to global memory.  The next tile's
 // copies start at the barrier that ends a tile and run during the next band's span pass; a tile's
 // wait is then 0.5-2 K cycles of about 65 K.  Measured on the 256 x 256, 6^8 search: two stages
-// filled by one warp 133.3 ms, one stage filled by one warp 128.6 ms, by all warps 116.1 ms.
+// filled by one warp 133.3 ms, one stage filled by one warp 128.6 ms, by all warps 116.1 ms (105.8 ms with
+// the cheaper task setup and span pass that came after).
 //
 // Sweep.  Lane l takes the tile's columns x0 + l + 32 k; each warp evaluates its G grid points
 // at every pixel, two points per packed FP32x2 instruction.  Blocks inside every point's inner

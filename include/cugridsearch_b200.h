@@ -105,7 +105,8 @@ typedef struct cgs_options {
 #define CGS_FLAG_TEXTURE_TAPS 16
 /* Span kernels (the default where they apply): in/out decisions per image row instead of per
  * sample.  They run zero-mean NCC (single channel) and MI (single channel, at most 32 bins) on fast
- * samples, and SAD_AVG, SQD_REF and NCC_REF (1 or 3 channels) on exact ones, unless a taps flag is
+ * samples, and SAD_AVG, SQD_REF and NCC_REF (1 or 3 channels) and MI of 3 channels (as many bins as fit
+ * shared memory, at most 32) on exact ones, unless a taps flag is
  * set (ZNCC: the texture flag).  ZNCC and the exact costs read their taps from per-block
  * moving-image windows in shared memory, MI keeps its histograms there.  They ignore
  * warps_per_block, and points_per_warp other than ZNCC's 2.  This flag selects the per-sample
