@@ -38,7 +38,7 @@
 // as in the per-sample kernel: equal counts give equal bits.
 //
 // Sums of the other costs.  Per lane and band of TH rows in FP32, then a warp sum into FP64 totals; the
-// fixed image's sum of squares comes from the row prefix sums.  SAD is formed in FP64, the NCC-like
+// fixed image's sum of squares comes from the row prefix sums (or the pixels: prefix_holds).  SAD is formed in FP64, the NCC-like
 // costs in FP32 from the rounded totals (finalize), so their special cases are the per-sample kernel's.  Costs do not depend on
 // the order of the points or on how many share a launch.
 #pragma once
@@ -227,31 +227,39 @@ __device__ __forceinline__ bool run_span_exact_task(const SearchParams &p, uint3
                 const int g = act ? i / TH : 0, r = i - g * TH;
                 double a[NS] = {}, s2 = 0.0;
                 int n = 0;
-                bool found = false;
+                bool found = false, sure = true;
+                const int y = y0 + r;
+                RowSpans sp{0, 0, 0, 0};
                 if (act) {
                     const SpanSlot &sl = my_slots[g];
-                    const int y = y0 + r;
-                    InnerSpan is{0, 0};
-                    if (y < fh && sl.valid && sl.ok) {
-                        const RowSpans sp = row_spans(sl, (float)y, fw, mov_wf, mov_hf);
-                        const int xa = sp.xa, len = sp.len, pa = sp.pa, plen = sp.plen;
-                        is = InnerSpan{xa, len};
-                        if (len > 0) {
-                            if constexpr (kFix) {
-                                const double2 *pr = p.fix_prefix + (int64_t)y * (fw + 1);
-                                s2 = pr[xa + len].y - pr[xa].y;
-                            }
-                            n = len;
+                    if (y < fh && sl.valid && sl.ok) sp = row_spans(sl, (float)y, fw, mov_wf, mov_hf);
+                    my_spans[g * TH + r] = InnerSpan{sp.xa, sp.len};
+                    n = sp.len;
+                    if constexpr (kFix) {
+                        if (sp.len > 0) {
+                            const double2 *pr = p.fix_prefix + (int64_t)y * (fw + 1) + sp.xa;
+                            const double to = pr[sp.len].y;
+                            s2 = to - pr[0].y;
+                            sure = prefix_holds(s2, to);
                         }
-                        // band pixels: the outer span outside the inner one, [pa, e0) and [e1, pa + plen)
-                        const int e0 = len > 0 ? xa : pa + plen, e1 = len > 0 ? xa + len : pa + plen;
-                        int nb = 0;
-                        for (int x = pa; x < e0; x++) nb += exact_sample(g, x, y, a, s2);
-                        for (int x = e1; x < pa + plen; x++) nb += exact_sample(g, x, y, a, s2);
-                        n += nb;
-                        found = nb > 0;
                     }
-                    my_spans[g * TH + r] = is;
+                }
+                if constexpr (kFix) {
+                    for (uint32_t m = __ballot_sync(0xffffffffu, !sure); m; m &= m - 1u) {
+                        const int l = __ffs(m) - 1;
+                        const double t = row_sums<C>(p.fix, __shfl_sync(0xffffffffu, y, l), __shfl_sync(0xffffffffu, sp.xa, l),
+                                                     __shfl_sync(0xffffffffu, sp.len, l)).y;
+                        if (lane == l) s2 = t;
+                    }
+                }
+                if (act) {
+                    // band pixels: the outer span outside the inner one, [pa, e0) and [e1, pa + plen)
+                    const int e0 = sp.len > 0 ? sp.xa : sp.pa + sp.plen, e1 = sp.len > 0 ? sp.xa + sp.len : sp.pa + sp.plen;
+                    int nb = 0;
+                    for (int x = sp.pa; x < e0; x++) nb += exact_sample(g, x, y, a, s2);
+                    for (int x = e1; x < sp.pa + sp.plen; x++) nb += exact_sample(g, x, y, a, s2);
+                    n += nb;
+                    found = nb > 0;
                 }
                 add_totals(g, act && r == 0, TH, a, s2, n, __any_sync(0xffffffffu, found));
             }
