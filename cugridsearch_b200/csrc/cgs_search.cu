@@ -293,51 +293,89 @@ __device__ __forceinline__ void prep_body(const PrepParams &q, int64_t tid, int6
 // The images' means for the ZNCC shifts, over a fixed subsample (at most kShiftSamples evenly
 // strided elements of each HWC image), summed in FP64 in a fixed order by one block of 256
 // threads: the same bits on every call.  shifts = {fixed mean, moving mean}.  A thread's 16 samples
-// are loaded at once (one after the other they took 8 of the staging kernel's 10 us).
+// are loaded at once (one after the other they took 8 of the staging kernel's 10 us).  Samples that are
+// not finite, or more than 2^16 above the geometric mean of the others (no-data values), are left
+// out: any shift gives the same cost, but one far from the pixels costs the sums their digits.
 constexpr int64_t kShiftSamples = 4096;
+constexpr int kShiftN = (int)(kShiftSamples / 256);
 
 template <class T>
-__device__ __forceinline__ double strided_sum(const void *src, int64_t stride, int count) {
-    constexpr int N = (int)(kShiftSamples / 256);
+__device__ __forceinline__ void strided_samples(const void *src, int64_t stride, int count, float (&f)[kShiftN]) {
     const T *v = static_cast<const T *>(src);
-    float f[N];
 #pragma unroll
-    for (int k = 0; k < N; k++) {
+    for (int k = 0; k < kShiftN; k++) {
         const int i = (int)threadIdx.x + 256 * k;
         f[k] = i < count ? (float)v[i * stride] : 0.0f;
     }
-    double s = 0.0;
-#pragma unroll
-    for (int k = 0; k < N; k++) s += (double)f[k];
-    return s;
 }
 
 __device__ void staging_means(const PrepParams &q) {
     __shared__ double part[2][8];
-    const int t = threadIdx.x;
-    double acc[2] = {0.0, 0.0};
+    __shared__ int scale[2][2][8], used[2][8];  // sums of exponents, their number; samples of the mean
+    const int t = threadIdx.x, warp = t >> 5;
+    float f[2][kShiftN];
+    int count[2];
+    auto magnitude = [](float v) { return __float_as_uint(v) & 0x7fffffffu; };
+#pragma unroll
     for (int k = 0; k < 2; k++) {
         const void *src = k == 0 ? q.fix_src : q.mov_src;
         const int pix = k == 0 ? q.fix_pix : q.mov_pix;
         const int64_t total = k == 0 ? (int64_t)q.fh * q.fw * q.c : (int64_t)q.mh * q.mw * q.c;
         const int64_t stride = total > kShiftSamples ? total / kShiftSamples : 1;
-        const int count = (int)(total > kShiftSamples ? kShiftSamples : total);
-        double s = pix == CGS_PIXEL_U8    ? strided_sum<uint8_t>(src, stride, count)
-                   : pix == CGS_PIXEL_F64 ? strided_sum<double>(src, stride, count)
-                   : pix == CGS_PIXEL_U16 ? strided_sum<uint16_t>(src, stride, count)
-                                          : strided_sum<float>(src, stride, count);
+        count[k] = (int)(total > kShiftSamples ? kShiftSamples : total);
+        if (pix == CGS_PIXEL_U8) strided_samples<uint8_t>(src, stride, count[k], f[k]);
+        else if (pix == CGS_PIXEL_F64) strided_samples<double>(src, stride, count[k], f[k]);
+        else if (pix == CGS_PIXEL_U16) strided_samples<uint16_t>(src, stride, count[k], f[k]);
+        else strided_samples<float>(src, stride, count[k], f[k]);
+        int es = 0, en = 0;
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if ((t & 31) == 0) part[k][t >> 5] = s;
-        acc[k] = (double)count;
+        for (int i = 0; i < kShiftN; i++) {
+            const uint32_t b = magnitude(f[k][i]);
+            const bool scaled = b >= 0x00800000u && b < 0x7f800000u;  // normal: neither zero nor special
+            es += scaled ? (int)(b >> 23) : 0;
+            en += scaled ? 1 : 0;
+        }
+        es = __reduce_add_sync(0xffffffffu, es);
+        en = __reduce_add_sync(0xffffffffu, en);
+        if ((t & 31) == 0) {
+            scale[k][0][warp] = es;
+            scale[k][1][warp] = en;
+        }
     }
     __syncthreads();
-    if (t == 0) {
-        for (int k = 0; k < 2; k++) {
-            double s = 0.0;
-            for (int w = 0; w < 8; w++) s += part[k][w];
-            q.shifts[k] = (float)(s / acc[k]);
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+        int es = 0, en = 0;
+        for (int w = 0; w < 8; w++) {
+            es += scale[k][0][w];
+            en += scale[k][1][w];
         }
+        const uint32_t most = en == 0 ? 0x7f7fffffu : (uint32_t)min(es / en + 16, 254) << 23 | 0x7fffffu;
+        double s = 0.0;
+        int n = 0;
+#pragma unroll
+        for (int i = 0; i < kShiftN; i++) {
+            const bool in = magnitude(f[k][i]) <= most;
+            s += in ? (double)f[k][i] : 0.0;
+            n += in && t + 256 * i < count[k] ? 1 : 0;
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        n = __reduce_add_sync(0xffffffffu, n);
+        if ((t & 31) == 0) {
+            part[k][warp] = s;
+            used[k][warp] = n;
+        }
+    }
+    __syncthreads();
+    if (t < 2) {
+        double s = 0.0;
+        int n = 0;
+        for (int w = 0; w < 8; w++) {
+            s += part[t][w];
+            n += used[t][w];
+        }
+        q.shifts[t] = n > 0 ? (float)(s / (double)n) : 0.0f;
     }
 }
 

@@ -17,8 +17,9 @@
 // those the guard's own bound is built from), which the 1.5 factor covers.
 //
 // Fixed-image sums.  sum f and sum f^2 over a point's overlap are the inner spans' sums, taken
-// from FP64 prefix sums of each fixed row (row_prefix_kernel), plus the band pixels found
-// inside; only the three sums that involve the moving image are accumulated per sample.
+// from FP64 prefix sums of each fixed row (span_prep_kernel; where a pixel before the span swamps
+// them, from the pixels: prefix_holds), plus the band pixels found inside; only the three sums that
+// involve the moving image are accumulated per sample.
 //
 // Tiles and windows.  The fixed image is walked in tiles of TW = 32 TX columns by TH rows.  For
 // every 32-column block of a tile the CTA's grid points map the block into a small region of
@@ -230,7 +231,8 @@ __device__ __forceinline__ RowSpans row_spans(const SpanSlot &k, float yf, int f
 
 // Prefix sums stand for the sums of an inner span only where the span's sum of squares d is not lost in the
 // rounding of the prefix `to` that it was taken from: a pixel before the span that is not finite or far
-// larger poisons the difference, and a span of zeros must sum to 0 exactly.  Above 2^-16 of the prefix the
+// larger poisons the difference, and a span of zeros must sum to 0 exactly.  The sum of f, at most
+// sqrt(W) times the root of that of squares, is then safe too.  Above 2^-16 of the prefix the
 // error, at most (5 + W / 32) 2^-53 of it, is below 2^-27 of the sum; below that the pixels are added
 // (row_sums).  Images without such pixels have next to no rows there.
 __device__ __forceinline__ bool prefix_holds(double d, double to) { return d > 0x1p-16 * to || to == 0.0; }
@@ -608,48 +610,60 @@ __device__ __forceinline__ bool run_span_task(const SearchParams &p, uint32_t un
                 const int g = act ? i / TH : 0, r = i - g * TH;
                 double s1 = 0.0, s2 = 0.0, sm = 0.0, smm = 0.0, sfm = 0.0;
                 int n = 0;
+                bool sure = true;
+                const int y = y0 + r;
+                const float yf = (float)y;
+                RowSpans sp{0, 0, 0, 0};
                 if (act) {
                     const SpanSlot &sl = my_slots[g];
-                    const int y = y0 + r;
-                    InnerSpan is{0, 0};
                     if (y < fh && sl.valid) {
-                        const float yf = (float)y;
-                        RowSpans sp{0, 0, 0, fw};  // ill-conditioned: every pixel exact
                         if (sl.ok) sp = row_spans(sl, yf, fw, mov_wf, mov_hf);
-                        const int xa = sp.xa, len = sp.len, pa = sp.pa, plen = sp.plen;
-                        is = InnerSpan{xa, len};
-                        if (len > 0) {
-                            const double2 *pr = p.fix_prefix + (int64_t)y * (fw + 1);
-                            const double2 a = pr[xa], b = pr[xa + len];
-                            s1 = b.x - a.x;
-                            s2 = b.y - a.y;
-                            n = len;
-                        }
-                        // band pixels: the outer span outside the inner one, [pa, e0) and [e1, pa + plen)
-                        const int e0 = len > 0 ? xa : pa + plen, e1 = len > 0 ? xa + len : pa + plen;
-                        const MapCoef kc{sl.A, sl.B, sl.P, sl.Q, sl.C1, sl.C2, sl.R, sl.S, sl.D1, sl.D2, sl.T, sl.U};
-                        const float *frow_g = fdata + (int64_t)y * fpitch;
-                        auto band = [&](int xs, int xe) {
-                            for (int x = xs; x < xe; x++) {
-                                float ex, ey;
-                                exact_map(kc, (float)x, yf, ex, ey);
-                                if (in_image(ey, ex, mov_wf, mov_hf)) {
-                                    const float m = bilinear_in(mdata, mpitch, ey, ex) - mshift;
-                                    const float f = frow_g[x];
-                                    const float fs = f - fshift;
-                                    s1 += (double)f;
-                                    s2 += (double)f * (double)f;
-                                    sm += (double)m;
-                                    smm += (double)m * (double)m;
-                                    sfm += (double)fs * (double)m;
-                                    n++;
-                                }
-                            }
-                        };
-                        band(pa, e0);
-                        band(e1, pa + plen);
+                        else sp.plen = fw;  // ill-conditioned: every pixel exact
                     }
-                    my_spans[g * TH + r] = is;
+                    my_spans[g * TH + r] = InnerSpan{sp.xa, sp.len};
+                    n = sp.len;
+                    if (sp.len > 0) {
+                        const double2 *pr = p.fix_prefix + (int64_t)y * (fw + 1) + sp.xa;
+                        const double2 a = pr[0], b = pr[sp.len];
+                        s1 = b.x - a.x;
+                        s2 = b.y - a.y;
+                        sure = prefix_holds(s2, b.y);
+                    }
+                }
+                for (uint32_t m = __ballot_sync(0xffffffffu, !sure); m; m &= m - 1u) {
+                    const int l = __ffs(m) - 1;
+                    const double2 t = row_sums<1>(p.fix, __shfl_sync(0xffffffffu, y, l), __shfl_sync(0xffffffffu, sp.xa, l),
+                                                  __shfl_sync(0xffffffffu, sp.len, l));
+                    if (lane == l) {
+                        s1 = t.x;
+                        s2 = t.y;
+                    }
+                }
+                if (act) {
+                    // band pixels: the outer span outside the inner one, [pa, e0) and [e1, pa + plen)
+                    const SpanSlot &sl = my_slots[g];
+                    const int e0 = sp.len > 0 ? sp.xa : sp.pa + sp.plen, e1 = sp.len > 0 ? sp.xa + sp.len : sp.pa + sp.plen;
+                    const MapCoef kc{sl.A, sl.B, sl.P, sl.Q, sl.C1, sl.C2, sl.R, sl.S, sl.D1, sl.D2, sl.T, sl.U};
+                    const float *frow_g = fdata + (int64_t)y * fpitch;
+                    auto band = [&](int xs, int xe) {
+                        for (int x = xs; x < xe; x++) {
+                            float ex, ey;
+                            exact_map(kc, (float)x, yf, ex, ey);
+                            if (in_image(ey, ex, mov_wf, mov_hf)) {
+                                const float m = bilinear_in(mdata, mpitch, ey, ex) - mshift;
+                                const float f = frow_g[x];
+                                const float fs = f - fshift;
+                                s1 += (double)f;
+                                s2 += (double)f * (double)f;
+                                sm += (double)m;
+                                smm += (double)m * (double)m;
+                                sfm += (double)fs * (double)m;
+                                n++;
+                            }
+                        }
+                    };
+                    band(sp.pa, e0);
+                    band(e1, sp.pa + sp.plen);
                 }
                 // sum over the TH lanes of each point (TH is 8, 16 or 32); the moving sums exist only
                 // where a band pixel was found inside, which is rare

@@ -1,7 +1,8 @@
 """Fixed pixels that are not finite, or so large that they swamp their row's sums in FP64, must not reach
 the cost of a grid point whose overlap misses them; a row of zeros beside other pixels sums to exactly 0.
 
-The fixed rows' sums over an overlap come from prefix sums (span kernels), which such pixels poison for
+Nor may they, in either image, move the shift of the zero-mean sums away from the pixels.  The fixed
+rows' sums over an overlap come from prefix sums (span kernels), which such pixels poison for
 the rest of their row.  Checked against the oracle, one and three channels, single and batch, whole and
 split tasks; tolerances as in conftest.close_costs.
 """
@@ -53,24 +54,31 @@ def _batch(cuda, p, cost):
     return costs.cpu().numpy()
 
 
+def _clear(p, fixed, moving):
+    """The points whose overlap misses the NaN pixels of the images (calcNCC and zero-mean NCC have the
+    same map; the oracle's zero-mean NCC takes whole images' means, so NaN spreads to all its points)."""
+    q = S.Pair(fixed, moving, p.gt, p.lo, p.hi, p.count)
+    clear = np.isfinite(_oracle(q, "NCC_REF", np.ascontiguousarray(fixed))[1])
+    assert 0.2 < clear.mean() < 0.8
+    return clear
+
+
 def _check(cuda, cost, h, w, channels, value):
     p = _pair(cost, h, w, channels)
-    # the points whose overlap misses the outliers: those that a NaN there leaves finite
-    clear = np.isfinite(_oracle(p, cost, _outliers(p, np.float32("nan")))[1])
-    assert 0.2 < clear.mean() < 0.8
+    clear = _clear(p, _outliers(p, np.float32("nan")), p.moving)
+    c32, c64 = _oracle(p, cost, p.fixed)  # at clear points the outliers' values are not read
     p.fixed = np.ascontiguousarray(_outliers(p, value))
-    c32, c64 = _oracle(p, cost, p.fixed)
     got = [_run(cuda, p, cost)[1]] + ([_batch(cuda, p, cost)] if channels == 1 else [])
     for c in got:
         bad = close_costs(c, c32, c64, cost) & clear
         assert not bad.any(), (int(bad.sum()), c[bad][:4], c64[bad][:4])
         if not np.isfinite(value):
-            np.testing.assert_array_equal(np.isfinite(c), np.isfinite(c64))
+            assert not np.isfinite(c[~clear]).any()
 
 
 @pytest.mark.parametrize("value", [float("nan"), float("inf"), float("-inf"), 1e10, LOWEST])
 @pytest.mark.parametrize("h,w,channels", [(30, 41, 1), (20, 300, 1), (30, 70, 3)])
-@pytest.mark.parametrize("cost", COSTS)
+@pytest.mark.parametrize("cost", COSTS + ["ZNCC"])
 def test_outliers_outside_the_overlap(cuda, lib, cost, h, w, channels, value):
     _check(cuda, cost, h, w, channels, value)
 
@@ -88,3 +96,19 @@ def test_overlap_of_zeros(cuda, lib, cost, channels):
     for c in [_run(cuda, p, cost)[1]] + ([_batch(cuda, p, cost)] if channels == 1 else []):
         bad = close_costs(c, c32, c64, cost)
         assert not bad.any(), (int(bad.sum()), c[bad][:4], c32[bad][:4], c64[bad][:4])
+
+
+@pytest.mark.parametrize("value", [float("nan"), 1e10, LOWEST])
+@pytest.mark.parametrize("channels", [1, 3])
+def test_moving_outliers_outside_the_overlap(cuda, lib, channels, value):
+    """Moving pixels that no sample of a point reads: its zero-mean cost is the oracle's."""
+    p = _pair("ZNCC", 30, 41, channels)
+    moving = p.moving.copy()
+    moving[::3, 30:32] = np.nan
+    clear = _clear(p, p.fixed, np.ascontiguousarray(moving))
+    c32, c64 = _oracle(p, "ZNCC", p.fixed)
+    moving[::3, 30:32] = value
+    p.moving = np.ascontiguousarray(moving)
+    c = _run(cuda, p, "ZNCC")[1]
+    bad = close_costs(c, c32, c64, "ZNCC") & clear
+    assert not bad.any(), (int(bad.sum()), c[bad][:4], c64[bad][:4])
