@@ -482,10 +482,13 @@ __device__ __forceinline__ void fold_band(const SearchParams &p, uint32_t task, 
     __syncwarp();
 }
 
-// After a part's bands: whether this CTA completed the task, whose totals and counts it then holds.
-template <int G, int NW>
+// After a part's bands: whether this CTA completed the task, whose totals and counts it then holds.  The
+// self-checking build's finding is reported for every part, before the part counts as done (a CTA
+// barrier precedes the call).
+template <int G, int NW, bool CHECK>
 __device__ __forceinline__ bool join_parts(const SearchParams &p, uint32_t task, int part, const SpanSmem &ss, double *my_dtot,
                                            int *my_cnt) {
+    if (CHECK && threadIdx.x == 0 && *ss.bounds_flag) atomicOr(p.status, kStatusSpanBounds);
     if (p.splits <= 1) return true;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     int *cnt = p.split_cnt + (size_t)task * p.splits * (NW * G) + warp * G;
@@ -910,7 +913,7 @@ __device__ __forceinline__ bool run_span_task(const SearchParams &p, uint32_t un
         if (more) issue_window<1, NW, TX>(p, ss, p.fix.data, t + kWinStages, st);
     }
 
-    if (!join_parts<G, NW>(p, task, part, ss, my_dtot, my_cnt)) return true;
+    if (!join_parts<G, NW, CHECK>(p, task, part, ss, my_dtot, my_cnt)) return true;
 
     // ---- per grid point: finalise, dump, argmin key (as the pixel-loop kernel)
     __syncwarp();
@@ -939,7 +942,6 @@ __device__ __forceinline__ bool run_span_task(const SearchParams &p, uint32_t un
     if (threadIdx.x == 0) {
         unsigned long long b = ~0ull;
         for (int w = 0; w < NW; w++) b = ss.wbest[w] < b ? ss.wbest[w] : b;
-        if (CHECK && *ss.bounds_flag) atomicOr(p.status, kStatusSpanBounds);
         retire_tasks(p, b, 1u, false);
     }
     return true;

@@ -494,7 +494,7 @@ __device__ __forceinline__ bool run_span_exact_task(const SearchParams &p, uint3
         if (more) issue_window<C, NW, TX>(p, ss, fsrc, t + kWinStages, st);
     }
 
-    if (!kMI && !join_parts<G, NW>(p, task, part, ss, my_dtot, my_cnt)) return true;
+    if (!join_parts<G, NW, CHECK>(p, task, part, ss, my_dtot, my_cnt)) return true;  // MI: never split
 
     // ---- per grid point: the cost from the totals or the counts, dump, argmin key
     __syncwarp();
@@ -537,7 +537,6 @@ __device__ __forceinline__ bool run_span_exact_task(const SearchParams &p, uint3
     if (threadIdx.x == 0) {
         unsigned long long b = ~0ull;
         for (int w = 0; w < NW; w++) b = ss.wbest[w] < b ? ss.wbest[w] : b;
-        if (CHECK && *ss.bounds_flag) atomicOr(p.status, kStatusSpanBounds);
         retire_tasks(p, b, 1u, false);
     }
     return true;
