@@ -468,6 +468,8 @@ __device__ __forceinline__ void span_windows(const SearchParams &p, const SpanSm
 // that completes a task's parts adds them in band order: the sums, and their order, are those of an
 // unsplit task.
 
+constexpr unsigned kPartLost = 1u << 16;  // in a task's count of done parts: one more was not run
+
 // The band's sums of a warp's points (my_band, cleared) into the task totals, or to global memory.
 template <int G, int NW>
 __device__ __forceinline__ void fold_band(const SearchParams &p, uint32_t task, int band, double *my_dtot, double *my_band) {
@@ -496,7 +498,14 @@ __device__ __forceinline__ bool join_parts(const SearchParams &p, uint32_t task,
     __threadfence();
     __syncthreads();
     volatile int &s_last = *(ss.bounds_flag + 2);
-    if (threadIdx.x == 0) s_last = atomicAdd(p.split_done + task, 1u) + 1u == (unsigned)p.splits;
+    if (threadIdx.x == 0) {
+        const unsigned done = atomicAdd(p.split_done + task, 1u) + 1u;
+        s_last = (done & (kPartLost - 1u)) == (unsigned)p.splits;
+        if (s_last && done >= kPartLost) {  // totals are missing: the task has no costs
+            retire_tasks(p, ~0ull, 1u, true);
+            s_last = 0;
+        }
+    }
     __syncthreads();
     if (!s_last) return false;
     __threadfence();
@@ -515,8 +524,8 @@ __device__ __forceinline__ bool join_parts(const SearchParams &p, uint32_t task,
     return true;
 }
 
-// Thread 0 of a CTA that stops: the parts it will not run count as done, and a task whose parts are all
-// done is retired with the timeout status.
+// Thread 0 of a CTA that stops: the parts it will not run count as done and lost (join_parts: nobody
+// adds their totals), and a task whose parts are all done is retired with the timeout status.
 __device__ __forceinline__ void retire_parts(const SearchParams &p, uint32_t unit, uint32_t step, uint32_t units) {
     for (uint32_t u = unit; u < units; u += step) {
         if (p.splits <= 1) {
@@ -525,7 +534,8 @@ __device__ __forceinline__ void retire_parts(const SearchParams &p, uint32_t uni
         }
         atomicOr(p.status, (unsigned)CGS_ERROR_DEVICE_TIMEOUT);
         __threadfence();
-        if (atomicAdd(p.split_done + u / p.splits, 1u) + 1u == (unsigned)p.splits) retire_tasks(p, ~0ull, 1u, true);
+        const unsigned done = atomicAdd(p.split_done + u / p.splits, kPartLost + 1u) + 1u;
+        if ((done & (kPartLost - 1u)) == (unsigned)p.splits) retire_tasks(p, ~0ull, 1u, true);
     }
 }
 

@@ -1,6 +1,8 @@
 // Device functions of the span kernels by themselves: span_check CASE prints the words that
 // tests/test_span_device_gpu.py compares.
 //   bounds     status after a part that found a bad address and was not its task's last one
+//   lost       a part after one that a CTA that gave up did not run, and that order turned around:
+//              what join_parts returned, tasks done, status, whether the argmin key is untouched
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -87,9 +89,26 @@ static void bounds() {
     std::printf("%d %u %d %u\n", first, after & kStatusSpanBounds, last, value(p.status) & kStatusSpanBounds);
 }
 
+// What a CTA that gives up on part `part` does.
+__global__ void lose_kernel(const __grid_constant__ SearchParams p, int part) { retire_parts(p, (uint32_t)part, 2u, 2u); }
+
+static void lost() {
+    for (int first = 0; first < 2; first++) {
+        const SearchParams p = two_parts();
+        int joined = 0;
+        if (first == 1) joined = join(p, 1, 0);
+        lose_kernel<<<1, 1>>>(p, 0);
+        check(cudaGetLastError());
+        check(cudaDeviceSynchronize());
+        if (first == 0) joined = join(p, 1, 0);
+        std::printf("%d %u %u %d\n", joined, value(p.done), value(p.status), value(p.key) == ~0ull);
+    }
+}
+
 int main(int argc, char **argv) {
     const std::string c = argc > 1 ? argv[1] : "";
     if (c == "bounds") bounds();
+    else if (c == "lost") lost();
     else return 1;
     return 0;
 }

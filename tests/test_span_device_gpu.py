@@ -24,3 +24,12 @@ def test_every_part_reports_a_bad_address(cuda, lib):
     first, after, last, status = _run("bounds")
     assert (first, last) == (0, 1)
     assert after == status == 0x100
+
+
+def test_a_task_with_a_lost_part_has_no_costs(cuda, lib):
+    """A part that a CTA which gave up did not run: the task is retired with the timeout status, by whichever
+    comes last, and its totals, never written, form no cost."""
+    out = _run("lost")
+    for joined, done, status, untouched in (out[:4], out[4:]):
+        assert (joined, done, untouched) == (0, 1, 1)
+        assert status == 7  # CGS_ERROR_DEVICE_TIMEOUT
