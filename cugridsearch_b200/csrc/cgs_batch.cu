@@ -306,6 +306,16 @@ static double pair_work(const SearchParams &p) {
     return w * (double)p.n * (double)p.fix.w * (double)p.fix.h;
 }
 
+// Window stage (quads) of the multi-pair span kernel for pairs of up to `tiles` tiles, or 0 where its
+// shared memory, laid out for every cost of the group, does not hold a useful one.  A single search's
+// layout can be smaller (zero-mean NCC has no row products), so a pair may fit its own span kernel alone.
+static int group_cap(const SpanPlan &g, int tiles) {
+    const size_t budget = 227 * 1024;
+    const int least = kMinSpanCap + g.TH * 32 * g.TX / 4;  // after the fixed rows
+    if (span_kernel_smem(g.G, g.NW, g.TH, g.TX, tiles, least, true, 0) > budget) return 0;
+    return (int)((budget - span_kernel_smem(g.G, g.NW, g.TH, g.TX, tiles, 0, true, 0)) / (16 * kWinStages));
+}
+
 }  // namespace cgs
 
 extern "C" {
@@ -355,21 +365,24 @@ cgs_status cgs_batch_create(const cgs_pair *pairs, int32_t n, const cgs_batch_pl
         const cgs_pair &q = pairs[i];
         Pending &pd = pend[i];
         // pairs that cgs_search runs on a tiled span kernel share one multi-pair span launch (same
-        // kernel plan); MI pairs on its MI span kernel are searched by their own launches once
-        // their grid fills the GPU by itself (a few tasks per SM), and stay in the persistent
-        // kernel below that (a refinement level's local grids, balanced there many at once)
+        // kernel plan); one that does not fit the group's shared memory is searched by its own
+        // launches.  So are MI pairs on its MI span kernel once their grid fills the GPU by itself
+        // (a few tasks per SM); they stay in the persistent kernel below that (a refinement level's
+        // local grids, balanced there many at once)
         uint32_t ppt = 0;
         SpanPlan zp;
-        if (span_plan(q.moving, q.fixed, q.options, pd.mi_bins, &zp) &&
-            kernel_span_batch(zp.G, zp.NW, zp.TX, zp.check) != nullptr &&
-            (!have_group || (zp.G == gplan.G && zp.NW == gplan.NW && zp.TX == gplan.TX && zp.TH == gplan.TH &&
-                             zp.pitch_mod == gplan.pitch_mod))) {
+        const bool group = span_plan(q.moving, q.fixed, q.options, pd.mi_bins, &zp) &&
+                           kernel_span_batch(zp.G, zp.NW, zp.TX, zp.check) != nullptr &&
+                           (!have_group || (zp.G == gplan.G && zp.NW == gplan.NW && zp.TX == gplan.TX &&
+                                            zp.TH == gplan.TH && zp.pitch_mod == gplan.pitch_mod));
+        const bool fits = group && group_cap(zp, zp.tiles_x * zp.tiles_y) > 0;
+        if (fits) {
             pd.route = 1;
             pd.zp = zp;
             if (!have_group) gplan = zp;
             have_group = true;
         } else if ((q.options.cost == CGS_COST_ZNCC || q.options.cost == CGS_COST_MI) &&
-                   span_route_bytes(q, &pd.span_bytes, &ppt) && (uint64_t)pd.p.n >= route_tasks * ppt) {
+                   span_route_bytes(q, &pd.span_bytes, &ppt) && (group || (uint64_t)pd.p.n >= route_tasks * ppt)) {
             pd.route = 2;
         }
         // ZNCC pairs of the persistent kernel on the fast sampling path read pre-gathered tap
@@ -435,18 +448,7 @@ cgs_status cgs_batch_create(const cgs_pair *pairs, int32_t n, const cgs_batch_pl
             gn++;
             gtiles = std::max(gtiles, pend[i].zp.tiles_x * pend[i].zp.tiles_y);
         }
-    int gcap = 0;
-    if (gn > 0) {
-        const size_t budget = 227 * 1024;
-        const size_t fixed = span_kernel_smem(gplan.G, gplan.NW, gplan.TH, gplan.TX, gtiles, 0, true, 0);
-        gcap = fixed + (size_t)kMinSpanCap * 16 * kWinStages > budget ? 0 : (int)((budget - fixed) / (16 * kWinStages));
-        gcap = std::max(gcap, kMinSpanCap + gplan.TH * 32 * gplan.TX / 4);
-        const size_t gsm = span_kernel_smem(gplan.G, gplan.NW, gplan.TH, gplan.TX, gtiles, gcap, true, 0);
-        if (fixed + (size_t)kMinSpanCap * 16 * kWinStages > budget || gsm > budget) {
-            for (int32_t i = 0; i < n; i++) pend[i].route = pend[i].route == 1 ? 0 : pend[i].route;
-            gn = 0;  // cannot happen for the sizes span_plan admits; the pairs go to the persistent kernel
-        }
-    }
+    const int gcap = gn > 0 ? group_cap(gplan, gtiles) : 0;
     const size_t gpar_off = off;
     off = align_up(off + gn * sizeof(SearchParams), 256);
     const size_t gtb_off = off;

@@ -304,3 +304,25 @@ def test_batch_zncc_group_of_mixed_sizes(cuda, lib):
     for (c_ref, r_ref), (c, r), it in zip(ref, got, its):
         np.testing.assert_array_equal(c.view(np.uint32), c_ref.view(np.uint32))
         assert r.index == r_ref.index and r.status == 0 and r.valid == r_ref.valid
+
+
+def test_batch_pair_too_large_for_the_group(cuda, lib):
+    """A ZNCC pair of 900 tiles fits its own span kernel but not the multi-pair one: it is searched by its
+    own launches and the others keep their group, every cost cgs_search's bit for bit."""
+    import torch
+    import cugridsearch_b200 as cgs
+    its = _make(cuda, [("SAD_AVG", 40, 44, 3), ("ZNCC", 56, 52, 3), ("NCC_REF", 36, 38, 3), ("SQD_REF", 28, 28, 3)])
+    yy, xx = np.mgrid[0:960, 0:3840]
+    img = (120 + 60 * np.sin(xx / 17.0) * np.cos(yy / 13.0)).astype(np.float32)[:, :, None]
+    mov, fix = (torch.from_numpy(np.ascontiguousarray(a)).to(cuda) for a in (np.roll(img, 3, 1), img))
+    grid = cgs.CudaGrid.from_ranges([0, 1, 1, 0, -3, 0, 0, 0], [0, 1, 1, 0, 3, 0, 0, 0], [1, 1, 1, 1, 5, 1, 1, 1])
+    its.append(dict(cost="ZNCC", mov=cgs.CudaImage(mov), fix=cgs.CudaImage(fix), grid=grid,
+                    costs=torch.empty(5, device=cuda), result=cgs.result_buffer(cuda)))
+    ref = _single(cuda, its)
+    with cgs.Batch(_batch_pairs(its)) as b:
+        b.launch()
+        torch.cuda.synchronize()
+        got = _read(its)
+    for (c_ref, r_ref), (c, r), it in zip(ref, got, its):
+        np.testing.assert_array_equal(c.view(np.uint32), c_ref.view(np.uint32), err_msg=it["cost"])
+        assert r.index == r_ref.index and r.status == 0 and r.valid == r_ref.valid
