@@ -1114,7 +1114,10 @@ static cgs_status search_core(const cgs_image *mov, const cgs_image *fix, const 
     const bool spans = span || span_mi;
     const bool quads = spans || (o.flags & CGS_FLAG_QUAD_TAPS) || (fast_path && !(o.flags & CGS_FLAG_TEXTURE_TAPS));
     const void *kfn = spans ? sp.kfn : getter(C, pl.G, pl.NW, quads);
-    if (!kfn) return fail(CGS_ERROR_UNSUPPORTED, "no kernel for this channel count / tuning");
+    // a request's tuning has to be one of the per-sample kernel's, though the exact span kernel ignores it
+    const bool tuned = span && sp.exact && (o.points_per_warp != 0 || o.warps_per_block != 0);
+    if (!kfn || (tuned && !getter(C, pl.G, pl.NW, false)))
+        return fail(CGS_ERROR_UNSUPPORTED, "no kernel for this channel count / tuning");
     if (ext && !spans) return fail(CGS_ERROR_UNSUPPORTED, "caller scratch: span searches only");
 
     DeviceInfo di;
@@ -1136,10 +1139,11 @@ static cgs_status search_core(const cgs_image *mov, const cgs_image *fix, const 
     // staged layout
     const Staging st = staging_layout(*mov, *fix, di.tex_align, di.tex_pitch_align, false, false, quads);
     const int64_t stage_bytes = set_chunks(&p, st, C, fix->height);
-    const size_t smem = spans ? sp.smem
-                              : cta_smem_bytes(pl.G, pl.NW, (size_t)stage_bytes,
-                                              acc_bytes(cost, pl.G, pl.NW, false, mi_bins));
-    if (smem > 227 * 1024) return fail(CGS_ERROR_UNSUPPORTED, "shared-memory plan exceeds 227 KB");
+    const size_t per_sample_smem = cta_smem_bytes(pl.G, pl.NW, (size_t)stage_bytes,
+                                                  acc_bytes(cost, pl.G, pl.NW, false, mi_bins));
+    const size_t smem = spans ? sp.smem : per_sample_smem;
+    if (smem > 227 * 1024 || (tuned && per_sample_smem > 227 * 1024))
+        return fail(CGS_ERROR_UNSUPPORTED, "shared-memory plan exceeds 227 KB");
     if (spans) {
         p.tile_h = sp.TH;
         p.tiles_x = sp.tiles_x;

@@ -127,3 +127,18 @@ def test_split_tasks_equal_whole_ones(cuda, lib, cost):
     np.testing.assert_array_equal(costs.cpu().numpy().view(np.uint32), c.view(np.uint32))
     assert cgs.read_result(out).index == res.index
     _oracle_agrees(pair, cost, c)
+
+
+@pytest.mark.parametrize("cost,channels,tuning", [("SAD_AVG", 1, {"warps_per_block": 5}),
+                                                  ("SQD_REF", 3, {"warps_per_block": 32}),
+                                                  ("NCC_REF", 1, {"warps_per_block": 1}),
+                                                  ("MI", 3, {"points_per_warp": 4})])  # 278 KB of histograms
+def test_tunings_of_no_per_sample_kernel_are_refused(cuda, lib, cost, channels, tuning):
+    """As on the per-sample kernel, although the span kernel has its own plan."""
+    import cugridsearch_b200 as cgs
+    pair = _pair(3, cost, 20, 20, 20, 20, channels)
+    for per_sample in (False, True):
+        with pytest.raises(cgs.CgsError):
+            _run(cuda, pair, cost, per_sample_decisions=per_sample, **tuning)
+    for tuning in ({"warps_per_block": 8}, {"points_per_warp": 1}):
+        _run(cuda, pair, cost, **tuning)
