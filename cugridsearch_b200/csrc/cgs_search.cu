@@ -260,7 +260,8 @@ __device__ __forceinline__ void prep_body(const PrepParams &q, int64_t tid, int6
     }
     if (q.pair_dst) {
         // the fixed image's {P(y, x), P(y, x + 1) - P(y, x)}, P its padded plane.  A sample on row y reads
-        // row y + 1 with weight 0, which shows only where the rows' difference is not finite
+        // row y + 1 with weight 0, which shows only where one of the four differences between the taps is
+        // not finite (each by itself: two no-data pixels over two others are finite differences)
         const int64_t plane = (int64_t)q.fh * q.fw;
         auto P = [&](int c, int64_t y, int64_t x) -> float {
             const int64_t e = y * q.fw + x;  // column W: the next row's pixel 0
@@ -270,10 +271,11 @@ __device__ __forceinline__ void prep_body(const PrepParams &q, int64_t tid, int6
             const int c = (int)(i / plane);
             const int64_t e = i - (int64_t)c * plane;
             const int64_t y = e / q.fw, x = e - y * q.fw;
-            const float v0 = P(c, y, x), v1 = P(c, y, x + 1);
-            const float below = fabsf(P(c, y + 1, x) - v0) + fabsf(P(c, y + 1, x + 1) - v1);
-            const bool finite = below < __int_as_float(0x7f800000);
-            q.pair_dst[i] = make_float2(finite ? v0 : __int_as_float(0x7fffffff), v1 - v0);
+            const float v00 = P(c, y, x), v01 = P(c, y, x + 1), v10 = P(c, y + 1, x), v11 = P(c, y + 1, x + 1);
+            const float inf = __int_as_float(0x7f800000);
+            const bool finite = fabsf(v01 - v00) < inf && fabsf(v11 - v10) < inf && fabsf(v10 - v00) < inf &&
+                                fabsf(v11 - v01) < inf;
+            q.pair_dst[i] = make_float2(finite ? v00 : __int_as_float(0x7fffffff), v01 - v00);
         }
     }
     for (int64_t i = tid; i < q.zero_n; i += nthr) q.zero_dst[i] = 0u;

@@ -45,3 +45,16 @@ def test_wide_rows_step_explicitly(cuda, lib, cost):
     lo, hi = [0, 1, 1, 0, -0.25, 0, 0, 0], [0, 1, 1, 0, 0.25, 0, 0, 0]
     c = _run(cuda, cost, moving, fixed, lo, hi, [1, 1, 1, 1, 3, 1, 1, 1])
     assert (c != 123123.0).any()
+
+
+@pytest.mark.parametrize("channels", [1, 3])
+@pytest.mark.parametrize("cost", ["NCC_ALT", "SQD_ALT"])
+def test_no_data_pixels(cuda, lib, cost, channels):
+    """A block of the type's lowest value in the fixed image: finite samples, whose squares overflow as the
+    reference's do (calcNCCAlt 0, not NaN)."""
+    pair = S.small_pair(41, size=33, count=3, cost=cost, channels=channels)
+    pair.fixed = pair.fixed.copy()
+    pair.fixed[5:9, 10:20] = np.finfo(np.float32).min
+    with np.errstate(all="ignore"):
+        c = _run(cuda, cost, pair.moving, pair.fixed, *pair.grid_args())
+    assert np.isnan(c).any() == (cost == "SQD_ALT")
