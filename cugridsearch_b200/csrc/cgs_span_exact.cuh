@@ -75,6 +75,8 @@ __device__ __forceinline__ void accumulate64(double *a, float f, float m) {
     }
 }
 
+constexpr int kFewBand = 8;  // band pixels of a row that its lane samples by itself
+
 template <int COST, int C, int G, int NW, int TX, bool CHECK>
 __device__ __forceinline__ bool run_span_exact_task(const SearchParams &p, uint32_t unit, const SpanSmem &ss,
                                                     uint32_t &wit) {
@@ -178,18 +180,27 @@ __device__ __forceinline__ bool run_span_exact_task(const SearchParams &p, uint3
             my_cnt[g] += n;
         }
     };
-    // every pixel of the band's rows for the points without spans, all lanes over the columns
-    auto no_span_rows = [&](int y0, int y1) {
-        for (int g = 0; g < G; g++) {
-            const SpanSlot &sl = my_slots[g];
-            if (!sl.valid || sl.ok) continue;
-            double a[NS] = {}, s2 = 0.0;
-            int n = 0;
-            for (int y = y0; y < y1; y++)
-                for (int x = lane; x < fw; x += 32) n += exact_sample(g, x, y, a, s2);
-            add_totals(g, lane == 0, 32, a, s2, n, true);
-            __syncwarp();
+    // pixels [xs, xe) of rows [ya, ye) of point g, by the whole warp
+    auto sample_run = [&](int g, int ya, int ye, int xs, int xe) {
+        double a[NS] = {}, s2 = 0.0;
+        int n = 0;
+        const int w = xe - xs;
+        int x = xs + lane, y = ya;
+        while (y < ye) {
+            while (x >= xe && y < ye) {
+                x -= w;
+                y++;
+            }
+            if (y < ye) n += exact_sample(g, x, y, a, s2);
+            x += 32;
         }
+        add_totals(g, lane == 0, 32, a, s2, n, true);
+        __syncwarp();
+    };
+    // every pixel of the band's rows for the points without spans
+    auto no_span_rows = [&](int y0, int y1) {
+        for (int g = 0; g < G; g++)
+            if (my_slots[g].valid && !my_slots[g].ok) sample_run(g, y0, y1, 0, fw);
     };
 
     // ---- sweep
@@ -252,14 +263,25 @@ __device__ __forceinline__ bool run_span_exact_task(const SearchParams &p, uint3
                         if (lane == l) s2 = t;
                     }
                 }
-                if (act) {
-                    // band pixels: the outer span outside the inner one, [pa, e0) and [e1, pa + plen)
-                    const int e0 = sp.len > 0 ? sp.xa : sp.pa + sp.plen, e1 = sp.len > 0 ? sp.xa + sp.len : sp.pa + sp.plen;
+                // band pixels: the outer span outside the inner one, [pa, e0) and [e1, pe).  A few, sampled by
+                // the row's lane; of a row along an edge of the moving image all, sampled by the warp
+                const int pe = sp.pa + sp.plen, e0 = sp.len > 0 ? sp.xa : pe, e1 = sp.len > 0 ? sp.xa + sp.len : pe;
+                const bool many = (e0 - sp.pa) + (pe - e1) > kFewBand;
+                if (act && !many) {
                     int nb = 0;
                     for (int x = sp.pa; x < e0; x++) nb += exact_sample(g, x, y, a, s2);
-                    for (int x = e1; x < sp.pa + sp.plen; x++) nb += exact_sample(g, x, y, a, s2);
+                    for (int x = e1; x < pe; x++) nb += exact_sample(g, x, y, a, s2);
                     n += nb;
                     found = nb > 0;
+                }
+                for (uint32_t m = __ballot_sync(0xffffffffu, many); m; m &= m - 1u) {
+                    const int l = __ffs(m) - 1;
+                    const int gl = __shfl_sync(0xffffffffu, g, l), yl = __shfl_sync(0xffffffffu, y, l);
+                    for (int side = 0; side < 2; side++) {
+                        const int xs = __shfl_sync(0xffffffffu, side ? e1 : sp.pa, l);
+                        const int xe = __shfl_sync(0xffffffffu, side ? pe : e0, l);
+                        if (xe > xs) sample_run(gl, yl, yl + 1, xs, xe);
+                    }
                 }
                 add_totals(g, act && r == 0, TH, a, s2, n, __any_sync(0xffffffffu, found));
             }

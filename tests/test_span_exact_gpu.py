@@ -142,3 +142,20 @@ def test_tunings_of_no_per_sample_kernel_are_refused(cuda, lib, cost, channels, 
             _run(cuda, pair, cost, per_sample_decisions=per_sample, **tuning)
     for tuning in ({"warps_per_block": 8}, {"points_per_warp": 1}):
         _run(cuda, pair, cost, **tuning)
+
+
+@pytest.mark.parametrize("channels", [1, 3])
+@pytest.mark.parametrize("cost", COSTS + ["MI"])
+@pytest.mark.parametrize("h,w", [(1, 300), (9, 70), (70, 9), (33, 33)])
+def test_rows_along_the_moving_images_edges(cuda, lib, cost, channels, h, w):
+    """No rotation, unit scale and whole pixels: the edge rows are band pixels from end to end (1 to 300,
+    around the 8 that a lane takes by itself and the 32 of a warp), with and without a slight tilt."""
+    pair = _pair(900 + w, cost, h, w, h + 2, w + 1, channels, u8=channels == 3)
+    pair.lo[:] = [0, 1, 1, 0, -8, -2, 0, -2e-6]
+    pair.hi[:] = [2e-6, 1, 1, 0, 8, 2, 0, 0]
+    pair.count[:] = [2, 1, 1, 1, 5, 5, 1, 2]
+    _, c = _run(cuda, pair, cost)
+    if cost == "MI":
+        _, c0 = _run(cuda, pair, cost, per_sample_decisions=True)
+        np.testing.assert_array_equal(c.view(np.uint32), c0.view(np.uint32))
+    _oracle_agrees(pair, cost, c)
