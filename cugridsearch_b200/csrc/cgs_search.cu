@@ -838,18 +838,44 @@ bool span_plan(const cgs_image &mov, const cgs_image &fix, const cgs_options &o,
 }
 
 // Parts that a windowed span search's tasks are split into (see the span kernel): the number, at most one
-// per band and 16, with the least waves x (sweep share + setup), a part's setup (decode, windows, the
-// first copies) being about 12 K cycles and a task's sweep 8 (ZNCC) or 15 cycles per 32 evaluations.
-// Whole tasks unless that saves 3 %, or where the bands' totals would take over 64 MB.
+// per band and 16, with the shortest busiest CTA, a part's setup (decode, windows, the first copies) being
+// about 12 K cycles and a task's sweep 8 (ZNCC) or 15 cycles per 32 evaluations.  CTA b runs units b,
+// b + sms, ..; unit u is part u mod k of its task, and a part's share of the sweep is its rows': where sms and
+// k have a common factor some CTAs get only the long parts (48 x 72 pixels in parts of 1 and 2 bands took
+// 1.16 times as long as whole).  Whole tasks unless that saves 3 %, or where the bands' totals would take
+// over 64 MB.
 static int span_splits(const SpanPlan &sp, int cost, uint32_t tasks, const cgs_image &fix, int sms) {
     const double points = (double)sp.G * sp.NW;
     if (cost == CGS_COST_MI || (double)tasks * sp.tiles_y * points * 40.0 > 64e6) return 1;
     const double sweep = (double)fix.width * fix.height * fix.channels * points / 32.0 * (cost == CGS_COST_ZNCC ? 8.0 : 15.0);
     const double setup = 12000.0 / sweep;
-    auto waves = [&](int k) { return (double)(((uint64_t)tasks * k + sms - 1) / sms) * (1.0 / k + setup); };
+    auto busiest = [&](int k) {
+        double part[16], most = 0.0;
+        for (int i = 0; i < k; i++)
+            part[i] = (double)(std::min((i + 1) * sp.tiles_y / k * sp.TH, (int)fix.height) - i * sp.tiles_y / k * sp.TH) / fix.height + setup;
+        const uint32_t units = tasks * (uint32_t)k;
+        for (int b = 0; b < k && (uint32_t)b < units && b < sms; b++) {  // CTAs b, b + k, .. have equal loads, or one unit less
+            const uint32_t n = (units - (uint32_t)b - 1u) / (uint32_t)sms + 1u;
+            double turn = 0.0, rest = 0.0;  // k units in a row; the remaining ones
+            for (uint32_t i = 0; i < (uint32_t)k; i++) {
+                const double t = part[((uint32_t)b + i * (uint32_t)sms) % (uint32_t)k];
+                turn += t;
+                if (i < n % (uint32_t)k) rest += t;
+            }
+            most = std::max(most, (double)(n / (uint32_t)k) * turn + rest);
+        }
+        return most;
+    };
+    const double whole = busiest(1);
+    double least = 0.97 * whole;
     int best = 1;
-    for (int k = 2; k <= std::min(sp.tiles_y, 16); k++)
-        if (waves(k) < 0.97 * waves(1) && waves(k) < waves(best)) best = k;
+    for (int k = 2; k <= std::min(sp.tiles_y, 16); k++) {
+        const double t = busiest(k);
+        if (t < least) {
+            least = t;
+            best = k;
+        }
+    }
     return best;
 }
 
