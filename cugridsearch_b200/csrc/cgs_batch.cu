@@ -372,7 +372,7 @@ cgs_status cgs_batch_create(const cgs_pair *pairs, int32_t n, const cgs_batch_pl
         uint32_t ppt = 0;
         SpanPlan zp;
         const bool group = span_plan(q.moving, q.fixed, q.options, pd.mi_bins, &zp) &&
-                           kernel_span_batch(zp.G, zp.NW, zp.TX, zp.check) != nullptr &&
+                           kernel_span_batch(zp.G, zp.NW, zp.TX, false, zp.check) != nullptr &&
                            (!have_group || (zp.G == gplan.G && zp.NW == gplan.NW && zp.TX == gplan.TX &&
                                             zp.TH == gplan.TH && zp.pitch_mod == gplan.pitch_mod));
         const bool fits = group && group_cap(zp, zp.tiles_x * zp.tiles_y) > 0;
@@ -443,9 +443,11 @@ cgs_status cgs_batch_create(const cgs_pair *pairs, int32_t n, const cgs_batch_pl
     // tile count, one window stage size), as span_plan sizes it for one pair
     uint32_t gn = 0;
     int gtiles = 0;
+    bool gzncc = true;
     for (int32_t i = 0; i < n; i++)
         if (pend[i].route == 1) {
             gn++;
+            gzncc = gzncc && pairs[i].options.cost == CGS_COST_ZNCC;
             gtiles = std::max(gtiles, pend[i].zp.tiles_x * pend[i].zp.tiles_y);
         }
     const int gcap = gn > 0 ? group_cap(gplan, gtiles) : 0;
@@ -618,7 +620,7 @@ cgs_status cgs_batch_create(const cgs_pair *pairs, int32_t n, const cgs_batch_pl
         ga.tile_h = gplan.TH;
         ga.tiles = gtiles;
         ga.cap = gcap;
-        b->g_kfn = kernel_span_batch(gplan.G, gplan.NW, gplan.TX, gplan.check);
+        b->g_kfn = kernel_span_batch(gplan.G, gplan.NW, gplan.TX, gzncc, gplan.check);
         b->g_smem = span_kernel_smem(gplan.G, gplan.NW, gplan.TH, gplan.TX, gtiles, gcap, true, 0);
         e = cudaMemcpy(b->mem + gpar_off, gpar.data(), sizeof(SearchParams) * gn, cudaMemcpyHostToDevice);
         if (e == cudaSuccess) e = cudaMemcpy(b->mem + gtb_off, gtb.data(), 4 * gtb.size(), cudaMemcpyHostToDevice);

@@ -137,9 +137,9 @@ inline int span_quad_form(int cost, int channels) {
     return cost == CGS_COST_ZNCC || (cost == CGS_COST_MI && channels == 1) ? 1 : 2;
 }
 inline bool span_uses_prefix(int cost) { return cost != CGS_COST_SAD_AVG && cost != CGS_COST_MI; }
-// The multi-pair span kernel of batches for a plan (null where not instantiated), and the
-// staging step of many pairs in one launch.
-const void *kernel_span_batch(int G, int NW, int TX, bool check);
+// The multi-pair span kernel of batches for a plan (null where not instantiated; zncc: for ZNCC pairs
+// alone), and the staging step of many pairs in one launch.
+const void *kernel_span_batch(int G, int NW, int TX, bool zncc, bool check);
 cudaError_t launch_span_prep_batch(const SpanPrepArgs *args, int n, int blocks, cudaStream_t stream);
 
 // Span kernel of single-channel MI (cgs_span_mi.cuh): 2 points per warp, NW warps, histograms of B <= 32

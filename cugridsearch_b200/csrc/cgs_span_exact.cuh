@@ -9,7 +9,7 @@
 // between the real and the reference's coordinates, so every pixel of the inner span is inside for the
 // reference; band pixels are decided and sampled in the span pass.  A point without a guard, or whose
 // quotients could leave exact_quot2's range, has no spans: the whole warp samples all of its pixels
-// with IEEE divisions (no_span_rows).
+// with IEEE divisions (band_pixels).
 //
 // Sweep.  Lane l takes the columns x0 + 32 c + l of a tile, block c after block c and in each block
 // the rows that have samples there (two ballots per block sort the rows into full, masked and none).
@@ -77,7 +77,110 @@ __device__ __forceinline__ void accumulate64(double *a, float f, float m) {
 
 constexpr int kFewBand = 8;  // band pixels of a row that its lane samples by itself
 
-template <int COST, int C, int G, int NW, int TX, bool CHECK>
+// The band pixels of a row: the outer span outside the inner one, [pa, e0) and [e1, pe).
+struct RowBand {
+    int pa, e0, e1, pe;
+    __device__ __forceinline__ explicit RowBand(const RowSpans &s)
+        : pa(s.pa), e0(s.len > 0 ? s.xa : s.pa + s.plen), e1(s.len > 0 ? s.xa + s.len : s.pa + s.plen), pe(s.pa + s.plen) {}
+    __device__ __forceinline__ bool many() const { return (e0 - pa) + (pe - e1) > kFewBand; }
+};
+
+// The samples of a point outside its inner spans: the reference's sequence, scaled by kS.
+template <int COST, int C>
+struct SpanSampler {
+    static constexpr int NS = SpanSums<COST>::value;
+    MapCoef kc;
+    Plane mov, fix;
+    float mw, mh, kS;
+    uint32_t hist;  // shared address of the point's histogram
+    int B;
+    double a[NS] = {}, s2 = 0.0;  // the sums, sum f^2
+    int n = 0;
+    __device__ __forceinline__ SpanSampler(const SearchParams &p, const SpanSlot &sl, const uint32_t *h, float scale)
+        : kc{sl.A, sl.B, sl.P, sl.Q, sl.C1, sl.C2, sl.R, sl.S, sl.D1, sl.D2, sl.T, sl.U}, mov(p.mov), fix(p.fix),
+          mw(p.mov_wf), mh(p.mov_hf), kS(scale), hist(smem_addr(h)), B(p.mi_bins) {}
+    __device__ __forceinline__ void add(int x, int y) {
+        float ex, ey;
+        exact_map(kc, (float)x, (float)y, ex, ey);
+        if (!in_image(ey, ex, mw, mh)) return;
+#pragma unroll
+        for (int ch = 0; ch < C; ch++) {
+            const float m = bilinear_in(mov.data + ch * mov.plane, mov.pitch, ey, ex);
+            const float f = __ldg(fix.data + ch * fix.plane + (int64_t)y * fix.pitch + x);
+            if constexpr (COST == CGS_COST_MI) red_shared_add1(hist + 4u * (uint32_t)(mi_bin(f, kS, B) * (B + 1) + mi_bin(m, kS, B)));
+            else accumulate64<COST>(a, f * kS, m * kS);
+            if constexpr (COST == CGS_COST_SQD_REF || COST == CGS_COST_NCC_REF) s2 += (double)f * (double)f;
+        }
+        n++;
+    }
+};
+
+// What few bands of rows have: the band pixels of the rows from y0 of the warp's points, a few by the row's
+// lane, many (a row along an edge of the moving image has nothing else) by the warp, and every pixel of
+// the points without spans.  parts: a bit per 32 (point, row) entries that have band pixels.  A function
+// of its own, which leaves the sweep its registers (SAD 256 x 256 7.01 ms against 7.15-7.25 inlined).  The
+// multi-pair kernel, whose bodies share one register allocation, spills around such a call (8 % slower): it
+// samples the same pixels in the span pass itself.
+template <int COST, int C, int G>
+__device__ __noinline__ void band_pixels(const SearchParams &p, const SpanSlot *slots, double *band, int *cnt, uint32_t *hist,
+                                         float kS, int y0, uint32_t parts) {
+    using Sampler = SpanSampler<COST, C>;
+    const int lane = threadIdx.x & 31, TH = p.tile_h, fw = p.fix.w, fh = p.fix.h;
+    const int hsize = (p.mi_bins + 1) * (p.mi_bins + 1);
+    // the sums of groups of `width` lanes into their points' totals
+    auto add = [&](int g, Sampler &s, int width, bool leader) {
+        for (int o = 1; o < width; o <<= 1) {
+            if constexpr (COST != CGS_COST_MI) {
+                s.s2 += __shfl_xor_sync(0xffffffffu, s.s2, o);
+#pragma unroll
+                for (int j = 0; j < Sampler::NS; j++) s.a[j] += __shfl_xor_sync(0xffffffffu, s.a[j], o);
+            }
+            s.n += __shfl_xor_sync(0xffffffffu, s.n, o);
+        }
+        if (leader) {
+            if constexpr (COST != CGS_COST_MI) {
+                band[g * 5] += s.s2;
+#pragma unroll
+                for (int j = 0; j < Sampler::NS; j++) band[g * 5 + 1 + j] += s.a[j];
+            }
+            cnt[g] += s.n;
+        }
+        __syncwarp();
+    };
+    auto run = [&](int g, int ya, int ye, int xa, int xb, int xc, int xd) {  // pixels [xa, xb) and [xc, xd)
+        Sampler s(p, slots[g], hist + g * hsize, kS);
+        for (int y = ya; y < ye; y++) {
+#pragma unroll (COST == CGS_COST_MI ? 2 : 4)
+            for (int x = xa + lane; x < xb; x += 32) s.add(x, y);
+            for (int x = xc + lane; x < xd; x += 32) s.add(x, y);
+        }
+        add(g, s, 32, lane == 0);
+    };
+    for (; parts; parts &= parts - 1u) {
+        const int i = lane + 32 * (__ffs(parts) - 1);
+        const bool act = i < G * TH;
+        const int g = act ? i / TH : 0, y = y0 + i - g * TH;
+        RowSpans sp{0, 0, 0, 0};
+        if (act && y < fh && slots[g].valid && slots[g].ok) sp = row_spans(slots[g], (float)y, fw, p.mov_wf, p.mov_hf);
+        const RowBand b(sp);
+        Sampler s(p, slots[g], hist + g * hsize, kS);
+        if (!b.many()) {
+            for (int x = b.pa; x < b.e0; x++) s.add(x, y);
+            for (int x = b.e1; x < b.pe; x++) s.add(x, y);
+        }
+        if (__any_sync(0xffffffffu, s.n > 0)) add(g, s, TH, act && i == g * TH);
+        for (uint32_t m = __ballot_sync(0xffffffffu, b.many()); m; m &= m - 1u) {
+            const int l = __ffs(m) - 1, yl = __shfl_sync(0xffffffffu, y, l);
+            run(__shfl_sync(0xffffffffu, g, l), yl, yl + 1, __shfl_sync(0xffffffffu, b.pa, l),
+                __shfl_sync(0xffffffffu, b.e0, l), __shfl_sync(0xffffffffu, b.e1, l), __shfl_sync(0xffffffffu, b.pe, l));
+        }
+    }
+    for (int g = 0; g < G; g++)
+        if (slots[g].valid && !slots[g].ok) run(g, y0, min(y0 + TH, fh), 0, fw, 0, 0);
+}
+
+// MULTI: a body of the multi-pair kernel.
+template <int COST, int C, int G, int NW, int TX, bool CHECK, bool MULTI = false>
 __device__ __forceinline__ bool run_span_exact_task(const SearchParams &p, uint32_t unit, const SpanSmem &ss,
                                                     uint32_t &wit) {
     static_assert(G % 2 == 0, "the span path pairs grid points");
@@ -103,20 +206,9 @@ __device__ __forceinline__ bool run_span_exact_task(const SearchParams &p, uint3
     SpanSlot *my_slots = ss.slots + warp * G;
     span_points<COST, G, true>(p, (task * NW + warp) * G, my_slots);
     __syncwarp();
-    // w = ((A x + By) + P) + nQ, -X = ((nC1 x + nC2 y) + nR) + S, -Y alike
-    float2 P2[GP], nQ2[GP], nR2[GP], S2[GP], nT2[GP], U2[GP];
     bool nospan = false;  // some point of the warp has no spans
 #pragma unroll
-    for (int h = 0; h < GP; h++) {
-        const SpanSlot &a = my_slots[2 * h], &b = my_slots[2 * h + 1];
-        P2[h] = make_float2(a.P, b.P);
-        nQ2[h] = make_float2(-a.Q, -b.Q);
-        nR2[h] = make_float2(-a.R, -b.R);
-        S2[h] = make_float2(a.S, b.S);
-        nT2[h] = make_float2(-a.T, -b.T);
-        U2[h] = make_float2(a.U, b.U);
-        nospan |= (a.valid && !a.ok) || (b.valid && !b.ok);
-    }
+    for (int g = 0; g < G; g++) nospan |= my_slots[g].valid && !my_slots[g].ok;
     float2 *my_rows = ss.rowtab + (size_t)warp * TH * GP * 3;  // [TH][GP]{B y, -C2 y, -D2 y}
     uint32_t *my_hist = ss.hist + (size_t)warp * G * hsize;
     double *my_dtot = ss.dtot + warp * G * 5;  // {sum f^2, the sweep's NS sums} per point, stride 5
@@ -180,35 +272,41 @@ __device__ __forceinline__ bool run_span_exact_task(const SearchParams &p, uint3
             my_cnt[g] += n;
         }
     };
-    // pixels [xs, xe) of rows [ya, ye) of point g, by the whole warp
-    auto sample_run = [&](int g, int ya, int ye, int xs, int xe) {
-        double a[NS] = {}, s2 = 0.0;
-        int n = 0;
-        const int w = xe - xs;
-        int x = xs + lane, y = ya;
-        while (y < ye) {
-            while (x >= xe && y < ye) {
-                x -= w;
-                y++;
-            }
-            if (y < ye) n += exact_sample(g, x, y, a, s2);
-            x += 32;
-        }
-        add_totals(g, lane == 0, 32, a, s2, n, true);
-        __syncwarp();
-    };
-    // every pixel of the band's rows for the points without spans
+    // every pixel of the band's rows for the points without spans, all lanes over the columns
     auto no_span_rows = [&](int y0, int y1) {
-        for (int g = 0; g < G; g++)
-            if (my_slots[g].valid && !my_slots[g].ok) sample_run(g, y0, y1, 0, fw);
+        for (int g = 0; g < G; g++) {
+            const SpanSlot &sl = my_slots[g];
+            if (!sl.valid || sl.ok) continue;
+            double a[NS] = {}, s2 = 0.0;
+            int n = 0;
+            for (int y = y0; y < y1; y++)
+                for (int x = lane; x < fw; x += 32) n += exact_sample(g, x, y, a, s2);
+            add_totals(g, lane == 0, 32, a, s2, n, true);
+            __syncwarp();
+        }
     };
 
-    // ---- sweep
+    // ---- sweep.  The points' coefficients,
+    // w = ((A x + By) + P) + nQ, -X = ((nC1 x + nC2 y) + nR) + S, -Y alike,
+    // and the sums are set at the start of a band, after its span pass, which then has their registers (the
+    // multi-pair kernel, where that spills: once)
+    float2 P2[GP], nQ2[GP], nR2[GP], S2[GP], nT2[GP], U2[GP];
     float2 acc[GP][NS];
+    auto set_points = [&]() {
 #pragma unroll
-    for (int h = 0; h < GP; h++)
+        for (int h = 0; h < GP; h++) {
+            const SpanSlot &a = my_slots[2 * h], &b = my_slots[2 * h + 1];
+            P2[h] = make_float2(a.P, b.P);
+            nQ2[h] = make_float2(-a.Q, -b.Q);
+            nR2[h] = make_float2(-a.R, -b.R);
+            S2[h] = make_float2(a.S, b.S);
+            nT2[h] = make_float2(-a.T, -b.T);
+            U2[h] = make_float2(a.U, b.U);
 #pragma unroll
-        for (int j = 0; j < NS; j++) acc[h][j] = make_float2(0.0f, 0.0f);
+            for (int j = 0; j < NS; j++) acc[h][j] = make_float2(0.0f, 0.0f);
+        }
+    };
+    if constexpr (MULTI) set_points();
     InnerSpan *my_spans = ss.spans + warp * G * TH;
     RowRun *my_runs = ss.runs + warp * TH;
     const float2 magic2 = make_float2(kMagic, kMagic), minus1 = make_float2(-1.0f, -1.0f);
@@ -232,20 +330,18 @@ __device__ __forceinline__ bool run_span_exact_task(const SearchParams &p, uint3
         const int x1 = min(x0 + TW, fw) - 1;
         if (tx == 0) {
             // the band's rows: spans, the fixed sums of the inner ones, the band pixels
+            uint32_t parts = 0u;  // entries with band pixels
             for (int k = 0; 32 * k < G * TH; k++) {
                 const int i = lane + 32 * k;
                 const bool act = i < G * TH;
-                const int g = act ? i / TH : 0, r = i - g * TH;
-                double a[NS] = {}, s2 = 0.0;
-                int n = 0;
-                bool found = false, sure = true;
-                const int y = y0 + r;
+                const int g = act ? i / TH : 0, r = i - g * TH, y = y0 + r;
                 RowSpans sp{0, 0, 0, 0};
+                double s2 = 0.0;
+                bool sure = true;
                 if (act) {
                     const SpanSlot &sl = my_slots[g];
                     if (y < fh && sl.valid && sl.ok) sp = row_spans(sl, (float)y, fw, mov_wf, mov_hf);
                     my_spans[g * TH + r] = InnerSpan{sp.xa, sp.len};
-                    n = sp.len;
                     if constexpr (kFix) {
                         if (sp.len > 0) {
                             const double2 *pr = p.fix_prefix + (int64_t)y * (fw + 1) + sp.xa;
@@ -255,6 +351,7 @@ __device__ __forceinline__ bool run_span_exact_task(const SearchParams &p, uint3
                         }
                     }
                 }
+                parts |= (__any_sync(0xffffffffu, sp.plen > sp.len) ? 1u : 0u) << k;
                 if constexpr (kFix) {
                     for (uint32_t m = __ballot_sync(0xffffffffu, !sure); m; m &= m - 1u) {
                         const int l = __ffs(m) - 1;
@@ -263,27 +360,56 @@ __device__ __forceinline__ bool run_span_exact_task(const SearchParams &p, uint3
                         if (lane == l) s2 = t;
                     }
                 }
-                // band pixels: the outer span outside the inner one, [pa, e0) and [e1, pe).  A few, sampled by
-                // the row's lane; of a row along an edge of the moving image all, sampled by the warp
-                const int pe = sp.pa + sp.plen, e0 = sp.len > 0 ? sp.xa : pe, e1 = sp.len > 0 ? sp.xa + sp.len : pe;
-                const bool many = (e0 - sp.pa) + (pe - e1) > kFewBand;
-                if (act && !many) {
-                    int nb = 0;
-                    for (int x = sp.pa; x < e0; x++) nb += exact_sample(g, x, y, a, s2);
-                    for (int x = e1; x < pe; x++) nb += exact_sample(g, x, y, a, s2);
-                    n += nb;
-                    found = nb > 0;
-                }
-                for (uint32_t m = __ballot_sync(0xffffffffu, many); m; m &= m - 1u) {
-                    const int l = __ffs(m) - 1;
-                    const int gl = __shfl_sync(0xffffffffu, g, l), yl = __shfl_sync(0xffffffffu, y, l);
-                    for (int side = 0; side < 2; side++) {
-                        const int xs = __shfl_sync(0xffffffffu, side ? e1 : sp.pa, l);
-                        const int xe = __shfl_sync(0xffffffffu, side ? pe : e0, l);
-                        if (xe > xs) sample_run(gl, yl, yl + 1, xs, xe);
+                if constexpr (MULTI) {
+                    double a[NS] = {};
+                    int n = sp.len;
+                    // band pixels: the outer span outside the inner one, [pa, e0) and [e1, pe).  First every lane
+                    // its row's, if a few; then, row after row, the warp those of a row with many (one along an
+                    // edge of the moving image has nothing else)
+                    const int pe = sp.pa + sp.plen, e0 = sp.len > 0 ? sp.xa : pe, e1 = sp.len > 0 ? sp.xa + sp.len : pe;
+                    const bool many = (e0 - sp.pa) + (pe - e1) > kFewBand;
+                    uint32_t rows = __ballot_sync(0xffffffffu, many);
+                    int gc = g, yc = y, xa = sp.pa, xb = many ? sp.pa : e0, xc = e1, xd = many ? e1 : pe, step = 1, width = TH;
+                    bool first = act && r == 0;
+                    for (;;) {
+                        int nb = 0;
+                        for (int x = xa; x < xb; x += step) nb += exact_sample(gc, x, yc, a, s2);
+                        for (int x = xc; x < xd; x += step) nb += exact_sample(gc, x, yc, a, s2);
+                        add_totals(gc, first, width, a, s2, n + nb, __any_sync(0xffffffffu, nb > 0));
+                        if (rows == 0u) break;
+                        const int l = __ffs(rows) - 1;
+                        rows &= rows - 1u;
+                        gc = __shfl_sync(0xffffffffu, g, l);
+                        yc = __shfl_sync(0xffffffffu, y, l);
+                        xa = __shfl_sync(0xffffffffu, sp.pa, l) + lane;
+                        xb = __shfl_sync(0xffffffffu, e0, l);
+                        xc = __shfl_sync(0xffffffffu, e1, l) + lane;
+                        xd = __shfl_sync(0xffffffffu, pe, l);
+                        step = width = 32;
+                        first = lane == 0;
+                        n = 0;
+                        s2 = 0.0;
+#pragma unroll
+                        for (int j = 0; j < NS; j++) a[j] = 0.0;
+                        __syncwarp();
+                    }
+                } else {
+                    int n = sp.len;
+                    for (int o = 1; o < TH; o <<= 1) {
+                        if constexpr (kFix) s2 += __shfl_xor_sync(0xffffffffu, s2, o);
+                        n += __shfl_xor_sync(0xffffffffu, n, o);
+                    }
+                    if (act && r == 0) {
+                        if constexpr (kFix) my_band[g * 5] += s2;
+                        my_cnt[g] += n;
                     }
                 }
-                add_totals(g, act && r == 0, TH, a, s2, n, __any_sync(0xffffffffu, found));
+            }
+            __syncwarp();
+            if constexpr (MULTI) {
+                if (nospan) no_span_rows(y0, min(y0 + TH, fh));
+            } else if (parts || nospan) {
+                band_pixels<COST, C, G>(p, my_slots, my_band, my_cnt, my_hist, kS, y0, parts);
             }
             __syncwarp();
             if (lane < TH) {  // the rows' common inner run and the hull of the inner spans
@@ -312,7 +438,7 @@ __device__ __forceinline__ bool run_span_exact_task(const SearchParams &p, uint3
                 d[2] = make_float2(-xm(a.D2, yf), -xm(b.D2, yf));
             }
             __syncwarp();
-            if (nospan) no_span_rows(y0, min(y0 + TH, fh));
+            if constexpr (!MULTI) set_points();
         }
         const int st = (int)(wit % kWinStages);
         if (!mbar_wait_bounded(&ss.bars[st], (wit / kWinStages) & 1u, kWaitLimitNs)) *ss.abort_flag = 1;
@@ -502,7 +628,7 @@ __device__ __forceinline__ bool run_span_exact_task(const SearchParams &p, uint3
                         my_band[(2 * h) * 5 + 1 + j] += (double)s0;
                         my_band[(2 * h + 1) * 5 + 1 + j] += (double)s1;
                     }
-                    acc[h][j] = make_float2(0.0f, 0.0f);
+                    if constexpr (MULTI) acc[h][j] = make_float2(0.0f, 0.0f);
                 }
             fold_band<G, NW>(p, task, ty, my_dtot, my_band);
         }

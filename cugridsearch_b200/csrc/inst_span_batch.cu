@@ -4,9 +4,10 @@
 
 namespace cgs {
 
-const void *kernel_span_batch(int G, int NW, int TX, bool check) {
-    if (G == 4 && NW == 16 && TX == 8 && !check) return (const void *)span_batch_kernel<4, 16, 8, false>;
-    return nullptr;
+const void *kernel_span_batch(int G, int NW, int TX, bool zncc, bool check) {
+    if (G != 4 || NW != 16 || TX != 8 || check) return nullptr;
+    return zncc ? (const void *)span_batch_kernel<4, 16, 8, true, false>
+                : (const void *)span_batch_kernel<4, 16, 8, false, false>;
 }
 
 }  // namespace cgs
