@@ -372,6 +372,7 @@ cgs_status cgs_batch_create(const cgs_pair *pairs, int32_t n, const cgs_batch_pl
         uint32_t ppt = 0;
         SpanPlan zp;
         const bool group = span_plan(q.moving, q.fixed, q.options, pd.mi_bins, &zp) &&
+                           span_pays(&zp, q.options.cost, q.fixed, pd.p.n, di.sms) &&
                            kernel_span_batch(zp.G, zp.NW, zp.TX, false, zp.check) != nullptr &&
                            (!have_group || (zp.G == gplan.G && zp.NW == gplan.NW && zp.TX == gplan.TX &&
                                             zp.TH == gplan.TH && zp.pitch_mod == gplan.pitch_mod));

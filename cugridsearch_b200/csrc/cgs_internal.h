@@ -122,15 +122,18 @@ constexpr int kMinSpanCap = 1024;                   // smallest useful window st
 struct SpanPlan {
     int G = 4, NW = 16, TX = 2, TH = 16;
     int tiles_x = 0, tiles_y = 0, cap = 0, pitch_mod = 0;
+    int splits = 1;      // a single search's parts per task
     bool exact = false;  // cgs_span_exact.cuh
     int mi_bins = 0;     // MI: histogram bins
     bool check = false;
     size_t smem = 0;
     const void *kfn = nullptr;
 };
-// Whether cgs_search runs a request on a span kernel with windows (zero-mean NCC and three-channel MI in
+// Whether cgs_search can run a request on a span kernel with windows (zero-mean NCC and three-channel MI in
 // their default sampling mode, SAD_AVG, SQD_REF and NCC_REF on exact samples), with its plan.
 bool span_plan(const cgs_image &mov, const cgs_image &fix, const cgs_options &o, int mi_bins, SpanPlan *sp);
+// Whether it does so for a grid of `points` (narrow images: the per-sample kernel), and the plan's splits.
+bool span_pays(SpanPlan *sp, int cost, const cgs_image &fix, uint32_t points, int sms);
 // The staging form of the quads (PrepParams::quad_form) and whether the cost reads the fixed rows'
 // prefix sums.
 inline int span_quad_form(int cost, int channels) {

@@ -843,9 +843,10 @@ bool span_plan(const cgs_image &mov, const cgs_image &fix, const cgs_options &o,
 // b + sms, ..; unit u is part u mod k of its task, and a part's share of the sweep is its rows': where sms and
 // k have a common factor some CTAs get only the long parts (48 x 72 pixels in parts of 1 and 2 bands took
 // 1.16 times as long as whole).  Whole tasks unless that saves 3 %, or where the bands' totals would take
-// over 64 MB.
-static int span_splits(const SpanPlan &sp, int cost, uint32_t tasks, const cgs_image &fix, int sms) {
+// over 64 MB.  *gain: the busiest CTA's time with whole tasks over that with split ones.
+static int span_splits(const SpanPlan &sp, int cost, uint32_t tasks, const cgs_image &fix, int sms, double *gain) {
     const double points = (double)sp.G * sp.NW;
+    *gain = 1.0;
     if (cost == CGS_COST_MI || (double)tasks * sp.tiles_y * points * 40.0 > 64e6) return 1;
     const double sweep = (double)fix.width * fix.height * fix.channels * points / 32.0 * (cost == CGS_COST_ZNCC ? 8.0 : 15.0);
     const double setup = 12000.0 / sweep;
@@ -874,9 +875,33 @@ static int span_splits(const SpanPlan &sp, int cost, uint32_t tasks, const cgs_i
         if (t < least) {
             least = t;
             best = k;
+            *gain = whole / t;
         }
     }
     return best;
+}
+
+// Whether the windowed span kernel of a plan is the faster one for a grid of `points`, and its splits.  Its
+// lanes take the columns of 32-wide blocks, so narrow images leave lanes idle which the per-sample kernel,
+// dealing pixels to lanes in turn, does not: the span kernel of the exact costs pays where the share of
+// busy lanes, times what splitting gains over the per-sample kernel's whole tasks, is above a line.  Measured
+// on a full GPU, 100 rows, span over per-sample speed: one channel SAD (NCC) 8 columns 0.46 (0.48), 24
+// 0.84 (0.89), 28 0.94 (1.00), 33 0.72 (0.83), 44 0.90 (0.99), 48 0.95 (1.07), 65 1.01 (1.14); three channels
+// 16 0.83 (0.91), 20 0.98 (1.08), 33 0.97 (1.17); MI of three 20 0.94, 24 1.07, 33 0.97, 44 1.10.  One row
+// alone (nothing to split, one row per block) loses on a GPU that is not full: 1 x 3000 NCC 0.84.  ZNCC is
+// faster at every width.  The self-checking build runs wherever it can.
+bool span_pays(SpanPlan *sp, int cost, const cgs_image &fix, uint32_t points, int sms) {
+    const uint32_t per_task = (uint32_t)(sp->G * sp->NW), tasks = (points + per_task - 1) / per_task;
+    double gain;
+    sp->splits = span_splits(*sp, cost, tasks, fix, sms, &gain);
+    if (!sp->exact || sp->check) return true;
+    if (fix.height == 1 && tasks < (uint32_t)sms) return false;
+    const int blocks = (fix.width + 31) / 32;
+    const double busy = (double)fix.width / (32.0 * blocks) * gain;
+    const bool mi = cost == CGS_COST_MI, rgb = fix.channels == 3;
+    if (blocks == 1) return busy >= (mi ? 0.72 : rgb ? 0.6 : 0.85);
+    if (blocks == 2) return busy >= (mi ? 0.6 : rgb ? 0.0 : cost == CGS_COST_SAD_AVG ? 0.72 : 0.66);
+    return true;
 }
 
 // Launch plan of the MI span kernel: 16 warps of 2 points, bands of TH = 16 rows (CGS_SPAN_TH
@@ -1134,19 +1159,17 @@ static cgs_status search_core(const cgs_image *mov, const cgs_image *fix, const 
     // taps: pre-gathered quads where the fast sampling path runs (measured faster than texture
     // gathers there); texture gathers (MI: scalar loads) for exact sampling and for MI
     const bool fast_path = !exact_samples(cost, o.flags) && cost != CGS_COST_MI;
+    bool quads = (o.flags & CGS_FLAG_QUAD_TAPS) || (fast_path && !(o.flags & CGS_FLAG_TEXTURE_TAPS));
+    const void *kfn = getter(C, pl.G, pl.NW, quads);  // the per-sample kernel
     SpanPlan sp;  // the span kernels (decisions per image row)
-    const bool span = span_plan(*mov, *fix, o, mi_bins, &sp);
+    bool span = span_plan(*mov, *fix, o, mi_bins, &sp);
     const bool span_mi = !span && cost == CGS_COST_MI && !exact_samples(cost, o.flags) &&
                          !(o.flags & (CGS_FLAG_PER_SAMPLE_DECISIONS | CGS_FLAG_TEXTURE_TAPS | CGS_FLAG_QUAD_TAPS)) &&
                          span_mi_plan(*mov, *fix, o, mi_bins, &sp);
-    const bool spans = span || span_mi;
-    const bool quads = spans || (o.flags & CGS_FLAG_QUAD_TAPS) || (fast_path && !(o.flags & CGS_FLAG_TEXTURE_TAPS));
-    const void *kfn = spans ? sp.kfn : getter(C, pl.G, pl.NW, quads);
     // a request's tuning has to be one of the per-sample kernel's, though the exact span kernel ignores it
     const bool tuned = span && sp.exact && (o.points_per_warp != 0 || o.warps_per_block != 0);
-    if (!kfn || (tuned && !getter(C, pl.G, pl.NW, false)))
+    if (!kfn && !span_mi && !(span && !sp.exact))
         return fail(CGS_ERROR_UNSUPPORTED, "no kernel for this channel count / tuning");
-    if (ext && !spans) return fail(CGS_ERROR_UNSUPPORTED, "caller scratch: span searches only");
 
     DeviceInfo di;
     if ((s = device_info(&di)) != CGS_SUCCESS) return s;
@@ -1154,6 +1177,13 @@ static cgs_status search_core(const cgs_image *mov, const cgs_image *fix, const 
     SearchParams p;
     int64_t n64;
     if ((s = fill_params(mov, fix, grid, o, mi_bins, &p, &n64)) != CGS_SUCCESS) return s;
+    span = span && span_pays(&sp, cost, *fix, p.n, di.sms);
+    const bool spans = span || span_mi;
+    if (ext && !spans) return fail(CGS_ERROR_UNSUPPORTED, "caller scratch: span searches only");
+    if (spans) {
+        quads = true;
+        kfn = sp.kfn;
+    }
     if (n64 <= 0) {
         if (query) {
             ext->bytes = 0;
@@ -1190,7 +1220,7 @@ static cgs_status search_core(const cgs_image *mov, const cgs_image *fix, const 
     const uint32_t per_task = spans ? (uint32_t)(sp.NW * sp.G) : (uint32_t)(pl.NW * pl.G);
     p.num_tasks = (p.n + per_task - 1) / per_task;
     // split tasks: the bands' totals, the parts' counts, the parts done
-    p.splits = span ? span_splits(sp, cost, p.num_tasks, *fix, di.sms) : 1;
+    p.splits = span ? sp.splits : 1;
     const size_t tot_off = (size_t)round_up((int64_t)(prefix_off + prefix_bytes), 256);
     const size_t tot_bytes = (size_t)p.num_tasks * sp.tiles_y * per_task * 5 * sizeof(double);
     const size_t cnt_bytes = (size_t)round_up((int64_t)p.num_tasks * p.splits * per_task * (int64_t)sizeof(int), 256);

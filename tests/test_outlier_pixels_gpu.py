@@ -12,7 +12,7 @@ import pytest
 import oracle as O
 from conftest import close_costs
 from cugridsearch_b200 import synthetic as S
-from test_span_gpu import _run
+from test_span_gpu import _env, _run
 
 pytestmark = pytest.mark.gpu
 COSTS = ["SQD_REF", "NCC_REF"]
@@ -42,6 +42,16 @@ def _oracle(p, cost, fixed):
     return O.search(cost, O.make_grid(*p.grid_args()), O.Image(p.moving), O.Image(fixed))
 
 
+def _runs(cuda, p, cost):
+    """A search, one on the span kernel whatever the width (self-checking), and a batch."""
+    out = [_run(cuda, p, cost)[1]]
+    if p.fixed.shape[2] == 1:
+        with _env(CGS_SPAN_CHECK=1):
+            out.append(_run(cuda, p, cost)[1])
+        out.append(_batch(cuda, p, cost))
+    return out
+
+
 def _batch(cuda, p, cost):
     import torch
     import cugridsearch_b200 as cgs
@@ -68,8 +78,7 @@ def _check(cuda, cost, h, w, channels, value):
     clear = _clear(p, _outliers(p, np.float32("nan")), p.moving)
     c32, c64 = _oracle(p, cost, p.fixed)  # at clear points the outliers' values are not read
     p.fixed = np.ascontiguousarray(_outliers(p, value))
-    got = [_run(cuda, p, cost)[1]] + ([_batch(cuda, p, cost)] if channels == 1 else [])
-    for c in got:
+    for c in _runs(cuda, p, cost):
         bad = close_costs(c, c32, c64, cost) & clear
         assert not bad.any(), (int(bad.sum()), c[bad][:4], c64[bad][:4])
         if not np.isfinite(value):
@@ -93,7 +102,7 @@ def test_overlap_of_zeros(cuda, lib, cost, channels):
     p.fixed[:, 12:] = 0.0
     c32, c64 = _oracle(p, cost, p.fixed)
     assert 0.2 < (~np.isfinite(c64)).mean() < 0.8
-    for c in [_run(cuda, p, cost)[1]] + ([_batch(cuda, p, cost)] if channels == 1 else []):
+    for c in _runs(cuda, p, cost):
         bad = close_costs(c, c32, c64, cost)
         assert not bad.any(), (int(bad.sum()), c[bad][:4], c32[bad][:4], c64[bad][:4])
 

@@ -154,8 +154,28 @@ def test_rows_along_the_moving_images_edges(cuda, lib, cost, channels, h, w):
     pair.lo[:] = [0, 1, 1, 0, -8, -2, 0, -2e-6]
     pair.hi[:] = [2e-6, 1, 1, 0, 8, 2, 0, 0]
     pair.count[:] = [2, 1, 1, 1, 5, 5, 1, 2]
-    _, c = _run(cuda, pair, cost)
+    with _env(**({"CGS_SPAN_CHECK": 1} if channels == 1 and cost != "MI" else {})):  # narrow ones too
+        _, c = _run(cuda, pair, cost)
     if cost == "MI":
         _, c0 = _run(cuda, pair, cost, per_sample_decisions=True)
         np.testing.assert_array_equal(c.view(np.uint32), c0.view(np.uint32))
     _oracle_agrees(pair, cost, c)
+
+
+@pytest.mark.parametrize("channels", [1, 3])
+@pytest.mark.parametrize("cost", COSTS + ["MI"])
+@pytest.mark.parametrize("h,w", [(40, 8), (20, 16), (20, 24), (20, 28), (20, 33), (20, 44), (20, 48), (1, 300)])
+def test_narrow_images(cuda, lib, cost, channels, h, w):
+    """Widths around the lines of span_pays, which run on the per-sample kernel or the span kernel."""
+    pair = _pair(950 + w, cost, h, w, h, w, channels, u8=channels == 3)
+    _, c = _run(cuda, pair, cost)
+    _oracle_agrees(pair, cost, c)
+    if channels == 1 and cost != "MI":
+        with _env(CGS_SPAN_CHECK=1):  # the span kernel
+            _, c1 = _run(cuda, pair, cost)
+        _oracle_agrees(pair, cost, c1)
+        _, c2 = _run(cuda, pair, cost, per_sample_decisions=True)
+        if w < 28 or 33 <= w < 44:
+            np.testing.assert_array_equal(c.view(np.uint32), c2.view(np.uint32))
+        elif w in (28, 48):
+            np.testing.assert_array_equal(c.view(np.uint32), c1.view(np.uint32))
