@@ -181,6 +181,7 @@ __device__ __forceinline__ SpanSmem carve_span(unsigned char *smem, int TH, int 
 struct RowSpans {
     int xa, len, pa, plen;
 };
+constexpr int kFewBand = 8;  // band pixels of a row that its lane samples by itself (exact costs, MI)
 
 // The spans of row y (see the head of this file).  Each edge of the moving image gives a condition
 // s f(x) > 0 with f(x) = a x + b linear and s the sign of w; x = q solves f = 0.  f is the distance

@@ -75,8 +75,6 @@ __device__ __forceinline__ void accumulate64(double *a, float f, float m) {
     }
 }
 
-constexpr int kFewBand = 8;  // band pixels of a row that its lane samples by itself
-
 // The band pixels of a row: the outer span outside the inner one, [pa, e0) and [e1, pe).
 struct RowBand {
     int pa, e0, e1, pe;
