@@ -28,7 +28,7 @@ namespace cgs {
 
 namespace cg = cooperative_groups;
 
-constexpr int kVerifyCtas = 8;        // the portable cluster size
+constexpr int kVerifyCtas = 8;        // the portable cluster size; 1 for images of a few pixels (launch_verify)
 constexpr int kVerifyThreads = 512;   // per CTA
 
 struct VerifyHdr {
@@ -86,7 +86,7 @@ __device__ __forceinline__ void cluster_sum(double (&v)[N], double *red, double 
 #pragma unroll
         for (int j = 0; j < N; j++) {
             double s = 0.0;
-            for (int r = 0; r < kVerifyCtas; r++) s += cluster.map_shared_rank(part, r)[j];
+            for (int r = 0; r < (int)cluster.num_blocks(); r++) s += cluster.map_shared_rank(part, r)[j];
             v[j] = s;
         }
     }
@@ -97,7 +97,7 @@ __device__ __forceinline__ void cluster_sum(double (&v)[N], double *red, double 
 template <int COST>
 __device__ double rescore(const SearchParams &p, uint32_t idx, double *red, double *part, uint32_t *hist) {
     cg::cluster_group cluster = cg::this_cluster();
-    const int rank = (int)cluster.block_rank();
+    const int rank = (int)cluster.block_rank(), ctas = (int)cluster.num_blocks();
     int32_t ax[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     int32_t rem = (int32_t)idx;
     for (int a = p.dims - 1; a >= 0; a--) {
@@ -121,7 +121,7 @@ __device__ double rescore(const SearchParams &p, uint32_t idx, double *red, doub
     const double msh = COST == CGS_COST_ZNCC ? (double)p.shifts[1] : 0.0;
     double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0, s4 = 0.0, cnt = 0.0;
     const uint32_t npix = (uint32_t)fw * (uint32_t)fh;  // below 2^24
-    for (uint32_t i = (uint32_t)(rank * kVerifyThreads) + threadIdx.x; i < npix; i += kVerifyCtas * kVerifyThreads) {
+    for (uint32_t i = (uint32_t)(rank * kVerifyThreads) + threadIdx.x; i < npix; i += (uint32_t)(ctas * kVerifyThreads)) {
         const int y = (int)(i / (uint32_t)fw), x = (int)(i - (uint32_t)y * (uint32_t)fw);
         float ex, ey;
         exact_map(k, (float)x, (float)y, ex, ey);
@@ -166,7 +166,7 @@ __device__ double rescore(const SearchParams &p, uint32_t idx, double *red, doub
         const double n = v[0];
         if (rank == 0) {
             for (int i = threadIdx.x; i < B * B; i += blockDim.x)
-                for (int r = 1; r < kVerifyCtas; r++) hist[i] += cluster.map_shared_rank(hist, r)[i];
+                for (int r = 1; r < ctas; r++) hist[i] += cluster.map_shared_rank(hist, r)[i];
         }
         cluster.sync();
         double acc[1] = {0.0};
@@ -220,14 +220,13 @@ __device__ __forceinline__ bool fp64_less(double a, uint32_t ia, double b, uint3
 
 // One cluster per band point; the last cluster writes the verification fields of the result.
 template <int COST>
-__global__ void __cluster_dims__(kVerifyCtas, 1, 1) __launch_bounds__(kVerifyThreads)
-verify_kernel(const __grid_constant__ SearchParams p, VerifyHdr *h) {
+__global__ void __launch_bounds__(kVerifyThreads) verify_kernel(const __grid_constant__ SearchParams p, VerifyHdr *h) {
     extern __shared__ __align__(16) unsigned char vsm[];
     double *red = reinterpret_cast<double *>(vsm), *part = red + 6 * 32;
     uint32_t *hist = reinterpret_cast<uint32_t *>(part + 8);
     __shared__ unsigned int last;
     const cgs_argmin r0 = *p.result;
-    const unsigned int point = blockIdx.x / kVerifyCtas, rank = blockIdx.x % kVerifyCtas;
+    const unsigned int ctas = cg::this_cluster().num_blocks(), point = blockIdx.x / ctas, rank = blockIdx.x % ctas;
     const unsigned int found = r0.valid ? h->count : 0u;
     const unsigned int nc = min(found, (unsigned int)kVerifyMax);
     if (point < nc) {
@@ -237,7 +236,7 @@ verify_kernel(const __grid_constant__ SearchParams p, VerifyHdr *h) {
     if (rank != 0) return;
     if (threadIdx.x == 0) {
         __threadfence();
-        last = atomicAdd(&h->ticket, 1u) + 1u == gridDim.x / kVerifyCtas;
+        last = atomicAdd(&h->ticket, 1u) + 1u == gridDim.x / ctas;
     }
     __syncthreads();
     if (!last || threadIdx.x != 0) return;
@@ -292,8 +291,22 @@ cgs_status launch_verify(const SearchParams &p, void *hdr, cudaStream_t stream, 
     const size_t smem = (6 * 32 + 8) * sizeof(double) + (p.cost == CGS_COST_MI ? (size_t)p.mi_bins * p.mi_bins * 4 : 0);
     SearchParams pv = p;
     void *args[] = {&pv, &h};
+    // a few pixels per thread make a CTA's work: below that its cluster is one CTA (64 clusters of 8 took
+    // 12 us longer for a 1 x 1 image, whose points mostly tie)
+    const int ctas = (int64_t)p.fix.w * p.fix.h < 4 * kVerifyThreads ? 1 : kVerifyCtas;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = (unsigned)ctas;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)(kVerifyMax * ctas));
+    cfg.blockDim = dim3(kVerifyThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
     cudaError_t e = cudaGetLastError();
-    if (e == cudaSuccess) e = cudaLaunchKernel(kfn, dim3(kVerifyMax * kVerifyCtas), dim3(kVerifyThreads), args, smem, stream);
+    if (e == cudaSuccess) e = cudaLaunchKernelExC(&cfg, kfn, args);
     if (e != cudaSuccess) return cuda_fail(e, "verification pass");
     return CGS_SUCCESS;
 }
