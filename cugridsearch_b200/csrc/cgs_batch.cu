@@ -549,27 +549,28 @@ cgs_status cgs_batch_create(const cgs_pair *pairs, int32_t n, const cgs_batch_pl
             preps[j].quad_dst = reinterpret_cast<float4 *>(org + pd.st.quad_off);
             preps[j].qplane = pd.st.qplane;
         }
-        // the staged moving plane as a (W + 1) x (H + 1) texture (point sampling, border 0)
-        cudaResourceDesc rd;
-        memset(&rd, 0, sizeof(rd));
-        rd.resType = cudaResourceTypePitch2D;
-        rd.res.pitch2D.devPtr = mstage;
-        rd.res.pitch2D.desc = cudaCreateChannelDesc<float>();
-        rd.res.pitch2D.width = (size_t)q.moving.width + 1;
-        rd.res.pitch2D.height = (size_t)q.moving.height + 1;
-        rd.res.pitch2D.pitchInBytes = (size_t)pd.st.mpitch * 4;
-        cudaTextureDesc td;
-        memset(&td, 0, sizeof(td));
-        td.addressMode[0] = td.addressMode[1] = cudaAddressModeBorder;
-        td.filterMode = cudaFilterModePoint;
-        td.readMode = cudaReadModeElementType;
-        td.normalizedCoords = 0;
-        e = cudaCreateTextureObject(&b->tex[j], &rd, &td, nullptr);
-        if (e != cudaSuccess) {
-            release(b);
-            return cuda_fail(e, "cudaCreateTextureObject");
+        if (pd.route == 0) {  // the staged moving plane as a (W + 1) x (H + 1) texture (point sampling, border 0)
+            cudaResourceDesc rd;
+            memset(&rd, 0, sizeof(rd));
+            rd.resType = cudaResourceTypePitch2D;
+            rd.res.pitch2D.devPtr = mstage;
+            rd.res.pitch2D.desc = cudaCreateChannelDesc<float>();
+            rd.res.pitch2D.width = (size_t)q.moving.width + 1;
+            rd.res.pitch2D.height = (size_t)q.moving.height + 1;
+            rd.res.pitch2D.pitchInBytes = (size_t)pd.st.mpitch * 4;
+            cudaTextureDesc td;
+            memset(&td, 0, sizeof(td));
+            td.addressMode[0] = td.addressMode[1] = cudaAddressModeBorder;
+            td.filterMode = cudaFilterModePoint;
+            td.readMode = cudaReadModeElementType;
+            td.normalizedCoords = 0;
+            e = cudaCreateTextureObject(&b->tex[j], &rd, &td, nullptr);
+            if (e != cudaSuccess) {
+                release(b);
+                return cuda_fail(e, "cudaCreateTextureObject");
+            }
+            p.mov_tex = b->tex[j];
         }
-        p.mov_tex = b->tex[j];
         if (pd.route == 1) {
             // as cgs_search sets up its span kernels: quads in the cost's span form (ZNCC: with the
             // moving shift folded in), the fixed rows' prefix sums, tiles and the (common) window stage
@@ -623,11 +624,13 @@ cgs_status cgs_batch_create(const cgs_pair *pairs, int32_t n, const cgs_batch_pl
         ga.cap = gcap;
         b->g_kfn = kernel_span_batch(gplan.G, gplan.NW, gplan.TX, gzncc, gplan.check);
         b->g_smem = span_kernel_smem(gplan.G, gplan.NW, gplan.TH, gplan.TX, gtiles, gcap, true, 0);
-        e = cudaMemcpy(b->mem + gpar_off, gpar.data(), sizeof(SearchParams) * gn, cudaMemcpyHostToDevice);
-        if (e == cudaSuccess) e = cudaMemcpy(b->mem + gtb_off, gtb.data(), 4 * gtb.size(), cudaMemcpyHostToDevice);
-        if (e == cudaSuccess) e = cudaMemcpy(b->mem + gslot_off, gslot.data(), 4 * gn, cudaMemcpyHostToDevice);
-        if (e == cudaSuccess)
-            e = cudaMemcpy(b->d_gprep, gprep.data(), sizeof(SpanPrepArgs) * gn, cudaMemcpyHostToDevice);
+        // the four tables, neighbours in the block, in one copy (each of its own took the host 5 to 10 us)
+        std::vector<char> tables(gprep_off + gn * sizeof(SpanPrepArgs) - gpar_off);
+        memcpy(tables.data(), gpar.data(), sizeof(SearchParams) * gn);
+        memcpy(tables.data() + (gtb_off - gpar_off), gtb.data(), 4 * gtb.size());
+        memcpy(tables.data() + (gslot_off - gpar_off), gslot.data(), 4 * gn);
+        memcpy(tables.data() + (gprep_off - gpar_off), gprep.data(), sizeof(SpanPrepArgs) * gn);
+        e = cudaMemcpy(b->mem + gpar_off, tables.data(), tables.size(), cudaMemcpyHostToDevice);
         if (e == cudaSuccess)
             e = cudaFuncSetAttribute(b->g_kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b->g_smem);
         int per_sm = 0;
