@@ -33,3 +33,11 @@ def test_a_task_with_a_lost_part_has_no_costs(cuda, lib):
     for joined, done, status, untouched in (out[:4], out[4:]):
         assert (joined, done, untouched) == (0, 1, 1)
         assert status == 7  # CGS_ERROR_DEVICE_TIMEOUT
+
+
+def test_quotients_are_correctly_rounded(cuda, lib):
+    """exact_quot2 over 3.9e9 quotients: ends of the binade, few and many bits, mixed mantissas, exponents over
+    the range that quot_range admits."""
+    tried, wrong = _run("quotients")
+    assert tried > 3_000_000_000
+    assert wrong == 0

@@ -179,3 +179,37 @@ def test_narrow_images(cuda, lib, cost, channels, h, w):
             np.testing.assert_array_equal(c.view(np.uint32), c2.view(np.uint32))
         elif w in (28, 48):
             np.testing.assert_array_equal(c.view(np.uint32), c1.view(np.uint32))
+
+
+@pytest.mark.parametrize("cost", COSTS + ["MI"])
+@pytest.mark.parametrize("h,w,mh,mw", [(17, 65, 19, 61), (16, 64, 16, 64), (31, 129, 33, 140), (20, 24, 24, 20)])
+def test_three_channel_windows_are_in_bounds(cuda, lib, cost, h, w, mh, mw):
+    """The self-checking build finds every sample of three planes in its block's window, with the plain
+    build's bits, from windows and (a small stage) from global memory."""
+    pair = _pair(640 + w, cost, h, w, mh, mw, 3, u8=True)
+    with _env(CGS_SPAN_CHECK=1):
+        _, c = _run(cuda, pair, cost)
+        with _env(CGS_SPAN_CAP=1024):
+            _, c1 = _run(cuda, pair, cost)
+    np.testing.assert_array_equal(c1.view(np.uint32), c.view(np.uint32))
+    _oracle_agrees(pair, cost, c)
+    if w > 32:  # wide enough for the span kernel
+        _, c0 = _run(cuda, pair, cost)
+        np.testing.assert_array_equal(c0.view(np.uint32), c.view(np.uint32))
+
+
+@pytest.mark.parametrize("cost", COSTS)
+def test_three_channel_split_tasks(cuda, lib, cost):
+    """64 points of a tall image, one task split over its bands, and the same points among 148 tasks, which
+    fill the GPU whole: the same bits per point."""
+    pair = _pair(23, cost, 104, 66, 100, 68, 3)
+    pair.count[:] = [2, 1, 1, 1, 4, 4, 2, 1]
+    _, few = _run(cuda, pair, cost)
+    n = [2, 37, 2, 2, 4, 4, 2, 2]
+    pair.count[:] = n
+    for a, step in ((1, 0.001), (2, 0.01), (3, 0.01), (7, 1e-6)):  # the few's value is the first of the many's
+        pair.hi[a] = pair.lo[a] + step * (n[a] - 1)
+    _, many = _run(cuda, pair, cost)
+    pick = many.reshape(n[::-1])[0, :, :, :, 0, 0, 0, :].reshape(-1)
+    np.testing.assert_array_equal(pick.view(np.uint32), few.view(np.uint32))
+    _oracle_agrees(pair, cost, many)
