@@ -313,7 +313,7 @@ static int group_cap(const SpanPlan &g, int tiles) {
     const size_t budget = 227 * 1024;
     const int least = kMinSpanCap + g.TH * 32 * g.TX / 4;  // after the fixed rows
     if (span_kernel_smem(g.G, g.NW, g.TH, g.TX, tiles, least, true, 0) > budget) return 0;
-    return (int)((budget - span_kernel_smem(g.G, g.NW, g.TH, g.TX, tiles, 0, true, 0)) / (16 * kWinStages));
+    return (int)((budget - span_kernel_smem(g.G, g.NW, g.TH, g.TX, tiles, 0, true, 0)) / 16);
 }
 
 }  // namespace cgs

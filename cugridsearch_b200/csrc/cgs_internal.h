@@ -117,7 +117,6 @@ SpanPrepArgs span_prep_args(const float *fix, int fpitch, int64_t fplane, int ch
                             float4 *quads, int64_t nquads, const float *shifts, int *blocks);
 cudaError_t launch_span_prep(const SpanPrepArgs &a, int blocks, cudaStream_t stream);
 constexpr unsigned int kStatusSpanBounds = 0x100u;  // result status bit of the self-checking span build
-constexpr int kWinStages = 1;                      // window stages of the ZNCC span kernel
 constexpr int kMinSpanCap = 1024;                   // smallest useful window stage (quads)
 struct SpanPlan {
     int G = 4, NW = 16, TX = 2, TH = 16;

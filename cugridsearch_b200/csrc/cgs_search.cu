@@ -783,7 +783,7 @@ static Plan choose_plan(int cost, const cgs_options &o, int mi_bins) {
 // stage filling the shared memory that is left (at most CGS_SPAN_CAP 16-byte units when that is set; it
 // holds the tile's fixed rows and its blocks' windows, of every channel) and window rows padded to
 // CGS_SPAN_PITCH (mod 8) quads.  Tiles are as wide as the windows fit (a 32 x 16 block's takes about
-// 1.1 K quads per channel): 256 columns, MI 128 (4.8 K quads of stage), three channels 64; TH = 16.  The
+// 1.1 K quads per channel): 256 columns, three channels 64; TH = 16.  The
 // tuning variables CGS_SPAN_TX = 2 | 4 | 8 (ZNCC) and CGS_SPAN_TH = 8 | 16 | 32 say otherwise.
 // CGS_SPAN_CHECK=1 selects the self-checking build (every sample's quad address is checked against its
 // window; a miss sets status bit 0x100 and skips the sample).
@@ -815,7 +815,7 @@ bool span_plan(const cgs_image &mov, const cgs_image &fix, const cgs_options &o,
     sp->mi_bins = mi ? mi_bins : 0;
     sp->G = mi || (zncc && o.points_per_warp == 2) ? 2 : 4;
     sp->NW = 16;
-    sp->TX = zncc ? env_int("CGS_SPAN_TX", 8) : C == 3 ? 2 : mi ? 4 : 8;
+    sp->TX = zncc ? env_int("CGS_SPAN_TX", 8) : C == 3 ? 2 : 8;
     sp->TH = env_int("CGS_SPAN_TH", 16);
     if (!(sp->TX == 2 || sp->TX == 4 || sp->TX == 8) || !(sp->TH == 8 || sp->TH == 16 || sp->TH == 32)) return false;
     sp->check = env_int("CGS_SPAN_CHECK", 0) != 0;
@@ -827,8 +827,8 @@ bool span_plan(const cgs_image &mov, const cgs_image &fix, const cgs_options &o,
     const int tiles = sp->tiles_x * sp->tiles_y;
     const size_t budget = 227 * 1024;
     const size_t fixed = span_kernel_smem(sp->G, sp->NW, sp->TH, sp->TX, tiles, 0, sp->exact, sp->mi_bins);
-    if (fixed + (size_t)kMinSpanCap * 16 * kWinStages > budget) return false;
-    sp->cap = (int)((budget - fixed) / (16 * kWinStages));
+    if (fixed + (size_t)kMinSpanCap * 16 > budget) return false;
+    sp->cap = (int)((budget - fixed) / 16);
     // CGS_SPAN_CAP (quads) lowers the stage size, e.g. to exercise the global-memory path
     sp->cap = std::max(kMinSpanCap, std::min(sp->cap, env_int("CGS_SPAN_CAP", sp->cap)));
     sp->cap = std::max(sp->cap, kMinSpanCap + C * sp->TH * 32 * sp->TX / 4);  // room for the fixed rows

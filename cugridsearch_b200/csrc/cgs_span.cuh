@@ -113,11 +113,11 @@ __host__ __device__ constexpr size_t span_smem_bytes(int G, int NW, int TH, int 
     return span_head_bytes(NW) + (size_t)NW * G * sizeof(SpanSlot) + (size_t)NW * (G / 2) * sizeof(PairRow) +
            (size_t)tiles * TX * sizeof(BlockWin) + (size_t)NW * G * TH * sizeof(InnerSpan) +
            (size_t)NW * TH * sizeof(RowRun) + (size_t)NW * G * (10 * sizeof(double) + sizeof(int)) +
-           (size_t)kWinStages * cap * 16 + 144;
+           (size_t)cap * 16 + 144;
 }
 
 struct SpanSmem {
-    uint64_t *bars;   // [kWinStages]
+    uint64_t *bar;     // the window stage's barrier
     unsigned long long *wbest;
     int *abort_flag;
     int *bounds_flag;  // self-checking build: a sample's quad address fell outside its window
@@ -129,7 +129,7 @@ struct SpanSmem {
     double *dtot;      // [NW][G * 5] FP64 task totals {sum f, sum m', sum f^2, sum m'^2, sum f'm'}
     double *dband;     // [NW][G * 5] the same sums of the current band
     int *cnt;          // [NW][G] overlap counts of the warps' points
-    float4 *win;       // [kWinStages][cap]
+    float4 *win;       // [cap] the window stage
     int cap;
     float2 *rowtab;    // exact span kernel: [NW][TH][G / 2][3] products of the rows
     uint32_t *hist;    // exact span kernel, MI: [NW * G][(B + 1)^2]
@@ -140,7 +140,7 @@ template <int G, int NW>
 __device__ __forceinline__ SpanSmem carve_span(unsigned char *smem, int TH, int TX, int tiles, int cap,
                                                bool exact = false, int mi_bins = 0) {
     SpanSmem s;
-    s.bars = reinterpret_cast<uint64_t *>(smem);
+    s.bar = reinterpret_cast<uint64_t *>(smem);
     s.wbest = reinterpret_cast<unsigned long long *>(smem + 64);
     s.abort_flag = reinterpret_cast<int *>(smem + 64 + 8 * NW);
     s.bounds_flag = s.abort_flag + 1;
@@ -285,10 +285,10 @@ __device__ __forceinline__ void red_shared_add1(uint32_t addr) {
 // The reference's bin of value v: min(max(floor(v B / 256), 0), B - 1).
 __device__ __forceinline__ int mi_bin(float v, float sB, int B) { return min(max((int)floorf(v * sB), 0), B - 1); }
 
-// Thread 0: announce the bytes of tile t's copies on stage `st`'s barrier (its one arrival).  It
+// Thread 0: announce the bytes of tile t's copies on the stage's barrier (its one arrival).  It
 // comes before the CTA barrier after which every warp issues its part (issue_window).
 template <int C, int TX>
-__device__ __forceinline__ void expect_window(const SearchParams &p, const SpanSmem &ss, int t, int st) {
+__device__ __forceinline__ void expect_window(const SearchParams &p, const SpanSmem &ss, int t) {
     constexpr int TW = 32 * TX;
     const int x0 = (t % p.tiles_x) * TW, y0 = (t / p.tiles_x) * p.tile_h;
     const BlockWin *bw = ss.wins + t * TX;
@@ -297,29 +297,28 @@ __device__ __forceinline__ void expect_window(const SearchParams &p, const SpanS
     for (int c = 0; c < TX; c++)
         if (bw[c].h > 0 && bw[c].w > 0) bytes += (uint32_t)bw[c].w * (uint32_t)bw[c].h * 16u;
     bytes *= C;
-    mbar_arrive_expect_tx(&ss.bars[st], bytes);
+    mbar_arrive_expect_tx(ss.bar, bytes);
 }
 
-// Issue (every warp its part) the copies of tile t into stage `st`, completing on that stage's
+// Issue (every warp its part) the copies of tile t into the stage, completing on its
 // barrier: the tile's rows of the fixed plane(s) fsrc, of p.fix's pitch (TH x TW floats at the stage's start; columns
 // past the image's right edge are not copied) and the windows of its blocks (quads, after the
 // fixed tile).  A tile has about 220 row copies and a warp issues one in about 60 cycles, so one
 // warp would hold the others back for 14 K cycles per tile; shared by the CTA's warps it is 1 K.
 template <int C, int NW, int TX>
-__device__ __forceinline__ void issue_window(const SearchParams &p, const SpanSmem &ss, const float *fsrc, int t,
-                                             int st) {
+__device__ __forceinline__ void issue_window(const SearchParams &p, const SpanSmem &ss, const float *fsrc, int t) {
     constexpr int TW = 32 * TX;
     constexpr int WB = NW / TX;  // warps per block window
     static_assert(NW % TX == 0, "whole warps per block window");
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int TH = p.tile_h;
     const int x0 = (t % p.tiles_x) * TW, y0 = (t / p.tiles_x) * TH;
-    uint64_t *bar = &ss.bars[st];
+    uint64_t *bar = ss.bar;
     fence_proxy_async_smem();  // the stage's previous reads before the async refill
     if (lane == 31) {
         const int rows = min(TH, p.fix.h - y0);
         const uint32_t row_bytes = (uint32_t)((min(TW, p.fix.w - x0) * 4 + 15) & ~15);  // within the row pitch
-        float *fdst = reinterpret_cast<float *>(ss.win + (size_t)st * ss.cap);
+        float *fdst = reinterpret_cast<float *>(ss.win);
         for (int j = warp; j < rows; j += NW)
 #pragma unroll
             for (int ch = 0; ch < C; ch++)
@@ -328,7 +327,7 @@ __device__ __forceinline__ void issue_window(const SearchParams &p, const SpanSm
     }
     const BlockWin b = ss.wins[t * TX + warp / WB];
     if (b.h > 0 && b.w > 0) {
-        float4 *wdst = ss.win + (size_t)st * ss.cap + C * TH * TW / 4 + b.off;
+        float4 *wdst = ss.win + C * TH * TW / 4 + b.off;
         const float4 *src = p.mov_quad + (int64_t)b.y0 * p.quad_pitch + b.x0;
         for (int j = lane * WB + warp % WB; j < b.h; j += 32 * WB)
 #pragma unroll
@@ -541,8 +540,8 @@ __device__ __forceinline__ void retire_parts(const SearchParams &p, uint32_t uni
 }
 
 // One task, or part of a task, of the span path (ZNCC, one channel, quads staged): the G grid points of
-// each warp over the part's tiles of the fixed image.  `wit` counts window stages used by this CTA (their
-// barrier phases).  Returns false if a bounded wait gave up.
+// each warp over the part's tiles of the fixed image.  `wit` counts this CTA's tiles (the
+// barrier's phases).  Returns false if a bounded wait gave up.
 template <int G, int NW, int TX, bool CHECK>
 __device__ __forceinline__ bool run_span_task(const SearchParams &p, uint32_t unit, const SpanSmem &ss,
                                               uint32_t &wit) {
@@ -590,11 +589,9 @@ __device__ __forceinline__ bool run_span_task(const SearchParams &p, uint32_t un
 
     span_windows<1, G, NW, TX>(p, ss, t0, t1);
     __syncthreads();
-    if (threadIdx.x == 0)
-        for (int t = 0; t < kWinStages && t0 + t < t1; t++) expect_window<1, TX>(p, ss, t0 + t, (int)((wit + t) % kWinStages));
+    if (threadIdx.x == 0) expect_window<1, TX>(p, ss, t0);
     __syncthreads();
-    for (int t = 0; t < kWinStages && t0 + t < t1; t++)
-        issue_window<1, NW, TX>(p, ss, p.fix.data, t0 + t, (int)((wit + t) % kWinStages));
+    issue_window<1, NW, TX>(p, ss, p.fix.data, t0);
 
     // ---- sweep
     float2 part_sum[GP][3];  // {sum m', sum m'^2, sum f'm'} of each pair of points
@@ -725,11 +722,10 @@ __device__ __forceinline__ bool run_span_task(const SearchParams &p, uint32_t un
             __syncwarp();
         }
         // the tile's windows
-        const int st = (int)(wit % kWinStages);
-        if (!mbar_wait_bounded(&ss.bars[st], (wit / kWinStages) & 1u, kWaitLimitNs)) *ss.abort_flag = 1;
+        if (!mbar_wait_bounded(ss.bar, wit & 1u, kWaitLimitNs)) *ss.abort_flag = 1;
         const BlockWin *twin = ss.wins + t * TX;
-        const float *sfix = reinterpret_cast<const float *>(ss.win + (size_t)st * ss.cap);  // TH x TW
-        const uint32_t wbase = smem_addr(ss.win + (size_t)st * ss.cap + TH * TW / 4);
+        const float *sfix = reinterpret_cast<const float *>(ss.win);  // TH x TW
+        const uint32_t wbase = smem_addr(ss.win + TH * TW / 4);
         const uint32_t szero = smem_addr(ss.win);
 
         // one row: fast samples of G points at the lane's columns; EDGE masks by the inner spans
@@ -908,20 +904,14 @@ __device__ __forceinline__ bool run_span_task(const SearchParams &p, uint32_t un
                 }
             fold_band<G, NW>(p, task, ty, my_dtot, my_band);
         }
-        const bool more = t + kWinStages < t1;
-        if (threadIdx.x == 0 && more) expect_window<1, TX>(p, ss, t + kWinStages, st);
-        __syncthreads();  // every warp is done with this stage
-        if (*ss.abort_flag) {
-            // a wait gave up: let this stage's copies and the next stage's (already issued) land,
-            // within the same bound, before the CTA stops
-            if (threadIdx.x == 0) {
-                mbar_wait_bounded(&ss.bars[st], (wit / kWinStages) & 1u, kWaitLimitNs);
-                if (kWinStages > 1 && t + 1 < t1)
-                    mbar_wait_bounded(&ss.bars[(wit + 1) % kWinStages], ((wit + 1) / kWinStages) & 1u, kWaitLimitNs);
-            }
+        const bool more = t + 1 < t1;
+        if (threadIdx.x == 0 && more) expect_window<1, TX>(p, ss, t + 1);
+        __syncthreads();  // every warp is done with the stage
+        if (*ss.abort_flag) {  // a wait gave up: let the stage's copies land, within the same bound, before the CTA stops
+            if (threadIdx.x == 0) mbar_wait_bounded(ss.bar, wit & 1u, kWaitLimitNs);
             return false;
         }
-        if (more) issue_window<1, NW, TX>(p, ss, p.fix.data, t + kWinStages, st);
+        if (more) issue_window<1, NW, TX>(p, ss, p.fix.data, t + 1);
     }
 
     if (!join_parts<G, NW, CHECK>(p, task, part, ss, my_dtot, my_cnt)) return true;
@@ -964,7 +954,7 @@ __global__ void __launch_bounds__(NW * 32, 1) span_kernel(const __grid_constant_
     extern __shared__ __align__(128) unsigned char smem[];
     const SpanSmem ss = carve_span<G, NW>(smem, p.tile_h, TX, p.tiles_x * p.tiles_y, p.win_cap);
     if (threadIdx.x == 0) {
-        for (int s = 0; s < kWinStages; s++) mbar_init(&ss.bars[s], 1);
+        mbar_init(ss.bar, 1);
         fence_mbar_init();
         *ss.abort_flag = 0;
         *ss.bounds_flag = 0;

@@ -33,7 +33,7 @@ __global__ void __launch_bounds__(NW * 32, 1) span_batch_kernel(const __grid_con
     // dynamic carve may take all 227 KB)
     volatile uint32_t &s_task = *reinterpret_cast<volatile uint32_t *>(ss.bounds_flag + 1);
     if (threadIdx.x == 0) {
-        for (int s = 0; s < kWinStages; s++) mbar_init(&ss.bars[s], 1);
+        mbar_init(ss.bar, 1);
         fence_mbar_init();
         *ss.abort_flag = 0;
         *ss.bounds_flag = 0;

@@ -224,12 +224,9 @@ __device__ __forceinline__ bool run_span_exact_task(const SearchParams &p, uint3
     const float *fsrc = kMI ? p.span_rows : p.fix.data;
     span_windows<C, G, NW, TX>(p, ss, t0, t1);
     __syncthreads();
-    if (threadIdx.x == 0)
-        for (int t = 0; t < kWinStages && t0 + t < t1; t++)
-            expect_window<C, TX>(p, ss, t0 + t, (int)((wit + t) % kWinStages));
+    if (threadIdx.x == 0) expect_window<C, TX>(p, ss, t0);
     __syncthreads();
-    for (int t = 0; t < kWinStages && t0 + t < t1; t++)
-        issue_window<C, NW, TX>(p, ss, fsrc, t0 + t, (int)((wit + t) % kWinStages));
+    issue_window<C, NW, TX>(p, ss, fsrc, t0);
 
     // one sample of point g at (x, y) by the reference's sequence, into a (and f^2 into s2) or the
     // histogram if inside
@@ -438,11 +435,10 @@ __device__ __forceinline__ bool run_span_exact_task(const SearchParams &p, uint3
             __syncwarp();
             if constexpr (!MULTI) set_points();
         }
-        const int st = (int)(wit % kWinStages);
-        if (!mbar_wait_bounded(&ss.bars[st], (wit / kWinStages) & 1u, kWaitLimitNs)) *ss.abort_flag = 1;
+        if (!mbar_wait_bounded(ss.bar, wit & 1u, kWaitLimitNs)) *ss.abort_flag = 1;
         const BlockWin *twin = ss.wins + t * TX;
-        const float *sfix = reinterpret_cast<const float *>(ss.win + (size_t)st * ss.cap);  // C x TH x TW
-        const uint32_t wbase = smem_addr(ss.win + (size_t)st * ss.cap + C * TH * TW / 4);
+        const float *sfix = reinterpret_cast<const float *>(ss.win);  // C x TH x TW
+        const uint32_t wbase = smem_addr(ss.win + C * TH * TW / 4);
         const uint32_t szero = smem_addr(ss.win);
 
         // this lane's row of the band (lanes past it: none)
@@ -630,14 +626,14 @@ __device__ __forceinline__ bool run_span_exact_task(const SearchParams &p, uint3
                 }
             fold_band<G, NW>(p, task, ty, my_dtot, my_band);
         }
-        const bool more = t + kWinStages < t1;
-        if (threadIdx.x == 0 && more) expect_window<C, TX>(p, ss, t + kWinStages, st);
-        __syncthreads();  // every warp is done with this stage
+        const bool more = t + 1 < t1;
+        if (threadIdx.x == 0 && more) expect_window<C, TX>(p, ss, t + 1);
+        __syncthreads();  // every warp is done with the stage
         if (*ss.abort_flag) {
-            if (threadIdx.x == 0) mbar_wait_bounded(&ss.bars[st], (wit / kWinStages) & 1u, kWaitLimitNs);
+            if (threadIdx.x == 0) mbar_wait_bounded(ss.bar, wit & 1u, kWaitLimitNs);
             return false;
         }
-        if (more) issue_window<C, NW, TX>(p, ss, fsrc, t + kWinStages, st);
+        if (more) issue_window<C, NW, TX>(p, ss, fsrc, t + 1);
     }
 
     if (!join_parts<G, NW, CHECK>(p, task, part, ss, my_dtot, my_cnt)) return true;  // MI: never split
@@ -695,7 +691,7 @@ __global__ void __launch_bounds__(NW * 32, 1) span_exact_kernel(const __grid_con
     const SpanSmem ss = carve_span<G, NW>(smem, p.tile_h, TX, p.tiles_x * p.tiles_y, p.win_cap, true,
                                           COST == CGS_COST_MI ? p.mi_bins : 0);
     if (threadIdx.x == 0) {
-        for (int s = 0; s < kWinStages; s++) mbar_init(&ss.bars[s], 1);
+        mbar_init(ss.bar, 1);
         fence_mbar_init();
         *ss.abort_flag = 0;
         *ss.bounds_flag = 0;
