@@ -161,8 +161,8 @@ cgs_status launch_verify(const SearchParams &p, void *hdr, cudaStream_t stream, 
 bool verify_supported(int cost);
 
 // A search in a caller's scratch block (cgs_search.cu): for requests that cgs_search runs on a
-// span kernel (ZNCC or MI on the fast sampling path), the batch runs them with the same launches
-// and results.  span_route_bytes: whether cgs_search runs this pair on a span kernel, the
+// span kernel, the batch runs them with the same launches and results (MI pairs whose grids fill the GPU,
+// ZNCC pairs that do not fit the multi-pair kernel).  span_route_bytes: whether cgs_search runs this pair on a span kernel, the
 // scratch it then needs (staging, span tables, verification header) and the kernel's grid
 // points per task; span_route_enqueue: the search's launches on `stream` with that scratch
 // (tex_align-aligned, `bytes` long).

@@ -8,9 +8,10 @@
 // 128 -> 16 (8 centres in [-1, 1] grid-range units, 8 log-radii).
 //
 // Numerics.  Activations are NHWC BF16, weights FP32 masters with BF16 copies; every
-// convolution is an implicit GEMM on the BF16 tensor cores with FP32 accumulation: the forward
-// and the data gradient on tcgen05 (UMMA, TMEM accumulators; conv_umma_kernel), the weight
-// gradient on mma.sync m16n8k16; pooling, the MLP, the loss and Adam run in FP32.
+// convolution is an implicit GEMM on the BF16 tensor cores with FP32 accumulation, on tcgen05 (UMMA,
+// TMEM accumulators): the forward and the data gradient in conv_umma_kernel, the weight gradient in
+// conv_wgrad_umma_kernel (mma.sync versions of all three are kept for comparison); pooling, the MLP, the
+// loss and Adam run in FP32.
 //
 // Loss.  Laplace negative log-likelihood of the label y per parameter: |c - y| e^-s + s with
 // s clamped to [-6, 4] (no gradient outside), averaged over batch and parameters.

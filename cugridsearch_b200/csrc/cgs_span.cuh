@@ -341,9 +341,9 @@ __device__ __forceinline__ void issue_window(const SearchParams &p, const SpanSm
 // -X and -Y (the caller forms the negatives by negating coefficients, which is exact).  The reciprocal
 // r of w is the approximate one and a Newton step; the quotient q0 = X r is corrected by its exact
 // residual, q = q0 + (X - w q0) r (P. Markstein, "Computation of elementary functions on the IBM RISC
-// System/6000 processor", IBM J. Res. Dev. 34, 1990).  Checked against IEEE division for every pair of
-// 24-bit mantissas (2^46 quotients): r and q are always the correctly rounded values, provided that no
-// step leaves the normal range (quot_range).  Eight packed operations and two reciprocals replace four
+// System/6000 processor", IBM J. Res. Dev. 34, 1990).  r and q are the correctly rounded values, provided
+// that no step leaves the normal range (quot_range): one run over every pair of 24-bit mantissas (2^46
+// quotients) found none that differs from IEEE division; tests/native/span_check.cu repeats 3.9e9 of them.  Eight packed operations and two reciprocals replace four
 // divisions of about ten instructions and a branch each.
 __device__ __forceinline__ void exact_quot2(float2 w, float2 nX, float2 nY, float2 &x, float2 &y) {
     const float2 nr0 = make_float2(rcp_approx(-w.x), rcp_approx(-w.y));

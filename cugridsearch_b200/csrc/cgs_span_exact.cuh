@@ -25,9 +25,9 @@
 //
 // What bounds it: the FP32 pipe.  A pair of points takes 26 packed operations (two pipe cycles each)
 // and about 20 scalar ones per pixel and channel; the heavier of the two FP32 pipes is active on 72 % of
-// cycles (SAD, 256 x 256).  39 instructions per 32 evaluations, of which 5 are register moves.  SAD
-// 64 x 64, 4^8: 604 us against 842 on the per-sample kernel; calcNCC 203 x 157: 3.82 ms against 6.1.  Row
-// after row instead of block after block: 659 us and 4.2 ms.
+// cycles (SAD, 256 x 256).  39 instructions per 32 evaluations, of which 5 are register moves.  Whole
+// calls: SAD 64 x 64, 4^8, 645 us against 839 on the per-sample kernel; calcNCC 203 x 157 3.86 ms against 6.2.
+// Row after row instead of block after block 9 % slower.
 //
 // Three-channel MI runs here too (2.8 ms against 4.7 on the per-sample kernel for 301 x 211, 3^8); with
 // one channel the guarded fast samples of cgs_span_mi.cuh are faster.
@@ -38,9 +38,10 @@
 // as in the per-sample kernel: equal counts give equal bits.
 //
 // Sums of the other costs.  Per lane and band of TH rows in FP32, then a warp sum into FP64 totals; the
-// fixed image's sum of squares comes from the row prefix sums (or the pixels: prefix_holds).  SAD is formed in FP64, the NCC-like
-// costs in FP32 from the rounded totals (finalize), so their special cases are the per-sample kernel's.  Costs do not depend on
-// the order of the points or on how many share a launch.
+// fixed image's sum of squares comes from the row prefix sums (or the pixels: prefix_holds).  SAD is
+// formed in FP64, the NCC-like costs in FP32 from the rounded totals (finalize), so their special cases
+// are the per-sample kernel's.  Costs do not depend on the order of the points or on how many share a
+// launch.
 #pragma once
 #include "cgs_span.cuh"
 

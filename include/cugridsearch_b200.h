@@ -99,8 +99,8 @@ typedef struct cgs_options {
 /* Where the 2x2 bilinear taps come from.  QUAD: a staged copy of the moving image that holds
  * each pixel's footprint as one 16-byte element (4x the moving image in scratch); TEXTURE:
  * texture gathers (scalar loads for MI).  Default: quads for the fast sampling path of every
- * cost but MI, texture otherwise (the faster choice measured on B200).  Results are identical;
- * only speed and scratch size differ. */
+ * cost but MI and in the span kernels, texture otherwise (the faster choice measured on B200).  Results
+ * are identical; only speed and scratch size differ. */
 #define CGS_FLAG_QUAD_TAPS 8
 #define CGS_FLAG_TEXTURE_TAPS 16
 /* Span kernels (the default where they apply): in/out decisions per image row instead of per
@@ -108,10 +108,20 @@ typedef struct cgs_options {
  * samples, and SAD_AVG, SQD_REF and NCC_REF (1 or 3 channels) and MI of 3 channels (as many bins as fit
  * shared memory, at most 32) on exact ones, unless a taps flag is
  * set (ZNCC: the texture flag).  ZNCC and the exact costs read their taps from per-block
- * moving-image windows in shared memory, MI keeps its histograms there.  They ignore
- * warps_per_block, and points_per_warp other than ZNCC's 2.  This flag selects the per-sample
- * decision kernel instead.  Both make the same decisions and form the same samples (exact) and bins
- * (MI): costs agree within FP32 summation order, MI costs are bit-identical. */
+ * moving-image windows in shared memory, MI keeps its histograms there.  The exact ones leave narrow
+ * fixed images, whose columns would not fill blocks of 32, to the per-sample kernel (up to 27 and 33
+ * to 43 columns of one channel, fewer where few points split their tasks).  They ignore warps_per_block,
+ * and points_per_warp other than ZNCC's 2; the exact ones refuse values that the per-sample kernel
+ * does not have.  This flag selects the per-sample decision kernel instead.  Both make the same
+ * decisions and form the same samples (exact) and bins (MI): costs agree within FP32 summation order,
+ * MI costs are bit-identical.
+ *
+ * Scratch.  A search holds its staged images and tables in a block from the library's pool, freed to the
+ * pool in stream order: FP32 copies of both images; 16 bytes per moving pixel and channel where taps are
+ * quads (so in every span kernel); 16 bytes per fixed pixel of row sums for ZNCC, SQD_REF and NCC_REF in
+ * the span kernels, or 4 bytes per fixed pixel and channel for MI; and 24 bytes per pixel and channel
+ * for SQD_ALT and NCC_ALT, about 400 MB at the largest images accepted (2^24 elements).  Splitting the
+ * tasks of a small grid takes up to 64 MB more. */
 #define CGS_FLAG_PER_SAMPLE_DECISIONS 32
 /* Skip the FP64 verification pass (see cgs_argmin).  Without the pass the verification fields
  * read verified = 0, index_fp64 = -1, cost_fp64 = NaN. */
@@ -293,10 +303,14 @@ typedef struct cgs_pair {
     cgs_grid grid;
     cgs_options options;   /* cost: CGS_COST_SAD_AVG, _SQD_REF, _NCC_REF, _ZNCC or _MI; mi_bins,
                               overlap_gate and flags as for cgs_search.  points_per_warp and
-                              warps_per_block are ignored: the batch plan applies.  Taps:
-                              ZNCC pairs follow cgs_search's choice (quads on the fast
-                              sampling path unless CGS_FLAG_TEXTURE_TAPS); the other costs
-                              read texture gathers (MI: scalar loads), whatever the flags   */
+                              warps_per_block are ignored: the batch plan applies.  The flags
+                              choose the kernel as in cgs_search.  Taps: pairs of the
+                              multi-pair span kernel read quads (16 bytes of scratch per moving
+                              pixel); in the persistent kernel, which takes SAD, SQD and NCC
+                              pairs with a taps or per-sample flag or narrow images, ZNCC
+                              pairs follow cgs_search's choice (quads on the fast sampling path
+                              unless CGS_FLAG_TEXTURE_TAPS) and the other costs read texture
+                              gathers (MI: scalar loads)                                     */
     float *costs;          /* nullable DEVICE dump of this pair's grid (as cgs_search)       */
     cgs_argmin *result;    /* DEVICE result of this pair                                     */
 } cgs_pair;
@@ -327,7 +341,8 @@ typedef struct cgs_batch cgs_batch; /* opaque handle */
  * (cheapest first) and records one CUDA graph: clear scratch, stage every pair; the pairs that
  * cgs_search runs on a span kernel with windows (ZNCC on fast samples, SAD_AVG, SQD_REF and NCC_REF
  * on exact ones, no per-sample or taps flag) in one multi-pair span launch, with cgs_search's costs
- * and argmins bit for bit; the other pairs in the
+ * and argmins bit for bit (a pair of so many tiles that it fits that kernel's shared memory alone only
+ * is searched by cgs_search's own launches); the other pairs in the
  * persistent batch kernel, for the plan (NULL: 4 points per warp, 16 warps, warp-private
  * histograms; 2 points per warp, then block-shared histograms, where those do not fit); then,
  * pair after pair, cgs_search's own launches for MI pairs that it runs on its MI span kernel and
