@@ -888,14 +888,14 @@ static int span_splits(const SpanPlan &sp, int cost, uint32_t tasks, const cgs_i
 // on a full GPU, 100 rows, span over per-sample speed: one channel SAD (NCC) 8 columns 0.46 (0.48), 24
 // 0.84 (0.89), 28 0.94 (1.00), 33 0.72 (0.83), 44 0.90 (0.99), 48 0.95 (1.07), 65 1.01 (1.14); three channels
 // 16 0.83 (0.91), 20 0.98 (1.08), 33 0.97 (1.17); MI of three 20 0.94, 24 1.07, 33 0.97, 44 1.10.  One row
-// alone (nothing to split, one row per block) loses on a GPU that is not full: 1 x 3000 NCC 0.84.  ZNCC is
-// faster at every width.  The self-checking build runs wherever it can.
+// alone (nothing to split, one row per block) loses on a GPU that is not full: 1 x 3000 NCC 0.84; beyond 4,096
+// values it stays here, as it may not fit the per-sample kernel's row stages.  ZNCC is faster at every width.  The self-checking build runs wherever it can.
 bool span_pays(SpanPlan *sp, int cost, const cgs_image &fix, uint32_t points, int sms) {
     const uint32_t per_task = (uint32_t)(sp->G * sp->NW), tasks = (points + per_task - 1) / per_task;
     double gain;
     sp->splits = span_splits(*sp, cost, tasks, fix, sms, &gain);
     if (!sp->exact || sp->check) return true;
-    if (fix.height == 1 && tasks < (uint32_t)sms) return false;
+    if (fix.height == 1 && tasks < (uint32_t)sms && (int64_t)fix.width * fix.channels <= 4096) return false;
     const int blocks = (fix.width + 31) / 32;
     const double busy = (double)fix.width / (32.0 * blocks) * gain;
     const bool mi = cost == CGS_COST_MI, rgb = fix.channels == 3;

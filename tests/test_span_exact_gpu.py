@@ -213,3 +213,18 @@ def test_three_channel_split_tasks(cuda, lib, cost):
     pick = many.reshape(n[::-1])[0, :, :, :, 0, 0, 0, :].reshape(-1)
     np.testing.assert_array_equal(pick.view(np.uint32), few.view(np.uint32))
     _oracle_agrees(pair, cost, many)
+
+
+@pytest.mark.parametrize("channels", [1, 3])
+@pytest.mark.parametrize("cost", ["SAD_AVG", "NCC_REF", "MI"])
+def test_one_wide_row(cuda, lib, cost, channels):
+    """A row too wide for the per-sample kernel's shared memory, which one row of few points otherwise takes."""
+    rng = np.random.default_rng(9)
+    pair = _pair(3, cost, 1, 16, 3, 16, channels)
+    pair.fixed = rng.uniform(0, 255, (1, 30000, channels)).astype(np.float32)
+    pair.moving = np.ascontiguousarray(np.repeat(np.roll(pair.fixed, 2, axis=1), 3, axis=0))
+    pair.lo[:] = [0, 1, 1, 0, -3, -0.25, 0, 0]
+    pair.hi[:] = [0, 1, 1, 0, 3, 1.25, 0, 0]
+    pair.count[:] = [1, 1, 1, 1, 4, 3, 1, 1]
+    _, c = _run(cuda, pair, cost)
+    _oracle_agrees(pair, cost, c)
