@@ -665,7 +665,13 @@ __device__ __forceinline__ bool run_span_exact_task(const SearchParams &p, uint3
             a[2] = (float)(d[2] * k2);
         }
         // 0 / 0 is NaN, as in the reference
-        cost = COST == CGS_COST_SAD_AVG ? (float)(d[1] / (double)n) : finalize<COST>(a, n, p);
+        if constexpr (COST == CGS_COST_SAD_AVG) {
+            // a sum beyond FP32 is infinite, as the reference's and the per-sample kernel's
+            const double sum = (double)(float)d[1];
+            cost = (float)((isinf(sum) ? sum : d[1]) / (double)n);
+        } else {
+            cost = finalize<COST>(a, n, p);
+        }
     }
     if (lane < G) {
         const SpanSlot &sl = my_slots[lane];

@@ -121,3 +121,17 @@ def test_moving_outliers_outside_the_overlap(cuda, lib, channels, value):
     c = _run(cuda, p, "ZNCC")[1]
     bad = close_costs(c, c32, c64, "ZNCC") & clear
     assert not bad.any(), (int(bad.sum()), c[bad][:4], c64[bad][:4])
+
+
+@pytest.mark.parametrize("channels", [1, 3])
+def test_sad_beyond_fp32(cuda, lib, channels):
+    """No-data pixels of the type's lowest value inside the overlap: the reference's FP32 sum overflows, and the
+    cost is +inf on every kernel."""
+    p = S.small_pair(47, size=70, count=2, cost="SAD_AVG", channels=channels)
+    p.fixed = p.fixed.copy()
+    p.fixed[12, 30] = p.fixed[50, 40] = LOWEST  # a band each: its FP32 sums hold it
+    c32, c64 = _oracle(p, "SAD_AVG", np.ascontiguousarray(p.fixed))
+    assert np.isinf(c32).any()
+    for c in _runs(cuda, p, "SAD_AVG") + [_run(cuda, p, "SAD_AVG", per_sample_decisions=True)[1]]:
+        bad = close_costs(c, c32, c64, "SAD_AVG")
+        assert not bad.any(), (int(bad.sum()), c[bad][:4], c32[bad][:4], c64[bad][:4])
